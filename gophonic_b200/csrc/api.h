@@ -146,6 +146,10 @@ GB_API int gb_concat_cast(const float* h, const float* delta, const float* side,
 // matrix products: C[M, N] = A[M, K] W[N, K]^T
 GB_API int gb_gemm_simt(const void* A, int a_dtype, const void* W, int w_dtype, void* C, int c_dtype, int M, int N, int K, int64_t lda,
                         int64_t ldw, int64_t ldc, cudaStream_t stream);
+// the same for float32 operands of 16-byte chunks, the same additions in the same order
+bool gb_gemm_f32_accepts(const void* A, const void* W, int N, int K, int64_t lda, int64_t ldw);
+int gb_gemm_f32_launch(const float* A, const float* W, float* C, int M, int N, int K, int64_t lda, int64_t ldw, int64_t ldc,
+                       cudaStream_t stream);
 GB_API int gb_gemm_skinny(const void* X, const void* W, void* Y, int c_dtype, int M, int N, int K, int64_t ldx, int64_t ldy, cudaStream_t stream);
 GB_API int gb_gemm_skinny_bias(const void* X, const void* W, void* Y, int c_dtype, int M, int N, int K, int64_t ldx, int64_t ldy,
                                const float* bias, cudaStream_t stream);

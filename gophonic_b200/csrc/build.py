@@ -40,6 +40,7 @@ SOURCES = [
     "elementwise.cu",
     "cache_fill.cu",
     "gemm_simt.cu",
+    "gemm_f32.cu",
     "gemm_skinny.cu",
     "gemm_skinny_fold.cu",
     "gemm_tc5.cu",

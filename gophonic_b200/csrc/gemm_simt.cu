@@ -1,11 +1,13 @@
 // C[M, N] = A[M, K] * W[N, K]^T with fp32 multiply-add on the CUDA cores.
 //
-// This is the matrix product of the true 32-bit path (no tensor cores, no reduced-precision
-// mode) and the fallback for operand types or sizes the tensor-core kernels refuse (for
-// instance a weight the checkpoint stores in 32-bit while activations are bfloat16).
+// This is the fallback for operand types or sizes the tensor-core kernels refuse (for instance a
+// weight the checkpoint stores in 32-bit while activations are bfloat16), and the entry to the products
+// of the true 32-bit path (no tensor cores, no reduced-precision mode): float32 operands of 16-byte
+// chunks go on to gemm_f32.cu, the others stay here.
 // Every output element is the sum over k in ascending order in one fp32 accumulator, whatever M
 // is and wherever the element lies in a tile: rows do not depend on what else is in the batch.
 #include "common.cuh"
+#include "api.h"
 
 namespace {
 
@@ -84,6 +86,9 @@ GB_API int gb_gemm_simt(const void* A, int a_dtype, const void* W, int w_dtype, 
     if ((a_dtype | w_dtype | c_dtype) & ~1) GB_REFUSE("gemm_simt: unknown dtypes (%d, %d, %d)", a_dtype, w_dtype, c_dtype);
     typedef __nv_bfloat16 bf;
     int key = a_dtype * 4 + w_dtype * 2 + c_dtype;
+    // all float32, rows of 16-byte chunks: the kernels of gemm_f32.cu, which add in the same order
+    if (key == 0 && M <= 65535 * BM && gb_gemm_f32_accepts(A, W, N, K, lda, ldw))
+        return gb_gemm_f32_launch((const float*)A, (const float*)W, (float*)C, M, N, K, lda, ldw, ldc, stream);
     switch (key) {
         case 0: return launch<float, float, float>(A, W, C, M, N, K, lda, ldw, ldc, stream);
         case 1: return launch<float, float, bf>(A, W, C, M, N, K, lda, ldw, ldc, stream);

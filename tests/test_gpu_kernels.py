@@ -234,6 +234,24 @@ def test_gemm_simt(ops, M, N, K, combo):
     close(out, a.double() @ w.double().T, 2e-5 if combo[2] == "f" else 6e-3)
 
 
+# float32 products: one row to the largest few-row batch on both sides of every choice of rows a thread, narrow and wide
+# outputs, remainders of the tiles and of the stages of K
+@pytest.mark.parametrize("M", [1, 2, 5, 8, 16, 17, 33, 64, 65, 129, 300])
+@pytest.mark.parametrize("N,K", [(1, 4), (70, 68), (333, 1028), (2050, 260), (14300, 132)])
+def test_float32_products_add_in_one_order(ops, M, N, K):
+    a, w = rnd(M, K, seed=6), rnd(N, K, scale=0.1, seed=7)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    ops.gemm_simt(a, w, out)
+    wide = torch.empty((M, K + 1), device=DEV)      # rows that are not 16-byte chunks: the general kernel
+    wide[:, :K] = a
+    want = torch.empty((M, N), device=DEV)
+    ops.gemm_simt(wide[:, :K], w, want)
+    assert torch.equal(out, want)
+    strided = torch.full((M, N + 3), float("nan"), device=DEV)
+    ops.gemm_simt(a, w, strided[:, 1:N + 1])
+    assert torch.equal(strided[:, 1:N + 1], want) and torch.isnan(strided[:, 0]).all() and torch.isnan(strided[:, N + 1:]).all()
+
+
 def test_gemm_simt_rows_do_not_depend_on_the_batch(ops):
     a, w = rnd(70, 200, seed=4), rnd(150, 200, seed=5)
     full = torch.empty((70, 150), device=DEV)
@@ -625,6 +643,37 @@ def test_attention_head_sizes_that_are_no_multiple_of_16(ops, dtype, heads, kvh,
         out, ref, used = attention_case(ops, dtype, heads, kvh, d, q_lens=[1, 1, 1], kv_lens=[1, 700, 65], splits=splits)
         assert used == "simt"
         close(out, ref, 1e-5 if dtype == torch.float32 else 1.2e-2)
+
+
+# float32 attention on planes whose rows are 16-byte chunks against the general kernel (planes that begin 4 bytes further): one
+# row a warp and four, heads that share a tile in groups of 1, 3 and 8, head sizes between the kernel's steps and one so wide
+# that a single stage is held, windows with kept first tokens, blocks, a sink, key splits
+@pytest.mark.parametrize("heads,kvh,d,dv", [(2, 1, 128, 128), (3, 1, 36, 20), (8, 1, 64, 200), (4, 4, 4, 4), (1, 1, 576, 512)])
+@pytest.mark.parametrize("q_lens,kv_lens,opts", [
+    ([1, 1, 1], [1, 31, 333], {}), ([1, 1], [64, 200], {"splits": 3}), ([1, 1, 1], [150, 33, 97], {"window": 40, "keep_first": 5}),
+    ([70, 5, 1], [70, 69, 130], {}), ([33, 90], [33, 190], {"window": 17, "keep_first": 3, "sink": True}), ([40, 3], [100, 65], {"chunk": 48})])
+def test_float32_attention_adds_in_one_order(ops, heads, kvh, d, dv, q_lens, kv_lens, opts):
+    splits = opts.get("splits", 1)
+    nseq, rows, n_pages = len(q_lens), sum(q_lens), 24
+    mk = lambda x: torch.tensor(list(x), dtype=torch.int32, device=DEV)
+    table = torch.randperm(n_pages, generator=torch.Generator().manual_seed(3)).to(torch.int32).view(4, 6).to(DEV)
+    q = rnd(rows, heads * d + 2, seed=8)[:, :heads * d]
+    k, v = rnd(n_pages, kvh, 64, d, seed=9), rnd(n_pages, kvh, 64, dv, seed=10)
+    outs = []
+    for shift in (0, 1):
+        planes = []
+        for t in (k, v):
+            flat = torch.empty(t.numel() + 1, device=DEV)
+            flat[shift:shift + t.numel()] = t.reshape(-1)
+            planes.append(flat[shift:shift + t.numel()].view(t.shape))
+        out = torch.full((rows, heads * dv), float("nan"), device=DEV)
+        scratch = torch.empty(ops.attention_scratch_floats(nseq, heads, dv, splits), device=DEV) if splits > 1 else None
+        used = ops.attention(q, out, planes[0], planes[1], table, mk(range(nseq)), mk([sum(q_lens[:i]) for i in range(nseq)]), mk(q_lens), mk(kv_lens),
+                             nseq, max(q_lens), heads, kvh, d, d ** -0.5, opts.get("window", 0), splits, scratch, value_dim=dv,
+                             keep_first=opts.get("keep_first", 0), sink=opts.get("sink", False), chunk=opts.get("chunk", 0))
+        assert used == "simt"
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and not torch.isnan(outs[0]).any()
 
 
 def test_attention_head_sizes_without_a_tensor_core_kernel_fall_back(ops):
