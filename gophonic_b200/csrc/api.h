@@ -192,6 +192,11 @@ GB_API int gb_attention_prefill_tc5(const AttnParams* p, int rows, int pages, cu
 GB_API int gb_attention_simt_x(const AttnParamsX* p, int dtype, cudaStream_t stream);
 GB_API int gb_attention_decode_mma_x(const AttnParamsX* p, cudaStream_t stream);
 GB_API int gb_attention_prefill_mma_x(const AttnParamsX* p, cudaStream_t stream);
+GB_API int gb_latent_gather(const void* plane, const int* block_table, int bt_stride, const int* seq_slot, const int* seq_q_len,
+                            const int* seq_kv_len, int nseq, int window, int d, int pages, int max_slots, int total_pages, void* out, int* base,
+                            cudaStream_t stream);
+GB_API int gb_attention_latent_tc5(const AttnParamsX* p, int rows, int kv_rows, const void* gathered, int gathered_cols, int rot_col, const int* base,
+                                   cudaStream_t stream);
 GB_API int gb_attention_prefill_tc5_x(const AttnParamsX* p, int rows, int pages, cudaStream_t stream);
 GB_API int gb_attention_algo_x(const AttnParamsX* p, int dtype);
 GB_API int gb_attention_latent_accepts(const AttnParamsX* p, int dtype);

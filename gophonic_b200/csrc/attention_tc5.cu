@@ -32,13 +32,21 @@ namespace {
 __device__ int g_status;
 
 typedef __nv_bfloat16 bf16;
-constexpr int HD = 128, BQ = 128, GROUPS = 2, BKV = 64, STAGES = 5, THREADS = 448;
+constexpr int HD = 128, BQ = 128, GROUPS = 2, BKV = 64, THREADS = 448;
 constexpr int FIRST_SOFTMAX_WARP = 1 + 2 * GROUPS;  // warp 0 loads queries and keys, then a scores issuer and a values issuer per group
 constexpr int VALUE_LOADER_WARP = FIRST_SOFTMAX_WARP + 4 * GROUPS;  // the last warp loads the values
 constexpr int QPANEL = 128 * 128;               // 128 rows of 128 bytes (64 head elements)
 constexpr int KPANEL = 64 * 128;                // 64 keys of 128 bytes
-constexpr int Q_BYTES = 2 * QPANEL;             // one group's query tile
-constexpr int K_BYTES = 2 * KPANEL, V_BYTES = 2 * KPANEL, STAGE_BYTES = K_BYTES + V_BYTES;
+// What a form of the kernel stages.  Keys of 128 channels straight from the paged cache, five pages deep; or keys of
+// 128 + 64 channels that were expanded from latents (the last 64, the rotated part, are the same for all heads), three.
+template <bool LATENT>
+struct Form {
+    static constexpr int PANELS = LATENT ? 3 : 2;              // of 64 channels, queries and keys
+    static constexpr int STAGES = LATENT ? 3 : 5;
+    static constexpr int Q_BYTES = PANELS * QPANEL;            // one group's query tile
+    static constexpr int K_BYTES = PANELS * KPANEL, V_BYTES = 2 * KPANEL, STAGE_BYTES = K_BYTES + V_BYTES;
+    static constexpr int SMEM = GROUPS * Q_BYTES + STAGES * STAGE_BYTES + 1024;
+};
 constexpr int TMEM_COLS = 512;                  // S: 2 groups x 2 buffers x 64; O: 2 groups x 128
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr int POLY_PAIRS = 1;                   // of every four pairs of scores, how many take the polynomial exponential (measured: 0 -> 55.5 us, 1 -> 52.9, 2 -> 56.8 at 2048 tokens)
@@ -155,11 +163,17 @@ __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t (&r)[3
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
-template <bool SIGMOID>
-__global__ void __launch_bounds__(THREADS) attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q,
-                                                                   const __grid_constant__ CUtensorMap map_k,
-                                                                   const __grid_constant__ CUtensorMap map_v, SigmoidAttnParams p,
-                                                                   int by_kv_head) {
+// What the form over expanded latents takes besides.
+struct LatentRows {
+    const int* base;   // [nseq]: the gathered row of the sequence's position 0 (rows of 64-aligned pages, so it may be negative)
+    int rot_col;       // column of the gathered rows where the rotated part begins
+};
+
+template <bool SIGMOID, bool LATENT>
+__device__ __forceinline__ void prefill_tc5(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_r,
+                                            const SigmoidAttnParams& p, int by_kv_head, const LatentRows& lat) {
+    using F = Form<LATENT>;
+    constexpr int STAGES = F::STAGES, PANELS = F::PANELS, Q_BYTES = F::Q_BYTES, K_BYTES = F::K_BYTES, V_BYTES = F::V_BYTES, STAGE_BYTES = F::STAGE_BYTES;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* Qs = base;                          // [GROUPS][Q_BYTES]
@@ -192,7 +206,8 @@ __global__ void __launch_bounds__(THREADS) attn_prefill_tc5_kernel(const __grid_
     const int past = kv_len - q_len;
     const int q_start = p.seq_q_start[seq];
     const int G = p.heads / p.kv_heads, kvh = head / G;
-    const int* bt = block_table_row(p.block_table, p.bt_stride, p.seq_slot[seq], p.max_slots);
+    const int* bt = LATENT ? nullptr : block_table_row(p.block_table, p.bt_stride, p.seq_slot[seq], p.max_slots);
+    const int lat_base = LATENT ? lat.base[seq] : 0;
 
     // pages each group walks: from the first page any of its rows may see to the page of its last row
     int lo_pos = 0;
@@ -257,8 +272,8 @@ __global__ void __launch_bounds__(THREADS) attn_prefill_tc5_kernel(const __grid_
             mbar_expect_tx(&q_full, GROUPS * Q_BYTES);
 #pragma unroll
             for (int g = 0; g < GROUPS; g++) {
-                tma_load_2d(Qs + g * Q_BYTES, &map_q, head * HD, q_start + q0 + g * BQ, &q_full);
-                tma_load_2d(Qs + g * Q_BYTES + QPANEL, &map_q, head * HD + 64, q_start + q0 + g * BQ, &q_full);
+#pragma unroll
+                for (int h = 0; h < PANELS; h++) tma_load_2d(Qs + g * Q_BYTES + h * QPANEL, &map_q, head * (64 * PANELS) + h * 64, q_start + q0 + g * BQ, &q_full);
             }
             // Keys and values travel separately: the keys of a page are free as soon as its scores are
             // done, long before its values are, so the key loads run further ahead than a shared
@@ -275,10 +290,17 @@ __global__ void __launch_bounds__(THREADS) attn_prefill_tc5_kernel(const __grid_
                 mbar_expect_tx(&k_full[s], K_BYTES);
                 unsigned char* ks = KVs + (size_t)s * STAGE_BYTES;
                 int lp = tile_of(j);
-                if (!gb_check(lp, p.bt_stride, GB_CHECK_LOGICAL_PAGE) || lp >= p.bt_stride) lp = p.bt_stride - 1;
-                const int row = ((int)page_of(bt, lp * BKV, p.bt_stride, p.pages) * p.kv_heads + kvh) * 64;
+                if (LATENT) {
+                    const int row = lat_base + lp * BKV;
 #pragma unroll
-                for (int h = 0; h < 2; h++) tma_load_2d(ks + h * KPANEL, &map_k, h * 64, row, &k_full[s]);
+                    for (int h = 0; h < 2; h++) tma_load_2d(ks + h * KPANEL, &map_k, head * HD + h * 64, row, &k_full[s]);
+                    tma_load_2d(ks + 2 * KPANEL, &map_r, lat.rot_col, row, &k_full[s]);
+                } else {
+                    if (!gb_check(lp, p.bt_stride, GB_CHECK_LOGICAL_PAGE) || lp >= p.bt_stride) lp = p.bt_stride - 1;
+                    const int row = ((int)page_of(bt, lp * BKV, p.bt_stride, p.pages) * p.kv_heads + kvh) * 64;
+#pragma unroll
+                    for (int h = 0; h < 2; h++) tma_load_2d(ks + h * KPANEL, &map_k, h * 64, row, &k_full[s]);
+                }
                 issued = j + 1;
             }
             if (*(volatile int*)&abort_s) {
@@ -301,12 +323,12 @@ __global__ void __launch_bounds__(THREADS) attn_prefill_tc5_kernel(const __grid_
                 mbar_expect_tx(&v_full[s], V_BYTES);
                 unsigned char* vs = KVs + (size_t)s * STAGE_BYTES + K_BYTES;
                 int lp = tile_of(j);
-                if (!gb_check(lp, p.bt_stride, GB_CHECK_LOGICAL_PAGE) || lp >= p.bt_stride) lp = p.bt_stride - 1;
+                if (!LATENT && (!gb_check(lp, p.bt_stride, GB_CHECK_LOGICAL_PAGE) || lp >= p.bt_stride)) lp = p.bt_stride - 1;
                 // consecutive key heads may read one value head
-                const int row = p.v_share > 1 ? ((int)page_of(bt, lp * BKV, p.bt_stride, p.pages) * (p.kv_heads / p.v_share) + kvh / p.v_share) * 64
+                const int row = LATENT ? lat_base + lp * BKV : p.v_share > 1 ? ((int)page_of(bt, lp * BKV, p.bt_stride, p.pages) * (p.kv_heads / p.v_share) + kvh / p.v_share) * 64
                                               : ((int)page_of(bt, lp * BKV, p.bt_stride, p.pages) * p.kv_heads + kvh) * 64;
 #pragma unroll
-                for (int h = 0; h < 2; h++) tma_load_2d(vs + h * KPANEL, &map_v, h * 64, row, &v_full[s]);
+                for (int h = 0; h < 2; h++) tma_load_2d(vs + h * KPANEL, &map_v, (LATENT ? head * HD : 0) + h * 64, row, &v_full[s]);
                 issued = j + 1;
             }
             if (*(volatile int*)&abort_s) {
@@ -354,7 +376,7 @@ __global__ void __launch_bounds__(THREADS) attn_prefill_tc5_kernel(const __grid_
                         const uint64_t kd = k_desc[j % STAGES];
                         const uint32_t d_tmem = tmem_base + (uint32_t)(g * 128 + b * 64);
 #pragma unroll
-                        for (int ks = 0; ks < HD / 16; ks++) {
+                        for (int ks = 0; ks < 4 * PANELS; ks++) {
                             // 64 head elements to a panel; 16 elements = 32 bytes = 2 address units inside it
                             umma(d_tmem, q_desc + (uint64_t)((ks >> 2) * (QPANEL >> 4) + (ks & 3) * 2),
                                  kd + (uint64_t)((ks >> 2) * (KPANEL >> 4) + (ks & 3) * 2), idesc_qk, ks > 0 ? 1u : 0u);
@@ -565,6 +587,54 @@ __global__ void __launch_bounds__(THREADS) attn_prefill_tc5_kernel(const __grid_
     }
 }
 
+template <bool SIGMOID>
+__global__ void __launch_bounds__(THREADS) attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q,
+                                                                   const __grid_constant__ CUtensorMap map_k,
+                                                                   const __grid_constant__ CUtensorMap map_v, SigmoidAttnParams p,
+                                                                   int by_kv_head) {
+    prefill_tc5<SIGMOID, false>(map_q, map_k, map_v, map_k, p, by_kv_head, LatentRows{nullptr, 0});
+}
+
+// Over keys and values that were expanded from latents for this step (gb_latent_gather and two products before it): heads
+// of 128 + 64 key channels and 128 value channels, every head its own keys.
+__global__ void __launch_bounds__(THREADS) attn_prefill_tc5_latent_kernel(const __grid_constant__ CUtensorMap map_q,
+                                                                          const __grid_constant__ CUtensorMap map_k,
+                                                                          const __grid_constant__ CUtensorMap map_v,
+                                                                          const __grid_constant__ CUtensorMap map_r, SigmoidAttnParams p,
+                                                                          LatentRows lat) {
+    prefill_tc5<false, true>(map_q, map_k, map_v, map_r, p, 0, lat);
+}
+
+// Cached latents of the sequences' visible pages, one sequence behind the other, each from a whole page on: CTA (i, part)
+// copies a quarter of gathered page i.  Behind a sequence's last token the rows are zeros (a weight of 0 times what a page
+// happens to hold there must be 0).  Bound by the copy: 3264 rows of 576, 7.5 MB moved.
+__global__ void __launch_bounds__(256) latent_gather_kernel(const bf16* __restrict__ plane, const int* __restrict__ block_table, int bt_stride,
+                                                            const int* __restrict__ seq_slot, const int* __restrict__ seq_q_len,
+                                                            const int* __restrict__ seq_kv_len, int nseq, int window, int d, int pages,
+                                                            int max_slots, bf16* __restrict__ out, int* __restrict__ base) {
+    pdl_wait();
+    pdl_trigger();
+    int before = 0, seq = 0, lp0 = 0, kv_len = 0;
+    for (;; seq++) {
+        if (seq >= nseq) return;
+        kv_len = seq_kv_len[seq];
+        const int first = window > 0 ? kv_len - seq_q_len[seq] - window + 1 : 0;   // first key that the sequence's first row sees
+        lp0 = first > 0 ? first / 64 : 0;
+        const int n = (kv_len + 63) / 64 - lp0;
+        if ((int)blockIdx.x < before + n) break;
+        before += n;
+    }
+    const int lp = lp0 + (int)blockIdx.x - before;
+    if (lp == lp0 && blockIdx.y == 0 && threadIdx.x == 0) base[seq] = (before - lp0) * 64;
+    const int* bt = block_table_row(block_table, bt_stride, seq_slot[seq], max_slots);
+    const int64_t page = page_of(bt, lp * 64, bt_stride, pages);
+    const int CH = d / 8, first_row = blockIdx.y * 16;
+    const uint4* src = (const uint4*)(plane + (page * 64 + first_row) * d);
+    uint4* dst = (uint4*)(out + ((int64_t)blockIdx.x * 64 + first_row) * d);
+    const int live = (kv_len - lp * 64 - first_row) * CH;
+    for (int i = threadIdx.x; i < 16 * CH; i += 256) dst[i] = i < live ? src[i] : make_uint4(0, 0, 0, 0);
+}
+
 // 2-D map over `rows` rows of `cols` bfloat16 with a row stride of ld elements; boxes of box_rows x 64
 int make_map(CUtensorMap* map, const void* base, int64_t rows, int cols, int64_t ld, int box_rows) {
     Tc5EncodeTiledFn fn = tc5_encode_fn();
@@ -622,7 +692,7 @@ static int launch_tc5(const SigmoidAttnParams& p, int rows, int pages, int sigmo
     if (((uintptr_t)p.k_plane & 15) || ((uintptr_t)p.v_plane & 15)) GB_REFUSE("%s: cache planes must be 16-byte aligned", who);
     if (rows <= 0 || pages <= 0) GB_REFUSE("%s: %d rows, %d pages", who, rows, pages);
     if ((int64_t)pages * p.kv_heads * 64 > 0x7fffffff) GB_REFUSE("%s: the cache plane has too many rows for one tensor map", who);
-    const int smem = GROUPS * Q_BYTES + STAGES * STAGE_BYTES + 1024;
+    const int smem = Form<false>::SMEM;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc5_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -640,6 +710,59 @@ static int launch_tc5(const SigmoidAttnParams& p, int rows, int pages, int sigmo
     const int by_kv_head = (int64_t)p.max_q_len * p.kv_heads * (4 * HD) > ((int64_t)48 << 20) ? 1 : 0;
     cudaError_t e = sigmoid ? launch_pdl(attn_prefill_tc5_kernel<true>, grid, dim3(THREADS), (size_t)smem, stream, map_q, map_k, map_v, p, by_kv_head)
                             : launch_pdl(attn_prefill_tc5_kernel<false>, grid, dim3(THREADS), (size_t)smem, stream, map_q, map_k, map_v, p, by_kv_head);
+    if (e != cudaSuccess) GB_REFUSE("%s: launch failed: %s", who, cudaGetErrorString(e));
+    return 0;
+}
+
+// Gathers the latents that a step's sequences can see into out[64 * total_pages, d] (see the kernel); base[nseq] receives
+// where each sequence's position 0 would stand.  total_pages is the caller's sum over the sequences.
+GB_API int gb_latent_gather(const void* plane, const int* block_table, int bt_stride, const int* seq_slot, const int* seq_q_len,
+                            const int* seq_kv_len, int nseq, int window, int d, int pages, int max_slots, int total_pages, void* out, int* base,
+                            cudaStream_t stream) {
+    if (nseq <= 0 || total_pages <= 0) return 0;
+    if (d <= 0 || (d & 7) || ((uintptr_t)plane & 15) || ((uintptr_t)out & 15)) GB_REFUSE("latent_gather: rows of %d channels must be 16-byte aligned", d);
+    if (window < 0) GB_REFUSE("latent_gather: window %d", window);
+    cudaError_t e = launch_pdl(latent_gather_kernel, dim3(total_pages, 4), dim3(256), 0, stream, (const bf16*)plane, block_table, bt_stride, seq_slot,
+                               seq_q_len, seq_kv_len, nseq, window, d, pages, max_slots, (bf16*)out, base);
+    if (e != cudaSuccess) GB_REFUSE("latent_gather: launch failed: %s", cudaGetErrorString(e));
+    return 0;
+}
+
+// Prompt attention over expanded latents.  p: q rows of heads x 192 (128 plain channels, 64 rotated ones), out rows of heads x 128,
+// k_plane / v_plane [kv_rows, heads x 128] the expanded keys and values, window, chunk, scale and the sequences; no block
+// table.  gathered [kv_rows, gathered_cols]: its columns from rot_col on are the rotated part of the keys.
+GB_API int gb_attention_latent_tc5(const AttnParamsX* pp, int rows, int kv_rows, const void* gathered, int gathered_cols, int rot_col, const int* base,
+                                   cudaStream_t stream) {
+    SigmoidAttnParams p;
+    static_cast<AttnParamsX&>(p) = *pp;
+    p.score_bias = nullptr;
+    p.gate = nullptr;
+    p.gate_stride = 0;
+    if (p.nseq <= 0 || p.max_q_len <= 0) return 0;
+    const char* who = "attention_latent_tc5";
+    if (p.heads <= 0 || p.kv_heads != p.heads || p.d != 192 || p.dv != HD) GB_REFUSE("%s: %d heads over %d of %d and %d channels", who, p.heads, p.kv_heads, p.d, p.dv);
+    if (p.num_splits != 1 || p.window < 0 || p.chunk < 0 || p.keep_first || p.sink || p.v_share > 1 || p.v_row_stride > 0) GB_REFUSE("%s: an option this form does not take", who);
+    if (((uintptr_t)p.q & 15) || (p.q_row_stride & 7) || ((uintptr_t)p.out & 15) || (p.out_row_stride & 7) || ((uintptr_t)p.k_plane & 15) ||
+        ((uintptr_t)p.v_plane & 15) || ((uintptr_t)gathered & 15) || (gathered_cols & 7) || (rot_col & 7) || rot_col + 64 > gathered_cols)
+        GB_REFUSE("%s: operands must be 16-byte aligned", who);
+    if (rows <= 0 || kv_rows <= 0) GB_REFUSE("%s: %d rows, %d key rows", who, rows, kv_rows);
+    static bool configured[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) GB_REFUSE("%s: no current device", who);
+    if (!configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc5_latent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Form<true>::SMEM);
+        if (e != cudaSuccess) GB_REFUSE("%s: cannot reserve %d bytes of shared memory: %s", who, Form<true>::SMEM, cudaGetErrorString(e));
+        configured[dev] = true;
+    }
+    CUtensorMap map_q, map_k, map_v, map_r;
+    if (int rc = make_map(&map_q, p.q, rows, p.heads * 192, p.q_row_stride, BQ)) return rc;
+    if (int rc = make_map(&map_k, p.k_plane, kv_rows, p.heads * HD, p.heads * HD, 64)) return rc;
+    if (int rc = make_map(&map_v, p.v_plane, kv_rows, p.heads * HD, p.heads * HD, 64)) return rc;
+    if (int rc = make_map(&map_r, gathered, kv_rows, gathered_cols, gathered_cols, 64)) return rc;
+    const dim3 grid(p.heads, ceil_div(p.max_q_len, GROUPS * BQ), p.nseq);
+    if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("%s: grid (%u, %u, %u) exceeds one launch", who, grid.x, grid.y, grid.z);
+    cudaError_t e = launch_pdl(attn_prefill_tc5_latent_kernel, grid, dim3(THREADS), (size_t)Form<true>::SMEM, stream, map_q, map_k, map_v, map_r, p,
+                               LatentRows{base, rot_col});
     if (e != cudaSuccess) GB_REFUSE("%s: launch failed: %s", who, cudaGetErrorString(e));
     return 0;
 }

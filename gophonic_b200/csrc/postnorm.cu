@@ -163,7 +163,8 @@ __global__ void __launch_bounds__(256) latent_prep_kernel(LatentPrepArgs p) {
 
 // q: [rows, heads, d + rot]; out: [rows, heads, out_head] whose last rot channels receive the rotated ones
 template <typename T>
-__global__ void latent_q_rot_kernel(const T* __restrict__ q, int64_t q_stride, T* __restrict__ out, int64_t out_stride, int heads, int d, int rot,
+__global__ void latent_q_rot_kernel(const T* q, int64_t q_stride, T* out, int64_t out_stride,   // out may be q itself
+                                     int heads, int d, int rot,
                                     int out_head, const float* __restrict__ cos_t, const float* __restrict__ sin_t, int table_positions,
                                     const int* __restrict__ row_pos) {
     const int64_t r = blockIdx.x;

@@ -44,6 +44,8 @@ class StepBatch:
     seq_kv_len: torch.Tensor   # [nseq] keys visible to the sequence's last row (= its length after them)
     device: torch.device = None
     sm_count: int = 148
+    # (tokens before, rows in this batch) of every sequence, where the host knows them (a replayed step's change)
+    extents: Optional[Sequence[Tuple[int, int]]] = None
     # launch plans of the step's mixers, by the mixer's identity (``Mixer.plan``); a mixer that is
     # not listed is asked when it first runs
     plans: Dict[int, object] = field(default_factory=dict)
@@ -139,7 +141,7 @@ def build_batch(pieces: Sequence[Tuple[int, Sequence[int], int]], device, sm_cou
                       row_pos=dev[rows:2 * rows], row_seq=dev[2 * rows:3 * rows],
                       seq_slot=dev[o:o + nseq], seq_q_start=dev[o + nseq:o + 2 * nseq],
                       seq_q_len=dev[o + 2 * nseq:o + 3 * nseq], seq_kv_len=dev[o + 3 * nseq:o2],
-                      device=torch.device(device), sm_count=sm_count)
+                      device=torch.device(device), sm_count=sm_count, extents=[(first, len(toks)) for _, toks, first in pieces])
     return batch, (dev[o2:] if nw else None)
 
 

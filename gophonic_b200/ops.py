@@ -730,6 +730,56 @@ def attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_plane
     return algo
 
 
+LATENT_TC5_MIN_ROWS = 65      # prompts whose longest sequence brings at least this many rows
+
+
+def latent_expanded_accepts(dtype: torch.dtype, head_dim: int, rot: int, value_dim: int, kv_rank: int, max_q_len: int) -> bool:
+    """Whether ``attention_latent_expanded`` takes heads of this geometry (bfloat16, 128 + 64 key and 128 value channels)."""
+    return dtype == torch.bfloat16 and (head_dim, rot, value_dim) == (128, 64, 128) and kv_rank % 8 == 0 and max_q_len >= LATENT_TC5_MIN_ROWS
+
+
+def latent_gather(plane: torch.Tensor, block_table: torch.Tensor, seq_slot: torch.Tensor, seq_q_len: torch.Tensor, seq_kv_len: torch.Tensor,
+                  nseq: int, window: int, out: torch.Tensor, base: torch.Tensor) -> None:
+    """The cached latents that the step's sequences can see, one sequence behind the other from whole pages on, into ``out``
+    [64 * pages of all of them, channels]; zeros behind a sequence's last token.  ``base`` [nseq] receives the row where
+    each sequence's position 0 would stand."""
+    _need(plane, "latents", torch.bfloat16, 4)
+    _need(out, "gathered latents", torch.bfloat16, 2)
+    _need(base, "gathered base", torch.int32, 1)
+    _need(block_table, "block table", torch.int32, 2)
+    for t, nm in ((seq_slot, "seq_slot"), (seq_q_len, "seq_q_len"), (seq_kv_len, "seq_kv_len"), (base, "gathered base")):
+        _need(t, nm, torch.int32, 1)
+        if t.numel() < nseq:
+            raise KernelError(f"latent_gather: {nm} has {t.numel()} entries for {nseq} sequences")
+    if plane.shape[1] != 1 or plane.shape[2] != PAGE or out.shape[1] != plane.shape[3] or out.shape[0] % PAGE:
+        raise KernelError(f"latent_gather: plane {tuple(plane.shape)}, out {tuple(out.shape)}")
+    _check(_lib.gb_latent_gather(_ptr(plane), _ptr(block_table), c_int(block_table.stride(0)), _ptr(seq_slot), _ptr(seq_q_len), _ptr(seq_kv_len),
+                                 c_int(nseq), c_int(window), c_int(plane.shape[3]), c_int(plane.shape[0]), c_int(block_table.shape[0]),
+                                 c_int(out.shape[0] // PAGE), _ptr(out), _ptr(base), _stream()))
+
+
+def attention_latent_expanded(q: torch.Tensor, out: torch.Tensor, keys: torch.Tensor, values: torch.Tensor, gathered: torch.Tensor,
+                              base: torch.Tensor, rot_col: int, seq_q_start: torch.Tensor, seq_q_len: torch.Tensor, seq_kv_len: torch.Tensor,
+                              nseq: int, max_q_len: int, heads: int, scale: float, window: int, chunk: int) -> None:
+    """Prompt attention over the keys and values of ``latent_gather``'s rows: q [rows, heads * 192], out, keys and values
+    [.., heads * 128]; the last 64 key channels of every head are columns ``rot_col`` on of ``gathered``."""
+    for t, nm in ((q, "q"), (out, "out"), (keys, "keys"), (values, "values"), (gathered, "gathered latents")):
+        _need(t, f"attention {nm}", torch.bfloat16, 2)
+    n = gathered.shape[0]
+    if (q.shape[1] != heads * 192 or out.shape != (q.shape[0], heads * 128) or keys.shape != (n, heads * 128) or values.shape != (n, heads * 128)
+            or rot_col < 0 or gathered.shape[1] < rot_col + 64):
+        raise KernelError(f"attention: q {tuple(q.shape)}, out {tuple(out.shape)}, keys {tuple(keys.shape)}, gathered {tuple(gathered.shape)}")
+    for t, nm in ((seq_q_start, "seq_q_start"), (seq_q_len, "seq_q_len"), (seq_kv_len, "seq_kv_len"), (base, "gathered base")):
+        _need(t, nm, torch.int32, 1)
+        if t.numel() < nseq:
+            raise KernelError(f"attention: {nm} has {t.numel()} entries for {nseq} sequences")
+    p = _AttnParams(q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), keys.data_ptr(), values.data_ptr(), 0, 0, 0, seq_q_start.data_ptr(),
+                    seq_q_len.data_ptr(), seq_kv_len.data_ptr(), nseq, heads, heads, 192, max_q_len, scale, window, 1, 0, 0, 0, 128, 0, 0, 0,
+                    int(chunk), 1, 0)
+    _check(_lib.gb_attention_latent_tc5(byref(p), c_int(q.shape[0]), c_int(n), _ptr(gathered), c_int(gathered.shape[1]), c_int(rot_col), _ptr(base),
+                                        _stream()))
+
+
 def attention_decode_rope_accepts(dtype: torch.dtype, head_dim: int, rotary_dim: int, max_q_len: int) -> bool:
     """Whether ``attention_decode_rope`` takes rows of this kind (bfloat16, one row a sequence, a head
     size the tensor-core single-token kernel takes)."""

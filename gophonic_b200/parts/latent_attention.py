@@ -6,7 +6,10 @@ How it runs.  A head's plain key is W_uk c and its value W_uv c, so a score is q
 from the keys to the queries and to the outputs, and attention itself runs over the cache as it is, as one key head of
 kv_rank + rot_dim channels that all query heads read and whose first kv_rank channels are also the values (the
 cache keeps no value plane: ``KVRequest.values_in_keys``).  Nothing is expanded per cached token, so prompts in
-portions, single tokens and batches are one path.
+portions, single tokens and batches are one path.  A prompt whose rows see the same keys many times over takes the other
+order in bfloat16: the latents that the step can see are gathered (``ops.latent_gather``), expanded to keys and values of every
+head by two products and attended to as such on the tcgen05 kernel (``ops.attention_latent_expanded``), three and a
+half times fewer operations a pair; the cache is the same.
 
 Per step: one product for both down-projections (and the output gate's pre-activations, if there is one); a row-wise kernel for the two RMS norms, the rotation of k_r and the
 cache write (``ops.latent_prep``); the query up-projection; the per-head product with W_uk and the rotation of the
@@ -27,6 +30,7 @@ from .base import KVRequest, Mixer, Runtime, TensorDecl
 
 class LatentAttention(Mixer):
     capturable = True
+    EXPANDED_KEYS_A_ROW, EXPANDED_BYTES = 12, 128 << 20
     ROWS_ONE_LAUNCH = 32      # up to this many rows the per-head products run as one launch for all heads
 
     @classmethod
@@ -114,6 +118,47 @@ class LatentAttention(Mixer):
         for h in range(heads):
             ops.gemm(a[:, h, :], w_nk[h], out[:, h, :])
 
+    def _expanded_pages(self, batch, cache) -> int:
+        """How many cache pages the step's rows see in all if it should run over expanded keys and values, else 0.
+
+        Over the latents a (row, key) pair of a head costs kv_rank + rot_dim + kv_rank multiply-adds, over expanded keys and
+        values head_dim + rot_dim + value_dim (1088 against 320 at a latent of 512), and the expansion itself
+        kv_rank (head_dim + value_dim) a key.  So it pays where a key is seen by enough rows.  Measured over eight layers (16
+        heads, a latent of 512, a window of 1024; ms a step, absorbed and expanded): 3244 rows over 3264 keys 8.4 and 4.9,
+        3741 over 12160 11.1 and 5.9, 1121 over 9280 6.3 and 3.4; 128 over 1152 and 70 over 1088 the same, 261 rows of
+        four sequences over 4352 3.5 and 3.6.  The expanded rows are scratch memory: no more of it than the absorbed queries
+        and outputs would take, or EXPANDED_BYTES."""
+        s, ops = self.spec, self.rt.ops
+        if batch.extents is None or not ops.latent_expanded_accepts(self.rt.act_dtype, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank, batch.max_q_len):
+            return 0
+        if self.uk_kn.dtype != torch.bfloat16 or self.uv_nk.dtype != torch.bfloat16:
+            return 0
+        window = int(s.window)
+        pages = 0
+        for known, rows in batch.extents:
+            pages += (known + rows + 63) // 64 - (max(0, known - window + 1) // 64 if window > 0 else 0)
+        expanded = 2 * 64 * pages * (self.key_dim + s.heads * (s.head_dim + s.value_dim))
+        absorbed = 2 * batch.rows * s.heads * (self.key_dim + s.kv_rank)
+        return pages if 64 * pages <= self.EXPANDED_KEYS_A_ROW * batch.rows and expanded <= max(absorbed, self.EXPANDED_BYTES) else 0
+
+    def _expanded(self, batch, q: torch.Tensor, cache, pages: int) -> torch.Tensor:
+        """Attention over keys and values made from the visible latents for this step: [rows, heads * value_dim]."""
+        ops, s = self.rt.ops, self.spec
+        H, R, dev = s.heads, s.kv_rank, q.device
+        cos, sin, _ = self.position.kernel_args()
+        ops.latent_q_rot(q, q, H, s.head_dim, s.rot_dim, cos, sin, batch.row_pos)
+        lat = torch.empty((64 * pages, self.key_dim), dtype=q.dtype, device=dev)
+        base = torch.empty((batch.nseq,), dtype=torch.int32, device=dev)
+        ops.latent_gather(cache.k, cache.block_table, batch.seq_slot, batch.seq_q_len, batch.seq_kv_len, batch.nseq, int(s.window), lat, base)
+        keys = torch.empty((64 * pages, H * s.head_dim), dtype=q.dtype, device=dev)
+        values = torch.empty((64 * pages, H * s.value_dim), dtype=q.dtype, device=dev)
+        ops.gemm(lat[:, :R], self.uk_kn.view(H * s.head_dim, R), keys)
+        ops.gemm(lat[:, :R], self.uv_nk.view(H * s.value_dim, R), values)
+        ctx = torch.empty((q.shape[0], H * s.value_dim), dtype=q.dtype, device=dev)
+        ops.attention_latent_expanded(q, ctx, keys, values, lat, base, R, batch.seq_q_start, batch.seq_q_len, batch.seq_kv_len, batch.nseq,
+                                      batch.max_q_len, H, float(s.scale), int(s.window), int(s.chunk))
+        return ctx
+
     def forward(self, batch, x: torch.Tensor, out: torch.Tensor, cache) -> None:
         ops, s = self.rt.ops, self.spec
         rows = x.shape[0]
@@ -131,6 +176,13 @@ class LatentAttention(Mixer):
                         cache.block_table, cache.k, cache.writable)
         q = torch.empty((rows, H * (d + dr)), dtype=x.dtype, device=x.device)
         ops.gemm(cq, self.uq, q)
+        pages = self._expanded_pages(batch, cache)
+        if pages:
+            ctx = self._expanded(batch, q, cache, pages)
+            if self.gated:
+                ops.head_norm_gate(ctx, made[:, Q + R + dr:], ctx, H, dv, ops.GATE_SIGMOID)
+            ops.gemm(ctx, self.o, out)
+            return
         qa = torch.empty((rows, H * self.key_dim), dtype=x.dtype, device=x.device)       # per head [W_uk^T q_plain | rotated part]
         self._per_head(q.view(rows, H, d + dr)[:, :, :d], self.uk_kn, self.uk_nk, qa.view(rows, H, self.key_dim)[:, :, :R])
         ops.latent_q_rot(q, qa, H, d, dr, cos, sin, batch.row_pos)

@@ -653,3 +653,66 @@ def test_the_command_line_writes_and_runs_a_named_configuration(tmp_path):
             logits = P.forward(cfg, w, ids)[-1]
             assert logits.max() - logits[t] <= 1e-5
             ids.append(t)
+
+
+@pytest.mark.parametrize("heads,kv_rank", [(3, 40), (16, 512)])
+@pytest.mark.parametrize("q_lens,kv_lens,window,chunk", [([65], [65], 0, 0), ([300, 1, 65], [300, 130, 700], 0, 0), ([129, 257], [700, 257], 150, 0),
+                                                         ([256, 70], [256, 128], 7, 0), ([200, 66], [333, 66], 0, 96), ([500, 65], [900, 65], 300, 100)])
+def test_prompts_over_expanded_latents(heads, kv_rank, q_lens, kv_lens, window, chunk):
+    """Gathered latents, expanded keys and values and the attention over them, against plain torch in 64 bits from the
+    same bfloat16 keys and values: whole prompts, prompts behind a context, a single row, windows and blocks that cut
+    pages, tiles and pages with remainders.  Rows behind a sequence's end hold NaN in the cache and must not be read."""
+    import torch
+    from gophonic_b200 import ops
+    dev, d, nseq = "cuda:0", kv_rank + 64, len(q_lens)
+    gen = torch.Generator(dev).manual_seed(5)
+    rnd = lambda *shape, scale=1.0: (torch.randn(shape, generator=gen, device=dev) * scale).to(torch.bfloat16)
+    i32 = lambda x: torch.tensor(list(x), dtype=torch.int32, device=dev)
+    most = max((n + 63) // 64 for n in kv_lens)
+    table = torch.randperm(nseq * most + 2, generator=torch.Generator().manual_seed(2))[:nseq * most].view(nseq, most).to(torch.int32).to(dev)
+    plane = torch.full((nseq * most + 2, 1, 64, d), float("nan"), dtype=torch.bfloat16, device=dev)
+    for i, n in enumerate(kv_lens):
+        for at in range(0, n, 64):
+            plane[table[i, at // 64].item(), 0, :min(64, n - at)] = rnd(min(64, n - at), d)
+    rows = sum(q_lens)
+    q = rnd(rows, heads * 192)
+    uk, uv = rnd(heads * 128, kv_rank, scale=kv_rank ** -0.5), rnd(heads * 128, kv_rank, scale=kv_rank ** -0.5)
+    firsts = [max(0, n - m - window + 1) // 64 if window else 0 for m, n in zip(q_lens, kv_lens)]
+    spans = [(n + 63) // 64 - f for n, f in zip(kv_lens, firsts)]
+    lat = torch.full((64 * sum(spans), d), float("nan"), dtype=torch.bfloat16, device=dev)
+    base = i32([-1] * nseq)
+    ql, kl = i32(q_lens), i32(kv_lens)
+    ops.latent_gather(plane, table, i32(range(nseq)), ql, kl, nseq, window, lat, base)
+    at = 0
+    for i, (n, f, span) in enumerate(zip(kv_lens, firsts, spans)):
+        assert base[i].item() == at - 64 * f
+        live = n - 64 * f
+        whole = torch.cat([plane[table[i, p].item(), 0] for p in range(f, f + span)])
+        assert torch.equal(lat[at:at + live], whole[:live]) and not lat[at + live:at + 64 * span].any()
+        at += 64 * span
+    keys, values = (torch.empty((lat.shape[0], heads * 128), dtype=torch.bfloat16, device=dev) for _ in range(2))
+    ops.gemm(lat[:, :kv_rank], uk, keys)
+    ops.gemm(lat[:, :kv_rank], uv, values)
+    out = torch.full((rows, heads * 128), float("nan"), dtype=torch.bfloat16, device=dev)
+    scale = 192 ** -0.5
+    ops.attention_latent_expanded(q, out, keys, values, lat, base, kv_rank, i32([sum(q_lens[:i]) for i in range(nseq)]), ql, kl, nseq, max(q_lens),
+                                  heads, scale, window, chunk)
+    assert ops.tc5_status() == 0
+    r = 0
+    for i, (m, n, f) in enumerate(zip(q_lens, kv_lens, firsts)):
+        b = base[i].item()
+        k = torch.cat([keys[b + 64 * f:b + n].double().view(-1, heads, 128),
+                       lat[b + 64 * f:b + n, None, kv_rank:].double().expand(-1, heads, -1)], -1)
+        v = values[b + 64 * f:b + n].double().view(-1, heads, 128)
+        pos = torch.arange(n - m, n, device=dev)[:, None]
+        key = torch.arange(64 * f, n, device=dev)[None]
+        see = key <= pos
+        if window:
+            see &= key > pos - window
+        if chunk:
+            see &= key >= pos - pos % chunk
+        s = torch.einsum("ihd,jhd->hij", q[r:r + m].double().view(m, heads, 192), k) * scale
+        want = torch.einsum("hij,jhd->ihd", s.masked_fill(~see, -torch.inf).softmax(-1), v).reshape(m, -1)
+        # probabilities and outputs are rounded to bfloat16 (2^-9 each), the exponentials are good to 2e-4
+        assert (out[r:r + m].double() - want).abs().max() <= 1.2e-2 * want.abs().max()
+        r += m
