@@ -196,52 +196,92 @@ struct SampleParams {
 };
 
 // The walk over the k likeliest candidates, most likely first (cand[i] = key << 32 | ~index, sorted
-// descending): weights, nucleus cut, draw.  Thread 0 does the sums one after another in fp32, the
-// order the reference adds them in.
+// descending): weights, nucleus cut, draw.  The sums are taken one after another in fp32, the order
+// the reference adds them in, so the walk is a chain of up to 2 k additions; the weights of WALK
+// candidates are read ahead of the chain (one at a time, each addition waited for its operand: the
+// last kernel of 16 rows, eight of them with 1024 candidates, took 64 us, and 28 now, the sort among them).
+// prob holds MAXK weights, acc MAXK sums.
+constexpr int WALK = 16;
+static_assert(MAXK % WALK == 0, "whole rounds of the walk");
+
+__device__ __forceinline__ void walk_read(float (&v)[WALK], const float* prob, int i) {
+#pragma unroll
+    for (int j = 0; j < WALK; j += 4) *(float4*)(v + j) = *(const float4*)(prob + i + j);
+}
+
 __device__ void pick_from_sorted(const SampleParams& p, int r, int o, const float* __restrict__ row, int k, float temp,
-                                 const unsigned long long* cand, float* prob) {
+                                 const unsigned long long* cand, float* prob, float* acc) {
     const int tid = threadIdx.x;
     const float inv = 1.f / temp;
     const int top_i = (int)(0xFFFFFFFFu - (uint32_t)(cand[0] & 0xFFFFFFFFull));
     const float top = row[top_i];
-    for (int i = tid; i < k; i += ST) {
-        int idx = (int)(0xFFFFFFFFu - (uint32_t)(cand[i] & 0xFFFFFFFFull));
-        prob[i] = expf((row[idx] - top) * inv);
+    const int rounds = (k + WALK - 1) / WALK;
+    for (int i = tid; i < rounds * WALK; i += ST) {  // weights of 0 behind the last candidate change no sum
+        int idx = i < k ? (int)(0xFFFFFFFFu - (uint32_t)(cand[i] & 0xFFFFFFFFull)) : 0;
+        prob[i] = i < k ? expf((row[idx] - top) * inv) : 0.f;
     }
     __syncthreads();
-    if (tid == 0) {
-        float sum = 0.f;
-        for (int i = 0; i < k; i++) sum += prob[i];
-        int n = k;
-        float tp = p.top_p[o];
-        if (tp > 0.f && tp < 1.f) {
-            float acc = 0.f;
-            for (int i = 0; i < k; i++) {
-                acc += prob[i];
-                if (acc >= tp * sum) {
-                    n = i + 1;
-                    sum = acc;
-                    break;
-                }
-            }
+    if (tid >= 32) return;
+    // one warp: every lane runs the same chain, the searches are shared out
+    float v[WALK], next[WALK];
+    float sum = 0.f;
+    walk_read(v, prob, 0);
+    for (int c = 0; c < rounds; c++) {
+        if (c + 1 < rounds) walk_read(next, prob, (c + 1) * WALK);
+#pragma unroll
+        for (int j = 0; j < WALK; j++) {
+            sum += v[j];
+            v[j] = sum;
         }
-        float rr = draw01(p.seed[o], p.draw[o]) * sum;
-        int pick = n - 1;
-        for (int i = 0; i < n; i++) {
-            rr -= prob[i];
-            if (rr <= 0.f) {
-                pick = i;
+        if (tid == 0) {
+#pragma unroll
+            for (int j = 0; j < WALK; j += 4) *(float4*)(acc + c * WALK + j) = *(const float4*)(v + j);
+        }
+#pragma unroll
+        for (int j = 0; j < WALK; j++) v[j] = next[j];
+    }
+    __syncwarp();
+    int n = k;
+    const float tp = p.top_p[o];
+    if (tp > 0.f && tp < 1.f) {
+        const float reach = tp * sum;
+        for (int i = 0; i < k; i += 32) {
+            const uint32_t hit = __ballot_sync(0xffffffffu, i + tid < k && acc[i + tid] >= reach);
+            if (hit) {
+                n = i + __ffs(hit);
+                sum = acc[n - 1];
                 break;
             }
         }
+    }
+    float rr = draw01(p.seed[o], p.draw[o]) * sum;
+    int pick = n - 1;
+    walk_read(v, prob, 0);
+    for (int i = 0; i < n; i += WALK) {
+        if (i + WALK < n) walk_read(next, prob, i + WALK);
+        uint32_t hit = 0;
+#pragma unroll
+        for (int j = 0; j < WALK; j++) {
+            rr -= v[j];
+            hit |= rr <= 0.f ? 1u << j : 0u;
+        }
+        if (hit) {
+            const int at = i + __ffs(hit) - 1;
+            pick = at < n ? at : n - 1;
+            break;
+        }
+#pragma unroll
+        for (int j = 0; j < WALK; j++) v[j] = next[j];
+    }
+    if (tid == 0) {
         p.out[r] = (int)(0xFFFFFFFFu - (uint32_t)(cand[pick] & 0xFFFFFFFFull));
         if (p.advance) p.draw[o] += 1ull;
     }
 }
 
 // One CTA selects for one row by itself: radix select of the k-th largest logit over the whole row,
-// gather, sort.  `cand` holds at least MAXK entries, `prob` MAXK.
-__device__ void sample_row_full(const SampleParams& p, int r, int o, unsigned long long* cand, float* prob) {
+// gather, sort.  `cand` holds at least MAXK entries, `prob` and `acc` MAXK each.
+__device__ void sample_row_full(const SampleParams& p, int r, int o, unsigned long long* cand, float* prob, float* acc) {
     __shared__ float s_val[32];
     __shared__ int s_idx[32];
     __shared__ uint32_t bins[256];
@@ -329,14 +369,14 @@ __device__ void sample_row_full(const SampleParams& p, int r, int o, unsigned lo
             __syncthreads();
         }
     }
-    pick_from_sorted(p, r, o, row, k, temp, cand, prob);
+    pick_from_sorted(p, r, o, row, k, temp, cand, prob, acc);
 }
 
 __global__ void __launch_bounds__(ST) sample_kernel(SampleParams p) {
     __shared__ unsigned long long cand[MAXK];
-    __shared__ float prob[MAXK];
+    __shared__ __align__(16) float prob[MAXK], acc[MAXK];
     const int r = blockIdx.x;
-    sample_row_full(p, r, p.opt_row ? p.opt_row[r] : r, cand, prob);
+    sample_row_full(p, r, p.opt_row ? p.opt_row[r] : r, cand, prob, acc);
 }
 
 // ---- wide rows: three kernels ------------------------------------------------------------
@@ -364,99 +404,190 @@ __device__ __forceinline__ int row_k(const SampleParams& p, int o) {
 __global__ void __launch_bounds__(256) sample_hist_kernel(SampleParams p, uint32_t* __restrict__ hist) {
     __shared__ uint32_t sh[HB];
     const int r = blockIdx.y, tid = threadIdx.x;
+    pdl_trigger();
     for (int i = tid; i < HB; i += 256) sh[i] = 0;
     __syncthreads();
     const float* row = p.logits + (int64_t)r * p.stride;
     const int lo = blockIdx.x * WCHUNK, hi = lo + WCHUNK < p.vocab ? lo + WCHUNK : p.vocab;
-    for (int i = lo + tid; i < hi; i += 256) atomicAdd(&sh[order_key(row[i]) >> 20], 1u);
+    float v[WCHUNK / 256];
+#pragma unroll
+    for (int j = 0; j < WCHUNK / 256; j++) {
+        const int i = lo + tid + 256 * j;
+        v[j] = i < hi ? row[i] : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < WCHUNK / 256; j++)
+        if (lo + tid + 256 * j < hi) atomicAdd(&sh[order_key(v[j]) >> 20], 1u);
     __syncthreads();
     uint32_t* h = hist + (int64_t)r * HROW;
     for (int i = tid; i < HB; i += 256)
         if (sh[i]) atomicAdd(&h[i], sh[i]);
 }
 
+// The chunk's logits are requested before the histogram is complete, the bin is found by a sum over the CTA and a
+// CTA asks for its places in the list once (a place at a time and the histogram walked by one thread: 19 us
+// for 16 rows of 151936, 11 now, some of it beside the histogram).  The order of the list is that of arrival; its entries differ, so
+// what is sorted from it is the same.
 __global__ void __launch_bounds__(256) sample_gather_kernel(SampleParams p, uint32_t* __restrict__ hist,
                                                             unsigned long long* __restrict__ cands) {
-    __shared__ uint32_t sh[HB];
-    __shared__ uint32_t seg[256];
+    constexpr int SEG = HB / 256, PER = WCHUNK / 256;
+    __shared__ uint32_t part[8];
     __shared__ int s_bin;
-    const int r = blockIdx.y, tid = threadIdx.x;
+    __shared__ uint32_t s_first;
+    const int r = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int o = p.opt_row ? p.opt_row[r] : r;
-    uint32_t* h = hist + (int64_t)r * HROW;
-    uint32_t local = 0;
-    for (int i = 0; i < HB / 256; i++) {
-        uint32_t v = h[tid * (HB / 256) + i];
-        sh[tid * (HB / 256) + i] = v;
-        local += v;
+    const float* row = p.logits + (int64_t)r * p.stride;
+    const int lo = blockIdx.x * WCHUNK, hi = lo + WCHUNK < p.vocab ? lo + WCHUNK : p.vocab;
+    float v[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int i = lo + tid + 256 * j;
+        v[j] = i < hi ? row[i] : 0.f;
     }
-    seg[tid] = local;
-    __syncthreads();
-    if (tid == 0) {
-        const uint32_t k = (uint32_t)row_k(p, o);
-        uint32_t cum = 0;
+    if (tid == 0) s_bin = 0;
+    pdl_wait_cta();
+    pdl_trigger();
+    // counts before this thread's in the order of the warps' threads, with the CTA's total
+    auto scan = [&](uint32_t n, uint32_t& total) {
+        uint32_t inc = n;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += x;
+        }
+        if (lane == 31) part[warp] = inc;
+        __syncthreads();
+        uint32_t before = 0;
+        total = 0;
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            if (w < warp) before += part[w];
+            total += part[w];
+        }
+        __syncthreads();
+        return before + inc - n;
+    };
+    // thread 0 holds the highest bins: the lowest bin that the k likeliest logits reach
+    uint32_t* h = hist + (int64_t)r * HROW;
+    uint32_t bins[SEG], local = 0, total;
+    const int first_bin = HB - SEG * (tid + 1);
+#pragma unroll
+    for (int j = 0; j < SEG; j++) {
+        bins[j] = h[first_bin + j];
+        local += bins[j];
+    }
+    const uint32_t k = (uint32_t)row_k(p, o), above = scan(local, total);
+    if (above < k && above + local >= k) {
+        uint32_t cum = above;
         int bin = 0;
-        for (int t = 255; t >= 0; t--) {
-            if (cum + seg[t] >= k) {
-                for (int b = t * (HB / 256) + HB / 256 - 1; b >= t * (HB / 256); b--) {
-                    cum += sh[b];
-                    if (cum >= k) {
-                        bin = b;
-                        break;
-                    }
-                }
-                break;
+        bool found = false;
+#pragma unroll
+        for (int j = SEG - 1; j >= 0; j--) {
+            cum += bins[j];
+            if (!found && cum >= k) {
+                bin = first_bin + j;
+                found = true;
             }
-            cum += seg[t];
         }
         s_bin = bin;
     }
     __syncthreads();
     const uint32_t bin = (uint32_t)s_bin;
-    const float* row = p.logits + (int64_t)r * p.stride;
+    uint32_t hits = 0;
+#pragma unroll
+    for (int j = 0; j < PER; j++) hits += lo + tid + 256 * j < hi && (order_key(v[j]) >> 20) >= bin ? 1u : 0u;
+    const uint32_t mine = scan(hits, total);
+    if (total == 0) return;
+    if (tid == 0) s_first = atomicAdd(&h[HB], total);
+    __syncthreads();
+    uint32_t slot = s_first + mine;
     unsigned long long* c = cands + (int64_t)r * MAXC;
-    const int lo = blockIdx.x * WCHUNK, hi = lo + WCHUNK < p.vocab ? lo + WCHUNK : p.vocab;
-    for (int i = lo + tid; i < hi; i += 256) {
-        const uint32_t key = order_key(row[i]);
-        if ((key >> 20) >= bin) {
-            const uint32_t slot = atomicAdd(&h[HB], 1u);
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int i = lo + tid + 256 * j;
+        const uint32_t key = order_key(v[j]);
+        if (i < hi && (key >> 20) >= bin) {
             if (slot < (uint32_t)MAXC) c[slot] = ((unsigned long long)key << 32) | (uint32_t)(0xFFFFFFFFu - (uint32_t)i);
+            slot++;
         }
     }
 }
 
+__device__ __forceinline__ void exchange(unsigned long long& a, unsigned long long& b, bool descending) {
+    const unsigned long long hi = a > b ? a : b, lo = a > b ? b : a;
+    a = descending ? hi : lo;
+    b = descending ? lo : hi;
+}
+
+// Bitonic sort of c[0..n), n <= EPT ST, into cand, descending (empty slots are 0 and sink).  A thread keeps EPT neighbouring
+// entries in registers: only partners in another warp meet in shared memory, 15 of the 66 steps of 2048
+// entries.
+template <int EPT>
+__device__ void sort_candidates(const unsigned long long* __restrict__ c, int n, unsigned long long* cand) {
+    const int first = threadIdx.x * EPT;
+    int P = 32;
+    while (P < n) P <<= 1;
+    unsigned long long x[EPT];
+#pragma unroll
+    for (int e = 0; e < EPT; e++) x[e] = first + e < n ? c[first + e] : 0ull;
+    for (int size = 2; size <= P; size <<= 1) {
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            if (EPT == 4 && stride == 2) {
+                exchange(x[0], x[2 % EPT], (first & size) == 0);
+                exchange(x[1 % EPT], x[3 % EPT], ((first + 1) & size) == 0);
+                continue;
+            }
+            if (EPT > 1 && stride == 1) {
+#pragma unroll
+                for (int e = 0; e + 1 < EPT; e += 2) exchange(x[e], x[e + 1], ((first + e) & size) == 0);
+                continue;
+            }
+            unsigned long long other[EPT];
+            if (stride < 32 * EPT) {
+#pragma unroll
+                for (int e = 0; e < EPT; e++) other[e] = __shfl_xor_sync(0xffffffffu, x[e], stride / EPT);
+            } else {
+#pragma unroll
+                for (int e = 0; e < EPT; e++) cand[first + e] = x[e];
+                __syncthreads();
+#pragma unroll
+                for (int e = 0; e < EPT; e++) other[e] = cand[(first + e) ^ stride];
+                __syncthreads();
+            }
+#pragma unroll
+            for (int e = 0; e < EPT; e++) {
+                const bool larger = (((first + e) & size) == 0) == (((first + e) & stride) == 0);   // keeps the larger of the pair
+                x[e] = larger == (x[e] > other[e]) ? x[e] : other[e];
+            }
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < EPT; e++) cand[first + e] = x[e];
+    __syncthreads();
+}
+
 __global__ void __launch_bounds__(ST) sample_final_kernel(SampleParams p, const uint32_t* __restrict__ hist,
                                                           const unsigned long long* __restrict__ cands) {
-    __shared__ unsigned long long cand[MAXC];
-    __shared__ float prob[MAXK];
+    __shared__ __align__(16) unsigned long long cand[MAXC];
+    __shared__ __align__(16) float acc[MAXK];
+    float* prob = (float*)(cand + MAXK);  // behind the k first, which are all that is looked at once they are sorted
     const int r = blockIdx.x, tid = threadIdx.x;
+    pdl_wait_cta();
+    pdl_trigger();
     const int o = p.opt_row ? p.opt_row[r] : r;
     const uint32_t count = hist[(int64_t)r * HROW + HB];
     if (count > (uint32_t)MAXC) {
-        sample_row_full(p, r, o, cand, prob);
+        sample_row_full(p, r, o, cand, prob, acc);
         return;
     }
     const int n = (int)count;
-    int P = 1024;
-    while (P < n) P <<= 1;
     const unsigned long long* c = cands + (int64_t)r * MAXC;
-    for (int i = tid; i < P; i += ST) cand[i] = i < n ? c[i] : 0ull;
-    __syncthreads();
-    // bitonic sort, descending (empty slots are 0 and sink)
-    for (int size = 2; size <= P; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int t = tid; t < P / 2; t += ST) {
-                const int i = ((t & ~(stride - 1)) << 1) | (t & (stride - 1));
-                const int j = i | stride;
-                unsigned long long a = cand[i], b = cand[j];
-                const bool desc = (i & size) == 0;
-                if (desc ? (a < b) : (a > b)) {
-                    cand[i] = b;
-                    cand[j] = a;
-                }
-            }
-            __syncthreads();
-        }
-    }
+    if (n <= ST)
+        sort_candidates<1>(c, n, cand);
+    else if (n <= 2 * ST)
+        sort_candidates<2>(c, n, cand);
+    else
+        sort_candidates<4>(c, n, cand);
     const float* row = p.logits + (int64_t)r * p.stride;
     const float temp = p.temperature[o];
     if (!(temp > 0.f)) {
@@ -465,7 +596,7 @@ __global__ void __launch_bounds__(ST) sample_final_kernel(SampleParams p, const 
     }
     int k = row_k(p, o);
     if (k > n) k = n;
-    pick_from_sorted(p, r, o, row, k, temp, cand, prob);
+    pick_from_sorted(p, r, o, row, k, temp, cand, prob, acc);
 }
 
 // logits[r, v] -= presence[r] for every token v the reply of row r already holds
@@ -550,10 +681,9 @@ GB_API int gb_sample(const float* logits, int rows, int vocab, int64_t stride, c
     const dim3 grid(ceil_div(vocab, WCHUNK), rows);
     sample_hist_kernel<<<grid, 256, 0, stream>>>(p, hist);
     GB_CHECK_LAUNCH("sample_hist");
-    sample_gather_kernel<<<grid, 256, 0, stream>>>(p, hist, cands);
-    GB_CHECK_LAUNCH("sample_gather");
-    sample_final_kernel<<<rows, ST, 0, stream>>>(p, hist, cands);
-    GB_CHECK_LAUNCH("sample_final");
+    cudaError_t e = launch_pdl(sample_gather_kernel, grid, dim3(256), 0, stream, p, hist, cands);
+    if (e == cudaSuccess) e = launch_pdl(sample_final_kernel, dim3(rows), dim3(ST), 0, stream, p, (const uint32_t*)hist, (const unsigned long long*)cands);
+    if (e != cudaSuccess) GB_REFUSE("sample: launch failed: %s", cudaGetErrorString(e));
     return 0;
 }
 
