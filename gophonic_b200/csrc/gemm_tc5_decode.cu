@@ -35,6 +35,7 @@ __device__ int g_status;
 
 constexpr int BMW = 128, BK = 64, THREADS = 192;
 constexpr int W_BYTES = BMW * BK * 2;
+constexpr int MAX_SPLITS = 8;
 
 // the folded variants' extra operands (all null / 0 for the plain product)
 struct DecodeFold {
@@ -284,16 +285,23 @@ __global__ void __launch_bounds__(THREADS) gemm_tc5_decode_kernel(const __grid_c
     const uint32_t part_addr = s32(tiles);
     int j = 0;
     for (int bb = row0; bb < M; bb += row_step, j++) {
-        float v[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int sl = 0; sl < splits; sl++) {
+        // all slices are asked for before the first is added (single-token steps of 16 sequences took 4 % longer, of 50 1.5 %,
+        // while they were read and added one by one, each waiting for the cluster's
+        // shared memory in turn)
+        float x[MAX_SPLITS][4];
+#pragma unroll
+        for (int sl = 0; sl < MAX_SPLITS; sl++) {
+            if (sl >= splits) break;
             uint32_t remote;
             asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(part_addr + (uint32_t)((bb * BMW + nl) * 4)), "r"(sl));
-            float x0, x1, x2, x3;
-            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(x0), "=f"(x1), "=f"(x2), "=f"(x3) : "r"(remote) : "memory");
-            v[0] += x0;
-            v[1] += x1;
-            v[2] += x2;
-            v[3] += x3;
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(x[sl][0]), "=f"(x[sl][1]), "=f"(x[sl][2]), "=f"(x[sl][3]) : "r"(remote) : "memory");
+        }
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int sl = 0; sl < MAX_SPLITS; sl++) {
+            if (sl >= splits) break;
+#pragma unroll
+            for (int e = 0; e < 4; e++) v[e] += x[sl][e];
         }
         if (epi == 2) {
             float* hq = reinterpret_cast<float*>(Y) + (int64_t)bb * ldy + n0 + nl;
