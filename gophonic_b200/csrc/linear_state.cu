@@ -61,40 +61,61 @@ __global__ void forget_gate_kernel(float* __restrict__ q, int64_t q_stride, floa
 }
 
 // ------------------------------------------------------------------------------------------
-// gates of the matrix memory.  One warp per (sequence, head), 32 tokens at a time: the lanes take a
-// token each for the capped gates, the running maximum m_t = max(f_t + m_(t-1), i_t) is walked in
-// order through shuffles (an add and a max a token), then the lanes turn their token's values into
-// the factors keep_t = exp(f_t + m_(t-1) - m_t) and take_t = exp(i_t - m_t).
+// gates of the matrix memory.  One CTA per (sequence, head), 256 tokens at a time: the threads take a
+// token each for the capped gates, one thread walks the running maximum m_t = max(f_t + m_(t-1), i_t) in
+// order (an add and a max a token, their operands read eight tokens ahead), then the threads turn their token's
+// values into the factors keep_t = exp(f_t + m_(t-1) - m_t) and take_t = exp(i_t - m_t).  Bound by the walk
+// (1611 tokens: 44.6 us with one warp that passed every token's gates through shuffles, 25.5 now).
 // coef[r, h] = (keep, take, m_t, -): the last place is filled by the scan's normaliser column.
-__global__ void __launch_bounds__(32) mlstm_gates_kernel(LinearStateParams p) {
-    const int h = blockIdx.x, seq = blockIdx.y, lane = threadIdx.x;
+constexpr int GATE_TOKENS = 256;
+
+__global__ void __launch_bounds__(GATE_TOKENS) mlstm_gates_kernel(LinearStateParams p) {
+    __shared__ __align__(16) float f_s[GATE_TOKENS], i_s[GATE_TOKENS], m_s[GATE_TOKENS + 4];   // m_s[3 + t]: the maximum before token t
+    const int h = blockIdx.x, seq = blockIdx.y, tid = threadIdx.x;
     const int q_len = p.seq_q_len[seq], q_start = p.seq_q_start[seq];
     int slot = p.seq_slot[seq];
     if (!gb_check(slot, p.max_slots, GB_CHECK_SLOT)) slot = 0;
     float* m_state = p.state + (int64_t)slot * p.slot_stride + (int64_t)h * p.head_stride + (int64_t)p.d * p.dv + p.d;
-    float m = *m_state;
     const float cap = p.gate_cap, inv_cap = 1.f / p.gate_cap;
     const float bi = p.gate_bias ? p.gate_bias[h] : 0.f, bf = p.gate_bias ? p.gate_bias[p.heads + h] : 0.f;
-    for (int t0 = 0; t0 < q_len; t0 += 32) {
-        const int t = t0 + lane;
+    if (tid == 0) m_s[3] = *m_state;
+    for (int t0 = 0; t0 < q_len; t0 += GATE_TOKENS) {
+        const int t = t0 + tid, n = q_len - t0 < GATE_TOKENS ? q_len - t0 : GATE_TOKENS;
         float gi = 0.f, gf = 0.f;
         if (t < q_len) {
             const float* g = p.gates + (int64_t)(q_start + t) * p.gates_stride;
             gi = cap * tanhf((g[h] + bi) * inv_cap);
             gf = log_sigmoid(cap * tanhf((g[p.heads + h] + bf) * inv_cap));
         }
-        float m_before = 0.f, m_mine = 0.f;
-        const int n = q_len - t0 < 32 ? q_len - t0 : 32;
-        for (int j = 0; j < n; j++) {
-            const float fj = __shfl_sync(0xffffffffu, gf, j), ij = __shfl_sync(0xffffffffu, gi, j);
-            const float m_new = fmaxf(fj + m, ij);
-            if (lane == j) {
-                m_before = m;
-                m_mine = m_new;
+        i_s[tid] = gi;
+        f_s[tid] = gf;
+        __syncthreads();
+        if (tid == 0) {
+            float m = m_s[3];
+            float4 f[2], i[2];
+            f[0] = *(const float4*)f_s, f[1] = *(const float4*)(f_s + 4), i[0] = *(const float4*)i_s, i[1] = *(const float4*)(i_s + 4);
+            for (int j = 0; j < n; j += 8) {
+                const float4 fa = f[0], fb = f[1], ia = i[0], ib = i[1];
+                if (j + 8 < n) {
+                    f[0] = *(const float4*)(f_s + j + 8), f[1] = *(const float4*)(f_s + j + 12);
+                    i[0] = *(const float4*)(i_s + j + 8), i[1] = *(const float4*)(i_s + j + 12);
+                }
+                float4 a, b;
+                a.x = m = fmaxf(fa.x + m, ia.x);
+                a.y = m = fmaxf(fa.y + m, ia.y);
+                a.z = m = fmaxf(fa.z + m, ia.z);
+                a.w = m = fmaxf(fa.w + m, ia.w);
+                b.x = m = fmaxf(fb.x + m, ib.x);
+                b.y = m = fmaxf(fb.y + m, ib.y);
+                b.z = m = fmaxf(fb.z + m, ib.z);
+                b.w = m = fmaxf(fb.w + m, ib.w);
+                *(float4*)(m_s + 4 + j) = a;
+                *(float4*)(m_s + 8 + j) = b;
             }
-            m = m_new;
         }
+        __syncthreads();
         if (t < q_len) {
+            const float m_before = m_s[3 + tid], m_mine = m_s[4 + tid];
             float4 c;
             c.x = expf(gf + m_before - m_mine);
             c.y = expf(gi - m_mine);
@@ -102,8 +123,10 @@ __global__ void __launch_bounds__(32) mlstm_gates_kernel(LinearStateParams p) {
             c.w = 1.f;
             *reinterpret_cast<float4*>(p.coef + ((int64_t)(q_start + t) * p.heads + h) * 4) = c;
         }
+        __syncthreads();
+        if (tid == 0) m_s[3] = m_s[3 + n];
     }
-    if (lane == 0) *m_state = m;
+    if (tid == 0 && q_len > 0) *m_state = m_s[3];
 }
 
 // ------------------------------------------------------------------------------------------
@@ -325,16 +348,23 @@ __global__ void __launch_bounds__(THREADS) state_scan_kernel(LinearStateParams p
 
 // ------------------------------------------------------------------------------------------
 // The same scan for heads of 128 or 256 key channels, laid out so that shared memory is read once: a
-// warp owns 4 columns and its 32 lanes are 32 slices of the channels (RC = d / 32 each), a thread keeps
-// RC x 4 state elements.  A token's q, k and decay rows are then read by the warp as whole rows (every
+// warp owns CW columns and its 32 lanes are 32 slices of the channels (RC = d / 32 each), a thread keeps
+// RC x CW state elements.  A token's q, k and decay rows are then read by the warp as whole rows (every
 // lane its own 16 bytes, no two quarter-warps the same bytes), four times less shared-memory traffic
-// than with 8 slices and a column a thread, for the same registers.  A tile's 8 tokens x 4 columns of
-// sums are added up over the 32 slices by a five-step exchange that leaves each lane one of them.
+// than with 8 slices and a column a thread, for the same registers.  A tile's sums (WT tokens x CW columns, 32
+// or 16) are added up over the 32 slices by a five-step exchange that leaves each lane one of them.
+// Bound by the latency of a token's chain through a warp: the CTAs of 16 columns leave one a SM, so eight
+// warps of two columns (two a scheduler) and, where shared memory allows, tiles of 16 tokens (1611 tokens of 8 heads of
+// 128 x 256: 190 us with four warps of four columns and tiles of 8, 167 to 182 now).  The sums' order is the same.
+constexpr int WIDE_THREADS = 256;
+
 template <typename T, int RC, int MODE>
-__global__ void __launch_bounds__(THREADS) state_scan_wide_kernel(LinearStateParams p) {
+__global__ void __launch_bounds__(WIDE_THREADS) state_scan_wide_kernel(LinearStateParams p) {
     constexpr bool SCALAR = MODE == 1, WRITES = MODE == 2;
     constexpr int D = 32 * RC;          // key channels of a head
-    constexpr int CW = 4;               // columns a warp (and a thread) owns
+    constexpr int CW = 2;               // columns a warp (and a thread) owns
+    constexpr int TT = RC == 4 ? 16 : 8, THREADS = WIDE_THREADS;   // tokens a tile
+    static_assert(CW * WIDE_THREADS / 32 == COLS && TT * COLS <= THREADS, "the warps own the CTA's columns; a thread fetches a value");
     __shared__ __align__(16) float q_s[TT][D];
     __shared__ __align__(16) float k_s[WRITES ? 1 : TT][WRITES ? 4 : D];
     __shared__ __align__(16) float a_s[SCALAR ? 1 : TT][SCALAR ? 4 : D];
@@ -401,7 +431,7 @@ __global__ void __launch_bounds__(THREADS) state_scan_wide_kernel(LinearStatePar
             if (!WRITES) rk[e] = r[p.k_off + h * D + c];
             ra[e] = SCALAR ? p.coef[(row * H + h) * 4 + 1] : p.decay[row * p.decay_stride + h * D + c];
         }
-        {
+        if (tid < TT * COLS) {
             int t = tid / COLS, jj = j0 + tid % COLS;
             t = t < nt ? t : nt - 1;
             jj = jj < dv ? jj : dv - 1;
@@ -426,7 +456,7 @@ __global__ void __launch_bounds__(THREADS) state_scan_wide_kernel(LinearStatePar
             if (!WRITES) k_s[t][c] = there ? (SCALAR ? to_f32<T>(rk[e]) * ra[e] : to_f32<T>(rk[e])) : 0.f;
             if (!SCALAR) a_s[t][c] = there ? ra[e] : (WRITES ? 0.f : 1.f);
         }
-        {
+        if (tid < TT * COLS) {
             const int t = tid / COLS, jj = tid % COLS;
             float v = 0.f;
             if (t < nt) {
@@ -443,13 +473,13 @@ __global__ void __launch_bounds__(THREADS) state_scan_wide_kernel(LinearStatePar
         }
         __syncthreads();
         if (t0 + TT < q_len) fetch(t0 + TT);
-        float acc[TT * CW];     // index t * 4 + c
+        float acc[TT * CW];     // index t * CW + c
 #pragma unroll
         for (int t = 0; t < TT; t++) {
-            const float4 v4 = *reinterpret_cast<const float4*>(&v_s[t][warp * CW]);
-            const float vv[CW] = {v4.x, v4.y, v4.z, v4.w};
+            const float2 v2 = *reinterpret_cast<const float2*>(&v_s[t][warp * CW]);
+            const float vv[CW] = {v2.x, v2.y};
             const float keep = SCALAR ? keep_s[t] : 0.f;
-            float sum[CW] = {0.f, 0.f, 0.f, 0.f};
+            float sum[CW] = {0.f, 0.f};
 #pragma unroll
             for (int i = 0; i < RC; i += 4) {
                 const float4 q4 = *reinterpret_cast<const float4*>(&q_s[t][lane * RC + i]);
@@ -469,12 +499,15 @@ __global__ void __launch_bounds__(THREADS) state_scan_wide_kernel(LinearStatePar
 #pragma unroll
             for (int c = 0; c < CW; c++) acc[t * CW + c] = sum[c];
         }
-        // 32 sums a thread over 32 slices: halve the sums and the lanes five times
+        // the sums of a thread over 32 slices: halve the sums and the lanes; 16 sums meet whole across the first halves
+        constexpr int SUMS = TT * CW;
         float b16[16], b8[8], b4[4], b2[2], total;
         {
             const bool up = lane & 16;
 #pragma unroll
-            for (int j = 0; j < 16; j++) b16[j] = (up ? acc[j + 16] : acc[j]) + __shfl_xor_sync(0xffffffffu, up ? acc[j] : acc[j + 16], 16);
+            for (int j = 0; j < 16; j++)
+                b16[j] = SUMS == 32 ? (up ? acc[(j + 16) % SUMS] : acc[j]) + __shfl_xor_sync(0xffffffffu, up ? acc[j] : acc[(j + 16) % SUMS], 16)
+                                    : acc[j] + __shfl_xor_sync(0xffffffffu, acc[j], 16);
         }
         {
             const bool up = lane & 8;
@@ -495,7 +528,8 @@ __global__ void __launch_bounds__(THREADS) state_scan_wide_kernel(LinearStatePar
             const bool up = lane & 1;
             total = (up ? b2[1] : b2[0]) + __shfl_xor_sync(0xffffffffu, up ? b2[0] : b2[1], 1);
         }
-        o_s[lane >> 2][warp * CW + (lane & 3)] = total;     // lane l is left with sum number l = t * 4 + c
+        // lane l is left with sum number l % SUMS = t * CW + c
+        if (lane < SUMS) o_s[lane / CW][warp * CW + lane % CW] = total;
         __syncthreads();
         if (norm_col) {
             if (tid < nt) {
@@ -637,9 +671,9 @@ int launch_scan(const LinearStateParams& p, cudaStream_t stream) {
     if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("state_scan: grid (%u, %u, %u) exceeds one launch", grid.x, grid.y, grid.z);
     if (p.d == 128 || p.d == 256) {     // heads whose channels fill a warp's 32 slices: shared memory read once
         if (p.d == 128)
-            state_scan_wide_kernel<T, 4, MODE><<<grid, THREADS, 0, stream>>>(p);
+            state_scan_wide_kernel<T, 4, MODE><<<grid, WIDE_THREADS, 0, stream>>>(p);
         else
-            state_scan_wide_kernel<T, 8, MODE><<<grid, THREADS, 0, stream>>>(p);
+            state_scan_wide_kernel<T, 8, MODE><<<grid, WIDE_THREADS, 0, stream>>>(p);
         GB_CHECK_LAUNCH("state_scan");
         return 0;
     }
@@ -880,7 +914,7 @@ GB_API int gb_state_scan(const LinearStateParams* pp, int dtype, cudaStream_t st
     if (p.scalar_decay) {
         if (!p.coef || !p.gates || !(p.gate_cap > 0.f)) GB_REFUSE("state_scan: gates, their cap (%g) or room for the factors is missing", (double)p.gate_cap);
         if (p.head_stride < (int64_t)p.d * p.dv + p.d + 1) GB_REFUSE("state_scan: the state has no room for the normaliser and the maximum");
-        mlstm_gates_kernel<<<dim3(p.heads, p.nseq), 32, 0, stream>>>(p);
+        mlstm_gates_kernel<<<dim3(p.heads, p.nseq), GATE_TOKENS, 0, stream>>>(p);
         GB_CHECK_LAUNCH("mlstm_gates");
         if (dtype == GB_F32) return launch_scan<float, 1>(p, stream);
         if (dtype == GB_BF16) return launch_scan<__nv_bfloat16, 1>(p, stream);
