@@ -33,6 +33,8 @@ constexpr int PAGE_LIST = 512;     // tiles whose pages a CTA looks up ahead (32
 // LKT: keys a step stages (a page, or half a page); STAGES: steps staged at a time.
 template <int NT, int RG, int WG, int LKT, int STAGES>
 __global__ void __launch_bounds__(32 * WG * RG) attn_latent_mma_kernel(AttnParamsX p) {
+    pdl_wait();
+    pdl_trigger();
     constexpr int LROWS = 16 * RG, THREADS = 32 * WG * RG, LPS = LKT + 8;
     constexpr int KW = LKT / WG, J = KW / 8;      // keys a warp scores, in tiles of 8
     const int d = p.d, SD = d + 8, KS = d / 16;
@@ -318,7 +320,7 @@ int launch_latent(const AttnParamsX& p, cudaStream_t stream) {
         if (e != cudaSuccess) GB_REFUSE("attention_latent: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
         configured = 220 * 1024;
     }
-    attn_latent_mma_kernel<NT, RG, WG, LKT, STAGES><<<grid, 32 * WG * RG, smem, stream>>>(p);
+    launch_pdl(attn_latent_mma_kernel<NT, RG, WG, LKT, STAGES>, dim3(grid), dim3(32 * WG * RG), smem, stream, p);
     GB_CHECK_LAUNCH("attention_latent");
     if (p.num_splits > 1) return gb_attention_merge_launch(p.scratch, p.out, GB_BF16, p.out_row_stride, p.seq_q_start, p.nseq, p.heads, 8 * NT * WG, p.num_splits, 0, nullptr, stream);
     return 0;

@@ -909,6 +909,8 @@ GB_API int gb_qk_norm_rope_kv_write_x(const QkRopeParamsX* pp, int dtype, cudaSt
 // ------------------------------------------------------------------------------------------
 // out[r, :] += bias, float32: the bias of a projection whose product left float32 rows
 __global__ void add_bias_kernel(float* __restrict__ out, const float* __restrict__ bias, int n, int64_t total) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < total) out[i] += bias[i % n];
 }
@@ -918,7 +920,7 @@ GB_API int gb_add_bias(float* out, const float* bias, int rows, int n, cudaStrea
     const int64_t total = (int64_t)rows * n;
     const int64_t blocks = (total + 255) / 256;
     if (blocks > 0x7fffffff) GB_REFUSE("add_bias: %d x %d elements are too many", rows, n);
-    add_bias_kernel<<<(unsigned)blocks, 256, 0, stream>>>(out, bias, n, total);
+    launch_pdl(add_bias_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, out, bias, n, total);
     GB_CHECK_LAUNCH("add_bias");
     return 0;
 }

@@ -34,6 +34,8 @@ __device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.f) - l
 // ------------------------------------------------------------------------------------------
 // decay of gated linear attention, in place: z[r, c] <- sigmoid(z[r, c] + bias[c]) ^ (1 / tau)
 __global__ void gla_decay_kernel(float* __restrict__ z, const float* __restrict__ bias, int64_t total, int width, float inv_tau) {
+    pdl_wait();
+    pdl_trigger();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     float x = z[i] + (bias ? bias[i % width] : 0.f);
@@ -49,6 +51,8 @@ __device__ __forceinline__ float silu_f32(float x) { return x / (1.f + expf(-x))
 
 __global__ void forget_gate_kernel(float* __restrict__ q, int64_t q_stride, float* __restrict__ z, int64_t z_stride, const float* __restrict__ bias,
                                    const float* __restrict__ lower, int64_t total, int width) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const int64_t r = i / width;
@@ -70,6 +74,8 @@ __global__ void forget_gate_kernel(float* __restrict__ q, int64_t q_stride, floa
 constexpr int GATE_TOKENS = 256;
 
 __global__ void __launch_bounds__(GATE_TOKENS) mlstm_gates_kernel(LinearStateParams p) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ __align__(16) float f_s[GATE_TOKENS], i_s[GATE_TOKENS], m_s[GATE_TOKENS + 4];   // m_s[3 + t]: the maximum before token t
     const int h = blockIdx.x, seq = blockIdx.y, tid = threadIdx.x;
     const int q_len = p.seq_q_len[seq], q_start = p.seq_q_start[seq];
@@ -136,6 +142,8 @@ __global__ void __launch_bounds__(GATE_TOKENS) mlstm_gates_kernel(LinearStatePar
 // (p.decay), S <- S + u (v - S), with no key: one staged row less and the same arithmetic an element.
 template <typename T, int RC, int MODE>
 __global__ void __launch_bounds__(THREADS) state_scan_kernel(LinearStateParams p) {
+    pdl_wait();
+    pdl_trigger();
     constexpr bool SCALAR = MODE == 1, WRITES = MODE == 2;
     constexpr int P = (RC / 4) % 2 ? RC : RC + 4;   // slice stride in floats: P / 4 odd, so the 8 slices' 16-byte reads miss each other's banks
     constexpr int ROW = SLICES * P;
@@ -360,6 +368,8 @@ constexpr int WIDE_THREADS = 256;
 
 template <typename T, int RC, int MODE>
 __global__ void __launch_bounds__(WIDE_THREADS) state_scan_wide_kernel(LinearStateParams p) {
+    pdl_wait();
+    pdl_trigger();
     constexpr bool SCALAR = MODE == 1, WRITES = MODE == 2;
     constexpr int D = 32 * RC;          // key channels of a head
     constexpr int CW = 2;               // columns a warp (and a thread) owns
@@ -596,6 +606,8 @@ __global__ void __launch_bounds__(THREADS) state_step_kernel(LinearStateParams p
         const int c = g + SLICES * i;
         st[i] = (mine && c < d) ? (norm_col ? nvec[c] : S[(int64_t)c * dv + j]) : 0.f;
     }
+    pdl_wait();   // the state is this kernel's own, the rows come from the kernels ahead
+    pdl_trigger();
     const T* r = (const T*)p.qkv + row * p.row_stride;
     float keep = 0.f, take = 1.f, m = 0.f;
     if (SCALAR) {
@@ -654,11 +666,11 @@ int launch_step(const LinearStateParams& p, cudaStream_t stream) {
     dim3 grid((p.dv + COLS - 1) / COLS + (MODE == 1 ? 1 : 0), p.heads, p.nseq);
     if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("state_scan: grid (%u, %u, %u) exceeds one launch", grid.x, grid.y, grid.z);
     if (p.d <= 64)
-        state_step_kernel<T, 8, MODE><<<grid, THREADS, 0, stream>>>(p);
+        launch_pdl(state_step_kernel<T, 8, MODE>, dim3(grid), dim3(THREADS), 0, stream, p);
     else if (p.d <= 128)
-        state_step_kernel<T, 16, MODE><<<grid, THREADS, 0, stream>>>(p);
+        launch_pdl(state_step_kernel<T, 16, MODE>, dim3(grid), dim3(THREADS), 0, stream, p);
     else
-        state_step_kernel<T, 32, MODE><<<grid, THREADS, 0, stream>>>(p);
+        launch_pdl(state_step_kernel<T, 32, MODE>, dim3(grid), dim3(THREADS), 0, stream, p);
     GB_CHECK_LAUNCH("state_step");
     return 0;
 }
@@ -671,21 +683,21 @@ int launch_scan(const LinearStateParams& p, cudaStream_t stream) {
     if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("state_scan: grid (%u, %u, %u) exceeds one launch", grid.x, grid.y, grid.z);
     if (p.d == 128 || p.d == 256) {     // heads whose channels fill a warp's 32 slices: shared memory read once
         if (p.d == 128)
-            state_scan_wide_kernel<T, 4, MODE><<<grid, WIDE_THREADS, 0, stream>>>(p);
+            launch_pdl(state_scan_wide_kernel<T, 4, MODE>, dim3(grid), dim3(WIDE_THREADS), 0, stream, p);
         else
-            state_scan_wide_kernel<T, 8, MODE><<<grid, WIDE_THREADS, 0, stream>>>(p);
+            launch_pdl(state_scan_wide_kernel<T, 8, MODE>, dim3(grid), dim3(WIDE_THREADS), 0, stream, p);
         GB_CHECK_LAUNCH("state_scan");
         return 0;
     }
     switch (rc) {
-        case 4: state_scan_kernel<T, 4, MODE><<<grid, THREADS, 0, stream>>>(p); break;
-        case 8: state_scan_kernel<T, 8, MODE><<<grid, THREADS, 0, stream>>>(p); break;
-        case 12: state_scan_kernel<T, 12, MODE><<<grid, THREADS, 0, stream>>>(p); break;
-        case 16: state_scan_kernel<T, 16, MODE><<<grid, THREADS, 0, stream>>>(p); break;
-        case 20: state_scan_kernel<T, 20, MODE><<<grid, THREADS, 0, stream>>>(p); break;
-        case 24: state_scan_kernel<T, 24, MODE><<<grid, THREADS, 0, stream>>>(p); break;
-        case 28: state_scan_kernel<T, 28, MODE><<<grid, THREADS, 0, stream>>>(p); break;
-        case 32: state_scan_kernel<T, 32, MODE><<<grid, THREADS, 0, stream>>>(p); break;
+        case 4: launch_pdl(state_scan_kernel<T, 4, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
+        case 8: launch_pdl(state_scan_kernel<T, 8, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
+        case 12: launch_pdl(state_scan_kernel<T, 12, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
+        case 16: launch_pdl(state_scan_kernel<T, 16, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
+        case 20: launch_pdl(state_scan_kernel<T, 20, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
+        case 24: launch_pdl(state_scan_kernel<T, 24, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
+        case 28: launch_pdl(state_scan_kernel<T, 28, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
+        case 32: launch_pdl(state_scan_kernel<T, 32, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
         default: GB_REFUSE("state_scan: %d key channels a head; at most 256", p.d);
     }
     GB_CHECK_LAUNCH("state_scan");
@@ -731,6 +743,8 @@ __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, const fl
 // per (row, head): y = norm(x / div) * w * gate(g), everything optional but the gate.  One warp a head.
 template <typename TI, typename T>
 __global__ void __launch_bounds__(128) head_norm_gate_kernel(HeadGateParams p) {
+    pdl_wait();
+    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t r = blockIdx.x;
     const int h = blockIdx.y * 4 + warp;
@@ -803,6 +817,8 @@ __global__ void __launch_bounds__(128) head_norm_gate_kernel(HeadGateParams p) {
 // anything is computed: a head of 128 alone is too few bytes in flight a warp to keep the memory busy.
 template <typename TI, typename T>
 __global__ void __launch_bounds__(128) head_norm_gate_span_kernel(HeadGateParams p, int hb) {
+    pdl_wait();
+    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t r = blockIdx.x;
     const int h0 = (blockIdx.y * 4 + warp) * hb;
@@ -885,13 +901,13 @@ int launch_gate(const HeadGateParams& p, cudaStream_t stream) {
         const int hb = 512 / n;     // whole heads in a span of 512 elements
         dim3 grid(p.rows, (p.heads + 4 * hb - 1) / (4 * hb));
         if (grid.y > 65535) GB_REFUSE("head_norm_gate: %d heads exceed one launch", p.heads);
-        head_norm_gate_span_kernel<TI, T><<<grid, 128, 0, stream>>>(p, hb);
+        launch_pdl(head_norm_gate_span_kernel<TI, T>, dim3(grid), dim3(128), 0, stream, p, hb);
         GB_CHECK_LAUNCH("head_norm_gate");
         return 0;
     }
     dim3 grid(p.rows, (p.heads + 3) / 4);
     if (grid.y > 65535) GB_REFUSE("head_norm_gate: %d heads exceed one launch", p.heads);
-    head_norm_gate_kernel<TI, T><<<grid, 128, 0, stream>>>(p);
+    launch_pdl(head_norm_gate_kernel<TI, T>, dim3(grid), dim3(128), 0, stream, p);
     GB_CHECK_LAUNCH("head_norm_gate");
     return 0;
 }
@@ -902,7 +918,7 @@ GB_API int gb_gla_decay(float* z, const float* bias, int rows, int width, float 
     if (rows <= 0) return 0;
     if (width <= 0 || !(tau > 0.f)) GB_REFUSE("gla_decay: width %d, tau %g", width, (double)tau);
     const int64_t total = (int64_t)rows * width;
-    gla_decay_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(z, bias, total, width, 1.f / tau);
+    launch_pdl(gla_decay_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, z, bias, total, width, 1.f / tau);
     GB_CHECK_LAUNCH("gla_decay");
     return 0;
 }
@@ -914,7 +930,7 @@ GB_API int gb_state_scan(const LinearStateParams* pp, int dtype, cudaStream_t st
     if (p.scalar_decay) {
         if (!p.coef || !p.gates || !(p.gate_cap > 0.f)) GB_REFUSE("state_scan: gates, their cap (%g) or room for the factors is missing", (double)p.gate_cap);
         if (p.head_stride < (int64_t)p.d * p.dv + p.d + 1) GB_REFUSE("state_scan: the state has no room for the normaliser and the maximum");
-        mlstm_gates_kernel<<<dim3(p.heads, p.nseq), GATE_TOKENS, 0, stream>>>(p);
+        launch_pdl(mlstm_gates_kernel, dim3(dim3(p.heads, p.nseq)), dim3(GATE_TOKENS), 0, stream, p);
         GB_CHECK_LAUNCH("mlstm_gates");
         if (dtype == GB_F32) return launch_scan<float, 1>(p, stream);
         if (dtype == GB_BF16) return launch_scan<__nv_bfloat16, 1>(p, stream);
@@ -925,7 +941,7 @@ GB_API int gb_state_scan(const LinearStateParams* pp, int dtype, cudaStream_t st
             if (p.max_q_len != 1 && p.rows > 0) {
                 const int width = p.heads * p.d;
                 const int64_t total = (int64_t)p.rows * width;
-                forget_gate_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>((float*)p.qkv + p.q_off, p.row_stride, (float*)p.decay,
+                launch_pdl(forget_gate_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, (float*)p.qkv + p.q_off, p.row_stride, (float*)p.decay,
                                                                                        p.decay_stride, p.gate_bias, p.lower, total, width);
                 GB_CHECK_LAUNCH("forget_gate");
             }

@@ -67,6 +67,8 @@ __device__ __forceinline__ void drop_groups(float* key, float* strength, int E, 
 // CORRECTED: the choice goes by score + correction and, with groups, inside the best of them
 template <bool CORRECTED>
 __global__ void __launch_bounds__(128) moe_route_kernel(MoeRouteParams p) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float key_s[CORRECTED ? 4 : 1][CORRECTED ? 32 * MAX_EXPERTS_PER_LANE : 1];
     __shared__ float group_s[CORRECTED ? 4 : 1][CORRECTED ? 32 * MAX_EXPERTS_PER_LANE : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -178,6 +180,8 @@ __device__ __forceinline__ float expert_act(float z, float u, float w, int kind,
 template <typename T>
 __global__ void moe_act_kernel(const T* __restrict__ up, int64_t up_stride, const float* __restrict__ dense, T* __restrict__ act,
                                int64_t act_stride, int rows, int experts, int ff, int kind, int weight_input, float limit, float slope) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t n = (int64_t)experts * ff;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= rows * n) return;
@@ -196,10 +200,12 @@ __global__ void moe_act_kernel(const T* __restrict__ up, int64_t up_stride, cons
 
 // The same for bfloat16 rows of 16-byte chunks (ff and the strides multiples of 8): eight columns a thread, one read of
 // each operand, no division a column.  Bound by the bytes: 3244 rows of 2048 gated columns, 40 MB, 40.7 us with a
-// column a thread, ACT_US now.
+// column a thread, 11.6 now.
 __global__ void __launch_bounds__(256) moe_act_bf16x8_kernel(const __nv_bfloat16* __restrict__ up, int64_t up_stride, const float* __restrict__ dense,
                                                              __nv_bfloat16* __restrict__ act, int64_t act_stride, int experts, int ff, int kind,
                                                              int weight_input, float limit, float slope) {
+    pdl_wait();
+    pdl_trigger();
     const int c = (blockIdx.x * 256 + threadIdx.x) * 8;
     const int64_t r = blockIdx.y;
     if (c >= experts * ff) return;
@@ -253,6 +259,8 @@ __device__ __forceinline__ float warp_dot<__nv_bfloat16, __nv_bfloat16>(const __
 // few rows: act[r, k, i] = weight[r, k] * relu(W_up[index[r, k]][i, :] . x[r])^2, a warp a hidden unit
 template <typename T, typename TW>
 __global__ void __launch_bounds__(128) moe_up_rows_kernel(MoeRowsParams p) {
+    pdl_wait();
+    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = blockIdx.x * 4 + warp;
     const int pair = blockIdx.y;            // row * top + k
@@ -274,6 +282,8 @@ __global__ void __launch_bounds__(128) moe_up_rows_kernel(MoeRowsParams p) {
 // out[r, c] = sum_k W_down[index[r, k]][c, :] . act[r, k, :], a warp an output column of a row
 template <typename T, typename TW>
 __global__ void __launch_bounds__(128) moe_down_rows_kernel(MoeRowsParams p) {
+    pdl_wait();
+    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = blockIdx.x * 4 + warp;
     const int r = blockIdx.y;
@@ -295,6 +305,8 @@ __global__ void __launch_bounds__(128) moe_down_rows_kernel(MoeRowsParams p) {
 // at the pair's sorted place p, ys[p, c] = down_e[c] . act[p]; the weights are applied when the rows are added up.
 template <typename T, typename TW>
 __global__ void __launch_bounds__(128) moe_up_grouped_kernel(MoeRowsParams p, const int* __restrict__ offsets, const int* __restrict__ src_row) {
+    pdl_wait();
+    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = blockIdx.x * 4 + warp, e = blockIdx.y;
     const int lo = offsets[e], hi = offsets[e + 1];
@@ -317,6 +329,8 @@ __global__ void __launch_bounds__(128) moe_up_grouped_kernel(MoeRowsParams p, co
 
 template <typename T, typename TW>
 __global__ void __launch_bounds__(128) moe_down_grouped_kernel(MoeRowsParams p, const int* __restrict__ offsets, float* __restrict__ ys) {
+    pdl_wait();
+    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = blockIdx.x * 4 + warp, e = blockIdx.y;
     const int lo = offsets[e], hi = offsets[e + 1];
@@ -378,6 +392,8 @@ __device__ __forceinline__ void leave_fragment(float* __restrict__ mine, const f
 template <bool GATED>
 __global__ void __launch_bounds__(32 * MG_WARPS) moe_up_grouped_mma_kernel(MoeRowsParams p, const int* __restrict__ offsets,
                                                                            const int* __restrict__ src_row) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[GATED ? 2 : 1][MG_WARPS][16 * 8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int n0 = blockIdx.x * 16, e = blockIdx.y, K = p.hidden;
@@ -417,6 +433,8 @@ __global__ void __launch_bounds__(32 * MG_WARPS) moe_up_grouped_mma_kernel(MoeRo
 }
 
 __global__ void __launch_bounds__(32 * MG_WARPS) moe_down_grouped_mma_kernel(MoeRowsParams p, const int* __restrict__ offsets, float* __restrict__ ys) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[MG_WARPS][16 * 8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int n0 = blockIdx.x * 16, e = blockIdx.y, K = p.ff;
@@ -454,6 +472,8 @@ constexpr int GROUP_MAX_EXPERTS = 512;
 __global__ void __launch_bounds__(GROUP_THREADS) moe_group_kernel(const int* __restrict__ index, int pairs, int top, int experts,
                                                                  int* __restrict__ offsets, int* __restrict__ place, int* __restrict__ src_row,
                                                                  const float* __restrict__ weight, float* __restrict__ sorted_weight) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ int count[GROUP_MAX_EXPERTS], cursor[GROUP_MAX_EXPERTS];
     const int tid = threadIdx.x;
     for (int e = tid; e < experts; e += GROUP_THREADS) count[e] = 0;
@@ -481,6 +501,8 @@ __global__ void __launch_bounds__(GROUP_THREADS) moe_group_kernel(const int* __r
 // xs[p, :] = x[src_row[p], :], 16 bytes a thread where rows allow it
 template <typename T>
 __global__ void moe_gather_kernel(const T* __restrict__ x, int64_t x_stride, const int* __restrict__ src_row, T* __restrict__ xs, int hidden) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t p = blockIdx.x;
     const T* src = x + (int64_t)src_row[p] * x_stride;
     T* dst = xs + p * hidden;
@@ -516,6 +538,8 @@ __global__ void gelu_kernel(T* __restrict__ z, int64_t n) {
 
 template <typename T, int V>   // V elements a thread: one, or a 16-byte chunk
 __global__ void relu2_kernel(T* __restrict__ z, int64_t n) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
     if (i >= n) return;
     if (V > 1 && i + V <= n) {
@@ -536,10 +560,12 @@ __global__ void relu2_kernel(T* __restrict__ z, int64_t n) {
 }
 
 // out[r, :] = sum_k weight[r, k] * ys[place[r * top + k], :], in the order of k
-// Four columns a thread where rows are 16-byte chunks (V 4): 3244 rows of 2048, two a row, 21.5 us a column a thread, COMBINE_US so.
+// Four columns a thread where rows are 16-byte chunks (V 4): 3244 rows of 2048, two a row, 21.5 us a column a thread, 11.4 so.
 template <int V>
 __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ ys, const int* __restrict__ place, const float* __restrict__ weight,
                                    float* __restrict__ out, int64_t out_stride, int top, int hidden) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t r = blockIdx.x;
     for (int c = threadIdx.x * V; c < hidden; c += 256 * V) {
         float a[V];
@@ -577,7 +603,7 @@ GB_API int gb_moe_group_weights(const int* index, int rows, int top, int experts
     if (rows <= 0) return 0;
     if (experts <= 0 || experts > GROUP_MAX_EXPERTS || top <= 0) GB_REFUSE("moe_group: %d experts, %d a token", experts, top);
     if ((weight != nullptr) != (sorted_weight != nullptr)) GB_REFUSE("moe_group: weights in and out go together");
-    moe_group_kernel<<<1, GROUP_THREADS, 0, stream>>>(index, rows * top, top, experts, offsets, place, src_row, weight, sorted_weight);
+    launch_pdl(moe_group_kernel, dim3(1), dim3(GROUP_THREADS), 0, stream, index, rows * top, top, experts, offsets, place, src_row, weight, sorted_weight);
     GB_CHECK_LAUNCH("moe_group");
     return 0;
 }
@@ -585,9 +611,9 @@ GB_API int gb_moe_group_weights(const int* index, int rows, int top, int experts
 GB_API int gb_moe_gather(const void* x, int64_t x_stride, const int* src_row, void* xs, int pairs, int hidden, int dtype, cudaStream_t stream) {
     if (pairs <= 0) return 0;
     if (dtype == GB_F32)
-        moe_gather_kernel<float><<<pairs, 128, 0, stream>>>((const float*)x, x_stride, src_row, (float*)xs, hidden);
+        launch_pdl(moe_gather_kernel<float>, dim3(pairs), dim3(128), 0, stream, (const float*)x, x_stride, src_row, (float*)xs, hidden);
     else if (dtype == GB_BF16)
-        moe_gather_kernel<__nv_bfloat16><<<pairs, 128, 0, stream>>>((const __nv_bfloat16*)x, x_stride, src_row, (__nv_bfloat16*)xs, hidden);
+        launch_pdl(moe_gather_kernel<__nv_bfloat16>, dim3(pairs), dim3(128), 0, stream, (const __nv_bfloat16*)x, x_stride, src_row, (__nv_bfloat16*)xs, hidden);
     else
         GB_REFUSE("moe_gather: unknown dtype %d", dtype);
     GB_CHECK_LAUNCH("moe_gather");
@@ -600,13 +626,13 @@ GB_API int gb_relu2(void* z, int64_t n, int dtype, cudaStream_t stream) {
     const int64_t per = !vec ? 1 : dtype == GB_F32 ? 4 : 8;
     const unsigned blocks = (unsigned)((n + 256 * per - 1) / (256 * per));
     if (dtype == GB_F32 && vec)
-        relu2_kernel<float, 4><<<blocks, 256, 0, stream>>>((float*)z, n);
+        launch_pdl(relu2_kernel<float, 4>, dim3(blocks), dim3(256), 0, stream, (float*)z, n);
     else if (dtype == GB_F32)
-        relu2_kernel<float, 1><<<blocks, 256, 0, stream>>>((float*)z, n);
+        launch_pdl(relu2_kernel<float, 1>, dim3(blocks), dim3(256), 0, stream, (float*)z, n);
     else if (dtype == GB_BF16 && vec)
-        relu2_kernel<__nv_bfloat16, 8><<<blocks, 256, 0, stream>>>((__nv_bfloat16*)z, n);
+        launch_pdl(relu2_kernel<__nv_bfloat16, 8>, dim3(blocks), dim3(256), 0, stream, (__nv_bfloat16*)z, n);
     else if (dtype == GB_BF16)
-        relu2_kernel<__nv_bfloat16, 1><<<blocks, 256, 0, stream>>>((__nv_bfloat16*)z, n);
+        launch_pdl(relu2_kernel<__nv_bfloat16, 1>, dim3(blocks), dim3(256), 0, stream, (__nv_bfloat16*)z, n);
     else
         GB_REFUSE("relu2: unknown dtype %d", dtype);
     GB_CHECK_LAUNCH("relu2");
@@ -637,9 +663,9 @@ GB_API int gb_moe_combine(const float* ys, const int* place, const float* weight
                           cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (!((hidden | out_stride) & 3) && !(((uintptr_t)ys | (uintptr_t)out) & 15))
-        moe_combine_kernel<4><<<rows, 256, 0, stream>>>(ys, place, weight, out, out_stride, top, hidden);
+        launch_pdl(moe_combine_kernel<4>, dim3(rows), dim3(256), 0, stream, ys, place, weight, out, out_stride, top, hidden);
     else
-        moe_combine_kernel<1><<<rows, 256, 0, stream>>>(ys, place, weight, out, out_stride, top, hidden);
+        launch_pdl(moe_combine_kernel<1>, dim3(rows), dim3(256), 0, stream, ys, place, weight, out, out_stride, top, hidden);
     GB_CHECK_LAUNCH("moe_combine");
     return 0;
 }
@@ -653,9 +679,9 @@ GB_API int gb_moe_route(const MoeRouteParams* pp, cudaStream_t stream) {
     if (p.groups > 1 && (p.experts % p.groups || p.keep_groups <= 0 || p.keep_groups > p.groups || p.experts / p.groups * p.keep_groups < p.top))
         GB_REFUSE("moe_route: %d of %d experts a token out of the best %d of %d groups", p.top, p.experts, p.keep_groups, p.groups);
     if (p.correction || p.groups > 1)
-        moe_route_kernel<true><<<(p.rows + 3) / 4, 128, 0, stream>>>(p);
+        launch_pdl(moe_route_kernel<true>, dim3((p.rows + 3) / 4), dim3(128), 0, stream, p);
     else
-        moe_route_kernel<false><<<(p.rows + 3) / 4, 128, 0, stream>>>(p);
+        launch_pdl(moe_route_kernel<false>, dim3((p.rows + 3) / 4), dim3(128), 0, stream, p);
     GB_CHECK_LAUNCH("moe_route");
     return 0;
 }
@@ -682,12 +708,12 @@ GB_API int gb_moe_act_clamped(const void* up, int64_t up_stride, const float* de
     const unsigned blocks = (unsigned)((total + 255) / 256);
     if (dtype == GB_BF16 && !((ff | up_stride | act_stride) & 7) && !(((uintptr_t)up | (uintptr_t)act) & 15) && rows <= 65535 &&
         (int64_t)experts * ff < (1 << 30))
-        moe_act_bf16x8_kernel<<<dim3(ceil_div(experts * ff, 2048), rows), 256, 0, stream>>>(
+        launch_pdl(moe_act_bf16x8_kernel, dim3(dim3(ceil_div(experts * ff, 2048), rows)), dim3(256), 0, stream, 
             (const __nv_bfloat16*)up, up_stride, dense, (__nv_bfloat16*)act, act_stride, experts, ff, kind, weight_input, limit, slope);
     else if (dtype == GB_F32)
-        moe_act_kernel<float><<<blocks, 256, 0, stream>>>((const float*)up, up_stride, dense, (float*)act, act_stride, rows, experts, ff, kind, weight_input, limit, slope);
+        launch_pdl(moe_act_kernel<float>, dim3(blocks), dim3(256), 0, stream, (const float*)up, up_stride, dense, (float*)act, act_stride, rows, experts, ff, kind, weight_input, limit, slope);
     else if (dtype == GB_BF16)
-        moe_act_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)up, up_stride, dense, (__nv_bfloat16*)act, act_stride,
+        launch_pdl(moe_act_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (const __nv_bfloat16*)up, up_stride, dense, (__nv_bfloat16*)act, act_stride,
                                                                   rows, experts, ff, kind, weight_input, limit, slope);
     else
         GB_REFUSE("moe_act: unknown dtype %d", dtype);
@@ -703,11 +729,11 @@ GB_API int gb_moe_rows(const MoeRowsParams* pp, int dtype, int w_dtype, cudaStre
     dim3 ugrid((p.ff + 3) / 4, p.rows * p.top), dgrid((p.hidden + 3) / 4, p.rows);
     if (ugrid.y > 65535) GB_REFUSE("moe_rows: %d rows exceed one launch", p.rows);
     if (dtype == GB_BF16 && w_dtype == GB_BF16) {
-        moe_up_rows_kernel<__nv_bfloat16, __nv_bfloat16><<<ugrid, 128, 0, stream>>>(p);
-        moe_down_rows_kernel<__nv_bfloat16, __nv_bfloat16><<<dgrid, 128, 0, stream>>>(p);
+        launch_pdl(moe_up_rows_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(ugrid), dim3(128), 0, stream, p);
+        launch_pdl(moe_down_rows_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(dgrid), dim3(128), 0, stream, p);
     } else if (dtype == GB_F32 && w_dtype == GB_F32) {
-        moe_up_rows_kernel<float, float><<<ugrid, 128, 0, stream>>>(p);
-        moe_down_rows_kernel<float, float><<<dgrid, 128, 0, stream>>>(p);
+        launch_pdl(moe_up_rows_kernel<float, float>, dim3(ugrid), dim3(128), 0, stream, p);
+        launch_pdl(moe_down_rows_kernel<float, float>, dim3(dgrid), dim3(128), 0, stream, p);
     } else {
         GB_REFUSE("moe_rows: activations of dtype %d with weights of dtype %d", dtype, w_dtype);
     }
@@ -729,16 +755,16 @@ GB_API int gb_moe_rows_grouped(const MoeRowsParams* pp, const int* offsets, cons
     if (dtype == GB_BF16 && w_dtype == GB_BF16 && aligned) {
         dim3 um((p.ff + 15) / 16, p.experts), dm((p.hidden + 15) / 16, p.experts);
         if (p.act_kind != 0)
-            moe_up_grouped_mma_kernel<true><<<um, 32 * MG_WARPS, 0, stream>>>(p, offsets, src_row);
+            launch_pdl(moe_up_grouped_mma_kernel<true>, dim3(um), dim3(32 * MG_WARPS), 0, stream, p, offsets, src_row);
         else
-            moe_up_grouped_mma_kernel<false><<<um, 32 * MG_WARPS, 0, stream>>>(p, offsets, src_row);
-        moe_down_grouped_mma_kernel<<<dm, 32 * MG_WARPS, 0, stream>>>(p, offsets, ys);
+            launch_pdl(moe_up_grouped_mma_kernel<false>, dim3(um), dim3(32 * MG_WARPS), 0, stream, p, offsets, src_row);
+        launch_pdl(moe_down_grouped_mma_kernel, dim3(dm), dim3(32 * MG_WARPS), 0, stream, p, offsets, ys);
     } else if (dtype == GB_BF16 && w_dtype == GB_BF16) {
-        moe_up_grouped_kernel<__nv_bfloat16, __nv_bfloat16><<<ugrid, 128, 0, stream>>>(p, offsets, src_row);
-        moe_down_grouped_kernel<__nv_bfloat16, __nv_bfloat16><<<dgrid, 128, 0, stream>>>(p, offsets, ys);
+        launch_pdl(moe_up_grouped_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(ugrid), dim3(128), 0, stream, p, offsets, src_row);
+        launch_pdl(moe_down_grouped_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(dgrid), dim3(128), 0, stream, p, offsets, ys);
     } else if (dtype == GB_F32 && w_dtype == GB_F32) {
-        moe_up_grouped_kernel<float, float><<<ugrid, 128, 0, stream>>>(p, offsets, src_row);
-        moe_down_grouped_kernel<float, float><<<dgrid, 128, 0, stream>>>(p, offsets, ys);
+        launch_pdl(moe_up_grouped_kernel<float, float>, dim3(ugrid), dim3(128), 0, stream, p, offsets, src_row);
+        launch_pdl(moe_down_grouped_kernel<float, float>, dim3(dgrid), dim3(128), 0, stream, p, offsets, ys);
     } else {
         GB_REFUSE("moe_rows: activations of dtype %d with weights of dtype %d", dtype, w_dtype);
     }

@@ -39,11 +39,13 @@ constexpr int NSA_KEEP = 8;     // elements of y a thread keeps in registers (ro
 template <typename TO>
 __global__ void __launch_bounds__(256) norm_scale_add_kernel(float* __restrict__ h, const float* __restrict__ y, const float* __restrict__ w,
                                                              float eps, int n, TO* __restrict__ x_out) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float part[8];
     const int64_t row = blockIdx.x;
     const float* yr = y + row * n;
     float* hr = h + row * n;
-    // everything the row needs is asked for ahead of the sum (3244 rows of 2048: 20.5 us with h and w behind it, NORM_US now)
+    // everything the row needs is asked for ahead of the sum (3244 rows of 2048: 20.5 us with h and w behind it, 14.0 now)
     float keep[NSA_KEEP], before[NSA_KEEP], scale[NSA_KEEP];
     float ss = 0.f;
 #pragma unroll
@@ -80,6 +82,8 @@ __global__ void __launch_bounds__(256) norm_scale_add_kernel(float* __restrict__
 template <typename T>
 __global__ void __launch_bounds__(128) diff_combine_kernel(const T* __restrict__ ctx, int64_t ctx_stride, T* __restrict__ out, int64_t out_stride,
                                                            int rows, int heads, int per_group, int dv, float lambda, float eps, float factor) {
+    pdl_wait();
+    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t unit = (int64_t)blockIdx.x * 4 + warp;
     if (unit >= (int64_t)rows * heads) return;
@@ -99,9 +103,11 @@ __global__ void __launch_bounds__(128) diff_combine_kernel(const T* __restrict__
     for (int c = lane; c < dv; c += 32) o[c] = from_f32<T>((to_f32<T>(a1[c]) - lambda * to_f32<T>(a2[c])) * inv);
 }
 
-// V columns a thread: four where rows are 16-byte chunks (3244 rows of 2048: 18.5 us one by one, GATED_US so)
+// V columns a thread: four where rows are 16-byte chunks (3244 rows of 2048: 18.5 us one by one, 11.0 so)
 template <int V>
 __global__ void __launch_bounds__(256) add_rows_gated_kernel(float* __restrict__ out, const float* __restrict__ y, const float* __restrict__ z, int64_t z_stride, int n) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t r = blockIdx.x;
     const float g = 1.f / (1.f + expf(-z[r * z_stride]));
 #pragma unroll 2
@@ -138,11 +144,13 @@ struct LatentPrepArgs {
 };
 
 // Both latents are read once, kept (widths up to 256 LP_KEEP; wider ones are read again) and summed in one round of the CTA.
-// 3244 rows of 768 + 512 + 64: 18 us with a round each and two reads, PREP_US now.
+// 3244 rows of 768 + 512 + 64: 18 us with a round each and two reads, 13.6 now.
 constexpr int LP_KEEP = 4;
 
 template <typename T>
 __global__ void __launch_bounds__(256) latent_prep_kernel(LatentPrepArgs p) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float part[2][8];
     const int64_t r = blockIdx.x;
     const T* src = (const T*)p.lat + r * p.lat_stride;
@@ -223,6 +231,8 @@ __global__ void latent_q_rot_kernel(const T* q, int64_t q_stride, T* out, int64_
                                      int heads, int d, int rot,
                                     int out_head, const float* __restrict__ cos_t, const float* __restrict__ sin_t, int table_positions,
                                     const int* __restrict__ row_pos) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t r = blockIdx.x;
     const int half = rot / 2;
     const int pos = row_pos[r];
@@ -248,6 +258,8 @@ template <typename T, typename TW>
 __global__ void __launch_bounds__(32 * HG_WARPS) head_gemm_kernel(const T* __restrict__ a, int64_t a_row_stride, int64_t a_head_stride,
                                                                  const TW* __restrict__ w, T* __restrict__ out, int64_t o_row_stride,
                                                                  int64_t o_head_stride, int rows, int K, int N) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ float as[];   // [HG_ROWS][K], then [HG_WARPS][HG_ROWS][HG_COLS]
     float* red = as + HG_ROWS * K;
     const int hd = blockIdx.y;
@@ -303,6 +315,8 @@ constexpr int HM_T = 64, HM_S = HM_T + 8;
 __global__ void __launch_bounds__(128) head_gemm_mma_kernel(const __nv_bfloat16* __restrict__ a, int64_t a_row_stride, int64_t a_head_stride,
                                                             const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
                                                             int64_t o_row_stride, int64_t o_head_stride, int rows, int K, int N) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ __align__(16) __nv_bfloat16 As[2][HM_T][HM_S];
     __shared__ __align__(16) __nv_bfloat16 Ws[2][HM_T][HM_S];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
@@ -370,9 +384,9 @@ GB_API int gb_norm_scale_add(float* h, const float* y, const float* w, float eps
     if (n <= 0) GB_REFUSE("norm_scale_add: rows of %d", n);
     if (!h || !y || !w) GB_REFUSE("norm_scale_add: a tensor is missing");
     if (!x_out || x_dtype == GB_F32)
-        norm_scale_add_kernel<float><<<rows, 256, 0, stream>>>(h, y, w, eps, n, (float*)x_out);
+        launch_pdl(norm_scale_add_kernel<float>, dim3(rows), dim3(256), 0, stream, h, y, w, eps, n, (float*)x_out);
     else if (x_dtype == GB_BF16)
-        norm_scale_add_kernel<__nv_bfloat16><<<rows, 256, 0, stream>>>(h, y, w, eps, n, (__nv_bfloat16*)x_out);
+        launch_pdl(norm_scale_add_kernel<__nv_bfloat16>, dim3(rows), dim3(256), 0, stream, h, y, w, eps, n, (__nv_bfloat16*)x_out);
     else
         GB_REFUSE("norm_scale_add: unknown dtype %d", x_dtype);
     GB_CHECK_LAUNCH("norm_scale_add");
@@ -386,9 +400,9 @@ GB_API int gb_diff_combine(const void* ctx, int64_t ctx_stride, void* out, int64
     const int64_t units = (int64_t)rows * heads;
     const unsigned blocks = (unsigned)((units + 3) / 4);
     if (dtype == GB_F32)
-        diff_combine_kernel<float><<<blocks, 128, 0, stream>>>((const float*)ctx, ctx_stride, (float*)out, out_stride, rows, heads, per_group, dv, lambda, eps, factor);
+        launch_pdl(diff_combine_kernel<float>, dim3(blocks), dim3(128), 0, stream, (const float*)ctx, ctx_stride, (float*)out, out_stride, rows, heads, per_group, dv, lambda, eps, factor);
     else if (dtype == GB_BF16)
-        diff_combine_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>((const __nv_bfloat16*)ctx, ctx_stride, (__nv_bfloat16*)out, out_stride, rows, heads,
+        launch_pdl(diff_combine_kernel<__nv_bfloat16>, dim3(blocks), dim3(128), 0, stream, (const __nv_bfloat16*)ctx, ctx_stride, (__nv_bfloat16*)out, out_stride, rows, heads,
                                                                       per_group, dv, lambda, eps, factor);
     else
         GB_REFUSE("diff_combine: unknown dtype %d", dtype);
@@ -399,9 +413,9 @@ GB_API int gb_diff_combine(const void* ctx, int64_t ctx_stride, void* out, int64
 GB_API int gb_add_rows_gated(float* out, const float* y, const float* z, int64_t z_stride, int rows, int n, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (!(n & 3) && !(((uintptr_t)out | (uintptr_t)y) & 15))
-        add_rows_gated_kernel<4><<<rows, 256, 0, stream>>>(out, y, z, z_stride, n);
+        launch_pdl(add_rows_gated_kernel<4>, dim3(rows), dim3(256), 0, stream, out, y, z, z_stride, n);
     else
-        add_rows_gated_kernel<1><<<rows, 256, 0, stream>>>(out, y, z, z_stride, n);
+        launch_pdl(add_rows_gated_kernel<1>, dim3(rows), dim3(256), 0, stream, out, y, z, z_stride, n);
     GB_CHECK_LAUNCH("add_rows_gated");
     return 0;
 }
@@ -416,9 +430,9 @@ GB_API int gb_latent_prep(const void* lat, int64_t lat_stride, void* cq, const f
     LatentPrepArgs p{lat, lat_stride, cq, q_w, kv_w, eps, cos_t, sin_t, table_positions, row_pos, row_seq, seq_slot, block_table, bt_stride,
                      k_plane, write_kv, rows, q_rank, kv_rank, rot, pages, max_slots};
     if (dtype == GB_F32)
-        latent_prep_kernel<float><<<rows, 256, 0, stream>>>(p);
+        launch_pdl(latent_prep_kernel<float>, dim3(rows), dim3(256), 0, stream, p);
     else if (dtype == GB_BF16)
-        latent_prep_kernel<__nv_bfloat16><<<rows, 256, 0, stream>>>(p);
+        launch_pdl(latent_prep_kernel<__nv_bfloat16>, dim3(rows), dim3(256), 0, stream, p);
     else
         GB_REFUSE("latent_prep: unknown dtype %d", dtype);
     GB_CHECK_LAUNCH("latent_prep");
@@ -430,10 +444,10 @@ GB_API int gb_latent_q_rot(const void* q, int64_t q_stride, void* out, int64_t o
     if (rows <= 0 || rot <= 0) return 0;
     if ((rot & 1) || out_head < rot) GB_REFUSE("latent_q_rot: %d rotated channels into heads of %d", rot, out_head);
     if (dtype == GB_F32)
-        latent_q_rot_kernel<float><<<rows, 128, 0, stream>>>((const float*)q, q_stride, (float*)out, out_stride, heads, d, rot, out_head, cos_t, sin_t,
+        launch_pdl(latent_q_rot_kernel<float>, dim3(rows), dim3(128), 0, stream, (const float*)q, q_stride, (float*)out, out_stride, heads, d, rot, out_head, cos_t, sin_t,
                                                              table_positions, row_pos);
     else if (dtype == GB_BF16)
-        latent_q_rot_kernel<__nv_bfloat16><<<rows, 128, 0, stream>>>((const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, out_stride, heads, d, rot,
+        launch_pdl(latent_q_rot_kernel<__nv_bfloat16>, dim3(rows), dim3(128), 0, stream, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, out_stride, heads, d, rot,
                                                                      out_head, cos_t, sin_t, table_positions, row_pos);
     else
         GB_REFUSE("latent_q_rot: unknown dtype %d", dtype);
@@ -451,12 +465,12 @@ GB_API int gb_head_gemm(const void* a, int64_t a_row_stride, int64_t a_head_stri
     if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("head_gemm: %d heads, %d rows exceed one launch", heads, rows);
     if (dtype == GB_F32 && w_dtype == GB_F32) {
         if (smem > 48 * 1024) cudaFuncSetAttribute(head_gemm_kernel<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-        head_gemm_kernel<float, float><<<grid, 32 * HG_WARPS, smem, stream>>>((const float*)a, a_row_stride, a_head_stride, (const float*)w, (float*)out,
+        launch_pdl(head_gemm_kernel<float, float>, dim3(grid), dim3(32 * HG_WARPS), smem, stream, (const float*)a, a_row_stride, a_head_stride, (const float*)w, (float*)out,
                                                                              o_row_stride, o_head_stride, rows, K, N);
     } else if (dtype == GB_BF16 && w_dtype == GB_BF16) {
         if (smem > 48 * 1024)
             cudaFuncSetAttribute(head_gemm_kernel<__nv_bfloat16, __nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-        head_gemm_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 32 * HG_WARPS, smem, stream>>>((const __nv_bfloat16*)a, a_row_stride, a_head_stride,
+        launch_pdl(head_gemm_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(grid), dim3(32 * HG_WARPS), smem, stream, (const __nv_bfloat16*)a, a_row_stride, a_head_stride,
                                                                                              (const __nv_bfloat16*)w, (__nv_bfloat16*)out, o_row_stride,
                                                                                              o_head_stride, rows, K, N);
     } else {
@@ -481,7 +495,7 @@ GB_API int gb_head_gemm_mma(const void* a, int64_t a_row_stride, int64_t a_head_
         GB_REFUSE("head_gemm_mma: %d heads of %d x %d with these strides are not what this kernel takes", heads, K, N);
     dim3 grid((N + HM_T - 1) / HM_T, heads, (rows + HM_T - 1) / HM_T);
     if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("head_gemm_mma: %d heads, %d rows exceed one launch", heads, rows);
-    head_gemm_mma_kernel<<<grid, 128, 0, stream>>>((const __nv_bfloat16*)a, a_row_stride, a_head_stride, (const __nv_bfloat16*)w, (__nv_bfloat16*)out,
+    launch_pdl(head_gemm_mma_kernel, dim3(grid), dim3(128), 0, stream, (const __nv_bfloat16*)a, a_row_stride, a_head_stride, (const __nv_bfloat16*)w, (__nv_bfloat16*)out,
                                                    o_row_stride, o_head_stride, rows, K, N);
     GB_CHECK_LAUNCH("head_gemm_mma");
     return 0;

@@ -82,8 +82,8 @@ def more_splits(units: int, max_kv_len: int, mean_kv_len: int, sm_count: int, pa
 
 def choose_prompt_splits(tiles: int, max_kv_len: int, sm_count: int = 148) -> int:
     """How many pieces the tcgen05 kernel's CTAs (``tiles``: 256 query rows of a head each) cut their keys into: as many as fill
-    the SMs once, of at least four pages of 64 keys each.  A turn of 90 tokens behind 1000 (32 heads): the layer's attention 29 us
-    whole, SPLIT_US in four pieces with their merge."""
+    the SMs once, of at least four pages of 64 keys each.  A turn of 90 tokens behind 1000 (32 heads): the attention of a layer 29 us whole
+    on 32 CTAs; twelve layers 2051 us whole and 2005 in four pieces."""
     return max(1, min(sm_count // max(1, tiles), (max_kv_len + 63) // 64 // 4, 32))
 
 
