@@ -14,8 +14,8 @@ half times fewer operations a pair; the cache is the same.
 Per step: one product for both down-projections (and the output gate's pre-activations, if there is one); a row-wise kernel for the two RMS norms, the rotation of k_r and the
 cache write (``ops.latent_prep``); the query up-projection; the per-head product with W_uk and the rotation of the
 queries' rotated part into the absorbed queries; attention; the per-head product with W_uv; the output projection.
-The per-head products are one launch for all heads: on the CUDA cores for few rows and for float32, on the tensor cores
-(mma.sync) for prompts in bfloat16; operands that kernel cannot take run one product a head.
+The per-head products are one launch for all heads: on the tensor cores (mma.sync) in bfloat16, on the CUDA cores in float32
+and for few rows that kernel cannot take; what neither takes runs one product a head.
 """
 from __future__ import annotations
 
@@ -31,7 +31,7 @@ from .base import KVRequest, Mixer, Runtime, TensorDecl
 class LatentAttention(Mixer):
     capturable = True
     EXPANDED_KEYS_A_ROW, EXPANDED_BYTES = 12, 128 << 20
-    ROWS_ONE_LAUNCH = 32      # up to this many rows the per-head products run as one launch for all heads
+    ROWS_ONE_LAUNCH = 32      # up to this many rows the per-head products that the tensor cores do not take run as one launch
 
     @classmethod
     def declare(cls, spec, prefix: str) -> List[TensorDecl]:
@@ -109,11 +109,13 @@ class LatentAttention(Mixer):
         """out[:, h, :] = a[:, h, :] @ w_kn[h] for every head (``w_nk`` holds the same matrices transposed)."""
         ops = self.rt.ops
         rows, heads, K = a.shape
-        if (self.rt.is_fp32 or rows <= self.ROWS_ONE_LAUNCH) and K <= ops.HEAD_GEMM_MAX_K:
-            ops.head_gemm(a, w_kn, out)
-            return
+        # bfloat16: the tensor cores from one row on (16 heads, us: 128 x 512 one row 3.5 on the CUDA cores and 2.5, 24 rows 7.8 and
+        # 3.0; 512 x 128 7.7 and 5.6, 24 rows 9.8 and 5.9; the same error against 64 bits)
         if ops.head_gemm_mma_accepts(a, w_nk, out):
             ops.head_gemm_mma(a, w_nk, out)
+            return
+        if (self.rt.is_fp32 or rows <= self.ROWS_ONE_LAUNCH) and K <= ops.HEAD_GEMM_MAX_K:
+            ops.head_gemm(a, w_kn, out)
             return
         for h in range(heads):
             ops.gemm(a[:, h, :], w_nk[h], out[:, h, :])
