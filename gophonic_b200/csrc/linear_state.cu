@@ -593,6 +593,8 @@ __global__ void __launch_bounds__(THREADS) state_step_kernel(LinearStateParams p
     const int vblocks = (dv + COLS - 1) / COLS;
     const bool norm_col = SCALAR && (int)blockIdx.x == vblocks;
     const int j = blockIdx.x * COLS + jj;
+    pdl_wait();   // the kernel ahead may be this one, at work on the same state for the token before
+    pdl_trigger();
     const int64_t row = p.seq_q_start[seq];
     int slot = p.seq_slot[seq];
     if (!gb_check(slot, p.max_slots, GB_CHECK_SLOT)) slot = 0;
@@ -606,8 +608,6 @@ __global__ void __launch_bounds__(THREADS) state_step_kernel(LinearStateParams p
         const int c = g + SLICES * i;
         st[i] = (mine && c < d) ? (norm_col ? nvec[c] : S[(int64_t)c * dv + j]) : 0.f;
     }
-    pdl_wait();   // the state is this kernel's own, the rows come from the kernels ahead
-    pdl_trigger();
     const T* r = (const T*)p.qkv + row * p.row_stride;
     float keep = 0.f, take = 1.f, m = 0.f;
     if (SCALAR) {

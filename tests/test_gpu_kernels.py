@@ -897,3 +897,53 @@ def test_presence_penalty_and_seen_bitmap(ops):
     want[0, 5] = want[0, 64] = -1.5
     want[2, 33] = -2.0      # marked twice, penalised once; row 1 has no penalty
     assert torch.equal(logits.cpu(), want)
+
+
+# ---- matrix states ---------------------------------------------------------------------------
+# A portion of a prompt and then one token after the other on the same state with nothing in between, in one captured graph so
+# that the kernels follow one another as closely as they can, against the whole prompt in one call.  The single-token kernel
+# adds a head's channels in another order: 256 products of one size at most, each sum off by 2^-24 of it, make 1.6e-5.
+@pytest.mark.parametrize("form", ["decay", "lower", "gates"])
+@pytest.mark.parametrize("H,d,dv", [(4, 128, 256), (3, 24, 40), (2, 256, 33)])
+def test_states_token_after_token_with_nothing_in_between(ops, form, H, d, dv):
+    lengths, slots, first = [48, 48, 48], [2, 0, 3], 7
+    n, rows = len(lengths), sum(lengths)
+    mk = lambda x: torch.tensor(list(x), dtype=torch.int32, device=DEV)
+    x = rnd(rows, 2 * H * d + H * dv, seed=1, scale=0.5)
+    z = rnd(rows, H * d, seed=2)
+    bias, lower = rnd(H * d, seed=3) + 2.0, torch.sigmoid(rnd(H * d, seed=4))
+    gates, gate_bias = rnd(rows, 2 * H, seed=5), torch.cat([rnd(H, seed=6), rnd(H, seed=7) + 3.0])
+    room = d * dv + (d + 1 if form == "gates" else 0)
+
+    def call(x, z, state, out, starts, lens, most):
+        seq = (mk(slots), starts, lens, n)
+        if form == "gates":
+            coef = torch.empty((rows, H, 4), device=DEV)
+            return lambda: ops.state_scan(x, 0, H * d, 2 * H * d, H, d, dv, d ** -0.5, state, out, *seq, gates=gates, gate_bias=gate_bias,
+                                          gate_cap=15.0, coef=coef, max_q_len=most)
+        extra = dict(decay=torch.sigmoid(z + bias)) if form == "decay" else dict(decay=z, gate_bias=bias, lower=lower)
+        return lambda: ops.state_scan(x, 0, H * d, 2 * H * d, H, d, dv, d ** -0.5, state, out, *seq, max_q_len=most, **extra)
+
+    start = [sum(lengths[:i]) for i in range(n)]
+    start_state = rnd(4, H, room, seed=8, scale=0.1)
+    whole, want = start_state.clone(), torch.full((rows, H * dv), float("nan"), device=DEV)
+    call(x.clone(), z.clone(), whole, want, mk(start), mk(lengths), max(lengths))()
+
+    state, got = start_state.clone(), torch.full((rows, H * dv), float("nan"), device=DEV)
+    # the portion overwrites its rows and gates in one of the forms: it has copies
+    x1, z1 = x.clone(), z.clone()
+    calls = [call(x1, z1, state, got, mk(start), mk([first] * n), first)]
+    calls += [call(x, z, state, got, mk(s + t for s in start), mk([1] * n), 1) for t in range(first, max(lengths))]
+    for c in calls:
+        c()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for c in calls:
+            c()
+    for _ in range(5):
+        for t, now in ((state, start_state), (x1, x), (z1, z), (got, torch.full_like(got, float("nan")))):
+            t.copy_(now)
+        graph.replay()
+        assert (got - want).abs().max().item() <= 256 * 2.0 ** -24 * max(1.0, want.abs().max().item())
+        assert (state - whole).abs().max().item() <= 256 * 2.0 ** -24 * max(1.0, whole.abs().max().item())
