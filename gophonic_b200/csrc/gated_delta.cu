@@ -398,6 +398,8 @@ __global__ void __launch_bounds__(THREADS) gated_delta_step_kernel(GatedDeltaPar
     const int d = p.d, dv = p.dv, H = p.heads;
     const int h = blockIdx.y, seq = blockIdx.z, kh = h / (H / p.kv_heads);
     const int j = blockIdx.x * COLS + jt * V;
+    pdl_wait();   // the kernel ahead may be this one, at work on the same state for the token before
+    pdl_trigger();
     int slot = p.seq_slot[seq];
     if (!gb_check(slot, p.max_slots, GB_CHECK_SLOT)) slot = 0;
     float* S = p.state + (int64_t)slot * p.slot_stride + (int64_t)h * p.head_stride;
@@ -410,8 +412,6 @@ __global__ void __launch_bounds__(THREADS) gated_delta_step_kernel(GatedDeltaPar
         for (int u = 0; u < V; u++) st[i][u] = 0.f;
         if (mine && c < d) lds<V>(S + (int64_t)c * dv + j, st[i]);
     }
-    pdl_wait();                                // the state is this kernel's own; the rows come from the kernels ahead
-    pdl_trigger();
     const int64_t row = p.seq_q_start[seq];
     const float* in = p.rows_in + row * p.row_stride;
     const float rate = expf(p.a_log[h]);

@@ -947,3 +947,42 @@ def test_states_token_after_token_with_nothing_in_between(ops, form, H, d, dv):
         graph.replay()
         assert (got - want).abs().max().item() <= 256 * 2.0 ** -24 * max(1.0, want.abs().max().item())
         assert (state - whole).abs().max().item() <= 256 * 2.0 ** -24 * max(1.0, whole.abs().max().item())
+
+
+# The same of the gated delta rule: a decay a head and one a channel, value columns taken one and four at a time.
+@pytest.mark.parametrize("per_channel", [True, False])
+@pytest.mark.parametrize("H,G,d,dv", [(8, 4, 128, 256), (3, 3, 20, 33)])
+def test_gated_deltas_token_after_token_with_nothing_in_between(ops, per_channel, H, G, d, dv):
+    from types import SimpleNamespace
+    lengths, slots, first = [48, 48, 48], [2, 0, 3], 7
+    n, rows = len(lengths), sum(lengths)
+    mk = lambda x: torch.tensor(list(x), dtype=torch.int32, device=DEV)
+    unit = torch.nn.functional.normalize(rnd(rows, 2 * G, d, seed=1), dim=-1).reshape(rows, -1)
+    x, width = torch.cat([unit, rnd(rows, H * dv, seed=2)], -1), H * d if per_channel else H
+    decay, beta, bias, rate = rnd(rows, width, seed=3), rnd(rows, H, seed=4), rnd(width, seed=5) - 3.0, rnd(H, seed=6)
+    start = [sum(lengths[:i]) for i in range(n)]
+
+    def call(state, out, starts, lens):
+        batch = SimpleNamespace(nseq=n, max_q_len=max(lens), seq_slot=mk(slots), seq_q_start=mk(starts), seq_q_len=mk(lens),
+                                row_seq=mk(i for i in range(n) for _ in range(lengths[i])))
+        return lambda: ops.gated_delta(x, H, G, d, dv, decay, bias, rate, beta, state, out, batch)
+
+    start_state = rnd(4, H, d * dv, seed=8, scale=0.1)
+    whole, want = start_state.clone(), torch.full((rows, H * dv), float("nan"), device=DEV)
+    call(whole, want, start, lengths)()
+    state, got = start_state.clone(), torch.full((rows, H * dv), float("nan"), device=DEV)
+    calls = [call(state, got, start, [first] * n)] + [call(state, got, [s + t for s in start], [1] * n) for t in range(first, max(lengths))]
+    for c in calls:
+        c()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for c in calls:
+            c()
+    for _ in range(5):
+        state.copy_(start_state)
+        got.fill_(float("nan"))
+        graph.replay()
+        # a prompt's tokens are taken several at a time, through sums of d products of unit rows: the bound of the rule's own test
+        assert (got - want).abs().max().item() <= 2e-5 * max(1.0, want.abs().max().item())
+        assert (state - whole).abs().max().item() <= 2e-5 * max(1.0, whole.abs().max().item())
