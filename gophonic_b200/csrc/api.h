@@ -143,7 +143,8 @@ GB_API int gb_qk_norm_rope_kv_write_x(const QkRopeParamsX* p, int dtype, cudaStr
 GB_API int gb_add_bias(float* out, const float* bias, int rows, int n, cudaStream_t stream);
 GB_API int gb_concat_cast(const float* h, const float* delta, const float* side, void* out, int out_dtype, int rows, int n, cudaStream_t stream);
 
-// matrix products: C[M, N] = A[M, K] W[N, K]^T
+// matrix products: C[M, N] = A[M, K] W[N, K]^T.  The bfloat16 few-row kernels (skinny, skinny_fold, tc5_decode) request W ahead
+// of their wait for the kernel ahead: W must not be written by the launch directly ahead of theirs.  The others read both after it.
 GB_API int gb_gemm_simt(const void* A, int a_dtype, const void* W, int w_dtype, void* C, int c_dtype, int M, int N, int K, int64_t lda,
                         int64_t ldw, int64_t ldc, cudaStream_t stream);
 // the same for float32 operands of 16-byte chunks, the same additions in the same order

@@ -7,10 +7,11 @@
 // Few rows (single tokens, short prompts): bound by reading W once, and by a lane's chain of additions, 4
 // cycles a column of K.  A CTA owns nt columns of the output, nt chosen so that the CTAs fill the SMs in
 // whole waves, and streams its nt weight rows and the activations through shared memory in stages of KS
-// columns, several stages in flight; a thread owns one column and MPT rows.  The weights' first stages are
-// requested before the kernel ahead has finished.  Three rows, against tiles of 64 x 64 without any
-// stages ahead (us; floor of the weights' bytes): 4096 x 2048 160 -> 20 (5), 12288 x 2048 219 -> 37 (15),
-// 2048 x 6144 473 -> 33 (8), 151936 x 2048 1407 -> 233 (190).
+// columns, several stages in flight; a thread owns one column and MPT rows.  An ordinary launch: W may be what the
+// kernel ahead makes, and as a dependent launch the waiting CTAs took the place of those at work (three rows behind a
+// norm, 12288 x 2048: 41.0 us, with the weights requested ahead of the wait or not, and 30.8 so).  Three rows, one product behind
+// the other inside a graph, against tiles of 64 x 64 without any stages ahead (us; floor of the weights' bytes): 4096 x 2048 160
+// -> 13.5 (5), 12288 x 2048 219 -> 28 (15), 2048 x 6144 473 -> 27 (8), 151936 x 2048 1407 -> 220 (190).
 //
 // More rows: bound by the multiply-add rate.  Tiles of BM x BN in registers, operands transposed on their way
 // into shared memory, the global loads two stages and the fragments one column ahead of their use, two
@@ -54,11 +55,11 @@ __global__ void __launch_bounds__(ROWS_THREADS) gemm_f32_rows_kernel(const float
         }
     };
     const int ahead = stages - 1;
-    for (int s = 0; s < ahead && s < steps; s++) load(W, ldw, nt, N, n0, sm + s * stage_floats, s);
-    pdl_wait_cta();
-    pdl_trigger();
     for (int s = 0; s < ahead; s++) {
-        if (s < steps) load(A, lda, M, M, 0, sm + s * stage_floats + nt * PITCH, s);
+        if (s < steps) {
+            load(W, ldw, nt, N, n0, sm + s * stage_floats, s);
+            load(A, lda, M, M, 0, sm + s * stage_floats + nt * PITCH, s);
+        }
         cp_async_commit();
     }
 
@@ -147,9 +148,8 @@ int launch_rows_ks(const float* A, const float* W, float* C, int M, int N, int K
         if (e != cudaSuccess) GB_REFUSE("gemm_f32: cannot reserve %d bytes of shared memory: %s", ROWS_SMEM, cudaGetErrorString(e));
         configured[dev] = true;
     }
-    cudaError_t e = launch_pdl(gemm_f32_rows_kernel<MPT, KS>, dim3(ceil_div(N, nt)), dim3(ROWS_THREADS), (size_t)stages * stage, stream, A, W,
-                               C, M, N, K, lda, ldw, ldc, nt, stages);
-    if (e != cudaSuccess) GB_REFUSE("gemm_f32: launch failed: %s", cudaGetErrorString(e));
+    gemm_f32_rows_kernel<MPT, KS><<<ceil_div(N, nt), ROWS_THREADS, (size_t)stages * stage, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, nt, stages);
+    GB_CHECK_LAUNCH("gemm_f32");
     return 0;
 }
 

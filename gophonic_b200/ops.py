@@ -406,6 +406,10 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, algo: str = "auto"
     on a tile.  Everything else,
     and operands whose rows are not 16-byte aligned, goes to the fp32 CUDA-core kernel.  float32
     operands never touch a tensor core.
+
+    The bfloat16 kernels of few rows (up to 64, or 256 for narrow outputs) ask for their first weights while the kernel ahead
+    may still run: there ``w`` must not be what the launch directly ahead on the stream writes.  ``a`` may be, and so may both
+    operands of the other kernels.
     """
     _need(a, "gemm a", dim=2, contiguous=False)
     _need(w, "gemm w", dim=2)

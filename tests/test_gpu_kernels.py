@@ -252,6 +252,33 @@ def test_float32_products_add_in_one_order(ops, M, N, K):
     assert torch.equal(strided[:, 1:N + 1], want) and torch.isnan(strided[:, 0]).all() and torch.isnan(strided[:, N + 1:]).all()
 
 
+# a product whose second operand is what the kernel ahead has just made: another product, and a row-wise kernel that lets its
+# dependents start early; in one captured graph, so that they follow one another as closely as they can
+@pytest.mark.parametrize("M", [1, 16, 40, 200])
+def test_float32_products_of_a_matrix_just_made(ops, M):
+    N, K, inner = 1500, 516, 64
+    left, right, x = rnd(N, inner, seed=1), rnd(K, inner, seed=2), rnd(M, K, seed=3)
+    made, out, out2 = (torch.zeros(shape, device=DEV) for shape in ((N, K), (M, N), (M, N)))
+    before = rnd(N, K, seed=4)
+
+    def steps():
+        ops.gemm(left, right, made)
+        ops.gemm(x, made, out)
+        ops.relu2(made)
+        ops.gemm(x, made, out2)
+    steps()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        steps()
+    w = (left.double() @ right.double().T)
+    for _ in range(5):
+        made.copy_(before)
+        graph.replay()
+        close(out, x.double() @ w.T, 2e-5)
+        close(out2, x.double() @ (w.clamp(min=0) ** 2).T, 2e-5)
+
+
 def test_gemm_simt_rows_do_not_depend_on_the_batch(ops):
     a, w = rnd(70, 200, seed=4), rnd(150, 200, seed=5)
     full = torch.empty((70, 150), device=DEV)
