@@ -48,7 +48,7 @@ struct Form {
     static constexpr int SMEM = GROUPS * Q_BYTES + STAGES * STAGE_BYTES + 1024;
 };
 constexpr int TMEM_COLS = 512;                  // S: 2 groups x 2 buffers x 64; O: 2 groups x 128
-constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+constexpr float LOG2E = 1.4426950408889634f;
 constexpr int POLY_PAIRS = 1;                   // of every four pairs of scores, how many take the polynomial exponential (measured: 0 -> 55.5 us, 1 -> 52.9, 2 -> 56.8 at 2048 tokens)
 constexpr float RESCALE_AT = 8.0f;              // rescale O when the row maximum outgrew the scale by 2^8
 
@@ -191,9 +191,7 @@ __device__ __forceinline__ void prefill_tc5(const CUtensorMap& map_q, const CUte
     // causal prompt differ manyfold in work).  Long prompts, whose keys and values do not fit L2
     // together: one kv head after the other (the query heads that share it side by side, longest
     // tiles first), so that what runs together reads the same keys and values.
-    // Few CTAs (a short turn behind a long context): each walks a piece of the keys only and leaves its unnormalised rows in scratch.
-    const int splits = SIGMOID || LATENT ? 1 : p.num_splits;
-    const int seq = blockIdx.z / splits, split = blockIdx.z % splits;
+    const int seq = blockIdx.z;
     int head = blockIdx.x, qt = (int)gridDim.y - 1 - (int)blockIdx.y;
     if (by_kv_head) {
         const int G = p.heads / p.kv_heads, tiles = (int)gridDim.y;
@@ -226,8 +224,7 @@ __device__ __forceinline__ void prefill_tc5(const CUtensorMap& map_q, const CUte
     // with kept first tokens: the pages of keys [0, keep_first) first, then those of the window, each once
     int n_first = p.window > 0 && p.keep_first > 0 ? (p.keep_first + BKV - 1) / BKV : 0;
     if (n_first > t_lo) n_first = t_lo;
-    int j0 = 0;  // first of the pages of this piece
-    auto tile_of = [&](int j) { return j0 + j < n_first ? j0 + j : t_lo + (j0 + j - n_first); };
+    auto tile_of = [&](int j) { return j < n_first ? j : t_lo + (j - n_first); };
     int n_g[GROUPS];
 #pragma unroll
     for (int g = 0; g < GROUPS; g++) {
@@ -239,27 +236,7 @@ __device__ __forceinline__ void prefill_tc5(const CUtensorMap& map_q, const CUte
             n_g[g] = n_first + (past + last) / BKV - t_lo + 1;
         }
     }
-    int n = n_g[0] > n_g[1] ? n_g[0] : n_g[1];
-    if (splits > 1) {
-        const int per = (n + splits - 1) / splits;
-        j0 = split * per;
-        n = 0;
-#pragma unroll
-        for (int g = 0; g < GROUPS; g++) {
-            n_g[g] = n_g[g] - j0 < per ? n_g[g] - j0 : per;
-            if (n_g[g] < 0) n_g[g] = 0;
-            n = n_g[g] > n ? n_g[g] : n;
-        }
-        if (n == 0) {  // nothing in this piece: the whole CTA leaves before anything is allocated
-            const int qrow = q0 + (int)threadIdx.x;
-            if (threadIdx.x < GROUPS * BQ && qrow < q_len) {
-                float* sp = p.scratch + (((int64_t)(q_start + qrow) * p.heads + head) * splits + split) * (HD + 2);
-                sp[0] = -INFINITY;
-                sp[1] = 0.f;
-            }
-            return;
-        }
-    }
+    const int n = n_g[0] > n_g[1] ? n_g[0] : n_g[1];
 
     if (threadIdx.x == 0) {
         mbar_init(&q_full, 1);
@@ -568,23 +545,6 @@ __device__ __forceinline__ void prefill_tc5(const CUtensorMap& map_q, const CUte
         if (!ok) {
             atomicCAS(&g_status, 0, 4);
             abort_s = 1;
-        } else if (splits > 1) {
-            // the row as it is: maximum (natural logarithm, as the merge expects), sum and columns; an empty piece has neither
-            float* sp = p.scratch + (((int64_t)(q_start + qrow) * p.heads + head) * splits + split) * (HD + 2);
-            if (row_ok) *reinterpret_cast<float2*>(sp) = my_n > 0 && m_used != -INFINITY ? make_float2(m_used * LN2, l) : make_float2(-INFINITY, 0.f);
-            if (my_n > 0) {
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-#pragma unroll 1
-                for (int c0 = 0; c0 < HD; c0 += 32) {
-                    uint32_t o[32];
-                    tmem_ld32(o_addr + (uint32_t)c0, o);
-                    if (row_ok) {
-#pragma unroll
-                        for (int i = 0; i < 32; i += 2)
-                            *reinterpret_cast<float2*>(sp + 2 + c0 + i) = make_float2(__uint_as_float(o[i]), __uint_as_float(o[i + 1]));
-                    }
-                }
-            }
         } else if (my_n > 0) {
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             // a sink adds one unit to the denominator: a key of score 0, in the scale the sums are kept in
@@ -633,41 +593,6 @@ __global__ void __launch_bounds__(THREADS) attn_prefill_tc5_kernel(const __grid_
                                                                    const __grid_constant__ CUtensorMap map_v, SigmoidAttnParams p,
                                                                    int by_kv_head) {
     prefill_tc5<SIGMOID, false>(map_q, map_k, map_v, map_k, p, by_kv_head, LatentRows{nullptr, 0});
-}
-
-// Joins the pieces of a row and head: a warp each, a lane four columns, the pieces in order.
-__global__ void __launch_bounds__(256) attn_rows_merge_kernel(const float* __restrict__ scratch, bf16* __restrict__ out, int64_t out_row_stride, int rows,
-                                                              int heads, int splits, int sink, const float* __restrict__ sinks) {
-    pdl_wait();
-    pdl_trigger();
-    const int64_t unit = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (unit >= (int64_t)rows * heads) return;
-    const int64_t row = unit / heads;
-    const int head = (int)(unit - row * heads);
-    const float* sp = scratch + unit * splits * (HD + 2);
-    const float m = lane < splits ? sp[(int64_t)lane * (HD + 2)] : -INFINITY, sum = lane < splits ? sp[(int64_t)lane * (HD + 2) + 1] : 0.f;
-    float M = warp_max(m);
-    const float z = sinks ? sinks[head] : 0.f;
-    if (sink) M = fmaxf(M, z);
-    const float w = m != -INFINITY ? expf(m - M) : 0.f;
-    float L = warp_sum(w * sum);
-    if (sink) L += expf(z - M);
-    float a[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-    for (int s = 0; s < splits; s++) {
-        const float ws = __shfl_sync(0xffffffffu, w, s);
-        if (ws == 0.f) continue;   // also an empty piece, whose columns nobody wrote
-        const float2 lo = *reinterpret_cast<const float2*>(sp + (int64_t)s * (HD + 2) + 2 + 4 * lane);
-        const float2 hi = *reinterpret_cast<const float2*>(sp + (int64_t)s * (HD + 2) + 4 + 4 * lane);
-        a[0] += ws * lo.x;
-        a[1] += ws * lo.y;
-        a[2] += ws * hi.x;
-        a[3] += ws * hi.y;
-    }
-    const float inv = 1.f / L;
-    __nv_bfloat162 o[2] = {__floats2bfloat162_rn(a[0] * inv, a[1] * inv), __floats2bfloat162_rn(a[2] * inv, a[3] * inv)};
-    *reinterpret_cast<uint2*>(out + row * out_row_stride + (int64_t)head * HD + 4 * lane) = *reinterpret_cast<uint2*>(o);
 }
 
 // Over keys and values that were expanded from latents for this step (gb_latent_gather and two products before it): heads
@@ -756,8 +681,7 @@ static int launch_tc5(const SigmoidAttnParams& p, int rows, int pages, int sigmo
     const char* who = sigmoid ? "attention_sigmoid_tc5" : "attention_prefill_tc5";
     if (p.d != HD) GB_REFUSE("%s: head_dim %d; this kernel takes 128", who, p.d);
     if (p.heads <= 0 || p.kv_heads <= 0 || p.heads % p.kv_heads) GB_REFUSE("%s: %d heads over %d kv heads", who, p.heads, p.kv_heads);
-    if (p.num_splits < 1 || p.num_splits > 32 || (p.num_splits > 1 && (sigmoid || !p.scratch || ((uintptr_t)p.scratch & 7))))
-        GB_REFUSE("%s: %d key splits", who, p.num_splits);
+    if (p.num_splits != 1) GB_REFUSE("%s: key splits are for single-token rows", who);
     if (p.window < 0) GB_REFUSE("%s: window %d", who, p.window);
     if (p.dv && p.dv != p.d) GB_REFUSE("%s: values of another size than keys run on the CUDA-core kernel", who);
     if (p.keep_first < 0) GB_REFUSE("%s: %d kept first tokens", who, p.keep_first);
@@ -780,15 +704,12 @@ static int launch_tc5(const SigmoidAttnParams& p, int rows, int pages, int sigmo
     if (int rc = make_map(&map_q, p.q, rows, p.heads * HD, p.q_row_stride, BQ)) return rc;
     if (int rc = make_map(&map_k, p.k_plane, (int64_t)pages * p.kv_heads * 64, HD, HD, 64)) return rc;
     if (int rc = make_map(&map_v, p.v_plane, (int64_t)pages * (p.v_share > 1 ? p.kv_heads / p.v_share : p.kv_heads) * 64, HD, HD, 64)) return rc;
-    dim3 grid(p.heads, ceil_div(p.max_q_len, GROUPS * BQ), p.nseq * p.num_splits);
+    dim3 grid(p.heads, ceil_div(p.max_q_len, GROUPS * BQ), p.nseq);
     if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("%s: grid (%u, %u, %u) exceeds one launch", who, grid.x, grid.y, grid.z);
     // keys and values of the longest prompt, all kv heads: more than 48 MB do not stay in L2 beside the rest
     const int by_kv_head = (int64_t)p.max_q_len * p.kv_heads * (4 * HD) > ((int64_t)48 << 20) ? 1 : 0;
     cudaError_t e = sigmoid ? launch_pdl(attn_prefill_tc5_kernel<true>, grid, dim3(THREADS), (size_t)smem, stream, map_q, map_k, map_v, p, by_kv_head)
                             : launch_pdl(attn_prefill_tc5_kernel<false>, grid, dim3(THREADS), (size_t)smem, stream, map_q, map_k, map_v, p, by_kv_head);
-    if (e == cudaSuccess && p.num_splits > 1)
-        e = launch_pdl(attn_rows_merge_kernel, dim3((unsigned)(((int64_t)rows * p.heads + 7) / 8)), dim3(256), 0, stream, (const float*)p.scratch,
-                       (bf16*)p.out, p.out_row_stride, rows, p.heads, p.num_splits, p.sink, p.sinks);
     if (e != cudaSuccess) GB_REFUSE("%s: launch failed: %s", who, cudaGetErrorString(e));
     return 0;
 }

@@ -157,7 +157,7 @@ GB_API int gb_attention_algo_x(const AttnParamsX* p, int dtype) {
 GB_API int gb_attention_auto(const AttnParams* p, int dtype, int rows, int pages, int* algo, int* kernels, cudaStream_t stream) {
     const int a = gb_attention_algo(p, dtype);
     if (algo) *algo = a;
-    if (kernels) *kernels = (a == GB_ATTN_SIMT || a == GB_ATTN_DECODE_MMA || a == GB_ATTN_PREFILL_TC5) && p->num_splits > 1 ? 2 : 1;
+    if (kernels) *kernels = (a == GB_ATTN_SIMT || a == GB_ATTN_DECODE_MMA) && p->num_splits > 1 ? 2 : 1;
     switch (a) {
         case GB_ATTN_DECODE_MMA: return gb_attention_decode_mma(p, stream);
         case GB_ATTN_PREFILL_MMA: return gb_attention_prefill_mma(p, stream);

@@ -726,10 +726,7 @@ def attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_plane
     elif algo == "prefill_mma":
         _check(_lib.gb_attention_prefill_mma_x(byref(p), _stream()))
     elif algo == "prefill_tc5":
-        # pieces of a prompt's keys: partial results of every row, not of every sequence
-        if num_splits > 1 and scratch.numel() < attention_scratch_floats(q.shape[0], heads, head_dim, num_splits):
-            raise KernelError("attention: scratch is too small")
-        _check(_lib.gb_attention_prefill_tc5_x(byref(p), c_int(q.shape[0]), c_int(k_plane.shape[0]), _stream()), nk)
+        _check(_lib.gb_attention_prefill_tc5_x(byref(p), c_int(q.shape[0]), c_int(k_plane.shape[0]), _stream()))
     elif algo == "latent_mma":
         _check(_lib.gb_attention_latent_mma(byref(p), _stream()), nk)
     else:

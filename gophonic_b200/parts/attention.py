@@ -80,13 +80,6 @@ def more_splits(units: int, max_kv_len: int, mean_kv_len: int, sm_count: int, pa
     return s
 
 
-def choose_prompt_splits(tiles: int, max_kv_len: int, sm_count: int = 148) -> int:
-    """How many pieces the tcgen05 kernel's CTAs (``tiles``: 256 query rows of a head each) cut their keys into: as many as fill
-    the SMs once, of at least four pages of 64 keys each.  A turn of 90 tokens behind 1000 (32 heads): the attention of a layer 29 us whole
-    on 32 CTAs; twelve layers 2051 us whole and 2005 in four pieces."""
-    return max(1, min(sm_count // max(1, tiles), (max_kv_len + 63) // 64 // 4, 32))
-
-
 class Attention(Mixer):
     capturable = True
 
@@ -134,13 +127,10 @@ class Attention(Mixer):
         self.position.prepare(capacity)
 
     def plan(self, nseq: int, max_q_len: int, max_kv_len: int, sm_count: int):
-        """Into how many pieces the keys of each sequence are cut: single-token steps and, on the tcgen05 kernel,
-        short prompts (few sequences with long contexts would otherwise leave most SMs idle)."""
+        """Into how many pieces the keys of each sequence are cut: only single-token steps cut them
+        (few sequences with long contexts would otherwise leave most SMs idle)."""
         if max_q_len != 1:
-            if self.rt.is_fp32 or self.spec.head_dim != 128 or max_q_len < self.rt.ops.TC5_ATTENTION_MIN_ROWS:
-                return 1
-            seen = min(max_kv_len, self.spec.window + max_q_len) if self.spec.window > 0 else max_kv_len
-            return choose_prompt_splits(nseq * self.spec.heads * ((max_q_len + 255) // 256), seen, sm_count)
+            return 1
         elem = 4 if self.rt.is_fp32 else 2
         page_bytes = 2 * 64 * self.spec.head_dim * elem     # keys and values of one kv head for one page
         return choose_splits(nseq * self.spec.kv_heads, max_kv_len, sm_count, page_bytes)
@@ -190,9 +180,8 @@ class Attention(Mixer):
         splits = int(batch.plan_for(self) or 1)
         if splits <= 1:
             return 1, None
-        units = batch.nseq if batch.max_q_len == 1 else batch.rows
         return splits, batch.workspace(("attention key splits", s.heads, s.head_dim, splits),
-                                       self.rt.ops.attention_scratch_floats(units, s.heads, s.head_dim, splits))
+                                       self.rt.ops.attention_scratch_floats(batch.nseq, s.heads, s.head_dim, splits))
 
     def _context(self, batch, x: torch.Tensor, cache) -> torch.Tensor:
         """Everything up to the output projection: [rows, heads * head_dim] in the activation dtype."""

@@ -703,32 +703,6 @@ def test_float32_attention_adds_in_one_order(ops, heads, kvh, d, dv, q_lens, kv_
     assert torch.equal(outs[0], outs[1]) and not torch.isnan(outs[0]).any()
 
 
-# prompts whose keys are cut into pieces on the tcgen05 kernel: fewer pages than pieces, sequences of one row and of several tiles
-# in one call, windows with kept first tokens whose pieces hold nothing, a sink, blocks
-@pytest.mark.parametrize("heads,kvh", [(4, 1), (3, 3)])
-@pytest.mark.parametrize("splits", [2, 5, 32])
-@pytest.mark.parametrize("q_lens,kv_lens,opts", [([90], [1090], {}), ([65, 1, 300], [65, 700, 812], {}), ([70, 257], [900, 300], {"window": 100, "keep_first": 70}),
-                                                 ([66, 2], [500, 64], {"window": 20, "sink": True}), ([130], [700], {"chunk": 96})])
-def test_attention_prompts_in_pieces(ops, heads, kvh, splits, q_lens, kv_lens, opts):
-    nseq, rows, d, n_pages = len(q_lens), sum(q_lens), 128, 60
-    mk = lambda x: torch.tensor(list(x), dtype=torch.int32, device=DEV)
-    table = torch.randperm(n_pages, generator=torch.Generator().manual_seed(4))[:18 * nseq].to(torch.int32).view(nseq, 18).to(DEV)
-    q = rnd(rows, heads * d, dtype=torch.bfloat16, seed=8)
-    k, v = (rnd(n_pages, kvh, 64, d, dtype=torch.bfloat16, seed=s) for s in (9, 10))
-    outs = []
-    for n in (1, splits):
-        out = torch.full((rows, heads * d), float("nan"), dtype=torch.bfloat16, device=DEV)
-        scratch = torch.full((ops.attention_scratch_floats(rows, heads, d, n),), float("nan"), device=DEV) if n > 1 else None
-        ops.attention(q, out, k, v, table, mk(range(nseq)), mk([sum(q_lens[:i]) for i in range(nseq)]), mk(q_lens), mk(kv_lens), nseq, max(q_lens),
-                      heads, kvh, d, d ** -0.5, opts.get("window", 0), n, scratch, algo="prefill_tc5", keep_first=opts.get("keep_first", 0),
-                      sink=opts.get("sink", False), chunk=opts.get("chunk", 0))
-        outs.append(out.float())
-    assert ops.tc5_status() == 0
-    # a weight p is rounded to bfloat16 (2^-9 p) under another maximum, and may come from the other exponential (2e-4 p): either
-    # result is off by at most (2^-9 + 2e-4) max |v|, and each is rounded to bfloat16 once
-    assert ((outs[1] - outs[0]).abs() <= 2.0 ** -7 * outs[0].abs() + 2 * (2.0 ** -9 + 2e-4) * v.abs().max().item()).all()
-
-
 def test_attention_head_sizes_without_a_tensor_core_kernel_fall_back(ops):
     out, ref, used = attention_case(ops, torch.bfloat16, 2, 1, 144, q_lens=[40, 1], kv_lens=[40, 90])
     assert used == "simt"
