@@ -495,8 +495,8 @@ def probe(name, **opts):
         ints = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
         slot, start = ints(list(range(nseq))), ints([i * q_len for i in range(nseq)])
         ql, kl = ints([q_len] * nseq), ints([kv_len] * nseq)
-        from gophonic_b200.parts.attention import choose_splits
-        splits = 1 if q_len > 1 else choose_splits(nseq * kvh, kv_len)
+        from gophonic_b200.parts.attention import choose_splits, few_splits
+        splits = 1 if q_len > 1 else max(choose_splits(nseq * kvh, kv_len), few_splits(nseq * kvh, kv_len))
         scratch = torch.empty(ops.attention_scratch_floats(nseq, heads, d, splits), dtype=torch.float32, device=dev) if splits > 1 else None
 
         def fn():

@@ -98,13 +98,13 @@ class DecodeGraphs:
     def engine(self):
         return self._engine()
 
-    def get(self, nseq: int, max_kv_len: int, mean_kv_len: int) -> DecodeGraph:
-        """The captured step that serves ``nseq`` sequences which see at most ``max_kv_len`` keys, ``mean_kv_len`` on average: one
+    def get(self, nseq: int, max_kv_len: int) -> DecodeGraph:
+        """The captured step that serves ``nseq`` sequences which see at most ``max_kv_len`` keys: one
         graph per captured batch size and per answer of the model's mixers to ``plan`` (whatever
         those answers are).  At most ``max_graphs`` graphs are kept; the one unused longest goes."""
         eng = self.engine
         size = min(captured_size(nseq), max(self.max_batch, nseq))
-        plans = eng.model.step_plans(size, 1, max_kv_len, eng.sm_count, mean_kv_len)
+        plans = eng.model.step_plans(size, 1, max_kv_len, eng.sm_count)
         key = (size, plans)
         g = self.graphs.pop(key, None)
         if g is None:

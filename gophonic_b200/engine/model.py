@@ -114,10 +114,10 @@ class Model:
             out.append((registry.part_class("block", layer.block).cache_request(layer), entry.cache_of))
         return out
 
-    def step_plans(self, nseq: int, max_q_len: int, max_kv_len: int, sm_count: int, mean_kv_len: int) -> Tuple:
+    def step_plans(self, nseq: int, max_q_len: int, max_kv_len: int, sm_count: int) -> Tuple:
         """The launch plans of every mixer for a step of this shape, block by block: a hashable value
         the engine keys its captured steps on without looking inside."""
-        return tuple(m.plan_lengths(nseq, max_q_len, max_kv_len, sm_count, mean_kv_len) for b in self.blocks for m in b.mixers())
+        return tuple(m.plan(nseq, max_q_len, max_kv_len, sm_count) for b in self.blocks for m in b.mixers())
 
     def bind_plans(self, plans: Sequence) -> Dict[int, object]:
         """``step_plans``' answer in the form ``StepBatch.plans`` takes: by mixer."""

@@ -55,8 +55,7 @@ class StepBatch:
         """The launch plan of ``part`` for this step (asked once per step and part)."""
         key = id(part)
         if key not in self.plans:
-            mean = sum(known for known, _ in self.extents) // len(self.extents) + 1 if self.extents else self.max_kv_len
-            self.plans[key] = part.plan_lengths(self.nseq, self.max_q_len, self.max_kv_len, self.sm_count, mean)
+            self.plans[key] = part.plan(self.nseq, self.max_q_len, self.max_kv_len, self.sm_count)
         return self.plans[key]
 
     def workspace(self, key, numel: int, dtype: torch.dtype = torch.float32) -> torch.Tensor:
@@ -374,7 +373,7 @@ class Engine:
         size."""
         n = len(entries)
         firsts = [self.cache.length(slot) for slot, _ in entries]
-        g = self.graphs.get(n, max(firsts) + 1, sum(firsts) // n + 1)
+        g = self.graphs.get(n, max(firsts) + 1)
         if g.logits is None:
             # the capture runs the step's kernels on the graph's own input buffer: fill it first
             self._fill_graph_meta(g, entries, firsts)

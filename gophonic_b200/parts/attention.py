@@ -59,24 +59,14 @@ def choose_splits(units: int, max_kv_len: int, sm_count: int = 148, page_bytes: 
     return best
 
 
-def more_splits(units: int, max_kv_len: int, mean_kv_len: int, sm_count: int, page_bytes: int) -> int:
-    """Into how many pieces at least, beside ``choose_splits``, two kinds of steps cut their keys.
-
-    Few sequences: while one CTA an SM takes all pieces, pieces of 96 to 192 keys, a power of two of them (the count then
-    changes as seldom as the context doubles, and a changed count means another captured step).  Whole steps, us, in pieces
-    of at least 256 keys and in these: one sequence of 700 keys 1248 and 1186 (1.7B sizes), of 1500 1217 and 1207, four of 1000
-    1329 and 1284.
-    Unequal sequences, up to two CTAs an SM uncut: the model of ``choose_splits`` sees them as the fewer sequences of the longest one's
-    length that hold as many keys, because the longest alone sets the pace of a step that is not cut.  24 sequences of up to
-    2500 keys, 620 on average: 2835 us uncut and 2455 in five pieces; eight of up to 4096, 1800 on average (8B sizes): 1519 in
-    four and 1449 in six.  With more sequences the CTAs no longer run in step and the others fill the time (50 sequences of up
-    to 1900 keys: 3144 us uncut, 3242 in two pieces)."""
+def few_splits(units: int, max_kv_len: int, sm_count: int = 148) -> int:
+    """Into how many pieces at least, beside ``choose_splits``, a step of few sequences cuts its keys: a power of two (the count then
+    changes as seldom as the context doubles, and a changed count means another captured step), as long as a CTA an SM
+    takes all pieces, there are no more than 32 and a piece keeps at least 96 keys.  Whole steps (1.7B sizes), us, in pieces of at
+    least 256 keys and in these: one sequence of 700 keys 1248 and 1186, of 1500 1217 and 1207, four of 1000 1329 and 1284."""
     s = 1
     while 2 * s <= min(max_kv_len // 96, sm_count // max(1, units), 32):
         s *= 2
-    if units <= 2 * sm_count and mean_kv_len < max_kv_len:
-        r = choose_splits(max(1, round(units * mean_kv_len / max_kv_len)), max_kv_len, sm_count, page_bytes)
-        s = max(s, max(n for n in (1, 2, 3, 4, 6, 8, 12, 16) if n <= r))
     return s
 
 
@@ -131,16 +121,16 @@ class Attention(Mixer):
         (few sequences with long contexts would otherwise leave most SMs idle)."""
         if max_q_len != 1:
             return 1
+        splits = self.splits_of(nseq, max_kv_len, sm_count)
+        if self.rt.is_fp32:
+            return splits
+        seen = min(max_kv_len, self.spec.window) if self.spec.window > 0 else max_kv_len
+        return max(splits, few_splits(nseq * self.spec.kv_heads, seen, sm_count))
+
+    def splits_of(self, nseq: int, max_kv_len: int, sm_count: int) -> int:
         elem = 4 if self.rt.is_fp32 else 2
         page_bytes = 2 * 64 * self.spec.head_dim * elem     # keys and values of one kv head for one page
         return choose_splits(nseq * self.spec.kv_heads, max_kv_len, sm_count, page_bytes)
-
-    def plan_lengths(self, nseq: int, max_q_len: int, max_kv_len: int, sm_count: int, mean_kv_len: int):
-        splits = self.plan(nseq, max_q_len, max_kv_len, sm_count)
-        if max_q_len != 1 or self.rt.is_fp32 or type(self).plan is not Attention.plan:
-            return splits
-        seen = min(max_kv_len, self.spec.window) if self.spec.window > 0 else max_kv_len
-        return max(splits, more_splits(nseq * self.spec.kv_heads, seen, min(mean_kv_len, seen), sm_count, 2 * 64 * self.spec.head_dim * 2))
 
     def forward(self, batch, x: torch.Tensor, out: torch.Tensor, cache) -> None:
         self.rt.ops.gemm(self._context(batch, x, cache), self.o, out)

@@ -211,11 +211,6 @@ class Mixer(Part):
         with.  Scratch memory that the plan calls for comes from ``batch.workspace(key, n)``."""
         return None
 
-    def plan_lengths(self, nseq: int, max_q_len: int, max_kv_len: int, sm_count: int, mean_kv_len: int):
-        """``plan`` for a step whose sequences see ``mean_kv_len`` keys on average: what the engine asks where it knows
-        the lengths.  By default the longest alone decides."""
-        return self.plan(nseq, max_q_len, max_kv_len, sm_count)
-
     def folds_norm(self, rows: int, norm) -> bool:
         """True if, for a step of ``rows`` rows, ``forward_folded(batch, h, stats, norm, cache,
         next_norm)`` can run: the part then takes its activations from ``stats.prescaled`` (made for

@@ -172,7 +172,7 @@ class GatedAttention(Attention):
             return 1
         s = self.spec
         seen = min(max_kv_len, s.window + s.keep_first) if s.window > 0 else max_kv_len
-        return super().plan(nseq, max_q_len, seen, sm_count)
+        return self.splits_of(nseq, seen, sm_count)
 
     def key_splits(self, batch):
         s = self.spec
