@@ -120,46 +120,78 @@ class LatentAttention(Mixer):
         for h in range(heads):
             ops.gemm(a[:, h, :], w_nk[h], out[:, h, :])
 
-    def _expanded_pages(self, batch, cache) -> int:
-        """How many cache pages the step's rows see in all if it should run over expanded keys and values, else 0.
+    def runs(self, batch):
+        """The step's sequences in neighbouring runs (first sequence, end, first row, end, most rows of one, pages): ``pages`` of the
+        cache are what the run's rows see if it goes over expanded keys and values, 0 if over the latents.
 
         Over the latents a (row, key) pair of a head costs kv_rank + rot_dim + kv_rank multiply-adds, over expanded keys and
         values head_dim + rot_dim + value_dim (1088 against 320 at a latent of 512), and the expansion itself
         kv_rank (head_dim + value_dim) a key.  So it pays where a key is seen by enough rows.  Measured over eight layers (16
         heads, a latent of 512, a window of 1024; ms a step, absorbed and expanded): 3244 rows over 3264 keys 8.4 and 4.9,
         3741 over 12160 11.1 and 5.9, 1121 over 9280 6.3 and 3.4; 128 over 1152 and 70 over 1088 the same, 261 rows of
-        four sequences over 4352 3.5 and 3.6.  The expanded rows are scratch memory: no more of it than the absorbed queries
-        and outputs would take, or EXPANDED_BYTES."""
-        s, ops = self.spec, self.rt.ops
-        if batch.extents is None or not ops.latent_expanded_accepts(self.rt.act_dtype, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank, batch.max_q_len):
-            return 0
-        if self.uk_kn.dtype != torch.bfloat16 or self.uv_nk.dtype != torch.bfloat16:
-            return 0
-        window = int(s.window)
-        pages = 0
-        for known, rows in batch.extents:
-            pages += (known + rows + 63) // 64 - (max(0, known - window + 1) // 64 if window > 0 else 0)
-        expanded = 2 * 64 * pages * (self.key_dim + s.heads * (s.head_dim + s.value_dim))
-        absorbed = 2 * batch.rows * s.heads * (self.key_dim + s.kv_rank)
-        return pages if 64 * pages <= self.EXPANDED_KEYS_A_ROW * batch.rows and expanded <= max(absorbed, self.EXPANDED_BYTES) else 0
+        four sequences over 4352 3.5 and 3.6.
 
-    def _expanded(self, batch, q: torch.Tensor, cache, pages: int) -> torch.Tensor:
-        """Attention over keys and values made from the visible latents for this step: [rows, heads * value_dim]."""
+        Both forms round, at different places, so each sequence is judged by its own rows and keys alone: what it
+        gets must not depend on what else is in the step.  The expanded rows are scratch memory, no more of it at a time than the
+        absorbed queries and outputs of the same sequences would take, or EXPANDED_BYTES; a run that would is cut in two."""
+        s, ops = self.spec, self.rt.ops
+        if (batch.extents is None or not ops.latent_expanded_accepts(self.rt.act_dtype, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank, batch.max_q_len)
+                or self.uk_kn.dtype != torch.bfloat16 or self.uv_nk.dtype != torch.bfloat16):
+            return [(0, batch.nseq, 0, batch.rows, batch.max_q_len, 0)]
+        window = int(s.window)
+        page_bytes = 2 * 64 * (self.key_dim + s.heads * (s.head_dim + s.value_dim))
+        row_bytes = 2 * s.heads * (self.key_dim + s.kv_rank)
+        out, at = [], 0
+        for i, (known, rows) in enumerate(batch.extents):
+            pages = (known + rows + 63) // 64 - (max(0, known - window + 1) // 64 if window > 0 else 0)
+            if (rows < ops.LATENT_TC5_MIN_ROWS or 64 * pages > self.EXPANDED_KEYS_A_ROW * rows
+                    or pages * page_bytes > max(rows * row_bytes, self.EXPANDED_BYTES)):
+                pages = 0
+            if out and (out[-1][5] > 0) == (pages > 0):
+                first, _, lo, _, most, held = out[-1]
+                if not pages or (held + pages) * page_bytes <= max((at + rows - lo) * row_bytes, self.EXPANDED_BYTES):
+                    out[-1] = (first, i + 1, lo, at + rows, max(most, rows), held + pages)
+                    at += rows
+                    continue
+            out.append((i, i + 1, at, at + rows, rows, pages))
+            at += rows
+        return out
+
+    def _expanded(self, batch, q: torch.Tensor, ctx: torch.Tensor, cache, run) -> None:
+        """Attention of a run's rows over keys and values made from the visible latents for this step."""
         ops, s = self.rt.ops, self.spec
         H, R, dev = s.heads, s.kv_rank, q.device
+        first, end, lo, hi, most, pages = run
         cos, sin, _ = self.position.kernel_args()
-        ops.latent_q_rot(q, q, H, s.head_dim, s.rot_dim, cos, sin, batch.row_pos)
+        ops.latent_q_rot(q[lo:hi], q[lo:hi], H, s.head_dim, s.rot_dim, cos, sin, batch.row_pos[lo:hi])
         lat = torch.empty((64 * pages, self.key_dim), dtype=q.dtype, device=dev)
-        base = torch.empty((batch.nseq,), dtype=torch.int32, device=dev)
-        ops.latent_gather(cache.k, cache.block_table, batch.seq_slot, batch.seq_q_len, batch.seq_kv_len, batch.nseq, int(s.window), lat, base)
+        base = torch.empty((end - first,), dtype=torch.int32, device=dev)
+        q_len, kv_len = batch.seq_q_len[first:end], batch.seq_kv_len[first:end]
+        ops.latent_gather(cache.k, cache.block_table, batch.seq_slot[first:end], q_len, kv_len, end - first, int(s.window), lat, base)
         keys = torch.empty((64 * pages, H * s.head_dim), dtype=q.dtype, device=dev)
         values = torch.empty((64 * pages, H * s.value_dim), dtype=q.dtype, device=dev)
         ops.gemm(lat[:, :R], self.uk_kn.view(H * s.head_dim, R), keys)
         ops.gemm(lat[:, :R], self.uv_nk.view(H * s.value_dim, R), values)
-        ctx = torch.empty((q.shape[0], H * s.value_dim), dtype=q.dtype, device=dev)
-        ops.attention_latent_expanded(q, ctx, keys, values, lat, base, R, batch.seq_q_start, batch.seq_q_len, batch.seq_kv_len, batch.nseq,
-                                      batch.max_q_len, H, float(s.scale), int(s.window), int(s.chunk))
-        return ctx
+        ops.attention_latent_expanded(q, ctx, keys, values, lat, base, R, batch.seq_q_start[first:end], q_len, kv_len, end - first, most, H,
+                                      float(s.scale), int(s.window), int(s.chunk))
+
+    def _absorbed(self, batch, q: torch.Tensor, ctx: torch.Tensor, cache, run) -> None:
+        """Attention of a run's rows over the latents as they are cached."""
+        ops, s = self.rt.ops, self.spec
+        H, d, dr, dv, R = s.heads, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank
+        first, end, lo, hi, most, _ = run
+        rows, q, ctx = hi - lo, q[lo:hi], ctx[lo:hi]
+        cos, sin, _ = self.position.kernel_args()
+        qa = torch.empty((rows, H * self.key_dim), dtype=q.dtype, device=q.device)       # per head [W_uk^T q_plain | rotated part]
+        self._per_head(q.view(rows, H, d + dr)[:, :, :d], self.uk_kn, self.uk_nk, qa.view(rows, H, self.key_dim)[:, :, :R])
+        ops.latent_q_rot(q, qa, H, d, dr, cos, sin, batch.row_pos[lo:hi])
+        mixed = torch.empty((rows, H * R), dtype=q.dtype, device=q.device)               # per head sum_j p_j c_j
+        splits, scratch = self.key_splits(batch)
+        q_start = batch.seq_q_start[first:end] - lo if lo else batch.seq_q_start[first:end]   # rows of qa
+        ops.attention(qa, mixed, cache.k, cache.v, cache.block_table, batch.seq_slot[first:end], q_start, batch.seq_q_len[first:end],
+                      batch.seq_kv_len[first:end], end - first, most, H, 1, self.key_dim, float(s.scale), int(s.window), splits, scratch,
+                      value_dim=R, chunk=int(s.chunk))
+        self._per_head(mixed.view(rows, H, R), self.uv_kn, self.uv_nk, ctx.view(rows, H, dv))
 
     def forward(self, batch, x: torch.Tensor, out: torch.Tensor, cache) -> None:
         ops, s = self.rt.ops, self.spec
@@ -178,23 +210,9 @@ class LatentAttention(Mixer):
                         cache.block_table, cache.k, cache.writable)
         q = torch.empty((rows, H * (d + dr)), dtype=x.dtype, device=x.device)
         ops.gemm(cq, self.uq, q)
-        pages = self._expanded_pages(batch, cache)
-        if pages:
-            ctx = self._expanded(batch, q, cache, pages)
-            if self.gated:
-                ops.head_norm_gate(ctx, made[:, Q + R + dr:], ctx, H, dv, ops.GATE_SIGMOID)
-            ops.gemm(ctx, self.o, out)
-            return
-        qa = torch.empty((rows, H * self.key_dim), dtype=x.dtype, device=x.device)       # per head [W_uk^T q_plain | rotated part]
-        self._per_head(q.view(rows, H, d + dr)[:, :, :d], self.uk_kn, self.uk_nk, qa.view(rows, H, self.key_dim)[:, :, :R])
-        ops.latent_q_rot(q, qa, H, d, dr, cos, sin, batch.row_pos)
-        mixed = torch.empty((rows, H * R), dtype=x.dtype, device=x.device)               # per head sum_j p_j c_j
-        splits, scratch = self.key_splits(batch)
-        ops.attention(qa, mixed, cache.k, cache.v, cache.block_table, batch.seq_slot, batch.seq_q_start, batch.seq_q_len, batch.seq_kv_len,
-                      batch.nseq, batch.max_q_len, H, 1, self.key_dim, float(s.scale), int(s.window), splits, scratch, value_dim=R,
-                      chunk=int(s.chunk))
         ctx = torch.empty((rows, H * dv), dtype=x.dtype, device=x.device)
-        self._per_head(mixed.view(rows, H, R), self.uv_kn, self.uv_nk, ctx.view(rows, H, dv))
+        for run in self.runs(batch):
+            (self._expanded if run[5] else self._absorbed)(batch, q, ctx, cache, run)
         if self.gated:
             ops.head_norm_gate(ctx, made[:, Q + R + dr:], ctx, H, dv, ops.GATE_SIGMOID)
         ops.gemm(ctx, self.o, out)

@@ -716,3 +716,63 @@ def test_prompts_over_expanded_latents(heads, kv_rank, q_lens, kv_lens, window, 
         # probabilities and outputs are rounded to bfloat16 (2^-9 each), the exponentials are good to 2e-4
         assert (out[r:r + m].double() - want).abs().max() <= 1.2e-2 * want.abs().max()
         r += m
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_the_forms_of_latent_attention_inside_a_step(tmp_path, dtype):
+    """Models whose heads both forms take: prompts, portions behind contexts on both sides of the rule, short portions and single
+    tokens in one step, in every order; each sequence goes the way it goes alone, and both ways agree with the plain model."""
+    from gophonic_b200 import ops
+    from gophonic_b200.engine.model import Model
+    from gophonic_b200.engine.step import Engine
+    from gophonic_b200.parts.latent_attention import LatentAttention
+    sizes = dict(dim=128, rot_dim=64, vdim=128, q_rank=96, scale=0.07)
+    cfg = config([latent(heads=3, kv_rank=64, size=150, mlp=dense(64), **sizes), latent(heads=2, kv_rank=128, size=None, **sizes)], width=128, vocab=80)
+    w = P.random_weights(cfg, seed=290)
+    eng = Engine(Model.from_dir(P.write_model(str(tmp_path / "m"), cfg, w), dtype=dtype), max_tokens=8192)
+    parts = [m for b in eng.model.blocks for m in b.mixers()]
+    seqs = [(0, 200), (0, 9), (900, 66), (30, 129), (300, 64), (0, 65), (77, 1)]         # (tokens before, rows of the step)
+    tokens = [tokens_for(cfg, 30 + i, n + m) for i, (n, m) in enumerate(seqs)]
+    want = [P.forward(cfg, w, t)[n:] for t, (n, _) in zip(tokens, seqs)]
+    # the window of the first layer hides most of the 900 from 66 rows; the second sees them all, 16 pages of 64 for 66 rows
+    long_rows = {0: [0, 2, 3, 5], 1: [0, 3, 5]} if dtype == "bfloat16" else {0: [], 1: []}
+    went = []
+    orig = LatentAttention._expanded, LatentAttention._absorbed
+
+    def spy(f, kind):
+        def g(self, batch, q, ctx, cache, run):
+            went.extend((parts.index(self), i, kind) for i in range(run[0], run[1]))
+            return f(self, batch, q, ctx, cache, run)
+        return g
+
+    def step(order):
+        went.clear()
+        slots = [eng.new_sequence() for _ in order]
+        for s, i in zip(slots, order):
+            if seqs[i][0]:
+                eng.step([(s, tokens[i][:seqs[i][0]])])
+        went.clear()
+        got = eng.step([(s, tokens[i][seqs[i][0]:]) for s, i in zip(slots, order)], [list(range(seqs[i][1])) for i in order]).cpu().numpy()
+        for s in slots:
+            eng.end_sequence(s)
+        eng.check_kernels()
+        at = np.concatenate([[0], np.cumsum([seqs[i][1] for i in order])])
+        return {i: got[at[j]:at[j + 1]] for j, i in enumerate(order)}, {(l, order[j]): kind for l, j, kind in went}
+
+    LatentAttention._expanded, LatentAttention._absorbed = spy(orig[0], "expanded"), spy(orig[1], "absorbed")
+    most = ops.LATENT_TC5_MIN_ROWS
+    try:
+        for order in ([0, 1, 2, 3, 4, 5, 6], [6, 5, 4, 3, 2, 1, 0], [2, 0, 5, 3, 1, 4, 6], [1, 4, 6], [0, 3], [2], [5]):
+            got, ways = step(order)
+            for i in order:
+                if len(order) > 1 or seqs[i][1] > 1:
+                    assert [ways[l, i] for l in (0, 1)] == ["expanded" if i in long_rows[l] else "absorbed" for l in (0, 1)]
+                close(got[i], want[i], TOL[dtype])
+        ops.LATENT_TC5_MIN_ROWS = 1 << 30
+        got, ways = step([0, 2, 3])
+        assert set(ways.values()) == {"absorbed"}
+        for i in got:
+            close(got[i], want[i], TOL[dtype])
+    finally:
+        LatentAttention._expanded, LatentAttention._absorbed = orig
+        ops.LATENT_TC5_MIN_ROWS = most

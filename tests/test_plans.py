@@ -7,6 +7,7 @@ import torch
 from gophonic_b200.engine.step import build_batch
 from gophonic_b200.parts.attention import Attention, choose_splits, few_splits
 from gophonic_b200.parts.gated_attention import GatedAttention
+from gophonic_b200.parts.latent_attention import LatentAttention
 
 SIZES = [1, 2, 3, 5, 8, 13, 24, 50, 64, 128]
 LENGTHS = [1, 63, 64, 65, 100, 256, 700, 1500, 4096, 12000, 40960]
@@ -65,3 +66,51 @@ def test_a_batch_of_one_size_asks_for_few_captured_steps():
     a = part()
     for n, most in ((1, 16), (2, 14), (4, 8), (8, 4), (12, 3), (16, 2), (24, 2), (32, 1)):
         assert len({a.plan(n, 1, kv, 148) for kv in range(1, 8193, 7)}) <= most
+
+
+# ---- latent attention: which sequences of a step go over expanded keys and values -------------------------
+def latent_part(window=1024, dtype=torch.bfloat16, heads=16, kv_rank=512, dims=(128, 64, 128)):
+    from gophonic_b200 import ops
+    weights = torch.empty(0, dtype=dtype)
+    spec = SimpleNamespace(heads=heads, head_dim=dims[0], rot_dim=dims[1], value_dim=dims[2], kv_rank=kv_rank, window=window)
+    return SimpleNamespace(spec=spec, rt=SimpleNamespace(ops=ops, act_dtype=dtype), uk_kn=weights, uv_nk=weights, key_dim=kv_rank + dims[1],
+                           EXPANDED_KEYS_A_ROW=LatentAttention.EXPANDED_KEYS_A_ROW, EXPANDED_BYTES=LatentAttention.EXPANDED_BYTES)
+
+
+def runs_of(extents, **kw):
+    batch, _ = build_batch([(i, [5] * rows, known) for i, (known, rows) in enumerate(extents)], torch.device("cpu"))
+    return LatentAttention.runs(latent_part(**kw), batch)
+
+
+STEPS = [[(0, 65)], [(0, 64)], [(700, 1)], [(0, 2048), (0, 1196)], [(0, 70), (5, 1), (0, 64), (3000, 65), (3000, 90), (3000, 100), (11, 1000)],
+         [(40000, 1000), (0, 100)], [(40000, 4000)] * 5, [(i * 37 % 5000, 1 + i * 61 % 400) for i in range(40)]]
+
+
+@pytest.mark.parametrize("window", [0, 100, 1024])
+@pytest.mark.parametrize("extents", STEPS)
+def test_each_sequence_is_judged_by_itself(extents, window):
+    """A sequence's form does not depend on its neighbours; runs follow one another without a gap, the pages are what the gather
+    kernel walks, and no run's expanded rows take more scratch memory than is allowed."""
+    runs, at, row = runs_of(extents, window=window), 0, 0
+    for k, (first, end, lo, hi, most, pages) in enumerate(runs):
+        assert (first, lo) == (at, row) and end > first
+        mine = extents[first:end]
+        at, row = end, row + sum(r for _, r in mine)
+        assert hi == row and most == max(r for _, r in mine)
+        alone = [runs_of([e], window=window)[0][5] for e in mine]
+        assert all((p > 0) == (pages > 0) for p in alone) and sum(alone) == pages
+        if pages:
+            # as the kernel counts: from the page of the first key that the first row sees to the last token's
+            assert pages == sum(-(-(n + r) // 64) - (max(0, n - window + 1) // 64 if window else 0) for n, r in mine)
+            assert 128 * pages * (576 + 16 * 256) <= max((hi - lo) * 32 * (576 + 512), LatentAttention.EXPANDED_BYTES)
+        assert k == 0 or (runs[k - 1][5] > 0) != (pages > 0) or pages > 0
+    assert at == len(extents)
+
+
+def test_the_rule_of_expanded_latents():
+    expanded = lambda known, rows, **kw: runs_of([(known, rows)], **kw)[0][5] > 0
+    assert expanded(0, 65) and not expanded(0, 64)                             # the fewest rows the kernel is for
+    assert expanded(1052, 100, window=0) and not expanded(1053, 100, window=0)  # at most 1200 keys for 100 rows, in whole pages: 1152 and 1216
+    assert expanded(100000, 2000) and not expanded(100000, 2000, window=0)     # what the window hides is not expanded
+    assert not expanded(0, 500, dtype=torch.float32) and not expanded(0, 500, dims=(64, 64, 128)) and not expanded(0, 500, kv_rank=516)
+    assert runs_of([(0, 100), (9, 3)], dtype=torch.float32) == [(0, 2, 0, 103, 100, 0)]
