@@ -46,10 +46,12 @@ struct Form {
     static constexpr int Q_BYTES = PANELS * QPANEL;            // one group's query tile
     static constexpr int K_BYTES = PANELS * KPANEL, V_BYTES = 2 * KPANEL, STAGE_BYTES = K_BYTES + V_BYTES;
     static constexpr int SMEM = GROUPS * Q_BYTES + STAGES * STAGE_BYTES + 1024;
+    // of every four pairs of scores, how many take the polynomial exponential (measured: 0 -> 55.5 us, 1 -> 52.9, 2 -> 56.8 at
+    // 2048 tokens); none over latents, whose exponentials are good to float32 on the kernel that works on them as cached too
+    static constexpr int POLY_PAIRS = LATENT ? 0 : 1;
 };
 constexpr int TMEM_COLS = 512;                  // S: 2 groups x 2 buffers x 64; O: 2 groups x 128
 constexpr float LOG2E = 1.4426950408889634f;
-constexpr int POLY_PAIRS = 1;                   // of every four pairs of scores, how many take the polynomial exponential (measured: 0 -> 55.5 us, 1 -> 52.9, 2 -> 56.8 at 2048 tokens)
 constexpr float RESCALE_AT = 8.0f;              // rescale O when the row maximum outgrew the scale by 2^8
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -517,7 +519,7 @@ __device__ __forceinline__ void prefill_tc5(const CUtensorMap& map_q, const CUte
                         asm("tanh.approx.f32 %0, %1;" : "=f"(p1) : "f"(t1));
                         p0 = a == 0xff800000u ? 0.f : fmaf(p0, 0.5f, 0.5f);
                         p1 = bb == 0xff800000u ? 0.f : fmaf(p1, 0.5f, 0.5f);
-                    } else if (e < POLY_PAIRS) {
+                    } else if (e < F::POLY_PAIRS) {
                         exp2_poly_x2(t0, t1, p0, p1);
                     } else {
                         p0 = fast_exp2(t0);

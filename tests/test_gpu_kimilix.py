@@ -713,9 +713,27 @@ def test_prompts_over_expanded_latents(heads, kv_rank, q_lens, kv_lens, window, 
             see &= key >= pos - pos % chunk
         s = torch.einsum("ihd,jhd->hij", q[r:r + m].double().view(m, heads, 192), k) * scale
         want = torch.einsum("hij,jhd->ihd", s.masked_fill(~see, -torch.inf).softmax(-1), v).reshape(m, -1)
-        # probabilities and outputs are rounded to bfloat16 (2^-9 each), the exponentials are good to 2e-4
+        # probabilities and outputs are rounded to bfloat16 (2^-9 each)
         assert (out[r:r + m].double() - want).abs().max() <= 1.2e-2 * want.abs().max()
         r += m
+
+
+def test_the_exponentials_over_expanded_latents_are_good_to_float32():
+    """All scores 0, so every weight is 1; values of 1 and 1 + 2^-7 in turn, so a mean over 2^k keys is 1 + 2^-8, half way between
+    two bfloat16 numbers, and rounds to the even one, 1.  Weights that are a little small in float32 but 1 in bfloat16 would
+    leave too small a sum of weights and round to the other."""
+    import torch
+    from gophonic_b200 import ops
+    dev, rows, heads = "cuda:0", 512, 2
+    bf, i32 = dict(dtype=torch.bfloat16, device=dev), lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    values = torch.ones((rows, heads * 128), **bf)
+    values[1::2] += 2.0 ** -7
+    out = torch.full((rows, heads * 128), float("nan"), **bf)
+    ops.attention_latent_expanded(torch.zeros((rows, heads * 192), **bf), out, torch.randn((rows, heads * 128), device=dev).to(torch.bfloat16), values,
+                                  torch.randn((rows, 128), device=dev).to(torch.bfloat16), i32([0]), 64, i32([0]), i32([rows]), i32([rows]), 1, rows, heads,
+                                  192 ** -0.5, 0, 0)
+    for n in (2, 4, 8, 16, 32, 64, 128, 256, 512):
+        assert (out[n - 1] == 1.0).all()
 
 
 @pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
