@@ -11,7 +11,7 @@
 //                   the key part (neighbouring channels turn together), both into the key plane at the row's position.
 // latent_q_rot:     the rotated channels of every query head, rotated and copied behind the head's absorbed channels.
 // head_gemm:        out[r, h, :] = a[r, h, :] W_h for every head h in one launch, W [heads, K, N]; float32 sums.
-// head_gemm_mma:    the same for many bfloat16 rows on the tensor cores, W [heads, N, K].
+// head_gemm_mma:    the same for bfloat16 rows on the tensor cores, W [heads, N, K].
 //
 // Everything is computed in float32 whatever the activation dtype; a row's result depends on that row alone and the
 // order of every sum is fixed by the row's width.
@@ -308,10 +308,16 @@ __global__ void __launch_bounds__(32 * HG_WARPS) head_gemm_kernel(const T* __res
     }
 }
 
-// The same product for many rows on the tensor cores (bf16 mma.sync), W as [heads][N][K]: a CTA takes 64 rows and 64
+// The same product on the tensor cores (bf16 mma.sync), W as [heads][N][K]: a CTA takes 64 rows and 64
 // columns of one head, a warp 16 of the rows; K in pieces of 64, double-buffered with cp.async.
+// FINE (up to HM_FINE_ROWS rows, where the other kernel adds in float32 multiply-adds): every 16 products are added up from zero
+// and the sums added in float32, because the tensor cores' own running sum is coarser (16 heads, K 512, 786432 outputs: 230 are not
+// the bfloat16 number nearest to the 64-bit sum, 66 so, 66 by float32 multiply-adds).  It costs 24 rows of 128 x 512
+// nothing (2.57 us), of 512 x 128 5.58 -> 5.80; 3244 rows would pay 31.7 -> 34.5.
 constexpr int HM_T = 64, HM_S = HM_T + 8;
+constexpr int HM_FINE_ROWS = 32;
 
+template <bool FINE>
 __global__ void __launch_bounds__(128) head_gemm_mma_kernel(const __nv_bfloat16* __restrict__ a, int64_t a_row_stride, int64_t a_head_stride,
                                                             const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
                                                             int64_t o_row_stride, int64_t o_head_stride, int rows, int K, int N) {
@@ -356,8 +362,19 @@ __global__ void __launch_bounds__(128) head_gemm_mma_kernel(const __nv_bfloat16*
             for (int jp = 0; jp < 4; jp++) {
                 uint32_t b[4];
                 ldmatrix_x4(b, &Ws[buf][jp * 16 + (lane & 7) + (lane >> 4) * 8][ks * 16 + ((lane >> 3) & 1) * 8]);
-                mma_bf16_16816(acc[jp * 2], af[0], af[1], af[2], af[3], b[0], b[1]);
-                mma_bf16_16816(acc[jp * 2 + 1], af[0], af[1], af[2], af[3], b[2], b[3]);
+                if (FINE) {
+                    float part[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                    mma_bf16_16816(part[0], af[0], af[1], af[2], af[3], b[0], b[1]);
+                    mma_bf16_16816(part[1], af[0], af[1], af[2], af[3], b[2], b[3]);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        acc[jp * 2][e] += part[0][e];
+                        acc[jp * 2 + 1][e] += part[1][e];
+                    }
+                } else {
+                    mma_bf16_16816(acc[jp * 2], af[0], af[1], af[2], af[3], b[0], b[1]);
+                    mma_bf16_16816(acc[jp * 2 + 1], af[0], af[1], af[2], af[3], b[2], b[3]);
+                }
             }
         }
     }
@@ -495,8 +512,8 @@ GB_API int gb_head_gemm_mma(const void* a, int64_t a_row_stride, int64_t a_head_
         GB_REFUSE("head_gemm_mma: %d heads of %d x %d with these strides are not what this kernel takes", heads, K, N);
     dim3 grid((N + HM_T - 1) / HM_T, heads, (rows + HM_T - 1) / HM_T);
     if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("head_gemm_mma: %d heads, %d rows exceed one launch", heads, rows);
-    launch_pdl(head_gemm_mma_kernel, dim3(grid), dim3(128), 0, stream, (const __nv_bfloat16*)a, a_row_stride, a_head_stride, (const __nv_bfloat16*)w, (__nv_bfloat16*)out,
-                                                   o_row_stride, o_head_stride, rows, K, N);
+    launch_pdl(rows <= HM_FINE_ROWS ? head_gemm_mma_kernel<true> : head_gemm_mma_kernel<false>, grid, dim3(128), 0, stream, (const __nv_bfloat16*)a, a_row_stride,
+               a_head_stride, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, o_row_stride, o_head_stride, rows, K, N);
     GB_CHECK_LAUNCH("head_gemm_mma");
     return 0;
 }

@@ -109,8 +109,8 @@ class LatentAttention(Mixer):
         """out[:, h, :] = a[:, h, :] @ w_kn[h] for every head (``w_nk`` holds the same matrices transposed)."""
         ops = self.rt.ops
         rows, heads, K = a.shape
-        # bfloat16: the tensor cores from one row on (16 heads, us: 128 x 512 one row 3.5 on the CUDA cores and 2.5, 24 rows 7.8 and
-        # 3.0; 512 x 128 7.7 and 5.6, 24 rows 9.8 and 5.9; the same error against 64 bits)
+        # bfloat16: the tensor cores from one row on (16 heads, us inside a graph: 128 x 512 one row 3.3 on the CUDA cores and 2.4, 24
+        # rows 7.3 and 2.6; 512 x 128 7.4 and 5.6, 24 rows 11.4 and 5.8; as many outputs are the nearest to the 64-bit sum)
         if ops.head_gemm_mma_accepts(a, w_nk, out):
             ops.head_gemm_mma(a, w_nk, out)
             return

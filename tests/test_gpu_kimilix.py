@@ -542,6 +542,30 @@ def test_a_product_for_every_head_on_the_tensor_cores(shape):
     assert not ops.head_gemm_mma_accepts(a[:, :, 1:K + 1], w, out[:, :, :N])      # rows that do not start on 16 bytes
 
 
+@pytest.mark.parametrize("shape", [(1, 32, 512, 128), (7, 16, 512, 128), (17, 5, 136, 130), (32, 16, 512, 128), (32, 16, 128, 512)])
+def test_few_rows_add_as_finely_on_the_tensor_cores_as_on_the_cuda_cores(shape):
+    """How many outputs are not the bfloat16 number nearest to the 64-bit sum says how coarse the sums were ahead of that rounding: both
+    kernels add float32 numbers, in different orders, so the counts of rare, independent events may differ by chance: by half,
+    and by four deviations of a small count.  (A running sum inside the tensor cores leaves more than three times as many.)"""
+    import torch
+    from gophonic_b200 import ops
+    ops.use_device(0)
+    rows, heads, K, N = shape
+    counts = [0, 0]
+    for seed in range(16):
+        g = torch.Generator("cuda:0").manual_seed(seed)
+        a = torch.randn(rows, heads, K, generator=g, device="cuda:0").to(torch.bfloat16)
+        w = (torch.randn(heads, K, N, generator=g, device="cuda:0") * K ** -0.5).to(torch.bfloat16)
+        nearest = torch.einsum("rhk,hkn->rhn", a.double(), w.double()).to(torch.bfloat16)
+        outs = [torch.zeros((rows, heads, N), dtype=torch.bfloat16, device="cuda:0") for _ in range(2)]
+        ops.head_gemm(a, w, outs[0])
+        ops.head_gemm_mma(a, w.transpose(1, 2).contiguous(), outs[1])
+        for i in range(2):
+            assert (outs[i].double() - nearest.double()).abs().max().item() <= 2.0 ** -6       # one step of a number below 4
+            counts[i] += (outs[i] != nearest).sum().item()
+    assert counts[1] <= 1.5 * counts[0] + 4 * counts[0] ** 0.5 + 4
+
+
 def test_the_scaled_rotation_tables():
     """All three ranges of wavelengths (kept, blended, divided) in one table, against the plain frequencies."""
     import torch
