@@ -24,6 +24,88 @@ constexpr int KT = 32;      // keys per tile
 constexpr int SIMT_MAX_D = 640;    // widest key head (a latent of 512 and 128 rotated channels); what one CTA stages
 constexpr int SIMT_MAX_DV = 512;   // widest value head
 
+// What both kernels of this file share, so that a row's keys, their order and its sums are the same in either.
+
+// The tiles of keys that a CTA's rows q0 .. last_q visit in its share of the splits.  With kept first tokens they are those of
+// keys [0, keep_first) and then those of the window, each once and in order of position: tile index i < n_first is tile i, the
+// others follow from t_lo.
+struct KeyTiles {
+    int t_lo, n_first, my_lo, my_hi;
+    __device__ __forceinline__ KeyTiles(const AttnParamsX& p, int past, int q0, int last_q, int split) {
+        int lo_pos = 0;
+        if (p.window > 0) {
+            lo_pos = past + q0 - p.window + 1;
+            if (lo_pos < 0) lo_pos = 0;
+        }
+        if (p.chunk > 0) {
+            // the block of the tile's first row begins no later than any other row's
+            const int b = (past + q0) - (past + q0) % p.chunk;
+            if (b > lo_pos) lo_pos = b;
+        }
+        t_lo = lo_pos / KT;
+        n_first = p.window > 0 && p.keep_first > 0 ? (p.keep_first + KT - 1) / KT : 0;
+        if (n_first > t_lo) n_first = t_lo;
+        const int n_tiles = n_first + ((past + last_q) / KT + 1 - t_lo);
+        const int per = (n_tiles + p.num_splits - 1) / p.num_splits;
+        my_lo = split * per;
+        my_hi = my_lo + per < n_tiles ? my_lo + per : n_tiles;
+    }
+    __device__ __forceinline__ int tile(int i) const { return i < n_first ? i : t_lo + (i - n_first); }
+};
+
+__device__ __forceinline__ bool sees(const AttnParamsX& p, int pos, int key) {
+    return key <= pos && (p.window <= 0 || key > pos - p.window || key < p.keep_first) && (p.chunk <= 0 || key >= pos - pos % p.chunk);
+}
+
+// One tile's scores of a row, a key a lane, into its running maximum and sum; the lane's weight.
+template <int NE>
+__device__ __forceinline__ float weigh(bool valid, float score, float& m, float& l, float (&acc)[NE]) {
+    const float sv = valid ? score : -INFINITY;
+    const float m_new = fmaxf(m, warp_max(sv));
+    if (m_new == -INFINITY) return 0.f;
+    const float corr = expf(m - m_new);
+    const float pv = valid ? expf(sv - m_new) : 0.f;
+    l = l * corr + warp_sum(pv);
+#pragma unroll
+    for (int e = 0; e < NE; e++) acc[e] *= corr;
+    m = m_new;
+    return pv;
+}
+
+// A finished row: divided by its sum, or as it is into the scratch memory of the splits.
+template <typename T, int NE>
+__device__ __forceinline__ void leave_row(const AttnParamsX& p, int seq, int split, int64_t row, int head, int dv, int lane, float m, float l,
+                                          const float (&acc)[NE]) {
+    if (p.num_splits == 1) {
+        T* op = (T*)p.out + row * p.out_row_stride + (int64_t)head * dv;
+        float lsum = l, keep = 1.f;
+        if (p.sink) {
+            // one more term in the denominator: a key that has no value, of score 0 or the head's own
+            const float z = p.sinks ? p.sinks[head] : 0.f;
+            const float mf = fmaxf(m, z);
+            keep = expf(m - mf);
+            lsum = lsum * keep + expf(z - mf);
+        }
+        const float inv = keep / lsum;
+#pragma unroll
+        for (int e = 0; e < NE; e++) {
+            const int c = lane + 32 * e;
+            if (c < dv) op[c] = from_f32<T>(acc[e] * inv);
+        }
+    } else {
+        float* sp = p.scratch + (((int64_t)seq * p.heads + head) * p.num_splits + split) * (dv + 2);
+        if (lane == 0) {
+            sp[0] = m;
+            sp[1] = l;
+        }
+#pragma unroll
+        for (int e = 0; e < NE; e++) {
+            const int c = lane + 32 * e;
+            if (c < dv) sp[2 + c] = acc[e];
+        }
+    }
+}
+
 template <typename T, int NE>
 __global__ void __launch_bounds__(128) attn_simt_kernel(AttnParamsX p) {
     extern __shared__ float sm[];
@@ -76,28 +158,9 @@ __global__ void __launch_bounds__(128) attn_simt_kernel(AttnParamsX p) {
         row_pos[rr] = past + q0 + qi;
     }
 
-    int last_q = (q0 + QT < q_len ? q0 + QT : q_len) - 1;
+    const int last_q = (q0 + QT < q_len ? q0 + QT : q_len) - 1;
     const int hi_pos = past + last_q;
-    int lo_pos = 0;
-    if (p.window > 0) {
-        lo_pos = past + q0 - p.window + 1;
-        if (lo_pos < 0) lo_pos = 0;
-    }
-    if (p.chunk > 0) {
-        // the block of the tile's first row begins no later than any other row's
-        const int b = (past + q0) - (past + q0) % p.chunk;
-        if (b > lo_pos) lo_pos = b;
-    }
-    const int t_lo = lo_pos / KT, t_hi = hi_pos / KT + 1;
-    // With kept first tokens the tiles visited are those of keys [0, keep_first) and then those of the
-    // window, each once and in order of position: tile index i < n_first is tile i, the others follow
-    // from t_lo.
-    int n_first = p.window > 0 && p.keep_first > 0 ? (p.keep_first + KT - 1) / KT : 0;
-    if (n_first > t_lo) n_first = t_lo;
-    const int n_tiles = n_first + (t_hi - t_lo);
-    const int per = (n_tiles + p.num_splits - 1) / p.num_splits;
-    const int my_lo = split * per;
-    const int my_hi = my_lo + per < n_tiles ? my_lo + per : n_tiles;
+    const KeyTiles tiles(p, past, q0, last_q, split);
 
     float m[RW], l[RW], acc[RW][NE];
 #pragma unroll
@@ -108,8 +171,8 @@ __global__ void __launch_bounds__(128) attn_simt_kernel(AttnParamsX p) {
         for (int e = 0; e < NE; e++) acc[rr][e] = 0.f;
     }
 
-    for (int ti = my_lo; ti < my_hi; ti++) {
-        const int t = ti < n_first ? ti : t_lo + (ti - n_first);
+    for (int ti = tiles.my_lo; ti < tiles.my_hi; ti++) {
+        const int t = tiles.tile(ti);
         __syncthreads();
         // each warp stages 8 keys of the tile
         for (int jj = 0; jj < 8; jj++) {
@@ -142,23 +205,7 @@ __global__ void __launch_bounds__(128) attn_simt_kernel(AttnParamsX p) {
         const int key = t * KT + lane;
         float pr[RW];
 #pragma unroll
-        for (int rr = 0; rr < RW; rr++) {
-            bool valid = row_ok[rr] && key <= row_pos[rr] && (p.window <= 0 || key > row_pos[rr] - p.window || key < p.keep_first) &&
-                         (p.chunk <= 0 || key >= row_pos[rr] - row_pos[rr] % p.chunk);
-            float sv = valid ? s[rr] : -INFINITY;
-            float m_new = fmaxf(m[rr], warp_max(sv));
-            if (m_new == -INFINITY) {
-                pr[rr] = 0.f;
-                continue;
-            }
-            float corr = expf(m[rr] - m_new);
-            float pv = valid ? expf(sv - m_new) : 0.f;
-            l[rr] = l[rr] * corr + warp_sum(pv);
-#pragma unroll
-            for (int e = 0; e < NE; e++) acc[rr][e] *= corr;
-            m[rr] = m_new;
-            pr[rr] = pv;
-        }
+        for (int rr = 0; rr < RW; rr++) pr[rr] = weigh(row_ok[rr] && sees(p, row_pos[rr], key), s[rr], m[rr], l[rr], acc[rr]);
         for (int jj = 0; jj < KT; jj++) {
             const float* vrow = Vs + jj * vs;
 #pragma unroll
@@ -174,37 +221,8 @@ __global__ void __launch_bounds__(128) attn_simt_kernel(AttnParamsX p) {
     }
 
 #pragma unroll
-    for (int rr = 0; rr < RW; rr++) {
-        if (!row_ok[rr]) continue;
-        if (p.num_splits == 1) {
-            T* op = (T*)p.out + (int64_t)(q_start + row_q[rr]) * p.out_row_stride + (int64_t)row_head[rr] * dv;
-            float lsum = l[rr], keep = 1.f;
-            if (p.sink) {
-                // one more term in the denominator: a key that has no value, of score 0 or the head's own
-                const float z = p.sinks ? p.sinks[row_head[rr]] : 0.f;
-                const float mf = fmaxf(m[rr], z);
-                keep = expf(m[rr] - mf);
-                lsum = lsum * keep + expf(z - mf);
-            }
-            float inv = keep / lsum;
-#pragma unroll
-            for (int e = 0; e < NE; e++) {
-                int c = lane + 32 * e;
-                if (c < dv) op[c] = from_f32<T>(acc[rr][e] * inv);
-            }
-        } else {
-            float* sp = p.scratch + (((int64_t)seq * p.heads + row_head[rr]) * p.num_splits + split) * (dv + 2);
-            if (lane == 0) {
-                sp[0] = m[rr];
-                sp[1] = l[rr];
-            }
-#pragma unroll
-            for (int e = 0; e < NE; e++) {
-                int c = lane + 32 * e;
-                if (c < dv) sp[2 + c] = acc[rr][e];
-            }
-        }
-    }
+    for (int rr = 0; rr < RW; rr++)
+        if (row_ok[rr]) leave_row<T>(p, seq, split, q_start + row_q[rr], row_head[rr], dv, lane, m[rr], l[rr], acc[rr]);
 }
 
 // The same for float32 rows of 16-byte chunks (the true 32-bit path at the usual head sizes), with the
@@ -246,26 +264,12 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParamsX p, int stages
 
     const int last_q = (q0 + QT < q_len ? q0 + QT : q_len) - 1;
     const int hi_pos = past + last_q;
-    int lo_pos = 0;
-    if (p.window > 0) {
-        lo_pos = past + q0 - p.window + 1;
-        if (lo_pos < 0) lo_pos = 0;
-    }
-    if (p.chunk > 0) {
-        const int b = (past + q0) - (past + q0) % p.chunk;
-        if (b > lo_pos) lo_pos = b;
-    }
-    const int t_lo = lo_pos / KT, t_hi = hi_pos / KT + 1;
-    int n_first = p.window > 0 && p.keep_first > 0 ? (p.keep_first + KT - 1) / KT : 0;
-    if (n_first > t_lo) n_first = t_lo;
-    const int n_tiles = n_first + (t_hi - t_lo);
-    const int per = (n_tiles + p.num_splits - 1) / p.num_splits;
-    const int my_lo = split * per;
-    const int my_hi = my_lo + per < n_tiles ? my_lo + per : n_tiles;
+    const KeyTiles tiles(p, past, q0, last_q, split);
+    const int my_lo = tiles.my_lo, my_hi = tiles.my_hi;
 
     // a tile's 32 keys lie in one page (of 64, and tiles begin at multiples of 32); its first key is visible
     auto load = [&](int ti) {
-        const int t = ti < n_first ? ti : t_lo + (ti - n_first);
+        const int t = tiles.tile(ti);
         const int64_t page = page_of(bt, t * KT, p.bt_stride, p.pages);
         const int64_t at = (page * p.kv_heads + kvh) * GB_PAGE + (t * KT) % GB_PAGE;
         const float* kp = (const float*)p.k_plane + at * d;
@@ -320,7 +324,7 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParamsX p, int stages
     float* pw = Ps + warp * RW * KT;
     const float* qrow = Qs + warp * RW * d;
     for (int ti = my_lo; ti < my_hi; ti++) {
-        const int t = ti < n_first ? ti : t_lo + (ti - n_first);
+        const int t = tiles.tile(ti);
         if (stages == 1) {
             __syncthreads();  // all are done with the tile before
             load(ti);
@@ -355,23 +359,8 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParamsX p, int stages
         const int key = t * KT + lane;
         __syncwarp();         // the probabilities of the tile before have been read
 #pragma unroll
-        for (int rr = 0; rr < RW; rr++) {
-            bool valid = row_ok[rr] && key <= row_pos[rr] && (p.window <= 0 || key > row_pos[rr] - p.window || key < p.keep_first) &&
-                         (p.chunk <= 0 || key >= row_pos[rr] - row_pos[rr] % p.chunk);
-            float sv = valid ? s[rr] : -INFINITY;
-            float m_new = fmaxf(m[rr], warp_max(sv));
-            if (m_new == -INFINITY) {
-                pw[rr * KT + lane] = 0.f;
-                continue;
-            }
-            float corr = expf(m[rr] - m_new);
-            float pv = valid ? expf(sv - m_new) : 0.f;
-            l[rr] = l[rr] * corr + warp_sum(pv);
-#pragma unroll
-            for (int e = 0; e < NE; e++) acc[rr][e] *= corr;
-            m[rr] = m_new;
-            pw[rr * KT + lane] = pv;
-        }
+        for (int rr = 0; rr < RW; rr++)
+            pw[rr * KT + lane] = weigh(row_ok[rr] && sees(p, row_pos[rr], key), s[rr], m[rr], l[rr], acc[rr]);
         __syncwarp();
 #pragma unroll 2
         for (int j0 = 0; j0 < KT; j0 += 4) {
@@ -396,36 +385,8 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParamsX p, int stages
     cp_async_wait<0>();
 
 #pragma unroll
-    for (int rr = 0; rr < RW; rr++) {
-        if (!row_ok[rr]) continue;
-        if (p.num_splits == 1) {
-            float* op = (float*)p.out + (int64_t)(q_start + row_q[rr]) * p.out_row_stride + (int64_t)row_head[rr] * dv;
-            float lsum = l[rr], keep = 1.f;
-            if (p.sink) {
-                const float z = p.sinks ? p.sinks[row_head[rr]] : 0.f;
-                const float mf = fmaxf(m[rr], z);
-                keep = expf(m[rr] - mf);
-                lsum = lsum * keep + expf(z - mf);
-            }
-            float inv = keep / lsum;
-#pragma unroll
-            for (int e = 0; e < NE; e++) {
-                int c = lane + 32 * e;
-                if (c < dv) op[c] = acc[rr][e] * inv;
-            }
-        } else {
-            float* sp = p.scratch + (((int64_t)seq * p.heads + row_head[rr]) * p.num_splits + split) * (dv + 2);
-            if (lane == 0) {
-                sp[0] = m[rr];
-                sp[1] = l[rr];
-            }
-#pragma unroll
-            for (int e = 0; e < NE; e++) {
-                int c = lane + 32 * e;
-                if (c < dv) sp[2 + c] = acc[rr][e];
-            }
-        }
-    }
+    for (int rr = 0; rr < RW; rr++)
+        if (row_ok[rr]) leave_row<float>(p, seq, split, q_start + row_q[rr], row_head[rr], dv, lane, m[rr], l[rr], acc[rr]);
 }
 
 // out[seq, head, :] = sum_s exp(m_s - M) acc_s / sum_s exp(m_s - M) l_s over the key splits.
