@@ -320,7 +320,7 @@ int launch_latent(const AttnParamsX& p, cudaStream_t stream) {
         if (e != cudaSuccess) GB_REFUSE("attention_latent: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
         configured = 220 * 1024;
     }
-    launch_pdl(attn_latent_mma_kernel<NT, RG, WG, LKT, STAGES>, dim3(grid), dim3(32 * WG * RG), smem, stream, p);
+    launch_pdl(attn_latent_mma_kernel<NT, RG, WG, LKT, STAGES>, grid, dim3(32 * WG * RG), smem, stream, p);
     GB_CHECK_LAUNCH("attention_latent");
     if (p.num_splits > 1) return gb_attention_merge_launch(p.scratch, p.out, GB_BF16, p.out_row_stride, p.seq_q_start, p.nseq, p.heads, 8 * NT * WG, p.num_splits, 0, nullptr, stream);
     return 0;

@@ -130,7 +130,7 @@ static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // kernel after it may begin its own prologue; the kernels here do so after their own wait, so at
 // most two kernels overlap.  Both calls are no-ops for ordinary launches.
 // The row-wise kernels of the designs with matrix states, latents and mixtures are all launched so (their single-token
-// steps are 80 to 160 kernels of a few microseconds: 16 sequences 600 -> 583 us a step, 24 of the mixture design 1425 -> 1379).  Not
+// steps are 80 to 160 kernels of a few microseconds: 16 sequences 600 -> 590 us a step, 24 of the mixture design 1425 -> 1379).  Not
 // the float32 products and attention of the 32-bit path: their CTAs, early, took the place of the kernel at work
 // (three sequences 2452 -> 2735 us, prompts 8564 -> 9742).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }

@@ -666,11 +666,11 @@ int launch_step(const LinearStateParams& p, cudaStream_t stream) {
     dim3 grid((p.dv + COLS - 1) / COLS + (MODE == 1 ? 1 : 0), p.heads, p.nseq);
     if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("state_scan: grid (%u, %u, %u) exceeds one launch", grid.x, grid.y, grid.z);
     if (p.d <= 64)
-        launch_pdl(state_step_kernel<T, 8, MODE>, dim3(grid), dim3(THREADS), 0, stream, p);
+        launch_pdl(state_step_kernel<T, 8, MODE>, grid, dim3(THREADS), 0, stream, p);
     else if (p.d <= 128)
-        launch_pdl(state_step_kernel<T, 16, MODE>, dim3(grid), dim3(THREADS), 0, stream, p);
+        launch_pdl(state_step_kernel<T, 16, MODE>, grid, dim3(THREADS), 0, stream, p);
     else
-        launch_pdl(state_step_kernel<T, 32, MODE>, dim3(grid), dim3(THREADS), 0, stream, p);
+        launch_pdl(state_step_kernel<T, 32, MODE>, grid, dim3(THREADS), 0, stream, p);
     GB_CHECK_LAUNCH("state_step");
     return 0;
 }
@@ -683,21 +683,21 @@ int launch_scan(const LinearStateParams& p, cudaStream_t stream) {
     if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("state_scan: grid (%u, %u, %u) exceeds one launch", grid.x, grid.y, grid.z);
     if (p.d == 128 || p.d == 256) {     // heads whose channels fill a warp's 32 slices: shared memory read once
         if (p.d == 128)
-            launch_pdl(state_scan_wide_kernel<T, 4, MODE>, dim3(grid), dim3(WIDE_THREADS), 0, stream, p);
+            launch_pdl(state_scan_wide_kernel<T, 4, MODE>, grid, dim3(WIDE_THREADS), 0, stream, p);
         else
-            launch_pdl(state_scan_wide_kernel<T, 8, MODE>, dim3(grid), dim3(WIDE_THREADS), 0, stream, p);
+            launch_pdl(state_scan_wide_kernel<T, 8, MODE>, grid, dim3(WIDE_THREADS), 0, stream, p);
         GB_CHECK_LAUNCH("state_scan");
         return 0;
     }
     switch (rc) {
-        case 4: launch_pdl(state_scan_kernel<T, 4, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
-        case 8: launch_pdl(state_scan_kernel<T, 8, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
-        case 12: launch_pdl(state_scan_kernel<T, 12, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
-        case 16: launch_pdl(state_scan_kernel<T, 16, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
-        case 20: launch_pdl(state_scan_kernel<T, 20, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
-        case 24: launch_pdl(state_scan_kernel<T, 24, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
-        case 28: launch_pdl(state_scan_kernel<T, 28, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
-        case 32: launch_pdl(state_scan_kernel<T, 32, MODE>, dim3(grid), dim3(THREADS), 0, stream, p); break;
+        case 4: launch_pdl(state_scan_kernel<T, 4, MODE>, grid, dim3(THREADS), 0, stream, p); break;
+        case 8: launch_pdl(state_scan_kernel<T, 8, MODE>, grid, dim3(THREADS), 0, stream, p); break;
+        case 12: launch_pdl(state_scan_kernel<T, 12, MODE>, grid, dim3(THREADS), 0, stream, p); break;
+        case 16: launch_pdl(state_scan_kernel<T, 16, MODE>, grid, dim3(THREADS), 0, stream, p); break;
+        case 20: launch_pdl(state_scan_kernel<T, 20, MODE>, grid, dim3(THREADS), 0, stream, p); break;
+        case 24: launch_pdl(state_scan_kernel<T, 24, MODE>, grid, dim3(THREADS), 0, stream, p); break;
+        case 28: launch_pdl(state_scan_kernel<T, 28, MODE>, grid, dim3(THREADS), 0, stream, p); break;
+        case 32: launch_pdl(state_scan_kernel<T, 32, MODE>, grid, dim3(THREADS), 0, stream, p); break;
         default: GB_REFUSE("state_scan: %d key channels a head; at most 256", p.d);
     }
     GB_CHECK_LAUNCH("state_scan");
@@ -901,13 +901,13 @@ int launch_gate(const HeadGateParams& p, cudaStream_t stream) {
         const int hb = 512 / n;     // whole heads in a span of 512 elements
         dim3 grid(p.rows, (p.heads + 4 * hb - 1) / (4 * hb));
         if (grid.y > 65535) GB_REFUSE("head_norm_gate: %d heads exceed one launch", p.heads);
-        launch_pdl(head_norm_gate_span_kernel<TI, T>, dim3(grid), dim3(128), 0, stream, p, hb);
+        launch_pdl(head_norm_gate_span_kernel<TI, T>, grid, dim3(128), 0, stream, p, hb);
         GB_CHECK_LAUNCH("head_norm_gate");
         return 0;
     }
     dim3 grid(p.rows, (p.heads + 3) / 4);
     if (grid.y > 65535) GB_REFUSE("head_norm_gate: %d heads exceed one launch", p.heads);
-    launch_pdl(head_norm_gate_kernel<TI, T>, dim3(grid), dim3(128), 0, stream, p);
+    launch_pdl(head_norm_gate_kernel<TI, T>, grid, dim3(128), 0, stream, p);
     GB_CHECK_LAUNCH("head_norm_gate");
     return 0;
 }
@@ -930,7 +930,7 @@ GB_API int gb_state_scan(const LinearStateParams* pp, int dtype, cudaStream_t st
     if (p.scalar_decay) {
         if (!p.coef || !p.gates || !(p.gate_cap > 0.f)) GB_REFUSE("state_scan: gates, their cap (%g) or room for the factors is missing", (double)p.gate_cap);
         if (p.head_stride < (int64_t)p.d * p.dv + p.d + 1) GB_REFUSE("state_scan: the state has no room for the normaliser and the maximum");
-        launch_pdl(mlstm_gates_kernel, dim3(dim3(p.heads, p.nseq)), dim3(GATE_TOKENS), 0, stream, p);
+        launch_pdl(mlstm_gates_kernel, dim3(p.heads, p.nseq), dim3(GATE_TOKENS), 0, stream, p);
         GB_CHECK_LAUNCH("mlstm_gates");
         if (dtype == GB_F32) return launch_scan<float, 1>(p, stream);
         if (dtype == GB_BF16) return launch_scan<__nv_bfloat16, 1>(p, stream);

@@ -708,7 +708,7 @@ GB_API int gb_moe_act_clamped(const void* up, int64_t up_stride, const float* de
     const unsigned blocks = (unsigned)((total + 255) / 256);
     if (dtype == GB_BF16 && !((ff | up_stride | act_stride) & 7) && !(((uintptr_t)up | (uintptr_t)act) & 15) && rows <= 65535 &&
         (int64_t)experts * ff < (1 << 30))
-        launch_pdl(moe_act_bf16x8_kernel, dim3(dim3(ceil_div(experts * ff, 2048), rows)), dim3(256), 0, stream, 
+        launch_pdl(moe_act_bf16x8_kernel, dim3(ceil_div(experts * ff, 2048), rows), dim3(256), 0, stream,
             (const __nv_bfloat16*)up, up_stride, dense, (__nv_bfloat16*)act, act_stride, experts, ff, kind, weight_input, limit, slope);
     else if (dtype == GB_F32)
         launch_pdl(moe_act_kernel<float>, dim3(blocks), dim3(256), 0, stream, (const float*)up, up_stride, dense, (float*)act, act_stride, rows, experts, ff, kind, weight_input, limit, slope);
@@ -729,11 +729,11 @@ GB_API int gb_moe_rows(const MoeRowsParams* pp, int dtype, int w_dtype, cudaStre
     dim3 ugrid((p.ff + 3) / 4, p.rows * p.top), dgrid((p.hidden + 3) / 4, p.rows);
     if (ugrid.y > 65535) GB_REFUSE("moe_rows: %d rows exceed one launch", p.rows);
     if (dtype == GB_BF16 && w_dtype == GB_BF16) {
-        launch_pdl(moe_up_rows_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(ugrid), dim3(128), 0, stream, p);
-        launch_pdl(moe_down_rows_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(dgrid), dim3(128), 0, stream, p);
+        launch_pdl(moe_up_rows_kernel<__nv_bfloat16, __nv_bfloat16>, ugrid, dim3(128), 0, stream, p);
+        launch_pdl(moe_down_rows_kernel<__nv_bfloat16, __nv_bfloat16>, dgrid, dim3(128), 0, stream, p);
     } else if (dtype == GB_F32 && w_dtype == GB_F32) {
-        launch_pdl(moe_up_rows_kernel<float, float>, dim3(ugrid), dim3(128), 0, stream, p);
-        launch_pdl(moe_down_rows_kernel<float, float>, dim3(dgrid), dim3(128), 0, stream, p);
+        launch_pdl(moe_up_rows_kernel<float, float>, ugrid, dim3(128), 0, stream, p);
+        launch_pdl(moe_down_rows_kernel<float, float>, dgrid, dim3(128), 0, stream, p);
     } else {
         GB_REFUSE("moe_rows: activations of dtype %d with weights of dtype %d", dtype, w_dtype);
     }
@@ -755,16 +755,16 @@ GB_API int gb_moe_rows_grouped(const MoeRowsParams* pp, const int* offsets, cons
     if (dtype == GB_BF16 && w_dtype == GB_BF16 && aligned) {
         dim3 um((p.ff + 15) / 16, p.experts), dm((p.hidden + 15) / 16, p.experts);
         if (p.act_kind != 0)
-            launch_pdl(moe_up_grouped_mma_kernel<true>, dim3(um), dim3(32 * MG_WARPS), 0, stream, p, offsets, src_row);
+            launch_pdl(moe_up_grouped_mma_kernel<true>, um, dim3(32 * MG_WARPS), 0, stream, p, offsets, src_row);
         else
-            launch_pdl(moe_up_grouped_mma_kernel<false>, dim3(um), dim3(32 * MG_WARPS), 0, stream, p, offsets, src_row);
-        launch_pdl(moe_down_grouped_mma_kernel, dim3(dm), dim3(32 * MG_WARPS), 0, stream, p, offsets, ys);
+            launch_pdl(moe_up_grouped_mma_kernel<false>, um, dim3(32 * MG_WARPS), 0, stream, p, offsets, src_row);
+        launch_pdl(moe_down_grouped_mma_kernel, dm, dim3(32 * MG_WARPS), 0, stream, p, offsets, ys);
     } else if (dtype == GB_BF16 && w_dtype == GB_BF16) {
-        launch_pdl(moe_up_grouped_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(ugrid), dim3(128), 0, stream, p, offsets, src_row);
-        launch_pdl(moe_down_grouped_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(dgrid), dim3(128), 0, stream, p, offsets, ys);
+        launch_pdl(moe_up_grouped_kernel<__nv_bfloat16, __nv_bfloat16>, ugrid, dim3(128), 0, stream, p, offsets, src_row);
+        launch_pdl(moe_down_grouped_kernel<__nv_bfloat16, __nv_bfloat16>, dgrid, dim3(128), 0, stream, p, offsets, ys);
     } else if (dtype == GB_F32 && w_dtype == GB_F32) {
-        launch_pdl(moe_up_grouped_kernel<float, float>, dim3(ugrid), dim3(128), 0, stream, p, offsets, src_row);
-        launch_pdl(moe_down_grouped_kernel<float, float>, dim3(dgrid), dim3(128), 0, stream, p, offsets, ys);
+        launch_pdl(moe_up_grouped_kernel<float, float>, ugrid, dim3(128), 0, stream, p, offsets, src_row);
+        launch_pdl(moe_down_grouped_kernel<float, float>, dgrid, dim3(128), 0, stream, p, offsets, ys);
     } else {
         GB_REFUSE("moe_rows: activations of dtype %d with weights of dtype %d", dtype, w_dtype);
     }

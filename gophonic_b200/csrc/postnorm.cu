@@ -482,12 +482,12 @@ GB_API int gb_head_gemm(const void* a, int64_t a_row_stride, int64_t a_head_stri
     if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("head_gemm: %d heads, %d rows exceed one launch", heads, rows);
     if (dtype == GB_F32 && w_dtype == GB_F32) {
         if (smem > 48 * 1024) cudaFuncSetAttribute(head_gemm_kernel<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-        launch_pdl(head_gemm_kernel<float, float>, dim3(grid), dim3(32 * HG_WARPS), smem, stream, (const float*)a, a_row_stride, a_head_stride, (const float*)w, (float*)out,
+        launch_pdl(head_gemm_kernel<float, float>, grid, dim3(32 * HG_WARPS), smem, stream, (const float*)a, a_row_stride, a_head_stride, (const float*)w, (float*)out,
                                                                              o_row_stride, o_head_stride, rows, K, N);
     } else if (dtype == GB_BF16 && w_dtype == GB_BF16) {
         if (smem > 48 * 1024)
             cudaFuncSetAttribute(head_gemm_kernel<__nv_bfloat16, __nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-        launch_pdl(head_gemm_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(grid), dim3(32 * HG_WARPS), smem, stream, (const __nv_bfloat16*)a, a_row_stride, a_head_stride,
+        launch_pdl(head_gemm_kernel<__nv_bfloat16, __nv_bfloat16>, grid, dim3(32 * HG_WARPS), smem, stream, (const __nv_bfloat16*)a, a_row_stride, a_head_stride,
                                                                                              (const __nv_bfloat16*)w, (__nv_bfloat16*)out, o_row_stride,
                                                                                              o_head_stride, rows, K, N);
     } else {
