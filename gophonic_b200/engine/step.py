@@ -49,6 +49,8 @@ class StepBatch:
     # launch plans of the step's mixers, by the mixer's identity (``Mixer.plan``); a mixer that is
     # not listed is asked when it first runs
     plans: Dict[int, object] = field(default_factory=dict)
+    # what parts work out on the host once a step for all layers of one geometry, by a key of theirs
+    shared: Dict[object, object] = field(default_factory=dict)
     _workspaces: Dict[object, torch.Tensor] = field(default_factory=dict)
 
     def plan_for(self, part):

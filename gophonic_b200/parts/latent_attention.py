@@ -30,7 +30,7 @@ from .base import KVRequest, Mixer, Runtime, TensorDecl
 
 class LatentAttention(Mixer):
     capturable = True
-    EXPANDED_KEYS_A_ROW, EXPANDED_BYTES = 12, 128 << 20
+    EXPANDED_KEYS_A_ROW, EXPANDED_BYTES, FEW_ROWS_PAGES = 12, 128 << 20, 20
     ROWS_ONE_LAUNCH = 32      # up to this many rows the per-head products that the tensor cores do not take run as one launch
 
     @classmethod
@@ -131,21 +131,35 @@ class LatentAttention(Mixer):
         3741 over 12160 11.1 and 5.9, 1121 over 9280 6.3 and 3.4; 128 over 1152 and 70 over 1088 the same, 261 rows of
         four sequences over 4352 3.5 and 3.6.
 
-        Both forms round, at different places, so each sequence is judged by its own rows and keys alone: what it
-        gets must not depend on what else is in the step.  The expanded rows are scratch memory, no more of it at a time than the
-        absorbed queries and outputs of the same sequences would take, or EXPANDED_BYTES; a run that would is cut in two."""
+        Both forms round, at different places, so a sequence's form must not follow from the other sequences' contexts: the numbers of
+        sequences and rows, by which all kernels are chosen, decide for the step.  A key of a sequence is seen by as many rows as
+        the portion and the window have, so what counts is the mean portion: with a window so many rows that at most twelve
+        keys a row are visible, without one the 94 rows that a window of 1024 asks for.
+
+        A run of its own costs the host about 0.1 ms a layer (eight layers, us: 300, 9, 120 and 1 row behind 300 tokens 2855 in one
+        run, 4650 in four), so a sequence leaves the others' form only for its own sake: few rows behind so many keys that the
+        expansion costs more than that.  The expanded rows are scratch memory, no more of it at a time than the absorbed queries and
+        outputs of the same sequences would take, or EXPANDED_BYTES; a run that would is cut in two, a sequence that would
+        alone stays on the latents."""
+        s = self.spec
+        key = ("latent runs", s.heads, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank, s.window, self.uk_kn.dtype, self.uv_nk.dtype)
+        if key not in batch.shared:       # every layer of one geometry has the same answer
+            batch.shared[key] = self._runs(batch)
+        return batch.shared[key]
+
+    def _runs(self, batch):
         s, ops = self.spec, self.rt.ops
-        if (batch.extents is None or not ops.latent_expanded_accepts(self.rt.act_dtype, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank, batch.max_q_len)
-                or self.uk_kn.dtype != torch.bfloat16 or self.uv_nk.dtype != torch.bfloat16):
-            return [(0, batch.nseq, 0, batch.rows, batch.max_q_len, 0)]
         window = int(s.window)
+        if (batch.extents is None or not ops.latent_expanded_accepts(self.rt.act_dtype, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank, batch.max_q_len)
+                or self.uk_kn.dtype != torch.bfloat16 or self.uv_nk.dtype != torch.bfloat16
+                or batch.nseq * (window if window > 0 else 1024) > (self.EXPANDED_KEYS_A_ROW - 1) * batch.rows):
+            return [(0, batch.nseq, 0, batch.rows, batch.max_q_len, 0)]
         page_bytes = 2 * 64 * (self.key_dim + s.heads * (s.head_dim + s.value_dim))
         row_bytes = 2 * s.heads * (self.key_dim + s.kv_rank)
         out, at = [], 0
         for i, (known, rows) in enumerate(batch.extents):
             pages = (known + rows + 63) // 64 - (max(0, known - window + 1) // 64 if window > 0 else 0)
-            if (rows < ops.LATENT_TC5_MIN_ROWS or 64 * pages > self.EXPANDED_KEYS_A_ROW * rows
-                    or pages * page_bytes > max(rows * row_bytes, self.EXPANDED_BYTES)):
+            if (rows < ops.LATENT_TC5_MIN_ROWS and pages > self.FEW_ROWS_PAGES) or pages * page_bytes > max(rows * row_bytes, self.EXPANDED_BYTES):
                 pages = 0
             if out and (out[-1][5] > 0) == (pages > 0):
                 first, _, lo, _, most, held = out[-1]
@@ -157,40 +171,50 @@ class LatentAttention(Mixer):
             at += rows
         return out
 
+    @staticmethod
+    def _sequences(batch, run):
+        """(slots, first rows, rows, keys) of the run's sequences and the positions of its rows."""
+        first, end, lo, hi = run[:4]
+        if end - first == batch.nseq:
+            return batch.seq_slot, batch.seq_q_start, batch.seq_q_len, batch.seq_kv_len, batch.row_pos
+        return batch.seq_slot[first:end], batch.seq_q_start[first:end], batch.seq_q_len[first:end], batch.seq_kv_len[first:end], batch.row_pos[lo:hi]
+
     def _expanded(self, batch, q: torch.Tensor, ctx: torch.Tensor, cache, run) -> None:
         """Attention of a run's rows over keys and values made from the visible latents for this step."""
         ops, s = self.rt.ops, self.spec
         H, R, dev = s.heads, s.kv_rank, q.device
         first, end, lo, hi, most, pages = run
+        slot, q_start, q_len, kv_len, row_pos = self._sequences(batch, run)
         cos, sin, _ = self.position.kernel_args()
-        ops.latent_q_rot(q[lo:hi], q[lo:hi], H, s.head_dim, s.rot_dim, cos, sin, batch.row_pos[lo:hi])
+        mine = q if hi - lo == batch.rows else q[lo:hi]
+        ops.latent_q_rot(mine, mine, H, s.head_dim, s.rot_dim, cos, sin, row_pos)
         lat = torch.empty((64 * pages, self.key_dim), dtype=q.dtype, device=dev)
         base = torch.empty((end - first,), dtype=torch.int32, device=dev)
-        q_len, kv_len = batch.seq_q_len[first:end], batch.seq_kv_len[first:end]
-        ops.latent_gather(cache.k, cache.block_table, batch.seq_slot[first:end], q_len, kv_len, end - first, int(s.window), lat, base)
+        ops.latent_gather(cache.k, cache.block_table, slot, q_len, kv_len, end - first, int(s.window), lat, base)
         keys = torch.empty((64 * pages, H * s.head_dim), dtype=q.dtype, device=dev)
         values = torch.empty((64 * pages, H * s.value_dim), dtype=q.dtype, device=dev)
         ops.gemm(lat[:, :R], self.uk_kn.view(H * s.head_dim, R), keys)
         ops.gemm(lat[:, :R], self.uv_nk.view(H * s.value_dim, R), values)
-        ops.attention_latent_expanded(q, ctx, keys, values, lat, base, R, batch.seq_q_start[first:end], q_len, kv_len, end - first, most, H,
-                                      float(s.scale), int(s.window), int(s.chunk))
+        ops.attention_latent_expanded(q, ctx, keys, values, lat, base, R, q_start, q_len, kv_len, end - first, most, H, float(s.scale),
+                                      int(s.window), int(s.chunk))
 
     def _absorbed(self, batch, q: torch.Tensor, ctx: torch.Tensor, cache, run) -> None:
         """Attention of a run's rows over the latents as they are cached."""
         ops, s = self.rt.ops, self.spec
         H, d, dr, dv, R = s.heads, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank
         first, end, lo, hi, most, _ = run
-        rows, q, ctx = hi - lo, q[lo:hi], ctx[lo:hi]
+        slot, q_start, q_len, kv_len, row_pos = self._sequences(batch, run)
+        rows = hi - lo
+        if rows != batch.rows:
+            q, ctx, q_start = q[lo:hi], ctx[lo:hi], q_start - lo     # rows of qa
         cos, sin, _ = self.position.kernel_args()
         qa = torch.empty((rows, H * self.key_dim), dtype=q.dtype, device=q.device)       # per head [W_uk^T q_plain | rotated part]
         self._per_head(q.view(rows, H, d + dr)[:, :, :d], self.uk_kn, self.uk_nk, qa.view(rows, H, self.key_dim)[:, :, :R])
-        ops.latent_q_rot(q, qa, H, d, dr, cos, sin, batch.row_pos[lo:hi])
+        ops.latent_q_rot(q, qa, H, d, dr, cos, sin, row_pos)
         mixed = torch.empty((rows, H * R), dtype=q.dtype, device=q.device)               # per head sum_j p_j c_j
         splits, scratch = self.key_splits(batch)
-        q_start = batch.seq_q_start[first:end] - lo if lo else batch.seq_q_start[first:end]   # rows of qa
-        ops.attention(qa, mixed, cache.k, cache.v, cache.block_table, batch.seq_slot[first:end], q_start, batch.seq_q_len[first:end],
-                      batch.seq_kv_len[first:end], end - first, most, H, 1, self.key_dim, float(s.scale), int(s.window), splits, scratch,
-                      value_dim=R, chunk=int(s.chunk))
+        ops.attention(qa, mixed, cache.k, cache.v, cache.block_table, slot, q_start, q_len, kv_len, end - first, most, H, 1, self.key_dim,
+                      float(s.scale), int(s.window), splits, scratch, value_dim=R, chunk=int(s.chunk))
         self._per_head(mixed.view(rows, H, R), self.uv_kn, self.uv_nk, ctx.view(rows, H, dv))
 
     def forward(self, batch, x: torch.Tensor, out: torch.Tensor, cache) -> None:

@@ -762,8 +762,8 @@ def test_the_exponentials_over_expanded_latents_are_good_to_float32():
 
 @pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
 def test_the_forms_of_latent_attention_inside_a_step(tmp_path, dtype):
-    """Models whose heads both forms take: prompts, portions behind contexts on both sides of the rule, short portions and single
-    tokens in one step, in every order; each sequence goes the way it goes alone, and both ways agree with the plain model."""
+    """Models whose heads both forms take: prompts, portions behind contexts, short portions and single tokens in one step, in several
+    orders, on both sides of the rule and with both forms in one step; both agree with the plain model."""
     from gophonic_b200 import ops
     from gophonic_b200.engine.model import Model
     from gophonic_b200.engine.step import Engine
@@ -773,11 +773,13 @@ def test_the_forms_of_latent_attention_inside_a_step(tmp_path, dtype):
     w = P.random_weights(cfg, seed=290)
     eng = Engine(Model.from_dir(P.write_model(str(tmp_path / "m"), cfg, w), dtype=dtype), max_tokens=8192)
     parts = [m for b in eng.model.blocks for m in b.mixers()]
-    seqs = [(0, 200), (0, 9), (900, 66), (30, 129), (300, 64), (0, 65), (77, 1)]         # (tokens before, rows of the step)
+    seqs = [(0, 200), (0, 9), (900, 66), (30, 129), (300, 64), (0, 65), (77, 1), (1400, 3)]         # (tokens before, rows of the step)
     tokens = [tokens_for(cfg, 30 + i, n + m) for i, (n, m) in enumerate(seqs)]
     want = [P.forward(cfg, w, t)[n:] for t, (n, _) in zip(tokens, seqs)]
-    # the window of the first layer hides most of the 900 from 66 rows; the second sees them all, 16 pages of 64 for 66 rows
-    long_rows = {0: [0, 2, 3, 5], 1: [0, 3, 5]} if dtype == "bfloat16" else {0: [], 1: []}
+    # order of a step, the sequences whose rows go over expanded keys and values in the first layer (a window of 150: 14 rows a
+    # sequence suffice) and in the second (no window: 94, but not three rows behind 1400 tokens)
+    steps = [([0, 1, 2, 3, 4, 5, 6], range(7), []), ([6, 5, 4, 3, 2, 1, 0], range(7), []), ([1, 4, 6], [], []), ([0, 3], [0, 3], [0, 3]), ([2], [2], []),
+             ([5], [5], []), ([0, 3, 7], [0, 3, 7], [0, 3]), ([7, 3, 0], [0, 3, 7], [0, 3]), ([0, 7, 3], [0, 3, 7], [0, 3]), ([1, 0, 3], [0, 1, 3], [0, 1, 3])]
     went = []
     orig = LatentAttention._expanded, LatentAttention._absorbed
 
@@ -804,11 +806,11 @@ def test_the_forms_of_latent_attention_inside_a_step(tmp_path, dtype):
     LatentAttention._expanded, LatentAttention._absorbed = spy(orig[0], "expanded"), spy(orig[1], "absorbed")
     most = ops.LATENT_TC5_MIN_ROWS
     try:
-        for order in ([0, 1, 2, 3, 4, 5, 6], [6, 5, 4, 3, 2, 1, 0], [2, 0, 5, 3, 1, 4, 6], [1, 4, 6], [0, 3], [2], [5]):
+        for order, *expanded in steps:
             got, ways = step(order)
             for i in order:
-                if len(order) > 1 or seqs[i][1] > 1:
-                    assert [ways[l, i] for l in (0, 1)] == ["expanded" if i in long_rows[l] else "absorbed" for l in (0, 1)]
+                want_ways = ["expanded" if dtype == "bfloat16" and i in expanded[l] else "absorbed" for l in (0, 1)]
+                assert [ways[l, i] for l in (0, 1)] == want_ways
                 close(got[i], want[i], TOL[dtype])
         ops.LATENT_TC5_MIN_ROWS = 1 << 30
         got, ways = step([0, 2, 3])

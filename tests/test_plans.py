@@ -74,43 +74,52 @@ def latent_part(window=1024, dtype=torch.bfloat16, heads=16, kv_rank=512, dims=(
     weights = torch.empty(0, dtype=dtype)
     spec = SimpleNamespace(heads=heads, head_dim=dims[0], rot_dim=dims[1], value_dim=dims[2], kv_rank=kv_rank, window=window)
     return SimpleNamespace(spec=spec, rt=SimpleNamespace(ops=ops, act_dtype=dtype), uk_kn=weights, uv_nk=weights, key_dim=kv_rank + dims[1],
-                           EXPANDED_KEYS_A_ROW=LatentAttention.EXPANDED_KEYS_A_ROW, EXPANDED_BYTES=LatentAttention.EXPANDED_BYTES)
+                           EXPANDED_KEYS_A_ROW=LatentAttention.EXPANDED_KEYS_A_ROW, EXPANDED_BYTES=LatentAttention.EXPANDED_BYTES,
+                           FEW_ROWS_PAGES=LatentAttention.FEW_ROWS_PAGES)
 
 
 def runs_of(extents, **kw):
     batch, _ = build_batch([(i, [5] * rows, known) for i, (known, rows) in enumerate(extents)], torch.device("cpu"))
-    return LatentAttention.runs(latent_part(**kw), batch)
+    return LatentAttention._runs(latent_part(**kw), batch)
 
 
 STEPS = [[(0, 65)], [(0, 64)], [(700, 1)], [(0, 2048), (0, 1196)], [(0, 70), (5, 1), (0, 64), (3000, 65), (3000, 90), (3000, 100), (11, 1000)],
-         [(40000, 1000), (0, 100)], [(40000, 4000)] * 5, [(i * 37 % 5000, 1 + i * 61 % 400) for i in range(40)]]
+         [(40000, 1000), (0, 100)], [(40000, 4000)] * 5, [(i * 37 % 5000, 1 + i * 61 % 400) for i in range(40)], [(2000, 3), (0, 1000), (90, 3)]]
 
 
 @pytest.mark.parametrize("window", [0, 100, 1024])
 @pytest.mark.parametrize("extents", STEPS)
-def test_each_sequence_is_judged_by_itself(extents, window):
-    """A sequence's form does not depend on its neighbours; runs follow one another without a gap, the pages are what the gather
-    kernel walks, and no run's expanded rows take more scratch memory than is allowed."""
+def test_the_runs_of_a_step(extents, window):
+    """A sequence's form does not depend on the others' contexts; runs follow one another without a gap, the pages are what the
+    gather kernel walks, and no run's expanded rows take more scratch memory than is allowed."""
     runs, at, row = runs_of(extents, window=window), 0, 0
     for k, (first, end, lo, hi, most, pages) in enumerate(runs):
         assert (first, lo) == (at, row) and end > first
         mine = extents[first:end]
         at, row = end, row + sum(r for _, r in mine)
         assert hi == row and most == max(r for _, r in mine)
-        alone = [runs_of([e], window=window)[0][5] for e in mine]
-        assert all((p > 0) == (pages > 0) for p in alone) and sum(alone) == pages
         if pages:
             # as the kernel counts: from the page of the first key that the first row sees to the last token's
             assert pages == sum(-(-(n + r) // 64) - (max(0, n - window + 1) // 64 if window else 0) for n, r in mine)
             assert 128 * pages * (576 + 16 * 256) <= max((hi - lo) * 32 * (576 + 512), LatentAttention.EXPANDED_BYTES)
         assert k == 0 or (runs[k - 1][5] > 0) != (pages > 0) or pages > 0
     assert at == len(extents)
+    forms = lambda runs: [pages > 0 for first, end, _, _, _, pages in runs for _ in range(first, end)]
+    for i in range(len(extents)):                # the same rows, the others behind other contexts
+        for other in (0, 10, 777, 30000):
+            assert forms(runs_of([e if j == i else (other, e[1]) for j, e in enumerate(extents)], window=window))[i] == forms(runs)[i]
 
 
 def test_the_rule_of_expanded_latents():
     expanded = lambda known, rows, **kw: runs_of([(known, rows)], **kw)[0][5] > 0
-    assert expanded(0, 65) and not expanded(0, 64)                             # the fewest rows the kernel is for
-    assert expanded(1052, 100, window=0) and not expanded(1053, 100, window=0)  # at most 1200 keys for 100 rows, in whole pages: 1152 and 1216
-    assert expanded(100000, 2000) and not expanded(100000, 2000, window=0)     # what the window hides is not expanded
+    for window in (0, 1024):                                    # 1024 keys ahead of the portion, eleven a row
+        for known in (0, 700, 3000):
+            assert expanded(known, 94, window=window) and not expanded(known, 93, window=window)
+    assert expanded(0, 65, window=100) and not expanded(0, 64, window=100)     # the fewest rows the kernel is for
+    assert expanded(100000, 2000) and not expanded(100000, 2000, window=0)     # scratch memory: what the window hides takes none
+    assert len(runs_of([(300, 300), (300, 9), (300, 120), (300, 1)])) == 1 and runs_of([(0, 66), (0, 5)]) == [(0, 2, 0, 71, 66, 0)]
+    # few rows behind many keys leave the others, where the window does not hide them
+    assert [r[5] > 0 for r in runs_of([(0, 500), (2000, 3), (1200, 3)], window=0)] == [True, False, True]
+    assert [r[5] > 0 for r in runs_of([(0, 500), (2000, 3), (1200, 3)])] == [True]
     assert not expanded(0, 500, dtype=torch.float32) and not expanded(0, 500, dims=(64, 64, 128)) and not expanded(0, 500, kv_rank=516)
     assert runs_of([(0, 100), (9, 3)], dtype=torch.float32) == [(0, 2, 0, 103, 100, 0)]
