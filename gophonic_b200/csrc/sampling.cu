@@ -424,7 +424,8 @@ __global__ void __launch_bounds__(256) sample_hist_kernel(SampleParams p, uint32
         if (sh[i]) atomicAdd(&h[i], sh[i]);
 }
 
-// The chunk's logits are requested before the histogram is complete, the bin is found by a sum over the CTA and a
+// The chunk's logits are requested before the histogram is complete (its kernel is an ordinary launch, so whatever made the
+// logits has ended), the bin is found by a sum over the CTA and a
 // CTA asks for its places in the list once (a place at a time and the histogram walked by one thread: 19 us
 // for 16 rows of 151936, 11 now, some of it beside the histogram).  The order of the list is that of arrival; its entries differ, so
 // what is sorted from it is the same.

@@ -794,7 +794,9 @@ def attention_decode_rope(qkv: torch.Tensor, out: torch.Tensor, rope_args: tuple
     """``qk_norm_rope_kv_write(qkv, *rope_args)`` and ``attention(qkv[:, :heads * head_dim], out,
     *attn_args)`` for single-token rows in one kernel (plus the merge of key splits): the attention
     kernel norms and rotates its queries itself, takes the token's own key and value from the row and
-    stores them in the cache.  The same bits as the two calls."""
+    stores them in the cache.  The same bits as the two calls.  Without key splits it asks for the pages of earlier tokens
+    while the launch directly ahead may still run: that one must not write this cache (the product that makes ``qkv``, which stands
+    between two tokens of a sequence, does not)."""
     r = _rope_params(qkv, *rope_args)
     a = _attn_params(qkv[:, :r.heads * r.d], out, *attn_args)
     _check(_lib.gb_attention_decode_mma_rope(byref(a), byref(r), _stream()), 2 if a.num_splits > 1 else 1)

@@ -29,7 +29,7 @@ def choose_splits(units: int, max_kv_len: int, sm_count: int = 148, page_bytes: 
     of its bytes at the memory bandwidth and of one CTA's own pace (a little over a microsecond a page),
     so a thin last wave costs as much as a full one unless its CTAs are short; cutting the keys
     costs the merge kernel and the traffic of the partial results.  A piece keeps at least 256
-    keys.
+    keys (``few_splits`` goes further where there are few sequences).
     """
     units = max(1, units)
     pages = max(1, (max_kv_len + 63) // 64)
