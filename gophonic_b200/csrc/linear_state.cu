@@ -16,7 +16,7 @@
 // tokens of the step, the tokens' q, k and decay rows are staged in shared memory eight tokens at a
 // time, and a token's output is a shuffle sum over the 8 slices.
 #include "api.h"
-#include "common.cuh"
+#include "mma.cuh"
 
 #include <math.h>
 
@@ -142,8 +142,6 @@ __global__ void __launch_bounds__(GATE_TOKENS) mlstm_gates_kernel(LinearStatePar
 // (p.decay), S <- S + u (v - S), with no key: one staged row less and the same arithmetic an element.
 template <typename T, int RC, int MODE>
 __global__ void __launch_bounds__(THREADS) state_scan_kernel(LinearStateParams p) {
-    pdl_wait();
-    pdl_trigger();
     constexpr bool SCALAR = MODE == 1, WRITES = MODE == 2;
     constexpr int P = (RC / 4) % 2 ? RC : RC + 4;   // slice stride in floats: P / 4 odd, so the 8 slices' 16-byte reads miss each other's banks
     constexpr int ROW = SLICES * P;
@@ -330,6 +328,7 @@ __global__ void __launch_bounds__(THREADS) state_scan_kernel(LinearStateParams p
             }
         }
     }
+    pdl_trigger();   // not before: the CTAs of the kernel behind, parked beside the scan, would take its issue slots
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < RC; i++) st_s[slice * RC + i][col] = st[i];
@@ -359,22 +358,17 @@ __global__ void __launch_bounds__(THREADS) state_scan_kernel(LinearStateParams p
 // warp owns CW columns and its 32 lanes are 32 slices of the channels (RC = d / 32 each), a thread keeps
 // RC x CW state elements.  A token's q, k and decay rows are then read by the warp as whole rows (every
 // lane its own 16 bytes, no two quarter-warps the same bytes), four times less shared-memory traffic
-// than with 8 slices and a column a thread, for the same registers.  A tile's sums (WT tokens x CW columns, 32
-// or 16) are added up over the 32 slices by a five-step exchange that leaves each lane one of them.
-// Bound by the latency of a token's chain through a warp: the CTAs of 16 columns leave one a SM, so eight
-// warps of two columns (two a scheduler) and, where shared memory allows, tiles of 16 tokens (1611 tokens of 8 heads of
-// 128 x 256: 190 us with four warps of four columns and tiles of 8, 167 to 182 now).  The sums' order is the same.
-constexpr int WIDE_THREADS = 256;
-
-template <typename T, int RC, int MODE>
-__global__ void __launch_bounds__(WIDE_THREADS) state_scan_wide_kernel(LinearStateParams p) {
-    pdl_wait();
-    pdl_trigger();
+// than with 8 slices and a column a thread, for the same registers.  A tile's 32 sums (8 tokens x 4 columns, or 16 x 2)
+// are added up over the 32 slices by a five-step exchange that leaves each lane one of them, in one order in both forms.
+// Four columns a warp, four warps: every staged row is read four times a CTA, which is what binds several CTAs an SM.  Two columns, eight
+// warps, where a CTA has an SM to itself and is bound by the latency of a token's chain (launch_scan has the line).
+// The kernel behind may come up only when the tokens are done: its CTAs, parked beside the scan, take its issue slots.
+template <typename T, int RC, int MODE, int CW>
+__global__ void __launch_bounds__(32 * COLS / CW) state_scan_wide_kernel(LinearStateParams p) {
     constexpr bool SCALAR = MODE == 1, WRITES = MODE == 2;
     constexpr int D = 32 * RC;          // key channels of a head
-    constexpr int CW = 2;               // columns a warp (and a thread) owns
-    constexpr int TT = RC == 4 ? 16 : 8, THREADS = WIDE_THREADS;   // tokens a tile
-    static_assert(CW * WIDE_THREADS / 32 == COLS && TT * COLS <= THREADS, "the warps own the CTA's columns; a thread fetches a value");
+    constexpr int THREADS = 32 * COLS / CW, TT = 32 / CW;   // tokens a tile: a thread fetches one value of them
+    static_assert(TT * COLS == THREADS, "a value a thread");
     __shared__ __align__(16) float q_s[TT][D];
     __shared__ __align__(16) float k_s[WRITES ? 1 : TT][WRITES ? 4 : D];
     __shared__ __align__(16) float a_s[SCALAR ? 1 : TT][SCALAR ? 4 : D];
@@ -441,7 +435,7 @@ __global__ void __launch_bounds__(WIDE_THREADS) state_scan_wide_kernel(LinearSta
             if (!WRITES) rk[e] = r[p.k_off + h * D + c];
             ra[e] = SCALAR ? p.coef[(row * H + h) * 4 + 1] : p.decay[row * p.decay_stride + h * D + c];
         }
-        if (tid < TT * COLS) {
+        {
             int t = tid / COLS, jj = j0 + tid % COLS;
             t = t < nt ? t : nt - 1;
             jj = jj < dv ? jj : dv - 1;
@@ -466,7 +460,7 @@ __global__ void __launch_bounds__(WIDE_THREADS) state_scan_wide_kernel(LinearSta
             if (!WRITES) k_s[t][c] = there ? (SCALAR ? to_f32<T>(rk[e]) * ra[e] : to_f32<T>(rk[e])) : 0.f;
             if (!SCALAR) a_s[t][c] = there ? ra[e] : (WRITES ? 0.f : 1.f);
         }
-        if (tid < TT * COLS) {
+        {
             const int t = tid / COLS, jj = tid % COLS;
             float v = 0.f;
             if (t < nt) {
@@ -486,10 +480,14 @@ __global__ void __launch_bounds__(WIDE_THREADS) state_scan_wide_kernel(LinearSta
         float acc[TT * CW];     // index t * CW + c
 #pragma unroll
         for (int t = 0; t < TT; t++) {
-            const float2 v2 = *reinterpret_cast<const float2*>(&v_s[t][warp * CW]);
-            const float vv[CW] = {v2.x, v2.y};
+            float vv[CW], sum[CW];
+            if (CW == 4)
+                *reinterpret_cast<float4*>(vv) = *reinterpret_cast<const float4*>(&v_s[t][warp * CW]);
+            else
+                *reinterpret_cast<float2*>(vv) = *reinterpret_cast<const float2*>(&v_s[t][warp * CW]);
             const float keep = SCALAR ? keep_s[t] : 0.f;
-            float sum[CW] = {0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < CW; c++) sum[c] = 0.f;
 #pragma unroll
             for (int i = 0; i < RC; i += 4) {
                 const float4 q4 = *reinterpret_cast<const float4*>(&q_s[t][lane * RC + i]);
@@ -509,15 +507,12 @@ __global__ void __launch_bounds__(WIDE_THREADS) state_scan_wide_kernel(LinearSta
 #pragma unroll
             for (int c = 0; c < CW; c++) acc[t * CW + c] = sum[c];
         }
-        // the sums of a thread over 32 slices: halve the sums and the lanes; 16 sums meet whole across the first halves
-        constexpr int SUMS = TT * CW;
+        // 32 sums a thread over 32 slices: halve the sums and the lanes five times
         float b16[16], b8[8], b4[4], b2[2], total;
         {
             const bool up = lane & 16;
 #pragma unroll
-            for (int j = 0; j < 16; j++)
-                b16[j] = SUMS == 32 ? (up ? acc[(j + 16) % SUMS] : acc[j]) + __shfl_xor_sync(0xffffffffu, up ? acc[j] : acc[(j + 16) % SUMS], 16)
-                                    : acc[j] + __shfl_xor_sync(0xffffffffu, acc[j], 16);
+            for (int j = 0; j < 16; j++) b16[j] = (up ? acc[j + 16] : acc[j]) + __shfl_xor_sync(0xffffffffu, up ? acc[j] : acc[j + 16], 16);
         }
         {
             const bool up = lane & 8;
@@ -538,8 +533,7 @@ __global__ void __launch_bounds__(WIDE_THREADS) state_scan_wide_kernel(LinearSta
             const bool up = lane & 1;
             total = (up ? b2[1] : b2[0]) + __shfl_xor_sync(0xffffffffu, up ? b2[0] : b2[1], 1);
         }
-        // lane l is left with sum number l % SUMS = t * CW + c
-        if (lane < SUMS) o_s[lane / CW][warp * CW + lane % CW] = total;
+        o_s[lane / CW][warp * CW + lane % CW] = total;     // lane l is left with sum number l = t * CW + c
         __syncthreads();
         if (norm_col) {
             if (tid < nt) {
@@ -553,6 +547,7 @@ __global__ void __launch_bounds__(WIDE_THREADS) state_scan_wide_kernel(LinearSta
             }
         }
     }
+    pdl_trigger();
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < RC; i++)
@@ -675,6 +670,8 @@ int launch_step(const LinearStateParams& p, cudaStream_t stream) {
     return 0;
 }
 
+// The scans are ordinary launches: as dependents of the gates' kernels their CTAs came up where those had just left room, several on
+// one SM beside empty ones, for the whole of their long run (one prompt of 2048, write gates, 16 heads of 64 x 64: 214 and 263 us).
 template <typename T, int MODE>
 int launch_scan(const LinearStateParams& p, cudaStream_t stream) {
     if (p.max_q_len == 1) return launch_step<T, MODE>(p, stream);   // every sequence brings one token
@@ -682,22 +679,28 @@ int launch_scan(const LinearStateParams& p, cudaStream_t stream) {
     dim3 grid((p.dv + COLS - 1) / COLS + (MODE == 1 ? 1 : 0), p.heads, p.nseq);
     if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("state_scan: grid (%u, %u, %u) exceeds one launch", grid.x, grid.y, grid.z);
     if (p.d == 128 || p.d == 256) {     // heads whose channels fill a warp's 32 slices: shared memory read once
-        if (p.d == 128)
-            launch_pdl(state_scan_wide_kernel<T, 4, MODE>, grid, dim3(WIDE_THREADS), 0, stream, p);
+        // A CTA with an SM to itself: eight warps of two columns (one prompt of 2048, 8 heads of 128 x 256, us: write gates 213 -> 185, a
+        // decay a head with its gates' kernel 257 -> 237, a decay a channel 225 -> 230; of 300 tokens 39.9 -> 32.9, 46 -> 41, 40.3 -> 39.0).
+        // Several an SM, or 256 channels: four warps of four columns (eight prompts of 512, 16 heads of 128 x 128, a decay a channel, 302
+        // where eight warps take 354; one of 2048, 4 heads of 256 x 256, 438 and 641).
+        if (p.d == 256)
+            state_scan_wide_kernel<T, 8, MODE, 4><<<grid, 128, 0, stream>>>(p);
+        else if ((int64_t)grid.x * grid.y * grid.z <= gb_sm_count())
+            state_scan_wide_kernel<T, 4, MODE, 2><<<grid, 256, 0, stream>>>(p);
         else
-            launch_pdl(state_scan_wide_kernel<T, 8, MODE>, grid, dim3(WIDE_THREADS), 0, stream, p);
+            state_scan_wide_kernel<T, 4, MODE, 4><<<grid, 128, 0, stream>>>(p);
         GB_CHECK_LAUNCH("state_scan");
         return 0;
     }
     switch (rc) {
-        case 4: launch_pdl(state_scan_kernel<T, 4, MODE>, grid, dim3(THREADS), 0, stream, p); break;
-        case 8: launch_pdl(state_scan_kernel<T, 8, MODE>, grid, dim3(THREADS), 0, stream, p); break;
-        case 12: launch_pdl(state_scan_kernel<T, 12, MODE>, grid, dim3(THREADS), 0, stream, p); break;
-        case 16: launch_pdl(state_scan_kernel<T, 16, MODE>, grid, dim3(THREADS), 0, stream, p); break;
-        case 20: launch_pdl(state_scan_kernel<T, 20, MODE>, grid, dim3(THREADS), 0, stream, p); break;
-        case 24: launch_pdl(state_scan_kernel<T, 24, MODE>, grid, dim3(THREADS), 0, stream, p); break;
-        case 28: launch_pdl(state_scan_kernel<T, 28, MODE>, grid, dim3(THREADS), 0, stream, p); break;
-        case 32: launch_pdl(state_scan_kernel<T, 32, MODE>, grid, dim3(THREADS), 0, stream, p); break;
+        case 4: state_scan_kernel<T, 4, MODE><<<grid, THREADS, 0, stream>>>(p); break;
+        case 8: state_scan_kernel<T, 8, MODE><<<grid, THREADS, 0, stream>>>(p); break;
+        case 12: state_scan_kernel<T, 12, MODE><<<grid, THREADS, 0, stream>>>(p); break;
+        case 16: state_scan_kernel<T, 16, MODE><<<grid, THREADS, 0, stream>>>(p); break;
+        case 20: state_scan_kernel<T, 20, MODE><<<grid, THREADS, 0, stream>>>(p); break;
+        case 24: state_scan_kernel<T, 24, MODE><<<grid, THREADS, 0, stream>>>(p); break;
+        case 28: state_scan_kernel<T, 28, MODE><<<grid, THREADS, 0, stream>>>(p); break;
+        case 32: state_scan_kernel<T, 32, MODE><<<grid, THREADS, 0, stream>>>(p); break;
         default: GB_REFUSE("state_scan: %d key channels a head; at most 256", p.d);
     }
     GB_CHECK_LAUNCH("state_scan");

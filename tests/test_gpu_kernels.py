@@ -905,7 +905,7 @@ def test_presence_penalty_and_seen_bitmap(ops):
 # that the kernels follow one another as closely as they can, against the whole prompt in one call.  The single-token kernel
 # adds a head's channels in another order: 256 products of one size at most, each sum off by 2^-24 of it, make 1.6e-5.
 @pytest.mark.parametrize("form", ["decay", "lower", "gates"])
-@pytest.mark.parametrize("H,d,dv", [(4, 128, 256), (3, 24, 40), (2, 256, 33)])
+@pytest.mark.parametrize("H,d,dv", [(4, 128, 256), (1, 128, 40), (3, 24, 40), (2, 256, 33)])
 def test_states_token_after_token_with_nothing_in_between(ops, form, H, d, dv):
     lengths, slots, first = [48, 48, 48], [2, 0, 3], 7
     n, rows = len(lengths), sum(lengths)
