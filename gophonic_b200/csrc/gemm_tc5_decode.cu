@@ -35,7 +35,6 @@ __device__ int g_status;
 
 constexpr int BMW = 128, BK = 64, THREADS = 192;
 constexpr int W_BYTES = BMW * BK * 2;
-constexpr int MAX_SPLITS = 8;
 
 // the folded variants' extra operands (all null / 0 for the plain product)
 struct DecodeFold {
@@ -52,10 +51,62 @@ struct DecodeFold {
 };
 constexpr int FOLD_ROWS = GB_FOLD_MAX_ROWS;
 
+// x / (1 + exp(-x)) without overflow on either side, and without a branch: the lanes of a warp hold values of both signs
 __device__ __forceinline__ float silu_f(float x) {
-    if (x >= 0.f) return x / (1.f + expf(-x));
-    float e = expf(x);
-    return x * e / (1.f + e);
+    const float e = expf(-fabsf(x));
+    return (x >= 0.f ? x : x * e) / (1.f + e);
+}
+
+// Four neighbouring elements of a row, of which the first `have` exist (the others read as zero and are not written); `vec`:
+// the row's address allows one access of all four.
+__device__ __forceinline__ float4 load4(const float* p, int have, bool vec) {
+    if (vec && have >= 4) return *reinterpret_cast<const float4*>(p);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (have > 0) v.x = p[0];
+    if (have > 1) v.y = p[1];
+    if (have > 2) v.z = p[2];
+    if (have > 3) v.w = p[3];
+    return v;
+}
+__device__ __forceinline__ void store4(float* p, const float4& v, int have, bool vec) {
+    if (vec && have >= 4) {
+        *reinterpret_cast<float4*>(p) = v;
+        return;
+    }
+    if (have > 0) p[0] = v.x;
+    if (have > 1) p[1] = v.y;
+    if (have > 2) p[2] = v.z;
+    if (have > 3) p[3] = v.w;
+}
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float4& v, int have, bool vec) {
+    if (vec && have >= 4) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+        uint2 u;
+        u.x = *reinterpret_cast<const uint32_t*>(&lo);
+        u.y = *reinterpret_cast<const uint32_t*>(&hi);
+        *reinterpret_cast<uint2*>(p) = u;
+        return;
+    }
+    if (have > 0) p[0] = __float2bfloat16_rn(v.x);
+    if (have > 1) p[1] = __float2bfloat16_rn(v.y);
+    if (have > 2) p[2] = __float2bfloat16_rn(v.z);
+    if (have > 3) p[3] = __float2bfloat16_rn(v.w);
+}
+__device__ __forceinline__ void store2(float* p, float a, float b, bool vec) {
+    if (vec) {
+        *reinterpret_cast<float2*>(p) = make_float2(a, b);
+        return;
+    }
+    p[0] = a;
+    p[1] = b;
+}
+__device__ __forceinline__ void store2(__nv_bfloat16* p, float a, float b, bool vec) {
+    if (vec) {
+        *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b);
+        return;
+    }
+    p[0] = __float2bfloat16_rn(a);
+    p[1] = __float2bfloat16_rn(b);
 }
 
 // value v of (weight row n, batch row b) -> Y, plain or through the SwiGLU epilogue; `other` is the
@@ -69,13 +120,21 @@ __device__ __forceinline__ void store_out(TC* __restrict__ Y, int64_t ldy, int b
     }
 }
 
+// Slices of rows a warp gathers at once, 16 bytes a lane: shared memory for them lies behind the partial tile, and the
+// shallower variants, which are there to fit more CTAs on an SM, hold fewer.
+constexpr int gather_slices(int nb, int stages) { return nb == 64 && stages >= 4 ? 16 : 8; }
+
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
+
 template <typename TC, int NB, int STAGES>  // NB = batch columns of the instruction: 16 to 256; STAGES deep
-__global__ void __launch_bounds__(THREADS) gemm_tc5_decode_kernel(const __grid_constant__ CUtensorMap map_w,
+__global__ void __launch_bounds__(THREADS, NB <= 32 ? 4 : NB == 64 && STAGES >= 4 ? 2 : 3) gemm_tc5_decode_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                  const __grid_constant__ CUtensorMap map_x, TC* __restrict__ Y,
                                                                  int M, int N, int K, int64_t ldy, int splits, int kb_per_split,
-                                                                 int epi, DecodeFold fold) {
+                                                                 int epi, int vec, DecodeFold fold) {
     constexpr int X_BYTES = NB * BK * 2, STAGE_BYTES = W_BYTES + X_BYTES;
     constexpr int TMEM_COLS = NB < 32 ? 32 : NB;
+    constexpr int GATHER = gather_slices(NB, STAGES);
     extern __shared__ unsigned char smem_raw[];
     unsigned char* tiles = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], accum_bar;
@@ -92,6 +151,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc5_decode_kernel(const __grid_c
     const int KT = kb1 > kb0 ? kb1 - kb0 : 0;
 
     if (threadIdx.x == 0) {
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&map_x) : "memory");
         for (int s = 0; s < STAGES; s++) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
@@ -174,10 +234,10 @@ __global__ void __launch_bounds__(THREADS) gemm_tc5_decode_kernel(const __grid_c
         const int quad = warp & 3;
         const int n = n0 + quad * 32 + lane;  // this thread's weight row
         if (fold.stats_in != nullptr) {
-            // The norm factors.  Warp q of the four takes batch rows q, q + 4, ..., eight at a time
-            // so that their loads are in flight together; its lanes add every 32nd partial sum of a
-            // row and a tree adds the lanes: an order that does not depend on the other rows.
-            for (int b0 = quad; b0 < M; b0 += 32) {
+            // The norm factors of the rows this CTA finishes: with several slices of K every splits-th one.  Warp q of the
+            // four takes rows q, q + 4, ... of them, eight at a time so that their loads are in flight together; its lanes
+            // add every 32nd partial sum of a row and a tree adds the lanes: an order that does not depend on the other rows.
+            for (int k0 = quad; split + splits * k0 < M; k0 += 32) {
                 float t[8];
 #pragma unroll
                 for (int u = 0; u < 8; u++) t[u] = 0.f;
@@ -185,13 +245,13 @@ __global__ void __launch_bounds__(THREADS) gemm_tc5_decode_kernel(const __grid_c
                 for (int c = lane; c < fold.stats_count; c += 32) {
 #pragma unroll
                     for (int u = 0; u < 8; u++) {
-                        const int b = b0 + 4 * u;
+                        const int b = split + splits * (k0 + 4 * u);
                         if (b < M) t[u] += fold.stats_in[(int64_t)b * fold.stats_in_stride + c];
                     }
                 }
 #pragma unroll
                 for (int u = 0; u < 8; u++) {
-                    const int b = b0 + 4 * u;
+                    const int b = split + splits * (k0 + 4 * u);
                     const float total = warp_sum(t[u]);
                     if (lane == 0 && b < M) rs_s[b] = 1.0f / sqrtf(total / (float)fold.norm_n + fold.eps);
                 }
@@ -204,9 +264,27 @@ __global__ void __launch_bounds__(THREADS) gemm_tc5_decode_kernel(const __grid_c
             have = false;
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        if (splits > 1) {
+            // partial tile in this CTA's shared memory: part[b][row of the tile]; the operand
+            // stages are free, every product that read them has completed
+            constexpr int CH = NB < 32 ? 16 : 32;
+            float* part = reinterpret_cast<float*>(tiles) + quad * 32 + lane;
+#pragma unroll 1
+            for (int c0 = 0; c0 < M; c0 += CH) {
+                uint32_t r[CH];
+                if (have) {
+                    tmem_ld(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, r);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < CH; i++) r[i] = 0u;
+                }
+#pragma unroll
+                for (int i = 0; i < CH; i++) part[(c0 + i) * BMW] = __uint_as_float(r[i]);
+            }
+        }
 #pragma unroll 1
         for (int c0 = 0; c0 < NB; c0 += 16) {
-            if (c0 >= M) break;
+            if (c0 >= M || splits > 1) break;
             uint32_t r[16];
             if (have) {
                 tmem_ld16(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, r);
@@ -214,7 +292,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc5_decode_kernel(const __grid_c
 #pragma unroll
                 for (int i = 0; i < 16; i++) r[i] = 0u;
             }
-            if (splits == 1 && epi == 2) {
+            if (epi == 2) {
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
                     const int b = c0 + i;
@@ -229,7 +307,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc5_decode_kernel(const __grid_c
                     sq = warp_sum(sq);
                     if (lane == 0 && b < M) sq_part[quad][b] = sq;
                 }
-            } else if (splits == 1) {
+            } else {
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
                     float v = __uint_as_float(r[i]);
@@ -237,12 +315,6 @@ __global__ void __launch_bounds__(THREADS) gemm_tc5_decode_kernel(const __grid_c
                     float other = __shfl_down_sync(0xffffffffu, v, 8);
                     if (c0 + i < M) store_out<TC>(Y, ldy, c0 + i, n, N, v, other, epi);
                 }
-            } else {
-                // partial tile in this CTA's shared memory: part[b][row of the tile]; the operand
-                // stages are free, every product that read them has completed
-                float* part = reinterpret_cast<float*>(tiles);
-#pragma unroll
-                for (int i = 0; i < 16; i++) part[(c0 + i) * BMW + quad * 32 + lane] = __uint_as_float(r[i]);
             }
         }
         if (splits == 1 && epi == 2) {
@@ -253,88 +325,112 @@ __global__ void __launch_bounds__(THREADS) gemm_tc5_decode_kernel(const __grid_c
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
+    if (splits == 1) {
+        __syncthreads();
+        if (warp == 1) {
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+        }
+        return;
+    }
+
+    // All slices of the tile have left their partial tiles: add them.  CTA r of the cluster takes batch rows r, r + slices, ...: a
+    // warp a row, a lane four neighbouring rows of the tile.  What the residual variant reads from global memory is requested
+    // while the cluster gathers.  A warp asks the other CTAs for all slices of as many of its rows as GATHER holds, keeps
+    // what comes in its own shared memory and finishes one row after the other from there: read row by row, the way to
+    // the other CTAs' shared memory was paid for every row, and written out for all rows at once the code was slower than
+    // this loop (12288 x 2048 with SwiGLU, 50 rows in two slices: 7 us for this phase in either form).
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+    const int n = n0 + lane * 4, have = N - n;
+    const int row_step = splits * (THREADS / 32);
+    const int row0 = (int)rank + splits * warp;
+    const int log_splits = 31 - __clz(splits);
+    float4 ahead = make_float4(0.f, 0.f, 0.f, 0.f), next_w = ahead;   // epi 2: what the residual holds for the next row; the next norm's weight
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    if (epi == 2) {
+        if (fold.next_w != nullptr) next_w = load4(fold.next_w + n, have, vec);
+        if (row0 < M) ahead = load4(reinterpret_cast<const float*>(Y) + (int64_t)row0 * ldy + n, have, vec);
+    }
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     if (warp == 1) {
+        // the barrier was also this CTA's: its epilogue warps have read the accumulators
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }
-    if (splits == 1) return;
-
-    // All slices of the tile have left their partial tiles: add them.  CTA r of the cluster takes
-    // batch rows r, r + slices, ...: a warp a row, a lane four neighbouring rows of the tile.  What the
-    // residual variant reads from global memory is requested while the cluster gathers.
-    uint32_t rank;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
-    const int nl = lane * 4;
-    const int row_step = splits * (THREADS / 32);
-    const int row0 = (int)rank + splits * warp;
-    float pre_h[2][4], next_w[4];
-    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-    if (epi == 2) {
+    const uint32_t part_addr = s32(tiles) + (uint32_t)(lane * 16);
+    float4* mine = reinterpret_cast<float4*>(tiles + (size_t)NB * BMW * 4) + warp * GATHER * 32 + lane;
+    const int rows_a_batch = GATHER >> log_splits;
+#pragma unroll 1
+    for (int first = row0; first < M; first += rows_a_batch * row_step) {
+        float4 x[GATHER];
 #pragma unroll
-        for (int e = 0; e < 4; e++) next_w[e] = (fold.next_w != nullptr && n0 + nl + e < N) ? fold.next_w[n0 + nl + e] : 0.f;
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int bj = row0 + j * row_step;
-#pragma unroll
-            for (int e = 0; e < 4; e++)
-                pre_h[j][e] = (bj < M && n0 + nl + e < N) ? reinterpret_cast<const float*>(Y)[(int64_t)bj * ldy + n0 + nl + e] : 0.f;
-        }
-    }
-    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-    const uint32_t part_addr = s32(tiles);
-    int j = 0;
-    for (int bb = row0; bb < M; bb += row_step, j++) {
-        // all slices are asked for before the first is added (single-token steps of 16 sequences took 4 % longer, of 50 1.5 %,
-        // while they were read and added one by one, each waiting for the cluster's
-        // shared memory in turn)
-        float x[MAX_SPLITS][4];
-#pragma unroll
-        for (int sl = 0; sl < MAX_SPLITS; sl++) {
-            if (sl >= splits) break;
+        for (int f = 0; f < GATHER; f++) {
+            const int bb = first + (f >> log_splits) * row_step;
+            if (bb >= M) break;
             uint32_t remote;
-            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(part_addr + (uint32_t)((bb * BMW + nl) * 4)), "r"(sl));
-            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(x[sl][0]), "=f"(x[sl][1]), "=f"(x[sl][2]), "=f"(x[sl][3]) : "r"(remote) : "memory");
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(part_addr + (uint32_t)(bb * BMW * 4)), "r"(f & (splits - 1)));
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(x[f].x), "=f"(x[f].y), "=f"(x[f].z), "=f"(x[f].w) : "r"(remote) : "memory");
         }
-        float v[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int sl = 0; sl < MAX_SPLITS; sl++) {
-            if (sl >= splits) break;
-#pragma unroll
-            for (int e = 0; e < 4; e++) v[e] += x[sl][e];
+        for (int f = 0; f < GATHER; f++) {
+            if (first + (f >> log_splits) * row_step >= M) break;
+            mine[f * 32] = x[f];
         }
-        if (epi == 2) {
-            float* hq = reinterpret_cast<float*>(Y) + (int64_t)bb * ldy + n0 + nl;
-            float sq = 0.f;
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                if (n0 + nl + e < N) {
-                    const float before = j == 0 ? pre_h[0][e] : (j == 1 ? pre_h[1][e] : hq[e]);
-                    const float hn = before + v[e];
-                    hq[e] = hn;
-                    sq += hn * hn;
-                    if (fold.next_w != nullptr) fold.xn_out[(int64_t)bb * fold.ldxn + n0 + nl + e] = __float2bfloat16_rn(hn * next_w[e]);
-                }
+        if (first + rows_a_batch * row_step >= M) {
+            // this warp reads no other CTA's memory any more
+            __syncwarp();
+            asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+        }
+#pragma unroll 1
+        for (int j = 0; j < rows_a_batch; j++) {
+            const int bb = first + j * row_step;
+            if (bb >= M) break;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+            for (int sl = 0; sl < splits; sl++) {
+                const float4 p = mine[((j << log_splits) + sl) * 32];
+                v.x += p.x;
+                v.y += p.y;
+                v.z += p.z;
+                v.w += p.w;
             }
-            // the lanes of the warp hold the whole tile's share of this batch row
-            sq = warp_sum(sq);
-            if (lane == 0) fold.stats_out[(int64_t)bb * fold.stats_out_stride + blockIdx.x] = sq;
-            continue;
-        }
-        if (fold.stats_in != nullptr) {
-            const float rs = rs_s[bb];
-#pragma unroll
-            for (int e = 0; e < 4; e++) v[e] *= rs;
-        }
-        // the up rows of these four gate rows are eight rows on: two lanes on
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            float other = __shfl_down_sync(0xffffffffu, v[e], 2);
-            store_out<TC>(Y, ldy, bb, n0 + nl + e, N, v[e], other, epi);
+            if (epi == 2) {
+                float* hq = reinterpret_cast<float*>(Y) + (int64_t)bb * ldy + n;
+                const float4 h = make_float4(ahead.x + v.x, ahead.y + v.y, ahead.z + v.z, ahead.w + v.w);
+                if (bb + row_step < M) ahead = load4(hq + (int64_t)row_step * ldy, have, vec);
+                store4(hq, h, have, vec);
+                if (fold.next_w != nullptr) store4(fold.xn_out + (int64_t)bb * fold.ldxn + n, make_float4(h.x * next_w.x, h.y * next_w.y, h.z * next_w.z, h.w * next_w.w), have, vec);
+                // columns behind the last are zero.  The lanes of the warp hold the whole tile's share of this batch row
+                float sq = h.x * h.x;
+                sq += h.y * h.y;
+                sq += h.z * h.z;
+                sq += h.w * h.w;
+                sq = warp_sum(sq);
+                if (lane == 0) fold.stats_out[(int64_t)bb * fold.stats_out_stride + blockIdx.x] = sq;
+                continue;
+            }
+            if (fold.stats_in != nullptr) {
+                const float rs = rs_s[bb];
+                v = make_float4(v.x * rs, v.y * rs, v.z * rs, v.w * rs);
+            }
+            if (epi == 0) {
+                store4(Y + (int64_t)bb * ldy + n, v, have, vec);
+            } else {
+                // The up rows of four gate rows are eight rows on: two lanes on.  Each of the two lanes finishes two of the four.
+                const bool is_up = lane & 2;
+                const float give0 = is_up ? v.x : v.z, give1 = is_up ? v.y : v.w;
+                const float got0 = __shfl_xor_sync(0xffffffffu, give0, 2), got1 = __shfl_xor_sync(0xffffffffu, give1, 2);
+                const float z0 = silu_f(is_up ? got0 : v.x) * (is_up ? v.z : got0), z1 = silu_f(is_up ? got1 : v.y) * (is_up ? v.w : got1);
+                const int col = ((n >> 4) << 3) + (n & 7) + (is_up ? 2 : 0);
+                if (n < N) store2(Y + (int64_t)bb * ldy + col, z0, z1, vec);   // N is a multiple of 16
+            }
         }
     }
     // no CTA may leave while another still reads its shared memory
-    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    __syncwarp();
+    if (row0 >= M) asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
@@ -346,7 +442,7 @@ int launch(const void* X, const void* W, void* Y, int M, int N, int K, int64_t l
            const DecodeFold& fold, cudaStream_t stream) {
     constexpr int X_BYTES = NB * BK * 2;
     int smem = STAGES * (W_BYTES + X_BYTES) + 1024;
-    const int part = NB * BMW * 4 + 1024;
+    const int part = (NB + gather_slices(NB, STAGES) * (THREADS / 32)) * BMW * 4 + 1024;
     if (part > smem) smem = part;
     static bool configured = false;
     if (!configured) {
@@ -361,9 +457,11 @@ int launch(const void* X, const void* W, void* Y, int M, int N, int K, int64_t l
     const int KB = ceil_div(K, BK);
     while (splits > 1 && KB < splits) splits >>= 1;
     const int kb_per_split = ceil_div(KB, splits);
+    const uintptr_t rows = (uintptr_t)Y | (uintptr_t)fold.next_w | (uintptr_t)fold.xn_out | ((uintptr_t)(ldy | fold.ldxn) * 4);
+    const int vec = !(rows & 15);   // four neighbouring elements of every row in one access
     if (tiles > MAX_TILES) GB_REFUSE("gemm_tc5_decode: N = %d exceeds %d tiles", N, MAX_TILES);
     cudaError_t e = launch_pdl_cluster(gemm_tc5_decode_kernel<TC, NB, STAGES>, dim3(tiles, splits), dim3(THREADS), (size_t)smem, stream, 1,
-                                       (unsigned)splits, map_w, map_x, (TC*)Y, M, N, K, ldy, splits, kb_per_split, epi, fold);
+                                       (unsigned)splits, map_w, map_x, (TC*)Y, M, N, K, ldy, splits, kb_per_split, epi, vec, fold);
     if (e != cudaSuccess) GB_REFUSE("gemm_tc5_decode: launch failed: %s", cudaGetErrorString(e));
     return 0;
 }
