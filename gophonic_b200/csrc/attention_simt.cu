@@ -10,6 +10,7 @@
 // into steps or on what else is in the batch.
 #include "mma.cuh"
 #include "api.h"
+#include "attention_pieces.cuh"
 
 #include <math.h>
 
@@ -31,7 +32,7 @@ constexpr int SIMT_MAX_DV = 512;   // widest value head
 // others follow from t_lo.
 struct KeyTiles {
     int t_lo, n_first, my_lo, my_hi;
-    __device__ __forceinline__ KeyTiles(const AttnParamsX& p, int past, int q0, int last_q, int split) {
+    __device__ __forceinline__ KeyTiles(const AttnParamsX& p, int past, int q0, int last_q, int split, int pieces) {
         int lo_pos = 0;
         if (p.window > 0) {
             lo_pos = past + q0 - p.window + 1;
@@ -46,7 +47,7 @@ struct KeyTiles {
         n_first = p.window > 0 && p.keep_first > 0 ? (p.keep_first + KT - 1) / KT : 0;
         if (n_first > t_lo) n_first = t_lo;
         const int n_tiles = n_first + ((past + last_q) / KT + 1 - t_lo);
-        const int per = (n_tiles + p.num_splits - 1) / p.num_splits;
+        const int per = (n_tiles + pieces - 1) / pieces;
         my_lo = split * per;
         my_hi = my_lo + per < n_tiles ? my_lo + per : n_tiles;
     }
@@ -74,9 +75,9 @@ __device__ __forceinline__ float weigh(bool valid, float score, float& m, float&
 
 // A finished row: divided by its sum, or as it is into the scratch memory of the splits.
 template <typename T, int NE>
-__device__ __forceinline__ void leave_row(const AttnParamsX& p, int seq, int split, int64_t row, int head, int dv, int lane, float m, float l,
+__device__ __forceinline__ void leave_row(const AttnParamsX& p, int pieces, int seq, int split, int64_t row, int head, int dv, int lane, float m, float l,
                                           const float (&acc)[NE]) {
-    if (p.num_splits == 1) {
+    if (pieces == 1) {
         T* op = (T*)p.out + row * p.out_row_stride + (int64_t)head * dv;
         float lsum = l, keep = 1.f;
         if (p.sink) {
@@ -121,7 +122,11 @@ __global__ void __launch_bounds__(128) attn_simt_kernel(AttnParamsX p) {
     const int hchunks = (G + GC - 1) / GC;
     const int QT = ROWS / GC;
 
-    const int seq = blockIdx.z / p.num_splits, split = blockIdx.z % p.num_splits;
+    // sequences cut by their own lengths leave some CTAs nothing to do: those come last
+    const bool own = p.piece_tiles > 0;
+    const int seq = own ? blockIdx.z % p.nseq : blockIdx.z / p.num_splits, split = own ? blockIdx.z / p.nseq : blockIdx.z % p.num_splits;
+    const int pieces = own ? attn_pieces(attn_decode_span(p, p.seq_kv_len[seq] - 1).n_tiles, p.piece_tiles, p.num_splits) : p.num_splits;
+    if (split >= pieces) return;
     const int kvh = blockIdx.y / hchunks, chunk = blockIdx.y % hchunks;
     // consecutive key heads may read one value head: -1 if every key head has its own
     const int v_heads = p.v_share > 1 ? p.kv_heads / p.v_share : p.kv_heads, vh = p.v_share > 1 ? kvh / p.v_share : -1;
@@ -160,7 +165,7 @@ __global__ void __launch_bounds__(128) attn_simt_kernel(AttnParamsX p) {
 
     const int last_q = (q0 + QT < q_len ? q0 + QT : q_len) - 1;
     const int hi_pos = past + last_q;
-    const KeyTiles tiles(p, past, q0, last_q, split);
+    const KeyTiles tiles(p, past, q0, last_q, split, pieces);
 
     float m[RW], l[RW], acc[RW][NE];
 #pragma unroll
@@ -222,7 +227,7 @@ __global__ void __launch_bounds__(128) attn_simt_kernel(AttnParamsX p) {
 
 #pragma unroll
     for (int rr = 0; rr < RW; rr++)
-        if (row_ok[rr]) leave_row<T>(p, seq, split, q_start + row_q[rr], row_head[rr], dv, lane, m[rr], l[rr], acc[rr]);
+        if (row_ok[rr]) leave_row<T>(p, pieces, seq, split, q_start + row_q[rr], row_head[rr], dv, lane, m[rr], l[rr], acc[rr]);
 }
 
 // The same for float32 rows of 16-byte chunks (the true 32-bit path at the usual head sizes), with the
@@ -251,7 +256,11 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParamsX p, int stages
     const int hchunks = (G + GC - 1) / GC;
     const int QT = ROWS / GC;
 
-    const int seq = blockIdx.z / p.num_splits, split = blockIdx.z % p.num_splits;
+    // sequences cut by their own lengths leave some CTAs nothing to do: those come last
+    const bool own = p.piece_tiles > 0;
+    const int seq = own ? blockIdx.z % p.nseq : blockIdx.z / p.num_splits, split = own ? blockIdx.z / p.nseq : blockIdx.z % p.num_splits;
+    const int pieces = own ? attn_pieces(attn_decode_span(p, p.seq_kv_len[seq] - 1).n_tiles, p.piece_tiles, p.num_splits) : p.num_splits;
+    if (split >= pieces) return;
     const int kvh = blockIdx.y / hchunks, chunk = blockIdx.y % hchunks;
     const int v_heads = p.v_share > 1 ? p.kv_heads / p.v_share : p.kv_heads, vh = p.v_share > 1 ? kvh / p.v_share : -1;
     const int q_len = p.seq_q_len[seq], kv_len = p.seq_kv_len[seq];
@@ -264,7 +273,7 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParamsX p, int stages
 
     const int last_q = (q0 + QT < q_len ? q0 + QT : q_len) - 1;
     const int hi_pos = past + last_q;
-    const KeyTiles tiles(p, past, q0, last_q, split);
+    const KeyTiles tiles(p, past, q0, last_q, split, pieces);
     const int my_lo = tiles.my_lo, my_hi = tiles.my_hi;
 
     // a tile's 32 keys lie in one page (of 64, and tiles begin at multiples of 32); its first key is visible
@@ -386,7 +395,7 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParamsX p, int stages
 
 #pragma unroll
     for (int rr = 0; rr < RW; rr++)
-        if (row_ok[rr]) leave_row<float>(p, seq, split, q_start + row_q[rr], row_head[rr], dv, lane, m[rr], l[rr], acc[rr]);
+        if (row_ok[rr]) leave_row<float>(p, pieces, seq, split, q_start + row_q[rr], row_head[rr], dv, lane, m[rr], l[rr], acc[rr]);
 }
 
 // out[seq, head, :] = sum_s exp(m_s - M) acc_s / sum_s exp(m_s - M) l_s over the key splits.
@@ -394,16 +403,22 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParamsX p, int stages
 // at once and leaves the weights exp(m_s - M) in shared memory (maximum and normaliser by shuffle
 // trees, a fixed order); then thread c adds column c of the splits in split order.
 constexpr int MERGE_MAX_SPLITS = 256;
+constexpr int MERGE_THREADS = 512;
 
 template <typename T>
-__global__ void __launch_bounds__(128) attn_merge_kernel(const float* __restrict__ scratch, T* __restrict__ out, int64_t out_row_stride,
-                                                         const int* __restrict__ seq_q_start, int heads, int d, int num_splits, int sink,
-                                                         const float* __restrict__ sinks) {
+__global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(AttnParamsX p, int d) {
     __shared__ float w_s[MERGE_MAX_SPLITS];
     __shared__ float l_s;
     pdl_trigger();  // the product that follows may start fetching its weights
     const int head = blockIdx.x, seq = blockIdx.y;
-    const float* sp = scratch + ((int64_t)seq * heads + head) * num_splits * (d + 2);
+    const float* sinks = p.sinks;
+    const int sink = p.sink;
+    const float* sp = p.scratch + ((int64_t)seq * p.heads + head) * p.num_splits * (d + 2);
+    int num_splits = p.num_splits;
+    if (p.piece_tiles > 0) {
+        num_splits = attn_pieces(attn_decode_span(p, p.seq_kv_len[seq] - 1).n_tiles, p.piece_tiles, p.num_splits);
+        if (num_splits == 1) return;   // written by the attention kernel itself
+    }
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
         float M = -INFINITY;
@@ -424,7 +439,7 @@ __global__ void __launch_bounds__(128) attn_merge_kernel(const float* __restrict
     }
     __syncthreads();
     const float L = l_s;
-    T* op = out + (int64_t)seq_q_start[seq] * out_row_stride + (int64_t)head * d;
+    T* op = (T*)p.out + (int64_t)p.seq_q_start[seq] * p.out_row_stride + (int64_t)head * d;
     for (int c = threadIdx.x; c < d; c += blockDim.x) {
         float a = 0.f;
         // sixteen loads in flight at a time; the sum itself stays in split order
@@ -439,6 +454,9 @@ __global__ void __launch_bounds__(128) attn_merge_kernel(const float* __restrict
         op[c] = from_f32<T>(a / L);
     }
 }
+
+// a thread a value where there are that many (four rounds of loads one behind the other for heads of 512 took 6 us)
+int merge_threads(int dv) { return dv <= 128 ? 128 : dv < MERGE_THREADS ? (dv + 31) / 32 * 32 : MERGE_THREADS; }
 
 template <typename T, int NE>
 int launch_ne(const AttnParamsX& p, dim3 grid, size_t smem, cudaStream_t stream) {
@@ -522,8 +540,7 @@ int launch(const AttnParamsX& p, cudaStream_t stream) {
     }
     if (rc) return rc;
     if (p.num_splits > 1) {
-        attn_merge_kernel<T><<<dim3(p.heads, p.nseq), 128, 0, stream>>>(p.scratch, (T*)p.out, p.out_row_stride,
-                                                                        p.seq_q_start, p.heads, dv, p.num_splits, p.sink, p.sinks);
+        attn_merge_kernel<T><<<dim3(p.heads, p.nseq), merge_threads(dv), 0, stream>>>(p, dv);
         GB_CHECK_LAUNCH("attention_merge");
     }
     return 0;
@@ -532,14 +549,12 @@ int launch(const AttnParamsX& p, cudaStream_t stream) {
 }  // namespace
 
 // Merge of per-split partial results, shared with the tensor-core single-token kernel.
-int gb_attention_merge_launch(const float* scratch, void* out, int dtype, int64_t out_row_stride, const int* seq_q_start,
-                              int nseq, int heads, int d, int num_splits, int sink, const float* sinks, cudaStream_t stream) {
-    if (num_splits > MERGE_MAX_SPLITS) GB_REFUSE("attention: %d key splits; at most %d", num_splits, MERGE_MAX_SPLITS);
+int gb_attention_merge_launch(const AttnParamsX& p, int dv, int dtype, cudaStream_t stream) {
+    if (p.num_splits > MERGE_MAX_SPLITS) GB_REFUSE("attention: %d key splits; at most %d", p.num_splits, MERGE_MAX_SPLITS);
     if (dtype == GB_F32)
-        attn_merge_kernel<float><<<dim3(heads, nseq), 128, 0, stream>>>(scratch, (float*)out, out_row_stride, seq_q_start, heads, d, num_splits, sink, sinks);
+        attn_merge_kernel<float><<<dim3(p.heads, p.nseq), merge_threads(dv), 0, stream>>>(p, dv);
     else
-        attn_merge_kernel<__nv_bfloat16><<<dim3(heads, nseq), 128, 0, stream>>>(scratch, (__nv_bfloat16*)out, out_row_stride,
-                                                                                seq_q_start, heads, d, num_splits, sink, sinks);
+        attn_merge_kernel<__nv_bfloat16><<<dim3(p.heads, p.nseq), merge_threads(dv), 0, stream>>>(p, dv);
     GB_CHECK_LAUNCH("attention_merge");
     return 0;
 }
@@ -557,6 +572,7 @@ GB_API int gb_attention_simt_x(const AttnParamsX* pp, int dtype, cudaStream_t st
     if (p.num_splits < 1 || p.num_splits > MERGE_MAX_SPLITS) GB_REFUSE("attention: %d key splits; 1 to %d", p.num_splits, MERGE_MAX_SPLITS);
     if (p.num_splits > 1 && p.max_q_len != 1) GB_REFUSE("attention: key splits need single-token rows, got rows of up to %d", p.max_q_len);
     if (p.num_splits > 1 && !p.scratch) GB_REFUSE("attention: %d key splits without scratch memory", p.num_splits);
+    if (p.piece_tiles < 0 || (p.piece_tiles > 0 && (p.num_splits < 2 || p.max_q_len != 1))) GB_REFUSE("attention: pieces of %d pages", p.piece_tiles);
     if (p.window < 0) GB_REFUSE("attention: window %d", p.window);
     if (p.dv < 0 || p.dv > SIMT_MAX_DV || (p.dv == 0 && p.d > SIMT_MAX_DV)) GB_REFUSE("attention_simt: value size %d is outside [1, %d]", p.dv ? p.dv : p.d, SIMT_MAX_DV);
     if (p.chunk < 0) GB_REFUSE("attention: blocks of %d positions", p.chunk);

@@ -70,6 +70,27 @@ def few_splits(units: int, max_kv_len: int, sm_count: int = 148) -> int:
     return s
 
 
+def token_pieces(nseq: int):
+    """(pages a piece, most pieces a sequence) for single tokens whose sequences are cut by their own lengths: short pieces where
+    few sequences have to fill the GPU, longer ones where there are many.  The lines lie at batch sizes that steps are captured
+    at, so that a step of nine and the one of twelve that is replayed for it cut alike."""
+    pages = 1 if nseq <= 2 else 2 if nseq <= 8 else 4
+    return pages, 32 if nseq <= 8 else 16 if nseq <= 32 else 8
+
+
+def key_pieces(part, batch, heads: int, head_dim: int, value_dim: int):
+    """(pieces at most, scratch for their partial results or None, pages a piece or 0) for this step: single tokens in bfloat16
+    are cut sequence by sequence (``token_pieces``), whatever the plan says; what the tensor-core kernel does not take, by
+    the plan."""
+    ops = part.rt.ops
+    if (part.rt.is_fp32 or batch.nseq > ops.PIECES_MAX_SEQS or value_dim != head_dim
+            or not ops.attention_decode_rope_accepts(torch.bfloat16, head_dim, 0, batch.max_q_len)):
+        return part.key_splits(batch) + (0,)
+    pages, most = token_pieces(batch.nseq)
+    floats = ops.attention_scratch_floats(batch.nseq, heads, value_dim, most)
+    return most, batch.workspace(("attention key splits", heads, value_dim, most), floats), pages
+
+
 class Attention(Mixer):
     capturable = True
 
@@ -193,13 +214,13 @@ class Attention(Mixer):
         rope_args = (s.heads, s.kv_heads, s.head_dim, self.q_norm, self.k_norm, self.eps, cos, sin, rot, batch.row_pos,
                      batch.row_seq, batch.seq_slot, cache.block_table, cache.k, cache.v, cache.writable)
         ctx = torch.empty((rows, self.q_dim), dtype=x.dtype, device=x.device)
-        splits, scratch = self.key_splits(batch)
+        splits, scratch, pages = key_pieces(self, batch, s.heads, s.head_dim, s.head_dim)
         attn_args = (cache.k, cache.v, cache.block_table, batch.seq_slot, batch.seq_q_start, batch.seq_q_len, batch.seq_kv_len,
                      batch.nseq, batch.max_q_len, s.heads, s.kv_heads, s.head_dim, float(s.scale), int(s.window), splits, scratch)
         if ops.attention_decode_rope_accepts(x.dtype, s.head_dim, rot, batch.max_q_len):
             # single tokens: the attention kernel norms and rotates its queries and places the token's key and value itself
-            ops.attention_decode_rope(qkv, ctx, rope_args, attn_args)
+            ops.attention_decode_rope(qkv, ctx, rope_args, attn_args, piece_pages=pages)
         else:
             ops.qk_norm_rope_kv_write(qkv, *rope_args)
-            ops.attention(qkv[:, :self.q_dim], ctx, *attn_args)
+            ops.attention(qkv[:, :self.q_dim], ctx, *attn_args, piece_pages=pages)
         return ctx

@@ -5,7 +5,8 @@ import pytest
 import torch
 
 from gophonic_b200.engine.step import build_batch
-from gophonic_b200.parts.attention import Attention, choose_splits, few_splits
+from gophonic_b200.engine.graphs import captured_size
+from gophonic_b200.parts.attention import Attention, choose_splits, few_splits, token_pieces
 from gophonic_b200.parts.gated_attention import GatedAttention
 from gophonic_b200.parts.latent_attention import LatentAttention
 
@@ -66,6 +67,11 @@ def test_a_batch_of_one_size_asks_for_few_captured_steps():
     a = part()
     for n, most in ((1, 16), (2, 14), (4, 8), (8, 4), (12, 3), (16, 2), (24, 2), (32, 1)):
         assert len({a.plan(n, 1, kv, 148) for kv in range(1, 8193, 7)}) <= most
+
+
+def test_a_step_and_the_captured_one_that_is_replayed_for_it_cut_alike():
+    for n in range(1, 129):
+        assert token_pieces(n) == token_pieces(captured_size(n))
 
 
 # ---- latent attention: which sequences of a step go over expanded keys and values -------------------------
