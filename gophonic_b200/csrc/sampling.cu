@@ -567,10 +567,90 @@ __device__ void sort_candidates(const unsigned long long* __restrict__ c, int n,
     __syncthreads();
 }
 
+// The same by buckets, for lists long enough to pay for it: the span from the largest to the smallest order key is cut into
+// BUCKETS equal ones, every entry goes to its bucket and finds its place there by counting the larger entries beside it.  Entries
+// differ (each holds its index), so the result is the one descending order.  False, with cand undefined, where a bucket would
+// hold more than CROWD entries (nearly equal logits): the list is then sorted by exchanges.  The exchanges of 2048 entries
+// are 66 dependent steps, 15 of them with two barriers.
+constexpr int BUCKETS = 2 * ST;
+constexpr int CROWD = 48;
+constexpr int BUCKET_MIN = 256;   // fewer entries: at most 36 steps of few warps
+
+__device__ bool bucket_candidates(const unsigned long long* __restrict__ c, int n, unsigned long long* cand, uint32_t* count) {
+    constexpr int EPT = MAXC / ST;
+    __shared__ uint32_t part[ST / 32], part2[ST / 32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    unsigned long long x[EPT];
+    uint32_t most = 0u, least = 0xFFFFFFFFu;
+#pragma unroll
+    for (int e = 0; e < EPT; e++) {
+        const int i = tid + e * ST;
+        x[e] = i < n ? c[i] : 0ull;
+        if (i < n) {
+            const uint32_t key = (uint32_t)(x[e] >> 32);
+            most = most > key ? most : key;
+            least = least < key ? least : key;
+        }
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    least = __reduce_min_sync(0xffffffffu, least);
+    if (lane == 0) {
+        part[warp] = most;
+        part2[warp] = least;
+    }
+    count[tid] = 0u;
+    count[tid + ST] = 0u;
+    __syncthreads();
+    most = __reduce_max_sync(0xffffffffu, part[lane]);
+    least = __reduce_min_sync(0xffffffffu, part2[lane]);
+    const unsigned long long scale = ((unsigned long long)BUCKETS << 32) / ((unsigned long long)(most - least) + 1ull);
+    uint32_t at[EPT], slot[EPT];
+#pragma unroll
+    for (int e = 0; e < EPT; e++) {
+        at[e] = (uint32_t)(((unsigned long long)(most - (uint32_t)(x[e] >> 32)) * scale) >> 32);
+        if (tid + e * ST < n) slot[e] = atomicAdd(&count[at[e]], 1u);
+    }
+    __syncthreads();
+    // entries ahead of each bucket, two buckets a thread
+    const uint32_t n0 = count[2 * tid], n1 = count[2 * tid + 1];
+    uint32_t inc = n0 + n1;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= d) inc += v;
+    }
+    if (lane == 31) part[warp] = inc;
+    if (__syncthreads_or(n0 > CROWD || n1 > CROWD)) return false;
+    const uint32_t ahead = __reduce_add_sync(0xffffffffu, lane < warp ? part[lane] : 0u) + inc - n0 - n1;
+    count[2 * tid] = ahead;
+    count[2 * tid + 1] = ahead + n0;
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < EPT; e++)
+        if (tid + e * ST < n) cand[count[at[e]] + slot[e]] = x[e];
+    __syncthreads();
+    uint32_t place[EPT];
+#pragma unroll
+    for (int e = 0; e < EPT; e++) {
+        place[e] = 0;
+        if (tid + e * ST >= n) continue;
+        const uint32_t lo = count[at[e]], hi = at[e] + 1 < BUCKETS ? count[at[e] + 1] : (uint32_t)n;
+        place[e] = lo;
+        for (uint32_t j = lo; j < hi; j++) place[e] += cand[j] > x[e] ? 1u : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < EPT; e++)
+        if (tid + e * ST < n) cand[place[e]] = x[e];
+    __syncthreads();
+    return true;
+}
+
 __global__ void __launch_bounds__(ST) sample_final_kernel(SampleParams p, const uint32_t* __restrict__ hist,
                                                           const unsigned long long* __restrict__ cands) {
     __shared__ __align__(16) unsigned long long cand[MAXC];
     __shared__ __align__(16) float acc[MAXK];
+    __shared__ uint32_t count_s[BUCKETS];
     float* prob = (float*)(cand + MAXK);  // behind the k first, which are all that is looked at once they are sorted
     const int r = blockIdx.x, tid = threadIdx.x;
     pdl_wait_cta();
@@ -583,7 +663,9 @@ __global__ void __launch_bounds__(ST) sample_final_kernel(SampleParams p, const 
     }
     const int n = (int)count;
     const unsigned long long* c = cands + (int64_t)r * MAXC;
-    if (n <= ST)
+    if (n >= BUCKET_MIN && bucket_candidates(c, n, cand, count_s)) {
+        // sorted
+    } else if (n <= ST)
         sort_candidates<1>(c, n, cand);
     else if (n <= 2 * ST)
         sort_candidates<2>(c, n, cand);

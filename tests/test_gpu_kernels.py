@@ -916,6 +916,41 @@ def test_sampler_matches_the_plain_sampler(ops, V, wide):
                 assert abs(i - j) == 1, (r, got, tok)
 
 
+@pytest.mark.parametrize("kind", ["normal", "ramp", "cluster", "levels", "few", "spread"])
+def test_wide_rows_are_sorted_as_the_whole_row_is(ops, kind):
+    """The candidates' ways to be sorted, by buckets and, where logits crowd, by exchanges: the tokens that one CTA over the whole row
+    chooses, for lists around the lengths where the ways part."""
+    V, rows = 151936, 24
+    logits = rnd(rows, V, scale=3.0, seed=17)
+    if kind == "ramp":                       # every bucket alike
+        order = torch.randperm(V, generator=torch.Generator().manual_seed(1)).to(DEV)
+        logits = torch.linspace(0.0, 12.0, V, device=DEV)[order].repeat(rows, 1)
+    elif kind == "cluster":                  # from two to hundreds of equal logits among the likeliest
+        for r in range(rows):
+            logits[r, 7:7 + 2 + 20 * r] = 8.25
+    elif kind == "levels":                   # a few values only
+        logits = (logits * 40.0).round().clamp(-500, 330) / 40.0
+    elif kind == "few":                      # lists of 230 to 276 entries
+        logits.clamp_(max=1.0)
+        for r in range(rows):
+            logits[r, 1000:1000 + 230 + 2 * r] = 20.0 + torch.arange(230 + 2 * r, device=DEV) * 0.03125
+    elif kind == "spread":                   # one far ahead of the rest, and infinities
+        logits[:, 5] = 3.0e38
+        logits[::2, 6] = float("inf")
+        logits[:, 9] = -float("inf")
+    mk = lambda x, dt: torch.tensor(x, dtype=dt, device=DEV)
+    scratch = torch.zeros(ops.sample_scratch_bytes(rows, V), dtype=torch.uint8, device=DEV)
+    ks = [(0, 1024, 230, 256, 257, 40)[i % 6] for i in range(rows)]
+    for draw in range(4):
+        outs = []
+        for with_scratch in (scratch, None):
+            out = torch.empty(rows, dtype=torch.int32, device=DEV)
+            ops.sample(logits, mk([1.0] * rows, torch.float32), mk(ks, torch.int32), mk([0.0, 0.95] * (rows // 2), torch.float32),
+                       mk(list(range(rows)), torch.int64), mk([draw] * rows, torch.int64), out, scratch=with_scratch)
+            outs.append(out)
+        assert torch.equal(*outs)
+
+
 def test_sampler_distribution_and_batch_independence(ops):
     V = 300
     base = torch.full((V,), -30.0)
