@@ -322,8 +322,10 @@ struct DecodeItem {
 };
 
 // PIECES: the CTAs, as many as are resident at once, walk the pieces of all sequences, each sequence cut by its own length
-// (attention_pieces.cuh); a piece's first pages and queries are asked for before the piece ahead of it is merged.  Without:
-// one CTA a (split, kv head, sequence), every sequence cut into num_splits.
+// (attention_pieces.cuh).  A piece is short, so what it needs is on its way before the piece ahead has ended: its place is worked out
+// before that one's first page, its pages follow that one's in the ring and its queries take the place of that one's as soon as those
+// are in registers (asked for behind the last page instead, a piece of four pages took 11 us, and 7 of the pages).  Without
+// PIECES: one CTA a (split, kv head, sequence), every sequence cut into num_splits.
 template <int HD, bool QREG, bool PIECES>
 __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, RopeFuse f) {
     constexpr int SD = HD + 8, KS = HD / 16, NF = HD / 8;
@@ -412,13 +414,6 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
         load_page<HD>(st + 64 * SD, vbase + voff, tid, 128);
     };
     auto ring = [](int buf) { return buf >= DSTAGES ? buf - DSTAGES : buf; };
-    auto ask_tiles = [&](const DecodeItem& it, int first) {
-#pragma unroll
-        for (int s = 0; s < DSTAGES - 1; s++) {
-            if (s < it.n) load_tile(it, s, ring(first + s));
-            cp_async_commit();
-        }
-    };
     auto heads_of = [&](const DecodeItem& it) { return (G - it.chunk * GC) < GC ? (G - it.chunk * GC) : GC; };  // heads of this CTA
     auto ask_queries = [&](const DecodeItem& it) {
         constexpr int CH = HD / 8;
@@ -429,7 +424,18 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
             bool ok = row < nh;
             cp_async16(Qs + row * SD + c * 8, ok ? qsrc + (int64_t)row * HD + c * 8 : qsrc, ok ? 16 : 0);
         }
-        cp_async_commit();
+    };
+    // The CTA whose keys end with the token's own page has that key and value from the q/k/v product's
+    // row, not from the cache: the last tile is patched in shared memory, and one CTA per kv head also
+    // stores them in the cache for the steps to come.  A run that only reads another's cache finds the key there.
+    auto owns_last_of = [&](const DecodeItem& it) { return f.on && f.write_kv && it.n > 0 && it.my_lo + it.n == it.span.n_tiles; };
+    auto ask_fresh = [&](const DecodeItem& it) {
+        constexpr int CH = HD / 8;
+        const bf16* row = (const bf16*)p.q + (int64_t)it.q_row * p.q_row_stride;
+        for (int i = tid; i < 2 * CH; i += 128) {
+            const bf16* src = row + (int64_t)(p.heads + (i < CH ? it.kvh : p.kv_heads + it.kvh)) * HD + (i < CH ? i : i - CH) * 8;
+            cp_async16(fresh + i * 8, src, 16);
+        }
     };
 
     int index = PIECES ? blockIdx.x : 0;
@@ -442,31 +448,35 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
     int first = 0;   // buffer of the item's first tile
     // Without `f.on` the keys of this step were written by the kernel just ahead: nothing is fetched early.
     if (!f.on) pdl_wait();
-    ask_tiles(it, first);
+#pragma unroll
+    for (int s = 0; s < DSTAGES - 1; s++)
+        if (s < it.n) load_tile(it, s, s);
     if (f.on) pdl_wait();
     pdl_trigger();  // the product that follows may start fetching its weights
     ask_queries(it);
+    if (owns_last_of(it)) ask_fresh(it);
+    cp_async_commit();
 
     const float sc = p.scale * LOG2E;
     for (;;) {
         const int n = it.n, pos = it.span.pos, nh = heads_of(it);
         const int h0 = it.kvh * G + it.chunk * GC;            // first head of this CTA
-        // The CTA whose keys end with the token's own page has that key and value from the q/k/v product's
-        // row, not from the cache: the last tile is patched in shared memory, and one CTA per kv head also
-        // stores them in the cache for the steps to come.
-        const bool owns_last = f.on && f.write_kv && n > 0 && it.my_lo + n == it.span.n_tiles;  // a run that only reads another's cache finds the key there
+        const bool owns_last = owns_last_of(it);
+        bool more = false;
+        DecodeItem nx;
+        int asked = 0;   // pages of the next piece that are on their way
+        if (PIECES) {
+            index += gridDim.x;
+            more = index < total;
+            if (more) nx = item_of(index);
+            else nx.n = 0;
+        }
         if (f.on && n > 0) {
             const int half = f.rot / 2;
             // rows whose position lies beyond the table are refused on the host
             const int tpos = (half == 0 || gb_check(pos, f.table_positions, GB_CHECK_ROPE_POSITION)) ? pos : 0;
             const float* cs = f.cos_t + (int64_t)tpos * half;
             const float* sn = f.sin_t + (int64_t)tpos * half;
-            const bf16* row = (const bf16*)p.q + (int64_t)it.q_row * p.q_row_stride;
-            if (owns_last) {
-                const bf16* ksrc = row + (int64_t)(p.heads + it.kvh) * HD;
-                const bf16* vsrc = row + (int64_t)(p.heads + p.kv_heads + it.kvh) * HD;
-                for (int i = tid; i < 2 * HD; i += 128) fresh[i] = i < HD ? ksrc[i] : vsrc[i - HD];
-            }
             cp_async_wait<0>();  // the queries have landed (the first tiles were requested before them)
             __syncthreads();
             for (int task = warp; task < nh + (owns_last ? 1 : 0); task += 4) {
@@ -500,13 +510,19 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
 
         int buf = first;   // of tile i
         for (int i = 0; i < n; i++) {
-            // tile i has landed; the queries, requested last, only once every group has (first iteration)
+            // tile i has landed, and with the first one the queries
             if (i == 0)
                 cp_async_wait<0>();
             else
                 cp_async_wait<DSTAGES - 2>();
             __syncthreads();
-            if (i + DSTAGES - 1 < n) load_tile(it, i + DSTAGES - 1, ring(buf + DSTAGES - 1));
+            if (i + DSTAGES - 1 < n) {
+                load_tile(it, i + DSTAGES - 1, ring(buf + DSTAGES - 1));
+            } else if (PIECES) {
+                // the next piece's, in the places behind this piece's last
+                for (; asked < nx.n && asked < i + DSTAGES - n; asked++) load_tile(nx, asked, ring(ring(buf + n - i) + asked));
+            }
+            if (PIECES && QREG && i == 1 && more) ask_queries(nx);   // every warp has this piece's in registers
             cp_async_commit();
             if (QREG && i == 0) {
 #pragma unroll
@@ -594,25 +610,18 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
                 mma_bf16_16816(o[c * 2 + 1], pa[0], pa[1], pa[2], pa[3], b[2], b[3]);
             }
         }
-        cp_async_wait<0>();
+        if (n == 0) cp_async_wait<0>();   // an empty split's queries
         l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
         l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
         l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
         l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
         __syncthreads();  // every warp is done with the tiles: the last one's memory takes the merge
 
-        const DecodeItem done = it;
         const int free_buf = n > 0 ? ring(buf + DSTAGES - 1) : 0;
-        bool more = false;
-        if (PIECES) {
-            index += gridDim.x;
-            more = index < total;
-            if (more) {
-                it = item_of(index);
-                first = buf;
-                ask_tiles(it, first);
-                ask_queries(it);
-            }
+        if (PIECES && more) {
+            if (!QREG || n < 2) ask_queries(nx);
+            if (owns_last_of(nx)) ask_fresh(nx);
+            cp_async_commit();
         }
 
         // merge the four warps: Ms/Ls [4][16], Os [4][16][HD]; rows of the tile that are no head stay out
@@ -638,7 +647,7 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
             float M = fmaxf(fmaxf(Ms[r], Ms[16 + r]), fmaxf(Ms[32 + r], Ms[48 + r]));
             float L = 0.f;
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            const bool sink_here = p.sink && done.pieces == 1;   // with several pieces the merge kernel adds the sink's unit
+            const bool sink_here = p.sink && it.pieces == 1;   // with several pieces the merge kernel adds the sink's unit
             if (sink_here) {
                 const float z = p.sinks ? p.sinks[h0 + r] * LOG2E : 0.f;
                 M = fmaxf(M, z);
@@ -657,12 +666,12 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
                 }
             }
             const int head = h0 + r;
-            if (done.pieces == 1) {
-                uint32_t* op = reinterpret_cast<uint32_t*>((bf16*)p.out + (int64_t)done.q_row * p.out_row_stride + (int64_t)head * HD + c);
+            if (it.pieces == 1) {
+                uint32_t* op = reinterpret_cast<uint32_t*>((bf16*)p.out + (int64_t)it.q_row * p.out_row_stride + (int64_t)head * HD + c);
                 op[0] = pack_bf16(acc.x / L, acc.y / L);
                 op[1] = pack_bf16(acc.z / L, acc.w / L);
             } else {
-                float* sp = p.scratch + (((int64_t)done.seq * p.heads + head) * p.num_splits + done.piece) * (HD + 2);
+                float* sp = p.scratch + (((int64_t)it.seq * p.heads + head) * p.num_splits + it.piece) * (HD + 2);
                 if (c == 0) {
                     sp[0] = M == -INFINITY ? -INFINITY : M * LN2;  // natural-log units, as the merge kernel expects
                     sp[1] = L;
@@ -672,6 +681,8 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
             }
         }
         if (!more) return;
+        it = nx;
+        first = buf;
     }
 }
 

@@ -398,61 +398,65 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParamsX p, int stages
         if (row_ok[rr]) leave_row<float>(p, pieces, seq, split, q_start + row_q[rr], row_head[rr], dv, lane, m[rr], l[rr], acc[rr]);
 }
 
-// out[seq, head, :] = sum_s exp(m_s - M) acc_s / sum_s exp(m_s - M) l_s over the key splits.
-// One CTA of 128 threads per (sequence, head).  The first warp reads every split's maximum and sum
-// at once and leaves the weights exp(m_s - M) in shared memory (maximum and normaliser by shuffle
-// trees, a fixed order); then thread c adds column c of the splits in split order.
+// out[seq, head, :] = sum_s exp(m_s - M) acc_s / sum_s exp(m_s - M) l_s over the key splits, one CTA a (sequence, head) and a
+// thread a value.  Every warp finds the maximum, the normaliser and the weights for itself (a lane a split, shuffle trees, a fixed
+// order); thread c then adds value c of the splits in split order.  A chain of waits for memory and little else, so what it
+// reads is asked for at once: the first splits' values and all maxima while the sequence's length is still on its way, from which
+// the number of its own pieces follows (one behind the other, with the weights through shared memory: 10.7 us for 8
+// sequences of 32 heads in up to 32 pieces, 4.8 for 4 splits).
 constexpr int MERGE_MAX_SPLITS = 256;
 constexpr int MERGE_THREADS = 512;
+constexpr int MERGE_AHEAD = 8;    // splits whose values are asked for ahead
 
 template <typename T>
 __global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(AttnParamsX p, int d) {
-    __shared__ float w_s[MERGE_MAX_SPLITS];
-    __shared__ float l_s;
     pdl_trigger();  // the product that follows may start fetching its weights
-    const int head = blockIdx.x, seq = blockIdx.y;
-    const float* sinks = p.sinks;
-    const int sink = p.sink;
+    const int head = blockIdx.x, seq = blockIdx.y, lane = threadIdx.x & 31, c = threadIdx.x;
     const float* sp = p.scratch + ((int64_t)seq * p.heads + head) * p.num_splits * (d + 2);
-    int num_splits = p.num_splits;
+    const float* column = sp + 2 + (c < d ? c : 0);
+    int n = p.num_splits;
+    float m = lane < n ? sp[(int64_t)lane * (d + 2)] : -INFINITY, l = lane < n ? sp[(int64_t)lane * (d + 2) + 1] : 0.f;
+    float v[MERGE_AHEAD];
+#pragma unroll
+    for (int j = 0; j < MERGE_AHEAD; j++) v[j] = j < n ? column[(int64_t)j * (d + 2)] : 0.f;
     if (p.piece_tiles > 0) {
-        num_splits = attn_pieces(attn_decode_span(p, p.seq_kv_len[seq] - 1).n_tiles, p.piece_tiles, p.num_splits);
-        if (num_splits == 1) return;   // written by the attention kernel itself
+        n = attn_pieces(attn_decode_span(p, p.seq_kv_len[seq] - 1).n_tiles, p.piece_tiles, p.num_splits);
+        if (n == 1) return;   // written by the attention kernel itself
+        if (lane >= n) m = -INFINITY;
     }
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        float M = -INFINITY;
-        for (int s = lane; s < num_splits; s += 32) M = fmaxf(M, sp[(int64_t)s * (d + 2)]);
-        M = warp_max(M);
-        const float z = sinks ? sinks[head] : 0.f;  // the sink's score
-        if (sink) M = fmaxf(M, z);
-        float L = 0.f;
-        for (int s = lane; s < num_splits; s += 32) {
-            const float ms = sp[(int64_t)s * (d + 2)];
-            const float w = ms != -INFINITY ? expf(ms - M) : 0.f;
-            w_s[s] = w;
-            L += w * sp[(int64_t)s * (d + 2) + 1];
+    float M = m;
+    for (int s = lane + 32; s < n; s += 32) M = fmaxf(M, sp[(int64_t)s * (d + 2)]);
+    M = warp_max(M);
+    const float z = p.sinks ? p.sinks[head] : 0.f;  // the sink's score
+    if (p.sink) M = fmaxf(M, z);
+    const float w0 = m != -INFINITY ? expf(m - M) : 0.f;
+    float L = lane < n ? w0 * l : 0.f;
+    for (int s = lane + 32; s < n; s += 32) {
+        const float ms = sp[(int64_t)s * (d + 2)];
+        L += (ms != -INFINITY ? expf(ms - M) : 0.f) * sp[(int64_t)s * (d + 2) + 1];
+    }
+    L = warp_sum(L);
+    if (p.sink) L += expf(z - M);
+    float a = 0.f;
+    for (int s0 = 0; s0 < n; s0 += 32) {
+        float w = w0;
+        if (s0 > 0) {
+            const float ms = s0 + lane < n ? sp[(int64_t)(s0 + lane) * (d + 2)] : -INFINITY;
+            w = ms != -INFINITY ? expf(ms - M) : 0.f;
         }
-        L = warp_sum(L);
-        if (sink) L += expf(z - M);
-        if (lane == 0) l_s = L;
-    }
-    __syncthreads();
-    const float L = l_s;
-    T* op = (T*)p.out + (int64_t)p.seq_q_start[seq] * p.out_row_stride + (int64_t)head * d;
-    for (int c = threadIdx.x; c < d; c += blockDim.x) {
-        float a = 0.f;
-        // sixteen loads in flight at a time; the sum itself stays in split order
-        for (int s0 = 0; s0 < num_splits; s0 += 16) {
-            float v[16];
+        for (int s1 = s0; s1 < n && s1 < s0 + 32; s1 += MERGE_AHEAD) {
+            if (s1 > 0) {
 #pragma unroll
-            for (int j = 0; j < 16; j++) v[j] = s0 + j < num_splits ? sp[(int64_t)(s0 + j) * (d + 2) + 2 + c] : 0.f;
+                for (int j = 0; j < MERGE_AHEAD; j++) v[j] = s1 + j < n ? column[(int64_t)(s1 + j) * (d + 2)] : 0.f;
+            }
 #pragma unroll
-            for (int j = 0; j < 16; j++)
-                if (s0 + j < num_splits) a += w_s[s0 + j] * v[j];
+            for (int j = 0; j < MERGE_AHEAD; j++) {
+                const float wj = __shfl_sync(0xffffffffu, w, s1 - s0 + j);
+                if (s1 + j < n) a += wj * v[j];
+            }
         }
-        op[c] = from_f32<T>(a / L);
     }
+    if (c < d) ((T*)p.out)[(int64_t)p.seq_q_start[seq] * p.out_row_stride + (int64_t)head * d + c] = from_f32<T>(a / L);
 }
 
 // a thread a value where there are that many (four rounds of loads one behind the other for heads of 512 took 6 us)

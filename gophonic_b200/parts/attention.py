@@ -74,7 +74,7 @@ def token_pieces(nseq: int):
     """(pages a piece, most pieces a sequence) for single tokens whose sequences are cut by their own lengths: short pieces where
     few sequences have to fill the GPU, longer ones where there are many.  The lines lie at batch sizes that steps are captured
     at, so that a step of nine and the one of twelve that is replayed for it cut alike."""
-    pages = 1 if nseq <= 2 else 2 if nseq <= 8 else 4
+    pages = 1 if nseq <= 2 else 2 if nseq <= 4 else 4
     return pages, 32 if nseq <= 8 else 16 if nseq <= 32 else 8
 
 
