@@ -314,19 +314,7 @@ __device__ __forceinline__ void norm_rope_row(bf16* x, float* y, const float* __
     __syncwarp();
 }
 
-// One piece of a sequence's keys for the heads of one CTA.
-struct DecodeItem {
-    int seq, piece, pieces, kvh, chunk, q_row, my_lo, n;   // pieces of this sequence; tiles [my_lo, my_lo + n) of its list
-    DecodeSpan span;
-    const int* bt;
-};
-
-// PIECES: the CTAs, as many as are resident at once, walk the pieces of all sequences, each sequence cut by its own length
-// (attention_pieces.cuh).  A piece is short, so what it needs is on its way before the piece ahead has ended: its place is worked out
-// before that one's first page, its pages follow that one's in the ring and its queries take the place of that one's as soon as those
-// are in registers (asked for behind the last page instead, a piece of four pages took 11 us, and 7 of the pages).  Without
-// PIECES: one CTA a (split, kv head, sequence), every sequence cut into num_splits.
-template <int HD, bool QREG, bool PIECES>
+template <int HD, bool QREG>
 __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, RopeFuse f) {
     constexpr int SD = HD + 8, KS = HD / 16, NF = HD / 8;
     constexpr int STAGE = 2 * 64 * SD;  // elements: keys then values
@@ -335,7 +323,6 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
     bf16* KV = Qs + 16 * SD;                          // [DSTAGES][2][64][SD]
     float* Ys = reinterpret_cast<float*>(KV + DSTAGES * STAGE);  // [4 warps][HD]: scratch of norm_rope_row
     bf16* fresh = reinterpret_cast<bf16*>(Ys + 4 * HD);          // [2][HD]: the token's own key and value
-    __shared__ int behind_s[PIECES ? PIECES_MAX_SEQS + 1 : 1];   // pieces of the sequences ahead of each
 
     // Ahead of the dependency wait: the step's metadata and the pages of earlier steps, none of which
     // the kernel before this one writes (the step's metadata is uploaded before its first kernel,
@@ -345,344 +332,262 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
     const int G = p.heads / p.kv_heads;
     const int GC = G < 16 ? G : 16;
     const int hchunks = (G + GC - 1) / GC;
-    const int head_ctas = p.kv_heads * hchunks;
+    // Cut by their own lengths, most sequences have fewer pieces than the longest: a CTA without one leaves at once, and those come
+    // last (the pieces are the slowest dimension of the grid there).
+    const bool own = p.piece_tiles > 0;
+    const int split = own ? blockIdx.z : blockIdx.x, seq = own ? blockIdx.y : blockIdx.z;
+    const int head_cta = own ? blockIdx.x : blockIdx.y;
+    const int kvh = head_cta / hchunks, chunk = head_cta % hchunks;
+    const int kv_len = p.seq_kv_len[seq];
+    const int q_row = p.seq_q_start[seq];
+    const int pos = kv_len - 1;
+    const int* bt = block_table_row(p.block_table, p.bt_stride, p.seq_slot[seq], p.max_slots);
     const bf16* kbase = (const bf16*)p.k_plane;
     const bf16* vbase = (const bf16*)p.v_plane;
+    const int h0 = kvh * G + chunk * GC;            // first head of this CTA
+    const int nh = (G - chunk * GC) < GC ? (G - chunk * GC) : GC;  // heads of this CTA
+    const DecodeSpan span = attn_decode_span(p, pos);
+    const int n_tiles = span.n_tiles;
+    const int pieces = own ? attn_pieces(n_tiles, p.piece_tiles, p.num_splits) : p.num_splits;
+    if (split >= pieces) return;   // an ordinary launch: nothing waits for this CTA's own wait
+    const int per = (n_tiles + pieces - 1) / pieces;
+    const int my_lo = split * per;
+    const int my_hi = my_lo + per < n_tiles ? my_lo + per : n_tiles;
+    const int n = my_hi > my_lo ? my_hi - my_lo : 0;
 
-    int total = 1;
-    if (PIECES) {
-        int mine = 0;
-        if (tid < p.nseq) mine = attn_pieces(attn_decode_span(p, p.seq_kv_len[tid] - 1).n_tiles, p.piece_tiles, p.num_splits);
-        int upto = mine;   // of this warp's sequences up to this one
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, upto, o);
-            if (lane >= o) upto += v;
-        }
-        if (lane == 31) Ys[warp] = __int_as_float(upto);
-        __syncthreads();
-        int ahead = 0;
-#pragma unroll
-        for (int w = 0; w < 4; w++) {
-            const int v = __float_as_int(Ys[w]);
-            if (w < warp) ahead += v;
-        }
-        if (tid < p.nseq) behind_s[tid + 1] = ahead + upto;
-        if (tid == 0) behind_s[0] = 0;
-        __syncthreads();
-        total = behind_s[p.nseq] * head_ctas;
-    }
-    auto item_of = [&](int index) {
-        DecodeItem it;
-        int y;
-        if (PIECES) {
-            const int at = index / head_ctas;   // neighbouring CTAs take the heads of one piece: their pages lie together
-            y = index - at * head_ctas;
-            int lo = 0, hi = p.nseq;            // the sequence whose pieces hold this one
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (behind_s[mid] <= at) lo = mid;
-                else hi = mid;
-            }
-            it.seq = lo;
-            it.piece = at - behind_s[lo];
-            it.pieces = behind_s[lo + 1] - behind_s[lo];
-        } else {
-            y = blockIdx.y;
-            it.seq = blockIdx.z;
-            it.piece = blockIdx.x;
-            it.pieces = p.num_splits;
-        }
-        it.kvh = y / hchunks;
-        it.chunk = y - it.kvh * hchunks;
-        it.q_row = p.seq_q_start[it.seq];
-        it.span = attn_decode_span(p, p.seq_kv_len[it.seq] - 1);
-        it.bt = block_table_row(p.block_table, p.bt_stride, p.seq_slot[it.seq], p.max_slots);
-        const int per = (it.span.n_tiles + it.pieces - 1) / it.pieces;
-        it.my_lo = it.piece * per;
-        const int my_hi = it.my_lo + per < it.span.n_tiles ? it.my_lo + per : it.span.n_tiles;
-        it.n = my_hi > it.my_lo ? my_hi - it.my_lo : 0;
-        return it;
-    };
-    auto load_tile = [&](const DecodeItem& it, int i, int buf) {
-        const int t = it.span.tile_of(it.my_lo + i);
-        int64_t page = page_of(it.bt, t * 64, p.bt_stride, p.pages);
-        int64_t off = ((page * p.kv_heads + it.kvh) * 64) * (int64_t)HD;
-        int64_t voff = p.v_share > 1 ? ((page * (p.kv_heads / p.v_share) + it.kvh / p.v_share) * 64) * (int64_t)HD : off;
-        bf16* st = KV + buf * STAGE;
+    auto load_tile = [&](int i) {
+        int t = span.tile_of(my_lo + i);
+        int64_t page = page_of(bt, t * 64, p.bt_stride, p.pages);
+        int64_t off = ((page * p.kv_heads + kvh) * 64) * (int64_t)HD;
+        int64_t voff = p.v_share > 1 ? ((page * (p.kv_heads / p.v_share) + kvh / p.v_share) * 64) * (int64_t)HD : off;
+        bf16* st = KV + (i % DSTAGES) * STAGE;
         load_page<HD>(st, kbase + off, tid, 128);
         load_page<HD>(st + 64 * SD, vbase + voff, tid, 128);
     };
-    auto ring = [](int buf) { return buf >= DSTAGES ? buf - DSTAGES : buf; };
-    auto heads_of = [&](const DecodeItem& it) { return (G - it.chunk * GC) < GC ? (G - it.chunk * GC) : GC; };  // heads of this CTA
-    auto ask_queries = [&](const DecodeItem& it) {
+    // Without `f.on` the keys of this step were written by the kernel just ahead: nothing is fetched early.
+    if (!f.on) pdl_wait();
+#pragma unroll
+    for (int s = 0; s < DSTAGES - 1; s++) {
+        if (s < n) load_tile(s);
+        cp_async_commit();
+    }
+    if (f.on) pdl_wait();
+    pdl_trigger();  // the product that follows may start fetching its weights
+    {
         constexpr int CH = HD / 8;
-        const int h0 = it.kvh * G + it.chunk * GC, nh = heads_of(it);
-        const bf16* qsrc = (const bf16*)p.q + (int64_t)it.q_row * p.q_row_stride + (int64_t)h0 * HD;
+        const bf16* qsrc = (const bf16*)p.q + (int64_t)q_row * p.q_row_stride + (int64_t)h0 * HD;
         for (int idx = tid; idx < 16 * CH; idx += 128) {
             int row = idx / CH, c = idx - row * CH;
             bool ok = row < nh;
             cp_async16(Qs + row * SD + c * 8, ok ? qsrc + (int64_t)row * HD + c * 8 : qsrc, ok ? 16 : 0);
         }
-    };
+        cp_async_commit();
+    }
+
     // The CTA whose keys end with the token's own page has that key and value from the q/k/v product's
     // row, not from the cache: the last tile is patched in shared memory, and one CTA per kv head also
-    // stores them in the cache for the steps to come.  A run that only reads another's cache finds the key there.
-    auto owns_last_of = [&](const DecodeItem& it) { return f.on && f.write_kv && it.n > 0 && it.my_lo + it.n == it.span.n_tiles; };
-    auto ask_fresh = [&](const DecodeItem& it) {
-        constexpr int CH = HD / 8;
-        const bf16* row = (const bf16*)p.q + (int64_t)it.q_row * p.q_row_stride;
-        for (int i = tid; i < 2 * CH; i += 128) {
-            const bf16* src = row + (int64_t)(p.heads + (i < CH ? it.kvh : p.kv_heads + it.kvh)) * HD + (i < CH ? i : i - CH) * 8;
-            cp_async16(fresh + i * 8, src, 16);
+    // stores them in the cache for the steps to come.
+    const bool owns_last = f.on && f.write_kv && n > 0 && my_hi == n_tiles;  // a run that only reads another's cache finds the key there
+    if (f.on && n > 0) {
+        const int half = f.rot / 2;
+        // rows whose position lies beyond the table are refused on the host
+        const int tpos = (half == 0 || gb_check(pos, f.table_positions, GB_CHECK_ROPE_POSITION)) ? pos : 0;
+        const float* cs = f.cos_t + (int64_t)tpos * half;
+        const float* sn = f.sin_t + (int64_t)tpos * half;
+        const bf16* row = (const bf16*)p.q + (int64_t)q_row * p.q_row_stride;
+        if (owns_last) {
+            const bf16* ksrc = row + (int64_t)(p.heads + kvh) * HD;
+            const bf16* vsrc = row + (int64_t)(p.heads + p.kv_heads + kvh) * HD;
+            for (int i = tid; i < 2 * HD; i += 128) fresh[i] = i < HD ? ksrc[i] : vsrc[i - HD];
         }
-    };
-
-    int index = PIECES ? blockIdx.x : 0;
-    if (PIECES && index >= total) {
-        pdl_wait();
-        pdl_trigger();
-        return;
-    }
-    DecodeItem it = item_of(index);
-    int first = 0;   // buffer of the item's first tile
-    // Without `f.on` the keys of this step were written by the kernel just ahead: nothing is fetched early.
-    if (!f.on) pdl_wait();
-#pragma unroll
-    for (int s = 0; s < DSTAGES - 1; s++)
-        if (s < it.n) load_tile(it, s, s);
-    if (f.on) pdl_wait();
-    pdl_trigger();  // the product that follows may start fetching its weights
-    ask_queries(it);
-    if (owns_last_of(it)) ask_fresh(it);
-    cp_async_commit();
-
-    const float sc = p.scale * LOG2E;
-    for (;;) {
-        const int n = it.n, pos = it.span.pos, nh = heads_of(it);
-        const int h0 = it.kvh * G + it.chunk * GC;            // first head of this CTA
-        const bool owns_last = owns_last_of(it);
-        bool more = false;
-        DecodeItem nx;
-        int asked = 0;   // pages of the next piece that are on their way
-        if (PIECES) {
-            index += gridDim.x;
-            more = index < total;
-            if (more) nx = item_of(index);
-            else nx.n = 0;
-        }
-        if (f.on && n > 0) {
-            const int half = f.rot / 2;
-            // rows whose position lies beyond the table are refused on the host
-            const int tpos = (half == 0 || gb_check(pos, f.table_positions, GB_CHECK_ROPE_POSITION)) ? pos : 0;
-            const float* cs = f.cos_t + (int64_t)tpos * half;
-            const float* sn = f.sin_t + (int64_t)tpos * half;
-            cp_async_wait<0>();  // the queries have landed (the first tiles were requested before them)
-            __syncthreads();
-            for (int task = warp; task < nh + (owns_last ? 1 : 0); task += 4) {
-                if (task < nh)
-                    norm_rope_row<HD>(Qs + task * SD, Ys + warp * HD, f.q_w, f.eps, cs, sn, f.rot, lane, f.consecutive != 0);
-                else
-                    norm_rope_row<HD>(fresh, Ys + warp * HD, f.k_w, f.eps, cs, sn, f.rot, lane, f.consecutive != 0);
-            }
-            __syncthreads();
-            if (owns_last && it.chunk == 0) {
-                const int64_t page = page_of(it.bt, pos, p.bt_stride, p.pages);
-                const int64_t at = ((page * p.kv_heads + it.kvh) * 64 + (pos & 63)) * (int64_t)HD;
-                bf16* kdst = (bf16*)p.k_plane + at;
-                bf16* vdst = (bf16*)p.v_plane + at;
-                for (int i = tid; i < 2 * HD; i += 128) {
-                    if (i < HD)
-                        kdst[i] = fresh[i];
-                    else
-                        vdst[i - HD] = fresh[i];
-                }
-            }
-        }
-
-        float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-        float o[NF][4];
-#pragma unroll
-        for (int j = 0; j < NF; j++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) o[j][e] = 0.f;
-        uint32_t qf[QREG ? KS : 1][4];
-
-        int buf = first;   // of tile i
-        for (int i = 0; i < n; i++) {
-            // tile i has landed, and with the first one the queries
-            if (i == 0)
-                cp_async_wait<0>();
+        cp_async_wait<0>();  // the queries have landed (the first tiles were requested before them)
+        __syncthreads();
+        for (int task = warp; task < nh + (owns_last ? 1 : 0); task += 4) {
+            if (task < nh)
+                norm_rope_row<HD>(Qs + task * SD, Ys + warp * HD, f.q_w, f.eps, cs, sn, f.rot, lane, f.consecutive != 0);
             else
-                cp_async_wait<DSTAGES - 2>();
-            __syncthreads();
-            if (i + DSTAGES - 1 < n) {
-                load_tile(it, i + DSTAGES - 1, ring(buf + DSTAGES - 1));
-            } else if (PIECES) {
-                // the next piece's, in the places behind this piece's last
-                for (; asked < nx.n && asked < i + DSTAGES - n; asked++) load_tile(nx, asked, ring(ring(buf + n - i) + asked));
-            }
-            if (PIECES && QREG && i == 1 && more) ask_queries(nx);   // every warp has this piece's in registers
-            cp_async_commit();
-            if (QREG && i == 0) {
-#pragma unroll
-                for (int ks = 0; ks < KS; ks++)
-                    ldmatrix_x4(qf[QREG ? ks : 0], Qs + ((lane & 7) + ((lane >> 3) & 1) * 8) * SD + ks * 16 + (lane >> 4) * 8);
-            }
-            if (owns_last && i == n - 1) {
-                // the token's own key and value over whatever the cache held at its place
-                bf16* krow = KV + buf * STAGE + (pos & 63) * SD;
-                for (int idx = tid; idx < 2 * HD; idx += 128) {
-                    if (idx < HD)
-                        krow[idx] = fresh[idx];
-                    else
-                        krow[64 * SD + idx - HD] = fresh[idx];
-                }
-                __syncthreads();
-            }
-            const bf16* kt = KV + buf * STAGE;
-            const bf16* vt = kt + 64 * SD;
-            const int t = it.span.tile_of(it.my_lo + i);
-            buf = ring(buf + 1);
-            float s[2][4];
-#pragma unroll
-            for (int j = 0; j < 2; j++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) s[j][e] = 0.f;
-#pragma unroll
-            for (int ks = 0; ks < KS; ks++) {
-                uint32_t a[4], b[4];
-                if (QREG) {
-#pragma unroll
-                    for (int e = 0; e < 4; e++) a[e] = qf[QREG ? ks : 0][e];
-                } else {
-                    ldmatrix_x4(a, Qs + ((lane & 7) + ((lane >> 3) & 1) * 8) * SD + ks * 16 + (lane >> 4) * 8);
-                }
-                ldmatrix_x4(b, kt + (warp * 16 + (lane & 7) + (lane >> 4) * 8) * SD + ks * 16 + ((lane >> 3) & 1) * 8);
-                mma_bf16_16816(s[0], a[0], a[1], a[2], a[3], b[0], b[1]);
-                mma_bf16_16816(s[1], a[0], a[1], a[2], a[3], b[2], b[3]);
-            }
-            float mx0 = m0, mx1 = m1;
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    int key = t * 64 + warp * 16 + j * 8 + t4 * 2 + (e & 1);
-                    bool ok = key <= pos && (key >= it.span.lo_pos || key < p.keep_first);
-                    float v = ok ? s[j][e] * sc : -INFINITY;
-                    s[j][e] = v;
-                    if (e & 2) mx1 = fmaxf(mx1, v); else mx0 = fmaxf(mx0, v);
-                }
-            }
-            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-            const float base0 = mx0 == -INFINITY ? 0.f : mx0, base1 = mx1 == -INFINITY ? 0.f : mx1;
-            const float c0 = exp2f(m0 - base0), c1 = exp2f(m1 - base1);
-            m0 = mx0;
-            m1 = mx1;
-            l0 *= c0;
-            l1 *= c1;
-#pragma unroll
-            for (int j = 0; j < NF; j++) {
-                o[j][0] *= c0;
-                o[j][1] *= c0;
-                o[j][2] *= c1;
-                o[j][3] *= c1;
-            }
-            uint32_t pa[4];
-            {
-                float p00 = exp2f(s[0][0] - base0), p01 = exp2f(s[0][1] - base0), p02 = exp2f(s[0][2] - base1), p03 = exp2f(s[0][3] - base1);
-                float p10 = exp2f(s[1][0] - base0), p11 = exp2f(s[1][1] - base0), p12 = exp2f(s[1][2] - base1), p13 = exp2f(s[1][3] - base1);
-                l0 += p00 + p01 + p10 + p11;
-                l1 += p02 + p03 + p12 + p13;
-                pa[0] = pack_bf16(p00, p01);
-                pa[1] = pack_bf16(p02, p03);
-                pa[2] = pack_bf16(p10, p11);
-                pa[3] = pack_bf16(p12, p13);
-            }
-#pragma unroll
-            for (int c = 0; c < KS; c++) {
-                uint32_t b[4];
-                ldmatrix_x4_trans(b, vt + (warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * SD + c * 16 + (lane >> 4) * 8);
-                mma_bf16_16816(o[c * 2], pa[0], pa[1], pa[2], pa[3], b[0], b[1]);
-                mma_bf16_16816(o[c * 2 + 1], pa[0], pa[1], pa[2], pa[3], b[2], b[3]);
-            }
-        }
-        if (n == 0) cp_async_wait<0>();   // an empty split's queries
-        l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-        l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-        l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-        l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-        __syncthreads();  // every warp is done with the tiles: the last one's memory takes the merge
-
-        const int free_buf = n > 0 ? ring(buf + DSTAGES - 1) : 0;
-        if (PIECES && more) {
-            if (!QREG || n < 2) ask_queries(nx);
-            if (owns_last_of(nx)) ask_fresh(nx);
-            cp_async_commit();
-        }
-
-        // merge the four warps: Ms/Ls [4][16], Os [4][16][HD]; rows of the tile that are no head stay out
-        float* Ms = reinterpret_cast<float*>(KV + free_buf * STAGE);
-        float* Ls = Ms + 64;
-        float* Os = Ls + 64;
-        if (t4 == 0) {
-            Ms[warp * 16 + g] = m0;
-            Ms[warp * 16 + g + 8] = m1;
-            Ls[warp * 16 + g] = l0;
-            Ls[warp * 16 + g + 8] = l1;
-        }
-#pragma unroll
-        for (int j = 0; j < NF; j++) {
-            float* o0 = Os + ((size_t)warp * 16 + g) * HD + j * 8 + t4 * 2;
-            float* o1 = Os + ((size_t)warp * 16 + g + 8) * HD + j * 8 + t4 * 2;
-            if (g < nh) *reinterpret_cast<float2*>(o0) = make_float2(o[j][0], o[j][1]);
-            if (g + 8 < nh) *reinterpret_cast<float2*>(o1) = make_float2(o[j][2], o[j][3]);
+                norm_rope_row<HD>(fresh, Ys + warp * HD, f.k_w, f.eps, cs, sn, f.rot, lane, f.consecutive != 0);
         }
         __syncthreads();
-        for (int idx = tid; idx < nh * HD / 4; idx += 128) {
-            const int r = idx / (HD / 4), c = (idx - r * (HD / 4)) * 4;
-            float M = fmaxf(fmaxf(Ms[r], Ms[16 + r]), fmaxf(Ms[32 + r], Ms[48 + r]));
-            float L = 0.f;
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            const bool sink_here = p.sink && it.pieces == 1;   // with several pieces the merge kernel adds the sink's unit
-            if (sink_here) {
-                const float z = p.sinks ? p.sinks[h0 + r] * LOG2E : 0.f;
-                M = fmaxf(M, z);
-                L = exp2f(z - M);
-            }
-            if (M != -INFINITY) {
-#pragma unroll
-                for (int w = 0; w < 4; w++) {
-                    const float e = exp2f(Ms[w * 16 + r] - M);
-                    const float4 x = *reinterpret_cast<const float4*>(Os + ((size_t)w * 16 + r) * HD + c);
-                    L += e * Ls[w * 16 + r];
-                    acc.x += e * x.x;
-                    acc.y += e * x.y;
-                    acc.z += e * x.z;
-                    acc.w += e * x.w;
-                }
-            }
-            const int head = h0 + r;
-            if (it.pieces == 1) {
-                uint32_t* op = reinterpret_cast<uint32_t*>((bf16*)p.out + (int64_t)it.q_row * p.out_row_stride + (int64_t)head * HD + c);
-                op[0] = pack_bf16(acc.x / L, acc.y / L);
-                op[1] = pack_bf16(acc.z / L, acc.w / L);
-            } else {
-                float* sp = p.scratch + (((int64_t)it.seq * p.heads + head) * p.num_splits + it.piece) * (HD + 2);
-                if (c == 0) {
-                    sp[0] = M == -INFINITY ? -INFINITY : M * LN2;  // natural-log units, as the merge kernel expects
-                    sp[1] = L;
-                }
-                reinterpret_cast<float2*>(sp + 2 + c)[0] = make_float2(acc.x, acc.y);
-                reinterpret_cast<float2*>(sp + 2 + c)[1] = make_float2(acc.z, acc.w);
+        if (owns_last && chunk == 0) {
+            const int64_t page = page_of(bt, pos, p.bt_stride, p.pages);
+            const int64_t at = ((page * p.kv_heads + kvh) * 64 + (pos & 63)) * (int64_t)HD;
+            bf16* kdst = (bf16*)p.k_plane + at;
+            bf16* vdst = (bf16*)p.v_plane + at;
+            for (int i = tid; i < 2 * HD; i += 128) {
+                if (i < HD)
+                    kdst[i] = fresh[i];
+                else
+                    vdst[i - HD] = fresh[i];
             }
         }
-        if (!more) return;
-        it = nx;
-        first = buf;
+    }
+
+    const float sc = p.scale * LOG2E;
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+    float o[NF][4];
+#pragma unroll
+    for (int j = 0; j < NF; j++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) o[j][e] = 0.f;
+    uint32_t qf[QREG ? KS : 1][4];
+
+    for (int i = 0; i < n; i++) {
+        // tile i has landed; the queries, requested last, only once every group has (first iteration)
+        if (i == 0)
+            cp_async_wait<0>();
+        else
+            cp_async_wait<DSTAGES - 2>();
+        __syncthreads();
+        if (i + DSTAGES - 1 < n) load_tile(i + DSTAGES - 1);
+        cp_async_commit();
+        if (QREG && i == 0) {
+#pragma unroll
+            for (int ks = 0; ks < KS; ks++)
+                ldmatrix_x4(qf[QREG ? ks : 0], Qs + ((lane & 7) + ((lane >> 3) & 1) * 8) * SD + ks * 16 + (lane >> 4) * 8);
+        }
+        if (owns_last && i == n - 1) {
+            // the token's own key and value over whatever the cache held at its place
+            bf16* krow = KV + (i % DSTAGES) * STAGE + (pos & 63) * SD;
+            for (int idx = tid; idx < 2 * HD; idx += 128) {
+                if (idx < HD)
+                    krow[idx] = fresh[idx];
+                else
+                    krow[64 * SD + idx - HD] = fresh[idx];
+            }
+            __syncthreads();
+        }
+        const bf16* kt = KV + (i % DSTAGES) * STAGE;
+        const bf16* vt = kt + 64 * SD;
+        const int t = span.tile_of(my_lo + i);
+        float s[2][4];
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) s[j][e] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < KS; ks++) {
+            uint32_t a[4], b[4];
+            if (QREG) {
+#pragma unroll
+                for (int e = 0; e < 4; e++) a[e] = qf[QREG ? ks : 0][e];
+            } else {
+                ldmatrix_x4(a, Qs + ((lane & 7) + ((lane >> 3) & 1) * 8) * SD + ks * 16 + (lane >> 4) * 8);
+            }
+            ldmatrix_x4(b, kt + (warp * 16 + (lane & 7) + (lane >> 4) * 8) * SD + ks * 16 + ((lane >> 3) & 1) * 8);
+            mma_bf16_16816(s[0], a[0], a[1], a[2], a[3], b[0], b[1]);
+            mma_bf16_16816(s[1], a[0], a[1], a[2], a[3], b[2], b[3]);
+        }
+        float mx0 = m0, mx1 = m1;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                int key = t * 64 + warp * 16 + j * 8 + t4 * 2 + (e & 1);
+                bool ok = key <= pos && (key >= span.lo_pos || key < p.keep_first);
+                float v = ok ? s[j][e] * sc : -INFINITY;
+                s[j][e] = v;
+                if (e & 2) mx1 = fmaxf(mx1, v); else mx0 = fmaxf(mx0, v);
+            }
+        }
+        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+        const float base0 = mx0 == -INFINITY ? 0.f : mx0, base1 = mx1 == -INFINITY ? 0.f : mx1;
+        const float c0 = exp2f(m0 - base0), c1 = exp2f(m1 - base1);
+        m0 = mx0;
+        m1 = mx1;
+        l0 *= c0;
+        l1 *= c1;
+#pragma unroll
+        for (int j = 0; j < NF; j++) {
+            o[j][0] *= c0;
+            o[j][1] *= c0;
+            o[j][2] *= c1;
+            o[j][3] *= c1;
+        }
+        uint32_t pa[4];
+        {
+            float p00 = exp2f(s[0][0] - base0), p01 = exp2f(s[0][1] - base0), p02 = exp2f(s[0][2] - base1), p03 = exp2f(s[0][3] - base1);
+            float p10 = exp2f(s[1][0] - base0), p11 = exp2f(s[1][1] - base0), p12 = exp2f(s[1][2] - base1), p13 = exp2f(s[1][3] - base1);
+            l0 += p00 + p01 + p10 + p11;
+            l1 += p02 + p03 + p12 + p13;
+            pa[0] = pack_bf16(p00, p01);
+            pa[1] = pack_bf16(p02, p03);
+            pa[2] = pack_bf16(p10, p11);
+            pa[3] = pack_bf16(p12, p13);
+        }
+#pragma unroll
+        for (int c = 0; c < KS; c++) {
+            uint32_t b[4];
+            ldmatrix_x4_trans(b, vt + (warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * SD + c * 16 + (lane >> 4) * 8);
+            mma_bf16_16816(o[c * 2], pa[0], pa[1], pa[2], pa[3], b[0], b[1]);
+            mma_bf16_16816(o[c * 2 + 1], pa[0], pa[1], pa[2], pa[3], b[2], b[3]);
+        }
+    }
+    cp_async_wait<0>();
+    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
+    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+    __syncthreads();  // every warp is done with the tiles: reuse their memory for the merge
+
+    // merge the four warps: Ms/Ls [4][16], Os [4][16][HD]; rows of the tile that are no head stay out
+    float* Ms = reinterpret_cast<float*>(KV);
+    float* Ls = Ms + 64;
+    float* Os = Ls + 64;
+    if (t4 == 0) {
+        Ms[warp * 16 + g] = m0;
+        Ms[warp * 16 + g + 8] = m1;
+        Ls[warp * 16 + g] = l0;
+        Ls[warp * 16 + g + 8] = l1;
+    }
+#pragma unroll
+    for (int j = 0; j < NF; j++) {
+        float* o0 = Os + ((size_t)warp * 16 + g) * HD + j * 8 + t4 * 2;
+        float* o1 = Os + ((size_t)warp * 16 + g + 8) * HD + j * 8 + t4 * 2;
+        if (g < nh) *reinterpret_cast<float2*>(o0) = make_float2(o[j][0], o[j][1]);
+        if (g + 8 < nh) *reinterpret_cast<float2*>(o1) = make_float2(o[j][2], o[j][3]);
+    }
+    __syncthreads();
+    for (int idx = tid; idx < nh * HD / 4; idx += 128) {
+        const int r = idx / (HD / 4), c = (idx - r * (HD / 4)) * 4;
+        float M = fmaxf(fmaxf(Ms[r], Ms[16 + r]), fmaxf(Ms[32 + r], Ms[48 + r]));
+        float L = 0.f;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        const bool sink_here = p.sink && pieces == 1;   // with several pieces the merge kernel adds the sink's unit
+        if (sink_here) {
+            const float z = p.sinks ? p.sinks[h0 + r] * LOG2E : 0.f;
+            M = fmaxf(M, z);
+            L = exp2f(z - M);
+        }
+        if (M != -INFINITY) {
+#pragma unroll
+            for (int w = 0; w < 4; w++) {
+                const float e = exp2f(Ms[w * 16 + r] - M);
+                const float4 x = *reinterpret_cast<const float4*>(Os + ((size_t)w * 16 + r) * HD + c);
+                L += e * Ls[w * 16 + r];
+                acc.x += e * x.x;
+                acc.y += e * x.y;
+                acc.z += e * x.z;
+                acc.w += e * x.w;
+            }
+        }
+        const int head = h0 + r;
+        if (pieces == 1) {
+            uint32_t* op = reinterpret_cast<uint32_t*>((bf16*)p.out + (int64_t)q_row * p.out_row_stride + (int64_t)head * HD + c);
+            op[0] = pack_bf16(acc.x / L, acc.y / L);
+            op[1] = pack_bf16(acc.z / L, acc.w / L);
+        } else {
+            float* sp = p.scratch + (((int64_t)seq * p.heads + head) * p.num_splits + split) * (HD + 2);
+            if (c == 0) {
+                sp[0] = M == -INFINITY ? -INFINITY : M * LN2;  // natural-log units, as the merge kernel expects
+                sp[1] = L;
+            }
+            reinterpret_cast<float2*>(sp + 2 + c)[0] = make_float2(acc.x, acc.y);
+            reinterpret_cast<float2*>(sp + 2 + c)[1] = make_float2(acc.z, acc.w);
+        }
     }
 }
 
@@ -704,14 +609,16 @@ int launch_prefill(const AttnParamsX& p, cudaStream_t stream) {
     return 0;
 }
 
-template <int HD, bool PIECES>
-int launch_decode_form(const AttnParamsX& p, const RopeFuse& f, cudaStream_t stream) {
+template <int HD>
+int launch_decode(const AttnParamsX& p, const RopeFuse& f, cudaStream_t stream) {
     constexpr bool QREG = HD <= 128;
     constexpr int SD = HD + 8;
-    const int smem = (16 * SD + DSTAGES * 2 * 64 * SD) * 2 + 4 * HD * 4 + 2 * HD * 2;   // a stage holds the merge: 512 + 256 HD <= 256 SD bytes
+    int smem = (16 * SD + DSTAGES * 2 * 64 * SD) * 2 + 4 * HD * 4 + 2 * HD * 2;
+    const int merge = (128 + 64 * HD) * 4 + 16 * SD * 2;
+    if (merge > smem) smem = merge;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_decode_mma_kernel<HD, QREG, PIECES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(attn_decode_mma_kernel<HD, QREG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) GB_REFUSE("attention_decode_mma: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
         configured = true;
     }
@@ -719,29 +626,19 @@ int launch_decode_form(const AttnParamsX& p, const RopeFuse& f, cudaStream_t str
     const int GC = G < 16 ? G : 16;
     const int hchunks = (G + GC - 1) / GC;
     dim3 grid(p.num_splits, p.kv_heads * hchunks, p.nseq);
-    if (PIECES) {
-        const int resident = (227 * 1024) / (smem + 2048);   // CTAs an SM holds
-        const int64_t most = (int64_t)p.num_splits * p.kv_heads * hchunks * p.nseq;
-        const int64_t slots = (int64_t)(resident > 0 ? resident : 1) * gb_sm_count();
-        grid = dim3((unsigned)(most < slots ? most : slots), 1, 1);
-    }
+    if (p.piece_tiles > 0) grid = dim3(p.kv_heads * hchunks, p.nseq, p.num_splits);
     if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("attention_decode_mma: grid (%u, %u, %u) exceeds one launch", grid.x, grid.y, grid.z);
     // Measured at 1 to 64 sequences of 4096 keys: launched early, this kernel gains a little when it
     // is alone (one split, many CTAs) and loses when its CTAs and those of the merge behind it sit
     // waiting beside the kernels ahead (also when it fetches its first pages while it waits), so only
     // the single-split form is a dependent launch.
     if (p.num_splits == 1)
-        launch_pdl(attn_decode_mma_kernel<HD, QREG, PIECES>, grid, dim3(128), (size_t)smem, stream, p, f);
+        launch_pdl(attn_decode_mma_kernel<HD, QREG>, grid, dim3(128), (size_t)smem, stream, p, f);
     else
-        attn_decode_mma_kernel<HD, QREG, PIECES><<<grid, 128, smem, stream>>>(p, f);
+        attn_decode_mma_kernel<HD, QREG><<<grid, 128, smem, stream>>>(p, f);
     GB_CHECK_LAUNCH("attention_decode_mma");
     if (p.num_splits > 1) return gb_attention_merge_launch(p, p.d, GB_BF16, stream);
     return 0;
-}
-
-template <int HD>
-int launch_decode(const AttnParamsX& p, const RopeFuse& f, cudaStream_t stream) {
-    return p.piece_tiles > 0 ? launch_decode_form<HD, true>(p, f, stream) : launch_decode_form<HD, false>(p, f, stream);
 }
 
 int check(const AttnParamsX& p, const char* who) {
@@ -759,8 +656,7 @@ int check(const AttnParamsX& p, const char* who) {
 }
 
 int check_pieces(const AttnParamsX& p, const char* who) {
-    if (p.piece_tiles < 0 || (p.piece_tiles > 0 && (p.nseq > PIECES_MAX_SEQS || p.num_splits < 2)))
-        GB_REFUSE("%s: pieces of %d pages, at most %d, for %d sequences", who, p.piece_tiles, p.num_splits, p.nseq);
+    if (p.piece_tiles < 0 || (p.piece_tiles > 0 && p.num_splits < 2)) GB_REFUSE("%s: pieces of %d pages, at most %d", who, p.piece_tiles, p.num_splits);
     if (p.num_splits > 1 && ((uintptr_t)p.scratch & 7)) GB_REFUSE("%s: scratch must be 8-byte aligned", who);
     return 0;
 }

@@ -5,8 +5,6 @@
 #include "api.h"
 #include "common.cuh"
 
-constexpr int PIECES_MAX_SEQS = 128;   // sequences of a step that is cut so (one thread of a CTA counts one sequence's pieces)
-
 // The pages of the keys [0, keep_first) first, where a window leaves them visible, then those of [lo_pos, pos].
 struct DecodeSpan {
     int pos, lo_pos, t_lo, n_first, n_tiles;

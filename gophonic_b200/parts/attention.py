@@ -74,16 +74,22 @@ def token_pieces(nseq: int):
     """(pages a piece, most pieces a sequence) for single tokens whose sequences are cut by their own lengths: short pieces where
     few sequences have to fill the GPU, longer ones where there are many.  The lines lie at batch sizes that steps are captured
     at, so that a step of nine and the one of twelve that is replayed for it cut alike."""
-    pages = 1 if nseq <= 2 else 2 if nseq <= 4 else 4
-    return pages, 32 if nseq <= 8 else 16 if nseq <= 32 else 8
+    if nseq <= 2:
+        return 2, 32
+    if nseq <= 4:
+        return 3, 32
+    return (8, 8) if nseq <= 8 else (6, 8) if nseq <= 32 else (10, 4)
+
+
+LONG_CONTEXT = 512   # keys up to which a step's plan decides; captured steps are kept apart on either side of it
 
 
 def key_pieces(part, batch, heads: int, head_dim: int, value_dim: int):
     """(pieces at most, scratch for their partial results or None, pages a piece or 0) for this step: single tokens in bfloat16
-    are cut sequence by sequence (``token_pieces``), whatever the plan says; what the tensor-core kernel does not take, by
-    the plan."""
+    behind long contexts are cut sequence by sequence (``token_pieces``), whatever the plan says; the others, and what the
+    tensor-core kernel does not take, by the plan."""
     ops = part.rt.ops
-    if (part.rt.is_fp32 or batch.nseq > ops.PIECES_MAX_SEQS or value_dim != head_dim
+    if (part.rt.is_fp32 or batch.max_kv_len <= LONG_CONTEXT or value_dim != head_dim
             or not ops.attention_decode_rope_accepts(torch.bfloat16, head_dim, 0, batch.max_q_len)):
         return part.key_splits(batch) + (0,)
     pages, most = token_pieces(batch.nseq)
