@@ -796,7 +796,7 @@ def attention_decode_rope(qkv: torch.Tensor, out: torch.Tensor, rope_args: tuple
     """``qk_norm_rope_kv_write(qkv, *rope_args)`` and ``attention(qkv[:, :heads * head_dim], out,
     *attn_args)`` for single-token rows in one kernel (plus the merge of key splits): the attention
     kernel norms and rotates its queries itself, takes the token's own key and value from the row and
-    stores them in the cache.  The same bits as the two calls.  Without key splits it asks for the pages of earlier tokens
+    stores them in the cache.  The same bits as the two calls.  Without key splits, and with ``piece_pages``, it asks for the pages of earlier tokens
     while the launch directly ahead may still run: that one must not write this cache (the product that makes ``qkv``, which stands
     between two tokens of a sequence, does not)."""
     r = _rope_params(qkv, *rope_args)

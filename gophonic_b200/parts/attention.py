@@ -87,12 +87,18 @@ LONG_CONTEXT = 512   # keys up to which a step's plan decides; captured steps ar
 def key_pieces(part, batch, heads: int, head_dim: int, value_dim: int):
     """(pieces at most, scratch for their partial results or None, pages a piece or 0) for this step: single tokens in bfloat16
     behind long contexts are cut sequence by sequence (``token_pieces``), whatever the plan says; the others, and what the
-    tensor-core kernel does not take, by the plan."""
+    tensor-core kernel does not take, by the plan.  Of up to eight sequences in float32, whose keys a CTA walks at two
+    microseconds a page, so are all that are longer than two pages."""
     ops = part.rt.ops
-    if (part.rt.is_fp32 or batch.max_kv_len <= LONG_CONTEXT or value_dim != head_dim
+    if part.rt.is_fp32:
+        if batch.max_q_len != 1 or batch.nseq > 8:
+            return part.key_splits(batch) + (0,)
+        pages, most = 2, 32
+    elif (batch.max_kv_len <= LONG_CONTEXT or value_dim != head_dim
             or not ops.attention_decode_rope_accepts(torch.bfloat16, head_dim, 0, batch.max_q_len)):
         return part.key_splits(batch) + (0,)
-    pages, most = token_pieces(batch.nseq)
+    else:
+        pages, most = token_pieces(batch.nseq)
     floats = ops.attention_scratch_floats(batch.nseq, heads, value_dim, most)
     return most, batch.workspace(("attention key splits", heads, value_dim, most), floats), pages
 
