@@ -6,7 +6,7 @@ import torch
 
 from gophonic_b200.engine.step import build_batch
 from gophonic_b200.engine.graphs import captured_size
-from gophonic_b200.parts.attention import Attention, choose_splits, few_splits, token_pieces
+from gophonic_b200.parts.attention import Attention, choose_splits, context_class, few_splits, token_pieces
 from gophonic_b200.parts.gated_attention import GatedAttention
 from gophonic_b200.parts.latent_attention import LatentAttention
 
@@ -71,7 +71,8 @@ def test_a_batch_of_one_size_asks_for_few_captured_steps():
 
 def test_a_step_and_the_captured_one_that_is_replayed_for_it_cut_alike():
     for n in range(1, 129):
-        assert token_pieces(n) == token_pieces(captured_size(n))
+        for kv in (1, 512, 513, 2048, 2049, 40000):
+            assert token_pieces(n, kv) == token_pieces(captured_size(n), kv) == token_pieces(n, context_class(kv))
 
 
 # ---- latent attention: which sequences of a step go over expanded keys and values -------------------------
