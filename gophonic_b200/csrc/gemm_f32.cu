@@ -315,114 +315,6 @@ int launch_tile(const float* A, const float* W, float* C, int M, int N, int K, i
     return 0;
 }
 
-// ---- small tiles --------------------------------------------------------------------------
-// Where the larger tiles leave SMs idle in their last wave: 32 x 64 outputs, four CTAs to an SM.  A warp's lanes stand 4 x 8, a lane owns
-// four rows, 4 apart, and four columns, 8 apart.  With so few products a value the transposed stages of the tiles above are not worth
-// their stores: rows of both operands are staged as they lie in memory, by asynchronous copies two stages ahead, and read four
-// columns of K at a time, the next four while these are multiplied.  341 rows: 2048 x 2048 114.6 -> 96.8 us, 2048 x 6144 329.5
-// -> 277.8 (in larger tiles this form is slower than the one above: 128 x 128 of 12288 x 2048 430 against 364).
-constexpr int SM_BM = 32, SM_BN = 64, SM_T = 4, SM_BK = 32, SM_STAGES = 3;
-constexpr int SM_PITCH = SM_BK + 4;   // eight rows' 16-byte chunks meet no bank twice
-constexpr int SM_THREADS = (SM_BM / SM_T) * (SM_BN / SM_T);
-constexpr int SM_STAGE = (SM_BM + SM_BN) * SM_PITCH;
-
-__global__ void __launch_bounds__(SM_THREADS, 4) gemm_f32_small_tile_kernel(const float* __restrict__ A, const float* __restrict__ W,
-                                                                            float* __restrict__ C, int M, int N, int K, int64_t lda,
-                                                                            int64_t ldw, int64_t ldc) {
-    constexpr int WN = SM_BN / (8 * SM_T), CH = SM_BK / 4, COPIES = (SM_BM + SM_BN) * CH;
-    static_assert(COPIES % SM_THREADS == 0, "whole rounds of copies");
-    extern __shared__ __align__(16) float sm[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * SM_BM, n0 = blockIdx.y * SM_BN;
-    const int am = (warp / WN) * 4 * SM_T + (lane >> 3), wc = (warp % WN) * 8 * SM_T + (lane & 7);
-    auto load = [&](int kb, int stage) {
-        float* st = sm + stage * SM_STAGE;
-#pragma unroll
-        for (int i = 0; i < COPIES / SM_THREADS; i++) {
-            const int idx = tid + i * SM_THREADS;
-            const int r = idx / CH, c = idx % CH, k = kb * SM_BK + c * 4;
-            const bool of_a = r < SM_BM;
-            const int row = of_a ? m0 + r : n0 + r - SM_BM;
-            const bool there = k < K && row < (of_a ? M : N);
-            const float* src = of_a ? A + (int64_t)row * lda + k : W + (int64_t)row * ldw + k;
-            cp_async16(st + r * SM_PITCH + c * 4, there ? src : A, there ? 16 : 0);
-        }
-    };
-    float acc[SM_T][SM_T];
-#pragma unroll
-    for (int i = 0; i < SM_T; i++)
-#pragma unroll
-        for (int j = 0; j < SM_T; j++) acc[i][j] = 0.f;
-    const int KB = (K + SM_BK - 1) / SM_BK;
-#pragma unroll
-    for (int s = 0; s < SM_STAGES - 1; s++) {
-        if (s < KB) load(s, s);
-        cp_async_commit();
-    }
-    float4 a[2][SM_T], w[2][SM_T];
-    int stage = 0;
-    for (int kb = 0; kb < KB; kb++) {
-        cp_async_wait<SM_STAGES - 2>();
-        __syncthreads();   // stage kb has landed; everyone is done with the one before, whose place the next takes
-        if (kb + SM_STAGES - 1 < KB) load(kb + SM_STAGES - 1, stage == 0 ? SM_STAGES - 1 : stage - 1);
-        cp_async_commit();
-        const float* as = sm + stage * SM_STAGE + am * SM_PITCH;
-        const float* ws = sm + stage * SM_STAGE + (SM_BM + wc) * SM_PITCH;
-        auto read = [&](int h, int g) {
-#pragma unroll
-            for (int i = 0; i < SM_T; i++) {
-                a[h][i] = *(const float4*)(as + i * 4 * SM_PITCH + g * 4);
-                w[h][i] = *(const float4*)(ws + i * 8 * SM_PITCH + g * 4);
-            }
-        };
-        read(0, 0);
-#pragma unroll
-        for (int g = 0; g < CH; g++) {
-            if (g + 1 < CH) read((g + 1) & 1, g + 1);
-            const float4(&x)[SM_T] = a[g & 1];
-            const float4(&y)[SM_T] = w[g & 1];
-#pragma unroll
-            for (int i = 0; i < SM_T; i++)
-#pragma unroll
-                for (int j = 0; j < SM_T; j++) acc[i][j] = fmaf(x[i].x, y[j].x, acc[i][j]);
-#pragma unroll
-            for (int i = 0; i < SM_T; i++)
-#pragma unroll
-                for (int j = 0; j < SM_T; j++) acc[i][j] = fmaf(x[i].y, y[j].y, acc[i][j]);
-#pragma unroll
-            for (int i = 0; i < SM_T; i++)
-#pragma unroll
-                for (int j = 0; j < SM_T; j++) acc[i][j] = fmaf(x[i].z, y[j].z, acc[i][j]);
-#pragma unroll
-            for (int i = 0; i < SM_T; i++)
-#pragma unroll
-                for (int j = 0; j < SM_T; j++) acc[i][j] = fmaf(x[i].w, y[j].w, acc[i][j]);
-        }
-        if (++stage == SM_STAGES) stage = 0;
-    }
-    cp_async_wait<0>();
-#pragma unroll
-    for (int i = 0; i < SM_T; i++) {
-        const int m = m0 + am + 4 * i;
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < SM_T; j++) {
-            const int n = n0 + wc + 8 * j;
-            if (n < N) C[(int64_t)m * ldc + n] = acc[i][j];
-        }
-    }
-}
-
-int launch_small_tile(const float* A, const float* W, float* C, int M, int N, int K, int64_t lda, int64_t ldw, int64_t ldc, cudaStream_t stream) {
-    const dim3 grid(ceil_div(M, SM_BM), ceil_div(N, SM_BN));
-    if (grid.y > 65535) GB_REFUSE("gemm_f32: %d columns exceed one launch", N);
-    constexpr int SMEM = SM_STAGES * SM_STAGE * 4;   // 41472 bytes: what a kernel has without asking
-    static_assert(SMEM <= 48 * 1024, "");
-    gemm_f32_small_tile_kernel<<<grid, SM_THREADS, SMEM, stream>>>(A, W, C, M, N, K, lda, ldw, ldc);
-    GB_CHECK_LAUNCH("gemm_f32");
-    return 0;
-}
-
 }  // namespace
 
 // Rows of 16-byte chunks, and few enough columns for one launch of the narrowest tile.
@@ -444,17 +336,16 @@ int gb_gemm_f32_launch(const float* A, const float* W, float* C, int M, int N, i
         if (nt * ceil_div(M, 8) <= 128) return launch_rows<8>(A, W, C, M, N, K, lda, ldw, ldc, stream);
         if (M <= 16) return launch_rows<4>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     }
-    // The tile: what the busiest SM's tiles take, from one alone and from several side by side (us at K = 2048); the small ones
-    // measured 45, 75, 97, 160 and 444 us for 1, 2, 3, 5 and 15 to an SM.
+    // The tile: what the busiest SM's tiles take, from one alone and from several side by side (us at K = 2048).
     struct Tile {
         int bm, bn, alone, each;
     };
-    static const Tile tiles[4] = {{128, 128, 184, 184}, {64, 128, 115, 97}, {64, 64, 67, 56}, {SM_BM, SM_BN, 0, 0}};
+    static const Tile tiles[4] = {{128, 128, 184, 184}, {64, 128, 115, 97}, {64, 64, 78, 56}, {32, 64, 63, 41}};
     int64_t best = INT64_MAX;
     int pick = 0;
     for (int i = 0; i < 4; i++) {
         const int64_t n = ((int64_t)ceil_div(M, tiles[i].bm) * ceil_div(N, tiles[i].bn) + sms - 1) / sms;
-        const int64_t t = i == 3 ? 15 + (59 * n + 1) / 2 : n * tiles[i].each > tiles[i].alone ? n * tiles[i].each : tiles[i].alone;
+        const int64_t t = n * tiles[i].each > tiles[i].alone ? n * tiles[i].each : tiles[i].alone;
         if (t < best) {
             best = t;
             pick = i;
@@ -464,6 +355,6 @@ int gb_gemm_f32_launch(const float* A, const float* W, float* C, int M, int N, i
         case 0: return launch_tile<128, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, stream);
         case 1: return launch_tile<64, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, stream);
         case 2: return launch_tile<64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-        default: return launch_small_tile(A, W, C, M, N, K, lda, ldw, ldc, stream);
+        default: return launch_tile<32, 64, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     }
 }
