@@ -47,7 +47,7 @@ struct AttnParamsX : AttnParams {
     int v_share;     // > 1: this many consecutive key heads read one value head (the value plane holds kv_heads / v_share heads)
     int64_t v_row_stride;  // elements between the values of two tokens of a page; 0: dv.  A value plane that is a view of the key
                            // plane (the values are the first dv channels of the keys) has the keys' stride d.
-    int piece_tiles;       // > 0, single tokens: every sequence is cut by its own length into pieces of this many pages, or of
+    int piece_tiles;       // > 0, single tokens on the tensor cores: every sequence is cut by its own length into pieces of this many pages, or of
                            // more if they were more than num_splits (the room scratch has a sequence and head)
     int piece_reserved;    // 0; keeps the size a multiple of eight for what is derived from this
 };

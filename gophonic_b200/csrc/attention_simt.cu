@@ -32,7 +32,7 @@ constexpr int SIMT_MAX_DV = 512;   // widest value head
 // others follow from t_lo.
 struct KeyTiles {
     int t_lo, n_first, my_lo, my_hi;
-    __device__ __forceinline__ KeyTiles(const AttnParamsX& p, int past, int q0, int last_q, int split, int pieces) {
+    __device__ __forceinline__ KeyTiles(const AttnParamsX& p, int past, int q0, int last_q, int split) {
         int lo_pos = 0;
         if (p.window > 0) {
             lo_pos = past + q0 - p.window + 1;
@@ -47,7 +47,7 @@ struct KeyTiles {
         n_first = p.window > 0 && p.keep_first > 0 ? (p.keep_first + KT - 1) / KT : 0;
         if (n_first > t_lo) n_first = t_lo;
         const int n_tiles = n_first + ((past + last_q) / KT + 1 - t_lo);
-        const int per = (n_tiles + pieces - 1) / pieces;
+        const int per = (n_tiles + p.num_splits - 1) / p.num_splits;
         my_lo = split * per;
         my_hi = my_lo + per < n_tiles ? my_lo + per : n_tiles;
     }
@@ -75,9 +75,9 @@ __device__ __forceinline__ float weigh(bool valid, float score, float& m, float&
 
 // A finished row: divided by its sum, or as it is into the scratch memory of the splits.
 template <typename T, int NE>
-__device__ __forceinline__ void leave_row(const AttnParamsX& p, int pieces, int seq, int split, int64_t row, int head, int dv, int lane, float m, float l,
+__device__ __forceinline__ void leave_row(const AttnParamsX& p, int seq, int split, int64_t row, int head, int dv, int lane, float m, float l,
                                           const float (&acc)[NE]) {
-    if (pieces == 1) {
+    if (p.num_splits == 1) {
         T* op = (T*)p.out + row * p.out_row_stride + (int64_t)head * dv;
         float lsum = l, keep = 1.f;
         if (p.sink) {
@@ -122,11 +122,7 @@ __global__ void __launch_bounds__(128) attn_simt_kernel(AttnParamsX p) {
     const int hchunks = (G + GC - 1) / GC;
     const int QT = ROWS / GC;
 
-    // sequences cut by their own lengths leave some CTAs nothing to do: those come last
-    const bool own = p.piece_tiles > 0;
-    const int seq = own ? blockIdx.z % p.nseq : blockIdx.z / p.num_splits, split = own ? blockIdx.z / p.nseq : blockIdx.z % p.num_splits;
-    const int pieces = own ? attn_pieces(attn_decode_span(p, p.seq_kv_len[seq] - 1).n_tiles, p.piece_tiles, p.num_splits) : p.num_splits;
-    if (split >= pieces) return;
+    const int seq = blockIdx.z / p.num_splits, split = blockIdx.z % p.num_splits;
     const int kvh = blockIdx.y / hchunks, chunk = blockIdx.y % hchunks;
     // consecutive key heads may read one value head: -1 if every key head has its own
     const int v_heads = p.v_share > 1 ? p.kv_heads / p.v_share : p.kv_heads, vh = p.v_share > 1 ? kvh / p.v_share : -1;
@@ -165,7 +161,7 @@ __global__ void __launch_bounds__(128) attn_simt_kernel(AttnParamsX p) {
 
     const int last_q = (q0 + QT < q_len ? q0 + QT : q_len) - 1;
     const int hi_pos = past + last_q;
-    const KeyTiles tiles(p, past, q0, last_q, split, pieces);
+    const KeyTiles tiles(p, past, q0, last_q, split);
 
     float m[RW], l[RW], acc[RW][NE];
 #pragma unroll
@@ -227,7 +223,7 @@ __global__ void __launch_bounds__(128) attn_simt_kernel(AttnParamsX p) {
 
 #pragma unroll
     for (int rr = 0; rr < RW; rr++)
-        if (row_ok[rr]) leave_row<T>(p, pieces, seq, split, q_start + row_q[rr], row_head[rr], dv, lane, m[rr], l[rr], acc[rr]);
+        if (row_ok[rr]) leave_row<T>(p, seq, split, q_start + row_q[rr], row_head[rr], dv, lane, m[rr], l[rr], acc[rr]);
 }
 
 // The same for float32 rows of 16-byte chunks (the true 32-bit path at the usual head sizes), with the
@@ -256,11 +252,7 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParamsX p, int stages
     const int hchunks = (G + GC - 1) / GC;
     const int QT = ROWS / GC;
 
-    // sequences cut by their own lengths leave some CTAs nothing to do: those come last
-    const bool own = p.piece_tiles > 0;
-    const int seq = own ? blockIdx.z % p.nseq : blockIdx.z / p.num_splits, split = own ? blockIdx.z / p.nseq : blockIdx.z % p.num_splits;
-    const int pieces = own ? attn_pieces(attn_decode_span(p, p.seq_kv_len[seq] - 1).n_tiles, p.piece_tiles, p.num_splits) : p.num_splits;
-    if (split >= pieces) return;
+    const int seq = blockIdx.z / p.num_splits, split = blockIdx.z % p.num_splits;
     const int kvh = blockIdx.y / hchunks, chunk = blockIdx.y % hchunks;
     const int v_heads = p.v_share > 1 ? p.kv_heads / p.v_share : p.kv_heads, vh = p.v_share > 1 ? kvh / p.v_share : -1;
     const int q_len = p.seq_q_len[seq], kv_len = p.seq_kv_len[seq];
@@ -273,7 +265,7 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParamsX p, int stages
 
     const int last_q = (q0 + QT < q_len ? q0 + QT : q_len) - 1;
     const int hi_pos = past + last_q;
-    const KeyTiles tiles(p, past, q0, last_q, split, pieces);
+    const KeyTiles tiles(p, past, q0, last_q, split);
     const int my_lo = tiles.my_lo, my_hi = tiles.my_hi;
 
     // a tile's 32 keys lie in one page (of 64, and tiles begin at multiples of 32); its first key is visible
@@ -395,7 +387,7 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParamsX p, int stages
 
 #pragma unroll
     for (int rr = 0; rr < RW; rr++)
-        if (row_ok[rr]) leave_row<float>(p, pieces, seq, split, q_start + row_q[rr], row_head[rr], dv, lane, m[rr], l[rr], acc[rr]);
+        if (row_ok[rr]) leave_row<float>(p, seq, split, q_start + row_q[rr], row_head[rr], dv, lane, m[rr], l[rr], acc[rr]);
 }
 
 // out[seq, head, :] = sum_s exp(m_s - M) acc_s / sum_s exp(m_s - M) l_s over the key splits, one CTA a (sequence, head) and a
@@ -570,13 +562,13 @@ GB_API int gb_attention_simt(const AttnParams* pp, int dtype, cudaStream_t strea
 
 GB_API int gb_attention_simt_x(const AttnParamsX* pp, int dtype, cudaStream_t stream) {
     AttnParamsX p = *pp;
+    p.piece_tiles = 0;   // here every sequence is cut into num_splits
     if (p.nseq <= 0 || p.max_q_len <= 0) return 0;
     if (p.heads <= 0 || p.kv_heads <= 0 || p.heads % p.kv_heads) GB_REFUSE("attention: %d heads over %d kv heads", p.heads, p.kv_heads);
     if (p.d <= 0 || p.d > SIMT_MAX_D) GB_REFUSE("attention_simt: head_dim %d is outside [1, %d]", p.d, SIMT_MAX_D);
     if (p.num_splits < 1 || p.num_splits > MERGE_MAX_SPLITS) GB_REFUSE("attention: %d key splits; 1 to %d", p.num_splits, MERGE_MAX_SPLITS);
     if (p.num_splits > 1 && p.max_q_len != 1) GB_REFUSE("attention: key splits need single-token rows, got rows of up to %d", p.max_q_len);
     if (p.num_splits > 1 && !p.scratch) GB_REFUSE("attention: %d key splits without scratch memory", p.num_splits);
-    if (p.piece_tiles < 0 || (p.piece_tiles > 0 && (p.num_splits < 2 || p.max_q_len != 1))) GB_REFUSE("attention: pieces of %d pages", p.piece_tiles);
     if (p.window < 0) GB_REFUSE("attention: window %d", p.window);
     if (p.dv < 0 || p.dv > SIMT_MAX_DV || (p.dv == 0 && p.d > SIMT_MAX_DV)) GB_REFUSE("attention_simt: value size %d is outside [1, %d]", p.dv ? p.dv : p.d, SIMT_MAX_DV);
     if (p.chunk < 0) GB_REFUSE("attention: blocks of %d positions", p.chunk);

@@ -661,8 +661,8 @@ def _attn_params(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_pl
     start; ``v_share`` > 1: that many consecutive key heads read one value head (the value plane holds
     kv_heads / v_share heads).  The value plane may be a view whose tokens lie further apart than
     ``value_dim`` (the first channels of a wider plane, the key plane itself for instance); ``piece_pages`` > 0
-    (single tokens): every sequence is cut by its own length into pieces of that many cache pages, or of more where they
-    were more than ``num_splits``."""
+    (single tokens on the tensor cores): every sequence is cut by its own length into pieces of that many cache pages, or
+    of more where they were more than ``num_splits``."""
     _need(q, "attention q", dim=2, contiguous=False)
     _need(out, "attention out", q.dtype, 2, contiguous=False)
     dv = head_dim if value_dim is None else int(value_dim)

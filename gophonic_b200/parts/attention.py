@@ -16,7 +16,7 @@ from typing import List, Mapping, Optional
 import torch
 
 from .. import registry
-from .base import KVRequest, Mixer, RowStats, Runtime, TensorDecl, fold_weight, other_fold_buffers
+from .base import FOLD_ROWS, KVRequest, Mixer, RowStats, Runtime, TensorDecl, fold_weight, other_fold_buffers
 
 
 def choose_splits(units: int, max_kv_len: int, sm_count: int = 148, page_bytes: int = 32768) -> int:
@@ -85,12 +85,13 @@ def token_pieces(nseq: int, max_kv_len: int):
     """(pages a piece, most pieces a sequence) for single tokens whose sequences are cut by their own lengths, or None where the plan
     decides: short pieces where few sequences have to fill the GPU, longer ones where there are many; never more than four of more
     than four sequences, since a CTA costs some 5 us beside 1.4 a page (8 sequences of 4096 keys: 30.2 us in four pieces, as by the
-    plan, 35.0 in eight), and none of more than eight beyond 2048 keys (64 of 4096: 172 us uncut, 190 in four).  Unequal
+    plan, 35.0 in eight), and none of more than eight beyond 2048 keys (64 of 4096: 172 us uncut, 190 in four) nor of more than
+    64, whose layers the library issues in one call by the plan.  Unequal
     sequences, attention and merge, by the plan and so: 50 of 118 to 1900 keys 42.7 and 37.3, 16 of 93 to 1500 23.6 and 16.4, 8
     of 256 to 4096 26.6 and 24.6, one of 700 8.0 and 7.6.  The lines lie at batch sizes that steps are captured at, so that a
     step of nine and the one of twelve that is replayed for it cut alike."""
     line = context_class(max_kv_len)
-    if line == CONTEXT_LINES[0] or (line > CONTEXT_LINES[-1] and nseq > 8):
+    if line == CONTEXT_LINES[0] or nseq > FOLD_ROWS or (line > CONTEXT_LINES[-1] and nseq > 8):
         return None
     return (2, 16) if nseq <= 2 else (3, 8) if nseq <= 4 else (8, 4) if nseq <= 8 else (6, 4) if nseq <= 32 else (10, 4)
 
@@ -98,14 +99,10 @@ def token_pieces(nseq: int, max_kv_len: int):
 def key_pieces(part, batch, heads: int, head_dim: int, value_dim: int):
     """(pieces at most, scratch for their partial results or None, pages a piece or 0) for this step: single tokens in bfloat16 are cut
     sequence by sequence where ``token_pieces`` says so, whatever the plan says; the others, and what the tensor-core kernel
-    does not take, by the plan.  Of up to eight sequences in float32, whose keys a CTA walks at two microseconds a page, so are all
-    that are longer than two pages."""
+    does not take, by the plan."""
     ops = part.rt.ops
     pieces = None
-    if part.rt.is_fp32:
-        if batch.max_q_len == 1 and batch.nseq <= 8:
-            pieces = 2, 32
-    elif value_dim == head_dim and ops.attention_decode_rope_accepts(torch.bfloat16, head_dim, 0, batch.max_q_len):
+    if not part.rt.is_fp32 and value_dim == head_dim and ops.attention_decode_rope_accepts(torch.bfloat16, head_dim, 0, batch.max_q_len):
         pieces = token_pieces(batch.nseq, batch.max_kv_len)
     if pieces is None:
         return part.key_splits(batch) + (0,)

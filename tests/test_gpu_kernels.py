@@ -661,13 +661,11 @@ def test_single_token_attention_that_rotates_and_stores_the_token_itself(ops, he
 @pytest.mark.parametrize("heads,kvh,d", [(4, 2, 16), (32, 8, 128), (20, 1, 32), (2, 2, 256)])
 @pytest.mark.parametrize("pages,most", [(1, 32), (2, 8), (4, 2)])
 @pytest.mark.parametrize("opts", [{}, {"window": 100}, {"window": 130, "keep_first": 70, "sink": True}, {"chunk": 256}])
-@pytest.mark.parametrize("dtype,algo", [(torch.bfloat16, "decode_mma"), (torch.float32, "simt")])
-def test_single_tokens_cut_by_their_own_lengths(ops, heads, kvh, d, pages, most, opts, dtype, algo):
+def test_single_tokens_cut_by_their_own_lengths(ops, heads, kvh, d, pages, most, opts):
     """Pieces of a fixed number of pages, more of them the longer the sequence: lengths at the edges of pages and pieces, more
-    pieces than the GPU has places, the options of the uncut kernel.  The uncut kernel's result but for roundings, in bfloat16
+    pieces than the GPU has places, the options of the uncut kernel.  The uncut kernel's result but for roundings to bfloat16,
     2^-9 on either side: of every weight, whose reference point is the largest score of its own piece (together at most that
-    share of the weighted mean of |v|), and of the result; in float32 the order of sums of up to 2048 terms.  And the bits of
-    the sequence alone."""
+    share of the weighted mean of |v|), and of the result; and the bits of the sequence alone."""
     kv_lens = [1, 64, 65, 128, 129, 257, 700, 333, 2049, 512] * 6
     nseq, n_pages = len(kv_lens), sum((n + 63) // 64 for n in kv_lens)
     stride = max((n + 63) // 64 for n in kv_lens)
@@ -677,16 +675,16 @@ def test_single_tokens_cut_by_their_own_lengths(ops, heads, kvh, d, pages, most,
         table[i, :(n + 63) // 64] = perm[at:at + (n + 63) // 64]
         at += (n + 63) // 64
     table = table.to(DEV)
-    k, v = paged(n_pages, kvh, d, dtype, 4)
-    q = rnd(nseq, heads * d, dtype=dtype, seed=6)
+    k, v = paged(n_pages, kvh, d, torch.bfloat16, 4)
+    q = rnd(nseq, heads * d, dtype=torch.bfloat16, seed=6)
     mk = lambda x: torch.tensor(list(x), dtype=torch.int32, device=DEV)
 
     def run(seqs, splits, v=v, **more):
         n = len(seqs)
-        out = torch.full((n, heads * d), float("nan"), dtype=dtype, device=DEV)
+        out = torch.full((n, heads * d), float("nan"), dtype=torch.bfloat16, device=DEV)
         scratch = torch.full((ops.attention_scratch_floats(n, heads, d, splits),), float("nan"), device=DEV) if splits > 1 else None
         ops.attention(q[seqs].contiguous(), out, k, v, table, mk(seqs), mk(range(n)), mk([1] * n), mk(kv_lens[i] for i in seqs), n, 1, heads, kvh, d,
-                      d ** -0.5, opts.get("window", 0), splits, scratch, algo=algo, keep_first=opts.get("keep_first", 0),
+                      d ** -0.5, opts.get("window", 0), splits, scratch, algo="decode_mma", keep_first=opts.get("keep_first", 0),
                       sink=opts.get("sink", False), chunk=opts.get("chunk", 0), **more)
         return out
 
@@ -695,7 +693,7 @@ def test_single_tokens_cut_by_their_own_lengths(ops, heads, kvh, d, pages, most,
     want = run(everyone, 1).float()
     size = run(everyone, 1, v=v.abs()).float()
     assert torch.isfinite(got.float()).all()
-    assert ((got.float() - want).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 1e-5) * (size + want.abs()) + 1e-5).all()
+    assert ((got.float() - want).abs() <= 2.0 ** -8 * (size + want.abs()) + 1e-5).all()
     for i in range(0, 10):
         assert torch.equal(run([i], most, piece_pages=pages)[0], got[i]), kv_lens[i]
 
