@@ -20,8 +20,6 @@
 
 #include <math.h>
 
-#include <type_traits>
-
 namespace {
 
 constexpr int COLS = 16;     // value columns per CTA
@@ -365,41 +363,17 @@ __global__ void __launch_bounds__(THREADS) state_scan_kernel(LinearStateParams p
 // Four columns a warp, four warps: every staged row is read four times a CTA, which is what binds several CTAs an SM.  Two columns, eight
 // warps, where a CTA has an SM to itself and is bound by the latency of a token's chain (launch_scan has the line).
 // The kernel behind may come up only when the tokens are done: its CTAs, parked beside the scan, take its issue slots.
-// bfloat16 rows are staged as they are and widened by the reader, which halves what q and k take of shared memory's
-// bandwidth (it binds: a token of eight warps was 104 cycles of reads).  A key that carries the input gate of a scalar decay
-// is no bfloat16 any more and is staged in float32.
-template <int RC>
-__device__ __forceinline__ void staged_row(float (&v)[RC], const float* p) {
-#pragma unroll
-    for (int i = 0; i < RC; i += 4) *reinterpret_cast<float4*>(v + i) = *reinterpret_cast<const float4*>(p + i);
-}
-template <int RC>
-__device__ __forceinline__ void staged_row(float (&v)[RC], const __nv_bfloat16* p) {
-    static_assert(RC == 4 || RC == 8, "one access");
-    uint32_t u[RC / 2];
-    if (RC == 8)
-        *reinterpret_cast<uint4*>(u) = *reinterpret_cast<const uint4*>(p);
-    else
-        *reinterpret_cast<uint2*>(u) = *reinterpret_cast<const uint2*>(p);
-#pragma unroll
-    for (int i = 0; i < RC / 2; i++) {
-        v[2 * i] = __uint_as_float(u[i] << 16);
-        v[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
-    }
-}
-
 template <typename T, int RC, int MODE, int CW>
 __global__ void __launch_bounds__(32 * COLS / CW) state_scan_wide_kernel(LinearStateParams p) {
     constexpr bool SCALAR = MODE == 1, WRITES = MODE == 2;
-    constexpr bool PACKED = sizeof(T) == 2;
-    typedef typename std::conditional<SCALAR, float, T>::type KeyT;
     constexpr int D = 32 * RC;          // key channels of a head
     constexpr int THREADS = 32 * COLS / CW, TT = 32 / CW;   // tokens a tile: a thread fetches one value of them
     static_assert(TT * COLS == THREADS, "a value a thread");
-    __shared__ __align__(16) T q_s[TT][D];
-    __shared__ __align__(16) KeyT k_s[WRITES ? 1 : TT][WRITES ? 8 : D];
+    __shared__ __align__(16) float q_s[TT][D];
+    __shared__ __align__(16) float k_s[WRITES ? 1 : TT][WRITES ? 4 : D];
     __shared__ __align__(16) float a_s[SCALAR ? 1 : TT][SCALAR ? 4 : D];
     __shared__ __align__(16) float v_s[TT][COLS];
+    __shared__ float o_s[TT][COLS];
     __shared__ float keep_s[TT], m_s[TT];
     __shared__ float st_s[D][COLS + 1];
 
@@ -482,8 +456,8 @@ __global__ void __launch_bounds__(32 * COLS / CW) state_scan_wide_kernel(LinearS
             const int idx = tid + e * THREADS;
             const int t = idx / D, c = idx % D;
             const bool there = t < nt;
-            q_s[t][c] = from_f32<T>(!there ? 0.f : PACKED ? to_f32<T>(rq[e]) : to_f32<T>(rq[e]) * p.q_scale);
-            if (!WRITES) k_s[t][c] = from_f32<KeyT>(!there ? 0.f : SCALAR ? to_f32<T>(rk[e]) * ra[e] : to_f32<T>(rk[e]));
+            q_s[t][c] = there ? to_f32<T>(rq[e]) * p.q_scale : 0.f;
+            if (!WRITES) k_s[t][c] = there ? (SCALAR ? to_f32<T>(rk[e]) * ra[e] : to_f32<T>(rk[e])) : 0.f;
             if (!SCALAR) a_s[t][c] = there ? ra[e] : (WRITES ? 0.f : 1.f);
         }
         {
@@ -514,22 +488,22 @@ __global__ void __launch_bounds__(32 * COLS / CW) state_scan_wide_kernel(LinearS
             const float keep = SCALAR ? keep_s[t] : 0.f;
 #pragma unroll
             for (int c = 0; c < CW; c++) sum[c] = 0.f;
-            float qq[RC], kk[RC], aa[RC];
-            staged_row<RC>(qq, &q_s[t][lane * RC]);
-            if (PACKED) {
 #pragma unroll
-                for (int i = 0; i < RC; i++) qq[i] *= p.q_scale;
+            for (int i = 0; i < RC; i += 4) {
+                const float4 q4 = *reinterpret_cast<const float4*>(&q_s[t][lane * RC + i]);
+                float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (!WRITES) k4 = *reinterpret_cast<const float4*>(&k_s[t][lane * RC + i]);
+                float4 a4 = make_float4(keep, keep, keep, keep);
+                if (!SCALAR) a4 = *reinterpret_cast<const float4*>(&a_s[t][lane * RC + i]);
+                const float qq[4] = {q4.x, q4.y, q4.z, q4.w}, kk[4] = {k4.x, k4.y, k4.z, k4.w}, aa[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+#pragma unroll
+                    for (int c = 0; c < CW; c++) {
+                        st[i + u][c] = WRITES ? fmaf(aa[u], vv[c] - st[i + u][c], st[i + u][c]) : fmaf(aa[u], st[i + u][c], kk[u] * vv[c]);
+                        sum[c] = fmaf(st[i + u][c], qq[u], sum[c]);
+                    }
             }
-            if (!WRITES) staged_row<RC>(kk, &k_s[t][lane * RC]);
-            if (!SCALAR) staged_row<RC>(aa, &a_s[t][lane * RC]);
-#pragma unroll
-            for (int i = 0; i < RC; i++)
-#pragma unroll
-                for (int c = 0; c < CW; c++) {
-                    const float a = SCALAR ? keep : aa[i];
-                    st[i][c] = WRITES ? fmaf(a, vv[c] - st[i][c], st[i][c]) : fmaf(a, st[i][c], kk[i] * vv[c]);
-                    sum[c] = fmaf(st[i][c], qq[i], sum[c]);
-                }
 #pragma unroll
             for (int c = 0; c < CW; c++) acc[t * CW + c] = sum[c];
         }
@@ -559,16 +533,17 @@ __global__ void __launch_bounds__(32 * COLS / CW) state_scan_wide_kernel(LinearS
             const bool up = lane & 1;
             total = (up ? b2[1] : b2[0]) + __shfl_xor_sync(0xffffffffu, up ? b2[0] : b2[1], 1);
         }
-        // lane l is left with sum number l = t * CW + c, and writes it from there: a barrier a tile less than by way of shared memory
-        {
-            const int t = lane / CW, jj = warp * CW + lane % CW;
-            const int64_t row = q_start + t0 + t;
-            if (t < nt) {
-                if (norm_col) {
-                    if (jj == 0) p.coef[(row * H + h) * 4 + 3] = fmaxf(fabsf(total), expf(-m_s[t])) + 1e-6f;
-                } else if (j0 + jj < dv) {
-                    p.out[row * p.out_stride + h * dv + j0 + jj] = total;
-                }
+        o_s[lane / CW][warp * CW + lane % CW] = total;     // lane l is left with sum number l = t * CW + c
+        __syncthreads();
+        if (norm_col) {
+            if (tid < nt) {
+                const int64_t row = q_start + t0 + tid;
+                p.coef[(row * H + h) * 4 + 3] = fmaxf(fabsf(o_s[tid][0]), expf(-m_s[tid])) + 1e-6f;
+            }
+        } else {
+            for (int idx = tid; idx < nt * COLS; idx += THREADS) {
+                const int t = idx / COLS, jj = idx % COLS;
+                if (j0 + jj < dv) p.out[(int64_t)(q_start + t0 + t) * p.out_stride + h * dv + j0 + jj] = o_s[t][jj];
             }
         }
     }
