@@ -571,7 +571,8 @@ __device__ void sort_candidates(const unsigned long long* __restrict__ c, int n,
 // BUCKETS equal ones, every entry goes to its bucket and finds its place there by counting the larger entries beside it.  Entries
 // differ (each holds its index), so the result is the one descending order.  False, with cand undefined, where a bucket would
 // hold more than CROWD entries (nearly equal logits): the list is then sorted by exchanges.  The exchanges of 2048 entries
-// are 66 dependent steps, 15 of them with two barriers.
+// are 66 dependent steps, 15 of them with two barriers (16 rows of 151936, eight of them with 1024 candidates: the kernel 31 us by
+// exchanges, 22 so, the whole choice 44 and 35).
 constexpr int BUCKETS = 2 * ST;
 constexpr int CROWD = 48;
 constexpr int BUCKET_MIN = 256;   // fewer entries: at most 36 steps of few warps
