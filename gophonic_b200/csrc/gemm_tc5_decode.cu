@@ -128,7 +128,7 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tme
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
 
 template <typename TC, int NB, int STAGES>  // NB = batch columns of the instruction: 16 to 256; STAGES deep
-__global__ void __launch_bounds__(THREADS, NB <= 32 ? 4 : 3) gemm_tc5_decode_kernel(const __grid_constant__ CUtensorMap map_w,
+__global__ void __launch_bounds__(THREADS, NB <= 32 ? 4 : NB == 64 && STAGES >= 4 ? 2 : 3) gemm_tc5_decode_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                  const __grid_constant__ CUtensorMap map_x, TC* __restrict__ Y,
                                                                  int M, int N, int K, int64_t ldy, int splits, int kb_per_split,
                                                                  int epi, int vec, DecodeFold fold) {
