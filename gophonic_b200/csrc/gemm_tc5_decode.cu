@@ -35,6 +35,7 @@ __device__ int g_status;
 
 constexpr int BMW = 128, BK = 64, THREADS = 192;
 constexpr int W_BYTES = BMW * BK * 2;
+constexpr int MAX_SPLITS = 8;
 
 // the folded variants' extra operands (all null / 0 for the plain product)
 struct DecodeFold {
@@ -120,10 +121,6 @@ __device__ __forceinline__ void store_out(TC* __restrict__ Y, int64_t ldy, int b
     }
 }
 
-// Slices of rows a warp gathers at once, 16 bytes a lane: shared memory for them lies behind the partial tile, and the
-// shallower variants, which are there to fit more CTAs on an SM, hold fewer.
-constexpr int gather_slices(int nb, int stages) { return nb == 64 && stages >= 4 ? 16 : 8; }
-
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
 
@@ -134,7 +131,6 @@ __global__ void __launch_bounds__(THREADS, NB <= 32 ? 4 : NB == 64 && STAGES >= 
                                                                  int epi, int vec, DecodeFold fold) {
     constexpr int X_BYTES = NB * BK * 2, STAGE_BYTES = W_BYTES + X_BYTES;
     constexpr int TMEM_COLS = NB < 32 ? 32 : NB;
-    constexpr int GATHER = gather_slices(NB, STAGES);
     extern __shared__ unsigned char smem_raw[];
     unsigned char* tiles = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], accum_bar;
@@ -336,17 +332,15 @@ __global__ void __launch_bounds__(THREADS, NB <= 32 ? 4 : NB == 64 && STAGES >= 
 
     // All slices of the tile have left their partial tiles: add them.  CTA r of the cluster takes batch rows r, r + slices, ...: a
     // warp a row, a lane four neighbouring rows of the tile.  What the residual variant reads from global memory is requested
-    // while the cluster gathers.  A warp asks the other CTAs for all slices of as many of its rows as GATHER holds, keeps
-    // what comes in its own shared memory and finishes one row after the other from there: read row by row, the way to
-    // the other CTAs' shared memory was paid for every row, and written out for all rows at once the code was slower than
-    // this loop (12288 x 2048 with SwiGLU, 50 rows in two slices: 7 us of 18.4 for this phase in either form, 15.9 in all so; a
-    // layer's four products at 1.7B sizes, us, row by row and so: 16 rows 36.7 and 34.8, 32 43.1 and 39.3, 64 54.4 and 49.2).
+    // while the cluster gathers.  All slices of a row are asked for before the first is added, and added as they are: kept in the
+    // warp's own shared memory first, for several rows at once, the products took up to a tenth longer (us a call in a chain, that
+    // way and so: 9 x 1024 x 2048 4.6 and 4.2, 64 x 2048 x 6144 11.1 and 10.9, 256 x 2048 x 2048 14.6 and 11.8; a layer's four
+    // products at 1.7B sizes, 16 rows 34.7 and 33.2, 32 39.6 and 38.9, 64 47.0 and 44.3).
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
     const int n = n0 + lane * 4, have = N - n;
     const int row_step = splits * (THREADS / 32);
     const int row0 = (int)rank + splits * warp;
-    const int log_splits = 31 - __clz(splits);
     float4 ahead = make_float4(0.f, 0.f, 0.f, 0.f), next_w = ahead;   // epi 2: what the residual holds for the next row; the next norm's weight
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
@@ -361,72 +355,59 @@ __global__ void __launch_bounds__(THREADS, NB <= 32 ? 4 : NB == 64 && STAGES >= 
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }
     const uint32_t part_addr = s32(tiles) + (uint32_t)(lane * 16);
-    float4* mine = reinterpret_cast<float4*>(tiles + (size_t)NB * BMW * 4) + warp * GATHER * 32 + lane;
-    const int rows_a_batch = GATHER >> log_splits;
 #pragma unroll 1
-    for (int first = row0; first < M; first += rows_a_batch * row_step) {
-        float4 x[GATHER];
+    for (int bb = row0; bb < M; bb += row_step) {
+        float4 x[MAX_SPLITS];
 #pragma unroll
-        for (int f = 0; f < GATHER; f++) {
-            const int bb = first + (f >> log_splits) * row_step;
-            if (bb >= M) break;
+        for (int sl = 0; sl < MAX_SPLITS; sl++) {
+            if (sl >= splits) break;
             uint32_t remote;
-            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(part_addr + (uint32_t)(bb * BMW * 4)), "r"(f & (splits - 1)));
-            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(x[f].x), "=f"(x[f].y), "=f"(x[f].z), "=f"(x[f].w) : "r"(remote) : "memory");
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(part_addr + (uint32_t)(bb * BMW * 4)), "r"(sl));
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(x[sl].x), "=f"(x[sl].y), "=f"(x[sl].z), "=f"(x[sl].w) : "r"(remote) : "memory");
         }
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int f = 0; f < GATHER; f++) {
-            if (first + (f >> log_splits) * row_step >= M) break;
-            mine[f * 32] = x[f];
+        for (int sl = 0; sl < MAX_SPLITS; sl++) {
+            if (sl >= splits) break;
+            v.x += x[sl].x;
+            v.y += x[sl].y;
+            v.z += x[sl].z;
+            v.w += x[sl].w;
         }
-        if (first + rows_a_batch * row_step >= M) {
+        if (bb + row_step >= M) {
             // this warp reads no other CTA's memory any more
             __syncwarp();
             asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
         }
-#pragma unroll 1
-        for (int j = 0; j < rows_a_batch; j++) {
-            const int bb = first + j * row_step;
-            if (bb >= M) break;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 2
-            for (int sl = 0; sl < splits; sl++) {
-                const float4 p = mine[((j << log_splits) + sl) * 32];
-                v.x += p.x;
-                v.y += p.y;
-                v.z += p.z;
-                v.w += p.w;
-            }
-            if (epi == 2) {
-                float* hq = reinterpret_cast<float*>(Y) + (int64_t)bb * ldy + n;
-                const float4 h = make_float4(ahead.x + v.x, ahead.y + v.y, ahead.z + v.z, ahead.w + v.w);
-                if (bb + row_step < M) ahead = load4(hq + (int64_t)row_step * ldy, have, vec);
-                store4(hq, h, have, vec);
-                if (fold.next_w != nullptr) store4(fold.xn_out + (int64_t)bb * fold.ldxn + n, make_float4(h.x * next_w.x, h.y * next_w.y, h.z * next_w.z, h.w * next_w.w), have, vec);
-                // columns behind the last are zero.  The lanes of the warp hold the whole tile's share of this batch row
-                float sq = h.x * h.x;
-                sq += h.y * h.y;
-                sq += h.z * h.z;
-                sq += h.w * h.w;
-                sq = warp_sum(sq);
-                if (lane == 0) fold.stats_out[(int64_t)bb * fold.stats_out_stride + blockIdx.x] = sq;
-                continue;
-            }
-            if (fold.stats_in != nullptr) {
-                const float rs = rs_s[bb];
-                v = make_float4(v.x * rs, v.y * rs, v.z * rs, v.w * rs);
-            }
-            if (epi == 0) {
-                store4(Y + (int64_t)bb * ldy + n, v, have, vec);
-            } else {
-                // The up rows of four gate rows are eight rows on: two lanes on.  Each of the two lanes finishes two of the four.
-                const bool is_up = lane & 2;
-                const float give0 = is_up ? v.x : v.z, give1 = is_up ? v.y : v.w;
-                const float got0 = __shfl_xor_sync(0xffffffffu, give0, 2), got1 = __shfl_xor_sync(0xffffffffu, give1, 2);
-                const float z0 = silu_f(is_up ? got0 : v.x) * (is_up ? v.z : got0), z1 = silu_f(is_up ? got1 : v.y) * (is_up ? v.w : got1);
-                const int col = ((n >> 4) << 3) + (n & 7) + (is_up ? 2 : 0);
-                if (n < N) store2(Y + (int64_t)bb * ldy + col, z0, z1, vec);   // N is a multiple of 16
-            }
+        if (epi == 2) {
+            float* hq = reinterpret_cast<float*>(Y) + (int64_t)bb * ldy + n;
+            const float4 h = make_float4(ahead.x + v.x, ahead.y + v.y, ahead.z + v.z, ahead.w + v.w);
+            if (bb + row_step < M) ahead = load4(hq + (int64_t)row_step * ldy, have, vec);
+            store4(hq, h, have, vec);
+            if (fold.next_w != nullptr) store4(fold.xn_out + (int64_t)bb * fold.ldxn + n, make_float4(h.x * next_w.x, h.y * next_w.y, h.z * next_w.z, h.w * next_w.w), have, vec);
+            // columns behind the last are zero.  The lanes of the warp hold the whole tile's share of this batch row
+            float sq = h.x * h.x;
+            sq += h.y * h.y;
+            sq += h.z * h.z;
+            sq += h.w * h.w;
+            sq = warp_sum(sq);
+            if (lane == 0) fold.stats_out[(int64_t)bb * fold.stats_out_stride + blockIdx.x] = sq;
+            continue;
+        }
+        if (fold.stats_in != nullptr) {
+            const float rs = rs_s[bb];
+            v = make_float4(v.x * rs, v.y * rs, v.z * rs, v.w * rs);
+        }
+        if (epi == 0) {
+            store4(Y + (int64_t)bb * ldy + n, v, have, vec);
+        } else {
+            // The up rows of four gate rows are eight rows on: two lanes on.  Each of the two lanes finishes two of the four.
+            const bool is_up = lane & 2;
+            const float give0 = is_up ? v.x : v.z, give1 = is_up ? v.y : v.w;
+            const float got0 = __shfl_xor_sync(0xffffffffu, give0, 2), got1 = __shfl_xor_sync(0xffffffffu, give1, 2);
+            const float z0 = silu_f(is_up ? got0 : v.x) * (is_up ? v.z : got0), z1 = silu_f(is_up ? got1 : v.y) * (is_up ? v.w : got1);
+            const int col = ((n >> 4) << 3) + (n & 7) + (is_up ? 2 : 0);
+            if (n < N) store2(Y + (int64_t)bb * ldy + col, z0, z1, vec);   // N is a multiple of 16
         }
     }
     // no CTA may leave while another still reads its shared memory
@@ -443,7 +424,7 @@ int launch(const void* X, const void* W, void* Y, int M, int N, int K, int64_t l
            const DecodeFold& fold, cudaStream_t stream) {
     constexpr int X_BYTES = NB * BK * 2;
     int smem = STAGES * (W_BYTES + X_BYTES) + 1024;
-    const int part = (NB + gather_slices(NB, STAGES) * (THREADS / 32)) * BMW * 4 + 1024;
+    const int part = NB * BMW * 4 + 1024;
     if (part > smem) smem = part;
     static bool configured = false;
     if (!configured) {

@@ -309,6 +309,50 @@ def test_gemm_tensor_core_kernels(ops, algo, M, N, K, out_dtype):
     close(out, a.double() @ w.double().T, 2e-5 if out_dtype == torch.float32 else 6e-3)
 
 
+@pytest.mark.parametrize("M,N,K", [(9, 333, 2048), (16, 130, 1024), (24, 206, 2048), (40, 335, 4096), (64, 198, 2048), (130, 333, 2048)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_decode_product_in_slices_whose_rows_end_and_begin_anywhere(ops, M, N, K, out_dtype):
+    """Slices of K joined in a cluster, four neighbouring columns a lane: the same bits whether a row may be written four columns at
+    a time or not (its stride, its address), a last group of one to three columns, and nothing beside it."""
+    assert ops._lib.gb_gemm_tc5_decode_splits(M, N, K, ops._sms()) > 1
+    x, w = rnd(M, K, dtype=torch.bfloat16, seed=1), rnd(N, K, dtype=torch.bfloat16, scale=0.1, seed=2)
+    ref = x.double() @ w.double().T
+    inter = N // 16 * 8
+    gate_up = w[:2 * inter].contiguous()
+    z_ref = (x.double() @ gate_up.double().T).view(M, inter // 8, 2, 8)
+    z_ref = (z_ref[:, :, 0] / (1 + torch.exp(-z_ref[:, :, 0])) * z_ref[:, :, 1]).reshape(M, inter)
+    h0, nw = rnd(M, N, seed=3), 1 + 0.1 * rnd(N, seed=4)
+    plain, act, resid = [], [], []
+    for first, wide in ((0, 8), (0, 1), (1, 8)):    # aligned rows, an odd stride, an odd address
+        place = lambda n, dtype: torch.full((M, (n + 7) // 8 * 8 + wide), float("nan"), dtype=dtype, device=DEV)
+        whole = place(N, out_dtype)
+        out = whole[:, first:first + N]
+        ops.gemm(x, w, out, algo="tc5_decode")
+        assert whole.isnan().sum() == M * (whole.shape[1] - N)
+        plain.append(out.clone())
+        whole = place(inter, out_dtype)
+        out = whole[:, first:first + inter]
+        ops.gemm_swiglu(x, gate_up, out, algo="tc5_decode")
+        assert whole.isnan().sum() == M * (whole.shape[1] - inter)
+        act.append(out.clone())
+        if M <= ops.FOLD_ROWS:
+            whole, nxt = place(N, torch.float32), torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+            h = whole[:, first:first + N]
+            h.copy_(h0)
+            stats = torch.full((M, ops.fold_capacity(N)), float("nan"), device=DEV)
+            count = ops.gemm_residual(x, w, h, stats, nw, nxt)
+            assert whole.isnan().sum() == M * (whole.shape[1] - N)
+            resid.append(torch.cat([h, nxt.float(), stats[:, :count]], dim=1))
+    assert ops.tc5_status() == 0
+    for got in (plain, act, resid):
+        assert all(torch.equal(got[0], g) for g in got[1:])
+    close(plain[0], ref, 2e-5 if out_dtype == torch.float32 else 6e-3)
+    close(act[0], z_ref, 2e-5 if out_dtype == torch.float32 else 6e-3)
+    if resid:
+        close(resid[0][:, :N], h0.double() + ref, 2e-5)
+        close(resid[0][:, N:2 * N], (h0.double() + ref) * nw.double(), 6e-3)
+
+
 @pytest.mark.parametrize("M,N,K", [(192, 96, 64), (300, 1000, 512), (2048, 520, 1032), (257, 96, 4104)])
 def test_gemm_adds_into_the_residual(ops, M, N, K):
     """out += a w^T in the epilogue: the same bits as the product into a buffer and a float32 add."""
