@@ -589,8 +589,15 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
                 sp[0] = M == -INFINITY ? -INFINITY : M * LN2;  // natural-log units, as the merge kernel expects
                 sp[1] = L;
             }
-            reinterpret_cast<float2*>(sp + 2 + c)[0] = make_float2(acc.x, acc.y);
-            reinterpret_cast<float2*>(sp + 2 + c)[1] = make_float2(acc.z, acc.w);
+            if (!((uintptr_t)sp & 7)) {
+                reinterpret_cast<float2*>(sp + 2 + c)[0] = make_float2(acc.x, acc.y);
+                reinterpret_cast<float2*>(sp + 2 + c)[1] = make_float2(acc.z, acc.w);
+            } else {   // scratch is floats, wherever they begin
+                sp[2 + c] = acc.x;
+                sp[3 + c] = acc.y;
+                sp[4 + c] = acc.z;
+                sp[5 + c] = acc.w;
+            }
         }
     }
 }
@@ -661,7 +668,6 @@ int check(const AttnParamsX& p, const char* who) {
 
 int check_pieces(const AttnParamsX& p, const char* who) {
     if (p.piece_tiles < 0 || (p.piece_tiles > 0 && p.num_splits < 2)) GB_REFUSE("%s: pieces of %d pages, at most %d", who, p.piece_tiles, p.num_splits);
-    if (p.num_splits > 1 && ((uintptr_t)p.scratch & 7)) GB_REFUSE("%s: scratch must be 8-byte aligned", who);
     return 0;
 }
 

@@ -702,6 +702,28 @@ def test_single_token_attention_that_rotates_and_stores_the_token_itself(ops, he
     assert torch.equal(k_a, k0) != write and torch.equal(v_a, v0) != write
 
 
+@pytest.mark.parametrize("heads,kvh,d,dv", [(4, 2, 16, 16), (32, 8, 128, 128), (2, 2, 256, 256), (16, 1, 96, 64), (6, 3, 24, 24)])
+def test_partial_results_of_key_splits_may_begin_at_any_float(ops, heads, kvh, d, dv):
+    """Scratch is floats: the bits do not depend on where it begins (the tensor-core kernels' single tokens and latents, the CUDA cores)."""
+    kv_lens = [1, 64, 700, 333]
+    nseq, stride = len(kv_lens), 11
+    table = torch.randperm(nseq * stride, generator=torch.Generator().manual_seed(5)).to(torch.int32).reshape(nseq, stride).to(DEV)
+    k, v = paged(nseq * stride, kvh, d, torch.bfloat16, 4)
+    if dv != d:
+        v = k[..., :dv]
+    q = rnd(nseq, heads * d, dtype=torch.bfloat16, seed=6)
+    mk = lambda x: torch.tensor(list(x), dtype=torch.int32, device=DEV)
+    floats = ops.attention_scratch_floats(nseq, heads, dv, 4)
+    outs = []
+    for first in (0, 1):
+        out = torch.full((nseq, heads * dv), float("nan"), dtype=torch.bfloat16, device=DEV)
+        used = ops.attention(q, out, k, v, table, mk(range(nseq)), mk(range(nseq)), mk([1] * nseq), mk(kv_lens), nseq, 1, heads, kvh, d, d ** -0.5, 0, 4,
+                             torch.full((floats + 1,), float("nan"), device=DEV)[first:first + floats], value_dim=dv)
+        outs.append(out)
+    assert used == ("latent_mma" if dv != d else "simt" if d % 16 else "decode_mma")
+    assert torch.isfinite(outs[0].float()).all() and torch.equal(*outs)
+
+
 @pytest.mark.parametrize("heads,kvh,d", [(4, 2, 16), (32, 8, 128), (20, 1, 32), (2, 2, 256)])
 @pytest.mark.parametrize("pages,most", [(1, 32), (2, 8), (4, 2)])
 @pytest.mark.parametrize("opts", [{}, {"window": 100}, {"window": 130, "keep_first": 70, "sink": True}, {"chunk": 256}])
