@@ -47,9 +47,6 @@ struct AttnParamsX : AttnParams {
     int v_share;     // > 1: this many consecutive key heads read one value head (the value plane holds kv_heads / v_share heads)
     int64_t v_row_stride;  // elements between the values of two tokens of a page; 0: dv.  A value plane that is a view of the key
                            // plane (the values are the first dv channels of the keys) has the keys' stride d.
-    int piece_tiles;       // > 0, single tokens on the tensor cores: every sequence is cut by its own length into pieces of this many pages, or of
-                           // more if they were more than num_splits (the room scratch has a sequence and head)
-    int piece_reserved;    // 0; keeps the size a multiple of eight for what is derived from this
 };
 
 // Per-head q/k RMSNorm, rotary embedding and cache write on the rows of a fused q|k|v buffer.
@@ -192,7 +189,6 @@ GB_API int gb_attention_decode_mma(const AttnParams* p, cudaStream_t stream);
 GB_API int gb_attention_prefill_mma(const AttnParams* p, cudaStream_t stream);
 GB_API int gb_attention_decode_rope_accepts(int dtype, int d, int rot, int max_q_len);
 GB_API int gb_attention_decode_mma_rope(const AttnParams* p, const QkRopeParams* r, cudaStream_t stream);
-GB_API int gb_attention_decode_mma_rope_x(const AttnParamsX* p, const QkRopeParams* r, cudaStream_t stream);
 GB_API int gb_attention_prefill_tc5(const AttnParams* p, int rows, int pages, cudaStream_t stream);
 GB_API int gb_attention_simt_x(const AttnParamsX* p, int dtype, cudaStream_t stream);
 GB_API int gb_attention_decode_mma_x(const AttnParamsX* p, cudaStream_t stream);
@@ -215,7 +211,6 @@ static inline AttnParamsX gb_attn_widen(const AttnParams& a) {
     x.sinks = nullptr;
     x.chunk = x.v_share = 0;
     x.v_row_stride = 0;
-    x.piece_tiles = x.piece_reserved = 0;
     return x;
 }
 

@@ -13,7 +13,6 @@
 // sequence was cut into steps or on what else the batch holds.  Single-token steps may cut the keys into splits that a
 // merge kernel joins (the same scratch layout as the other attention kernels).
 #include "api.h"
-#include "attention_pieces.cuh"
 #include "common.cuh"
 #include "mma.cuh"
 
@@ -54,9 +53,7 @@ __global__ void __launch_bounds__(32 * WG * RG) attn_latent_mma_kernel(AttnParam
     const int H = p.heads;
     const int HC = H < LROWS ? H : LROWS;       // heads a CTA holds
     const int QT = LROWS / HC;                  // query positions a CTA holds
-    // cut by their own lengths, sequences with few pieces leave some CTAs nothing to do: those come last
-    const bool own = p.piece_tiles > 0;
-    const int seq = own ? blockIdx.z % p.nseq : blockIdx.z / p.num_splits, split = own ? blockIdx.z / p.nseq : blockIdx.z % p.num_splits;
+    const int seq = blockIdx.z / p.num_splits, split = blockIdx.z % p.num_splits;
     const int h0 = blockIdx.y * HC;
     const int q_len = p.seq_q_len[seq], kv_len = p.seq_kv_len[seq];
     const int q0 = blockIdx.x * QT;
@@ -90,9 +87,7 @@ __global__ void __launch_bounds__(32 * WG * RG) attn_latent_mma_kernel(AttnParam
     }
     const int t_lo = lo_pos / LKT, t_hi = hi_pos / LKT + 1;
     const int n_tiles = t_hi - t_lo;
-    const int pieces = own ? attn_pieces(n_tiles, p.piece_tiles, p.num_splits) : p.num_splits;   // a tile is a page there
-    if (own && split >= pieces) return;
-    const int per = (n_tiles + pieces - 1) / pieces;
+    const int per = (n_tiles + p.num_splits - 1) / p.num_splits;
     const int my_lo = t_lo + split * per;
     const int my_hi = my_lo + per < t_hi ? my_lo + per : t_hi;
     const int n = my_hi > my_lo ? my_hi - my_lo : 0;
@@ -289,7 +284,7 @@ __global__ void __launch_bounds__(32 * WG * RG) attn_latent_mma_kernel(AttnParam
     for (int e = 0; e < 2; e++) {
         if (!rok[e]) continue;
         const float L = e ? L1 : L0, M = e ? m1 : m0;
-        if (pieces == 1) {
+        if (p.num_splits == 1) {
             bf16* op = (bf16*)p.out + (int64_t)(q_start + rq[e]) * p.out_row_stride + (int64_t)rhead[e] * DV + warp * (NT * 8) + t4 * 2;
             const float inv = 1.f / L;
 #pragma unroll
@@ -346,7 +341,6 @@ GB_API int gb_attention_latent_mma(const AttnParamsX* pp, cudaStream_t stream) {
     if (p.nseq <= 0 || p.max_q_len <= 0) return 0;
     if (!gb_attention_latent_accepts(&p, GB_BF16)) GB_REFUSE("attention_latent: %d heads over %d key heads of %d with values of %d are not what this kernel takes", p.heads, p.kv_heads, p.d, p.dv);
     if (p.num_splits < 1 || (p.num_splits > 1 && (p.max_q_len != 1 || !p.scratch))) GB_REFUSE("attention_latent: %d key splits", p.num_splits);
-    if (p.piece_tiles < 0 || (p.piece_tiles > 0 && (p.num_splits < 2 || p.max_q_len != 1))) GB_REFUSE("attention_latent: pieces of %d pages", p.piece_tiles);
     if (p.window < 0 || p.chunk < 0) GB_REFUSE("attention_latent: window %d, blocks of %d", p.window, p.chunk);
     // two groups of rows share a staged page where a sequence brings that many (query position, head) pairs; a single group
     // (single tokens of up to 16 heads) gets eight warps, two a scheduler, where its value heads are wide enough to deal out.

@@ -15,7 +15,6 @@
 // bfloat16 for the second product, as the values are bfloat16.
 #include "mma.cuh"
 #include "api.h"
-#include "attention_pieces.cuh"
 
 #include <math.h>
 
@@ -332,12 +331,8 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
     const int G = p.heads / p.kv_heads;
     const int GC = G < 16 ? G : 16;
     const int hchunks = (G + GC - 1) / GC;
-    // Cut by their own lengths, most sequences have fewer pieces than the longest: a CTA without one leaves at once, and those come
-    // last (the pieces are the slowest dimension of the grid there).
-    const bool own = p.piece_tiles > 0;
-    const int split = own ? blockIdx.z : blockIdx.x, seq = own ? blockIdx.y : blockIdx.z;
-    const int head_cta = own ? blockIdx.x : blockIdx.y;
-    const int kvh = head_cta / hchunks, chunk = head_cta % hchunks;
+    const int split = blockIdx.x, seq = blockIdx.z;
+    const int kvh = blockIdx.y / hchunks, chunk = blockIdx.y % hchunks;
     const int kv_len = p.seq_kv_len[seq];
     const int q_row = p.seq_q_start[seq];
     const int pos = kv_len - 1;
@@ -346,21 +341,26 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
     const bf16* vbase = (const bf16*)p.v_plane;
     const int h0 = kvh * G + chunk * GC;            // first head of this CTA
     const int nh = (G - chunk * GC) < GC ? (G - chunk * GC) : GC;  // heads of this CTA
-    const DecodeSpan span = attn_decode_span(p, pos);
-    const int n_tiles = span.n_tiles;
-    const int pieces = own ? attn_pieces(n_tiles, p.piece_tiles, p.num_splits) : p.num_splits;
-    if (split >= pieces) {
-        pdl_wait();
-        pdl_trigger();
-        return;
+    int lo_pos = 0;
+    if (p.window > 0) {
+        lo_pos = pos - p.window + 1;
+        if (lo_pos < 0) lo_pos = 0;
     }
-    const int per = (n_tiles + pieces - 1) / pieces;
+    if (p.chunk > 0 && pos - pos % p.chunk > lo_pos) lo_pos = pos - pos % p.chunk;   // blocks of positions
+    const int t_lo = lo_pos / 64, t_hi = pos / 64 + 1;  // [t_lo, t_hi)
+    // with kept first tokens: the tiles of keys [0, keep_first) first, then those of the window; the
+    // splits cut this list of tiles
+    int n_first = p.window > 0 && p.keep_first > 0 ? (p.keep_first + 63) / 64 : 0;
+    if (n_first > t_lo) n_first = t_lo;
+    const int n_tiles = n_first + t_hi - t_lo;
+    auto tile_of = [&](int i) { return i < n_first ? i : t_lo + (i - n_first); };
+    const int per = (n_tiles + p.num_splits - 1) / p.num_splits;
     const int my_lo = split * per;
     const int my_hi = my_lo + per < n_tiles ? my_lo + per : n_tiles;
     const int n = my_hi > my_lo ? my_hi - my_lo : 0;
 
     auto load_tile = [&](int i) {
-        int t = span.tile_of(my_lo + i);
+        int t = tile_of(my_lo + i);
         int64_t page = page_of(bt, t * 64, p.bt_stride, p.pages);
         int64_t off = ((page * p.kv_heads + kvh) * 64) * (int64_t)HD;
         int64_t voff = p.v_share > 1 ? ((page * (p.kv_heads / p.v_share) + kvh / p.v_share) * 64) * (int64_t)HD : off;
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
         }
         const bf16* kt = KV + (i % DSTAGES) * STAGE;
         const bf16* vt = kt + 64 * SD;
-        const int t = span.tile_of(my_lo + i);
+        const int t = tile_of(my_lo + i);
         float s[2][4];
 #pragma unroll
         for (int j = 0; j < 2; j++)
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 int key = t * 64 + warp * 16 + j * 8 + t4 * 2 + (e & 1);
-                bool ok = key <= pos && (key >= span.lo_pos || key < p.keep_first);
+                bool ok = key <= pos && (key >= lo_pos || key < p.keep_first);
                 float v = ok ? s[j][e] * sc : -INFINITY;
                 s[j][e] = v;
                 if (e & 2) mx1 = fmaxf(mx1, v); else mx0 = fmaxf(mx0, v);
@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
         float M = fmaxf(fmaxf(Ms[r], Ms[16 + r]), fmaxf(Ms[32 + r], Ms[48 + r]));
         float L = 0.f;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        const bool sink_here = p.sink && pieces == 1;   // with several pieces the merge kernel adds the sink's unit
+        const bool sink_here = p.sink && p.num_splits == 1;   // with key splits the merge kernel adds the sink's unit
         if (sink_here) {
             const float z = p.sinks ? p.sinks[h0 + r] * LOG2E : 0.f;
             M = fmaxf(M, z);
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnParamsX p, Rop
             }
         }
         const int head = h0 + r;
-        if (pieces == 1) {
+        if (p.num_splits == 1) {
             uint32_t* op = reinterpret_cast<uint32_t*>((bf16*)p.out + (int64_t)q_row * p.out_row_stride + (int64_t)head * HD + c);
             op[0] = pack_bf16(acc.x / L, acc.y / L);
             op[1] = pack_bf16(acc.z / L, acc.w / L);
@@ -637,13 +637,12 @@ int launch_decode(const AttnParamsX& p, const RopeFuse& f, cudaStream_t stream) 
     const int GC = G < 16 ? G : 16;
     const int hchunks = (G + GC - 1) / GC;
     dim3 grid(p.num_splits, p.kv_heads * hchunks, p.nseq);
-    if (p.piece_tiles > 0) grid = dim3(p.kv_heads * hchunks, p.nseq, p.num_splits);
     if (grid.y > 65535 || grid.z > 65535) GB_REFUSE("attention_decode_mma: grid (%u, %u, %u) exceeds one launch", grid.x, grid.y, grid.z);
-    // Dependent launches: the single-split form, and sequences cut by their own lengths, whose CTAs are many and short, so that the
-    // way to their first pages shows (50 sequences of 118 to 1900 keys: a step 2.5 % faster so; one sequence, 8 and 16: no
-    // change).  Equal splits lose as such (measured at 1 to 64 sequences of 4096 keys: their CTAs and those of the merge behind sit
-    // waiting beside the kernels ahead), and so does the merge.
-    if (p.num_splits == 1 || p.piece_tiles > 0)
+    // Measured at 1 to 64 sequences of 4096 keys: launched early, this kernel gains a little when it
+    // is alone (one split, many CTAs) and loses when its CTAs and those of the merge behind it sit
+    // waiting beside the kernels ahead (also when it fetches its first pages while it waits), so only
+    // the single-split form is a dependent launch.
+    if (p.num_splits == 1)
         launch_pdl(attn_decode_mma_kernel<HD, QREG>, grid, dim3(128), (size_t)smem, stream, p, f);
     else
         attn_decode_mma_kernel<HD, QREG><<<grid, 128, smem, stream>>>(p, f);
@@ -663,11 +662,6 @@ int check(const AttnParamsX& p, const char* who) {
         GB_REFUSE("%s: blocks of %d positions, value heads shared by %d, value stride %lld", who, p.chunk, p.v_share, (long long)p.v_row_stride);
     if (((uintptr_t)p.q & 15) || (p.q_row_stride & 7)) GB_REFUSE("%s: query rows must be 16-byte aligned", who);
     if ((p.out_row_stride & 1) || ((uintptr_t)p.out & 3)) GB_REFUSE("%s: output rows must be 4-byte aligned", who);
-    return 0;
-}
-
-int check_pieces(const AttnParamsX& p, const char* who) {
-    if (p.piece_tiles < 0 || (p.piece_tiles > 0 && p.num_splits < 2)) GB_REFUSE("%s: pieces of %d pages, at most %d", who, p.piece_tiles, p.num_splits);
     return 0;
 }
 
@@ -712,7 +706,6 @@ GB_API int gb_attention_decode_mma_x(const AttnParamsX* pp, cudaStream_t stream)
     if (p.max_q_len != 1) GB_REFUSE("attention_decode_mma: rows of up to %d tokens; this kernel takes single tokens", p.max_q_len);
     if (p.num_splits < 1) GB_REFUSE("attention_decode_mma: %d key splits", p.num_splits);
     if (p.num_splits > 1 && !p.scratch) GB_REFUSE("attention_decode_mma: %d key splits without scratch memory", p.num_splits);
-    if (int rc = check_pieces(p, "attention_decode_mma")) return rc;
     const RopeFuse off = {};
     GB_DISPATCH_HD(launch_decode, off)
     GB_REFUSE("attention_decode_mma: head_dim %d", p.d);
@@ -730,12 +723,7 @@ GB_API int gb_attention_decode_rope_accepts(int dtype, int d, int rot, int max_q
 // sequence's last page takes the token's own key and value from the row, and one CTA per kv head
 // stores them in the cache.  The same bits as the two kernels one after the other.
 GB_API int gb_attention_decode_mma_rope(const AttnParams* pp, const QkRopeParams* rp, cudaStream_t stream) {
-    const AttnParamsX x = gb_attn_widen(*pp);
-    return gb_attention_decode_mma_rope_x(&x, rp, stream);
-}
-
-GB_API int gb_attention_decode_mma_rope_x(const AttnParamsX* pp, const QkRopeParams* rp, cudaStream_t stream) {
-    AttnParamsX p = *pp;
+    AttnParamsX p = gb_attn_widen(*pp);
     const QkRopeParams& r = *rp;
     if (p.nseq <= 0) return 0;
     const char* who = "attention_decode_mma_rope";
@@ -743,7 +731,6 @@ GB_API int gb_attention_decode_mma_rope_x(const AttnParamsX* pp, const QkRopePar
     if (p.max_q_len != 1) GB_REFUSE("%s: rows of up to %d tokens; this kernel takes single tokens", who, p.max_q_len);
     if (p.num_splits < 1) GB_REFUSE("%s: %d key splits", who, p.num_splits);
     if (p.num_splits > 1 && !p.scratch) GB_REFUSE("%s: %d key splits without scratch memory", who, p.num_splits);
-    if (int rc = check_pieces(p, who)) return rc;
     if (r.qkv != p.q || r.row_stride != p.q_row_stride || r.heads != p.heads || r.kv_heads != p.kv_heads || r.d != p.d ||
         r.rows != p.nseq || r.block_table != p.block_table || r.bt_stride != p.bt_stride)
         GB_REFUSE("%s: the two descriptions are not of the same rows", who);

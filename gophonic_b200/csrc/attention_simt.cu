@@ -10,7 +10,6 @@
 // into steps or on what else is in the batch.
 #include "mma.cuh"
 #include "api.h"
-#include "attention_pieces.cuh"
 
 #include <math.h>
 
@@ -393,9 +392,9 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParamsX p, int stages
 // out[seq, head, :] = sum_s exp(m_s - M) acc_s / sum_s exp(m_s - M) l_s over the key splits, one CTA a (sequence, head) and a
 // thread a value.  Every warp finds the maximum, the normaliser and the weights for itself (a lane a split, shuffle trees, a fixed
 // order); thread c then adds value c of the splits in split order.  A chain of waits for memory and little else, so what it
-// reads is asked for at once: the first splits' values and all maxima while the sequence's length is still on its way, from which
-// the number of its own pieces follows (one behind the other, with the weights through shared memory: 10.7 us for 8
-// sequences of 32 heads in up to 32 pieces, 4.9 so; one sequence of 16 heads in 4 splits 4.1, in 11 pieces 3.5 so).
+// reads is asked for at once: the first splits' values beside all maxima and sums (one behind the other, with the weights
+// through shared memory, and so; attention and merge in a chain, us: one sequence of 4096 keys, 32 heads of 128 in 16 splits 13.4
+// and 11.6, one of 4096 latents in 16 splits 28.0 and 21.9, 24 of 1500 in 5 splits 30.1 and 25.8).
 constexpr int MERGE_MAX_SPLITS = 256;
 constexpr int MERGE_THREADS = 512;
 constexpr int MERGE_AHEAD = 8;    // splits whose values are asked for ahead
@@ -406,16 +405,11 @@ __global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(AttnParamsX p
     const int head = blockIdx.x, seq = blockIdx.y, lane = threadIdx.x & 31, c = threadIdx.x;
     const float* sp = p.scratch + ((int64_t)seq * p.heads + head) * p.num_splits * (d + 2);
     const float* column = sp + 2 + (c < d ? c : 0);
-    int n = p.num_splits;
-    float m = lane < n ? sp[(int64_t)lane * (d + 2)] : -INFINITY, l = lane < n ? sp[(int64_t)lane * (d + 2) + 1] : 0.f;
+    const int n = p.num_splits;
+    const float m = lane < n ? sp[(int64_t)lane * (d + 2)] : -INFINITY, l = lane < n ? sp[(int64_t)lane * (d + 2) + 1] : 0.f;
     float v[MERGE_AHEAD];
 #pragma unroll
     for (int j = 0; j < MERGE_AHEAD; j++) v[j] = j < n ? column[(int64_t)j * (d + 2)] : 0.f;
-    if (p.piece_tiles > 0) {
-        n = attn_pieces(attn_decode_span(p, p.seq_kv_len[seq] - 1).n_tiles, p.piece_tiles, p.num_splits);
-        if (n == 1) return;   // written by the attention kernel itself
-        if (lane >= n) m = -INFINITY;
-    }
     float M = m;
     for (int s = lane + 32; s < n; s += 32) M = fmaxf(M, sp[(int64_t)s * (d + 2)]);
     M = warp_max(M);
@@ -562,7 +556,6 @@ GB_API int gb_attention_simt(const AttnParams* pp, int dtype, cudaStream_t strea
 
 GB_API int gb_attention_simt_x(const AttnParamsX* pp, int dtype, cudaStream_t stream) {
     AttnParamsX p = *pp;
-    p.piece_tiles = 0;   // here every sequence is cut into num_splits
     if (p.nseq <= 0 || p.max_q_len <= 0) return 0;
     if (p.heads <= 0 || p.kv_heads <= 0 || p.heads % p.kv_heads) GB_REFUSE("attention: %d heads over %d kv heads", p.heads, p.kv_heads);
     if (p.d <= 0 || p.d > SIMT_MAX_D) GB_REFUSE("attention_simt: head_dim %d is outside [1, %d]", p.d, SIMT_MAX_D);

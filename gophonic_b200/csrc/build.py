@@ -62,7 +62,7 @@ SOURCES = [
     "no_alloc.cu",
     "dispatch.cu",
 ]
-HEADERS = ["common.cuh", "mma.cuh", "tc5.cuh", "no_alloc.h", "api.h", "attention_pieces.cuh"]
+HEADERS = ["common.cuh", "mma.cuh", "tc5.cuh", "no_alloc.h", "api.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -16,12 +16,11 @@ from typing import Dict, Optional, Tuple
 
 import torch
 
-from ..parts.attention import context_class
 from .step import StepBatch
 
 
 class DecodeGraph:
-    def __init__(self, engine, nseq: int, plans, max_kv_len: int, pool):
+    def __init__(self, engine, nseq: int, plans, pool):
         # the engine owns its graphs; a strong reference back would make a cycle, and an engine
         # dropped by its user would then be freed by the collector at some later time, perhaps in
         # the middle of another engine's capture, where freeing device memory is an error
@@ -32,7 +31,7 @@ class DecodeGraph:
         self.meta = torch.zeros(8 * nseq, dtype=torch.int32, device=dev)
         n = nseq
         m = self.meta
-        self.batch = StepBatch(rows=n, nseq=n, max_q_len=1, max_kv_len=max_kv_len, ids=m[:n], row_pos=m[n:2 * n],
+        self.batch = StepBatch(rows=n, nseq=n, max_q_len=1, max_kv_len=0, ids=m[:n], row_pos=m[n:2 * n],
                                row_seq=m[2 * n:3 * n], seq_slot=m[3 * n:4 * n], seq_q_start=m[4 * n:5 * n],
                                seq_q_len=m[5 * n:6 * n], seq_kv_len=m[6 * n:7 * n], device=dev,
                                sm_count=engine.sm_count, plans=engine.model.bind_plans(plans))
@@ -101,18 +100,18 @@ class DecodeGraphs:
 
     def get(self, nseq: int, max_kv_len: int) -> DecodeGraph:
         """The captured step that serves ``nseq`` sequences which see at most ``max_kv_len`` keys: one
-        graph per captured batch size, per answer of the model's mixers to ``plan`` (whatever
-        those answers are) and per class of the longest context.  At most ``max_graphs`` graphs are kept; the one unused longest goes."""
+        graph per captured batch size and per answer of the model's mixers to ``plan`` (whatever
+        those answers are).  At most ``max_graphs`` graphs are kept; the one unused longest goes."""
         eng = self.engine
         size = min(captured_size(nseq), max(self.max_batch, nseq))
         plans = eng.model.step_plans(size, 1, max_kv_len, eng.sm_count)
-        key = (size, plans, context_class(max_kv_len))
+        key = (size, plans)
         g = self.graphs.pop(key, None)
         if g is None:
             if self.pool is None:
                 self.pool = torch.cuda.graph_pool_handle()
             while len(self.graphs) >= self.max_graphs:
                 self.graphs.pop(next(iter(self.graphs)))
-            g = DecodeGraph(eng, size, plans, key[2], self.pool)
+            g = DecodeGraph(eng, size, plans, self.pool)
         self.graphs[key] = g
         return g

@@ -640,7 +640,7 @@ class _AttnParams(Structure):
         ("seq_kv_len", c_void_p), ("nseq", c_int), ("heads", c_int), ("kv_heads", c_int), ("d", c_int),
         ("max_q_len", c_int), ("scale", c_float), ("window", c_int), ("num_splits", c_int), ("scratch", c_void_p),
         ("pages", c_int), ("max_slots", c_int), ("dv", c_int), ("keep_first", c_int), ("sink", c_int), ("sinks", c_void_p),
-        ("chunk", c_int), ("v_share", c_int), ("v_row_stride", c_int64), ("piece_tiles", c_int), ("piece_reserved", c_int),
+        ("chunk", c_int), ("v_share", c_int), ("v_row_stride", c_int64),
     ]
 
 
@@ -653,16 +653,14 @@ def _attn_params(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_pl
                  seq_q_len: torch.Tensor, seq_kv_len: torch.Tensor, nseq: int, max_q_len: int,
                  heads: int, kv_heads: int, head_dim: int, scale: float, window: int,
                  num_splits: int, scratch: Optional[torch.Tensor], value_dim: Optional[int] = None, keep_first: int = 0,
-                 sink: bool = False, sinks: Optional[torch.Tensor] = None, chunk: int = 0, v_share: int = 1, piece_pages: int = 0) -> "_AttnParams":
+                 sink: bool = False, sinks: Optional[torch.Tensor] = None, chunk: int = 0, v_share: int = 1) -> "_AttnParams":
     """``value_dim``: size of a value head if it is not ``head_dim``; ``keep_first``: with a window, keys
     at positions below it stay visible; ``sink``: one more unit in the softmax denominator; ``sinks``
     (float32 [heads]): head h's denominator holds exp(sinks[h]) instead of that unit; ``chunk`` > 0: row i
     sees key j <= i only if both lie in the same block of ``chunk`` positions counted from the sequence's
     start; ``v_share`` > 1: that many consecutive key heads read one value head (the value plane holds
     kv_heads / v_share heads).  The value plane may be a view whose tokens lie further apart than
-    ``value_dim`` (the first channels of a wider plane, the key plane itself for instance); ``piece_pages`` > 0
-    (single tokens on the tensor cores): every sequence is cut by its own length into pieces of that many cache pages, or
-    of more where they were more than ``num_splits``."""
+    ``value_dim`` (the first channels of a wider plane, the key plane itself for instance)."""
     _need(q, "attention q", dim=2, contiguous=False)
     _need(out, "attention out", q.dtype, 2, contiguous=False)
     dv = head_dim if value_dim is None else int(value_dim)
@@ -703,7 +701,7 @@ def _attn_params(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_pl
                     head_dim, max_q_len, scale, window, num_splits, 0 if scratch is None else scratch.data_ptr(),
                     k_plane.shape[0], block_table.shape[0], 0 if dv == head_dim else dv, int(keep_first) if window > 0 else 0,
                     1 if sink or sinks is not None else 0, 0 if sinks is None else sinks.data_ptr(),
-                    int(chunk), v_share, 0 if v_tok == dv else v_tok, int(piece_pages))
+                    int(chunk), v_share, 0 if v_tok == dv else v_tok)
     return p
 
 
@@ -713,11 +711,11 @@ def attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_plane
               heads: int, kv_heads: int, head_dim: int, scale: float, window: int = 0,
               num_splits: int = 1, scratch: Optional[torch.Tensor] = None, algo: str = "auto",
               value_dim: Optional[int] = None, keep_first: int = 0, sink: bool = False, sinks: Optional[torch.Tensor] = None,
-              chunk: int = 0, v_share: int = 1, piece_pages: int = 0) -> str:
+              chunk: int = 0, v_share: int = 1) -> str:
     """Causal GQA over the paged cache.  q is a [rows, >= heads*head_dim] view (row stride free),
     out is [rows, heads*value_dim].  Returns the kernel's name."""
     p = _attn_params(q, out, k_plane, v_plane, block_table, seq_slot, seq_q_start, seq_q_len, seq_kv_len, nseq, max_q_len,
-                     heads, kv_heads, head_dim, scale, window, num_splits, scratch, value_dim, keep_first, sink, sinks, chunk, v_share, piece_pages)
+                     heads, kv_heads, head_dim, scale, window, num_splits, scratch, value_dim, keep_first, sink, sinks, chunk, v_share)
     if algo == "auto":   # the library's own rule (head size, rows per sequence, alignment)
         algo = ("simt", "decode_mma", "prefill_mma", "prefill_tc5", "latent_mma")[int(_lib.gb_attention_algo_x(byref(p), _code(q.dtype)))]
     nk = 2 if num_splits > 1 else 1
@@ -792,16 +790,16 @@ def attention_decode_rope_accepts(dtype: torch.dtype, head_dim: int, rotary_dim:
     return dtype in (torch.float32, torch.bfloat16) and bool(_lib.gb_attention_decode_rope_accepts(_code(dtype), c_int(head_dim), c_int(rotary_dim), c_int(max_q_len)))
 
 
-def attention_decode_rope(qkv: torch.Tensor, out: torch.Tensor, rope_args: tuple, attn_args: tuple, piece_pages: int = 0) -> None:
+def attention_decode_rope(qkv: torch.Tensor, out: torch.Tensor, rope_args: tuple, attn_args: tuple) -> None:
     """``qk_norm_rope_kv_write(qkv, *rope_args)`` and ``attention(qkv[:, :heads * head_dim], out,
     *attn_args)`` for single-token rows in one kernel (plus the merge of key splits): the attention
     kernel norms and rotates its queries itself, takes the token's own key and value from the row and
-    stores them in the cache.  The same bits as the two calls.  Without key splits, and with ``piece_pages``, it asks for the pages of earlier tokens
+    stores them in the cache.  The same bits as the two calls.  Without key splits it asks for the pages of earlier tokens
     while the launch directly ahead may still run: that one must not write this cache (the product that makes ``qkv``, which stands
     between two tokens of a sequence, does not)."""
     r = _rope_params(qkv, *rope_args)
-    a = _attn_params(qkv[:, :r.heads * r.d], out, *attn_args, piece_pages=piece_pages)
-    _check(_lib.gb_attention_decode_mma_rope_x(byref(a), byref(r), _stream()), 2 if a.num_splits > 1 else 1)
+    a = _attn_params(qkv[:, :r.heads * r.d], out, *attn_args)
+    _check(_lib.gb_attention_decode_mma_rope(byref(a), byref(r), _stream()), 2 if a.num_splits > 1 else 1)
 
 
 # ---- mixers with a matrix state ------------------------------------------------------------

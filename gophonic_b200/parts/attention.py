@@ -16,7 +16,7 @@ from typing import List, Mapping, Optional
 import torch
 
 from .. import registry
-from .base import FOLD_ROWS, KVRequest, Mixer, RowStats, Runtime, TensorDecl, fold_weight, other_fold_buffers
+from .base import KVRequest, Mixer, RowStats, Runtime, TensorDecl, fold_weight, other_fold_buffers
 
 
 def choose_splits(units: int, max_kv_len: int, sm_count: int = 148, page_bytes: int = 32768) -> int:
@@ -68,47 +68,6 @@ def few_splits(units: int, max_kv_len: int, sm_count: int = 148) -> int:
     while 2 * s <= min(max_kv_len // 96, sm_count // max(1, units), 32):
         s *= 2
     return s
-
-
-# Lines in the longest context of a step, on either side of which single tokens are cut differently; captured steps are kept apart by
-# them.  Up to the first the plan decides: a sequence of one piece would pay for a merge that has nothing to do (32 of 300 keys:
-# 10.4 us by the plan, 14.5 otherwise).
-CONTEXT_LINES = (512, 2048)
-
-
-def context_class(max_kv_len: int) -> int:
-    """The smallest of ``CONTEXT_LINES`` that holds ``max_kv_len``, or the last one's successor."""
-    return next((n for n in CONTEXT_LINES if max_kv_len <= n), CONTEXT_LINES[-1] + 1)
-
-
-def token_pieces(nseq: int, max_kv_len: int):
-    """(pages a piece, most pieces a sequence) for single tokens whose sequences are cut by their own lengths, or None where the plan
-    decides: short pieces where few sequences have to fill the GPU, longer ones where there are many; never more than four of more
-    than four sequences, since a CTA costs some 5 us beside 1.4 a page (8 sequences of 4096 keys: 30.2 us in four pieces, as by the
-    plan, 35.0 in eight), and none of more than eight beyond 2048 keys (64 of 4096: 172 us uncut, 190 in four) nor of more than
-    64, whose layers the library issues in one call by the plan.  Unequal
-    sequences, attention and merge, by the plan and so: 50 of 118 to 1900 keys 42.7 and 37.3, 16 of 93 to 1500 23.6 and 16.4, 8
-    of 256 to 4096 26.6 and 24.6, one of 700 8.0 and 7.6.  The lines lie at batch sizes that steps are captured at, so that a
-    step of nine and the one of twelve that is replayed for it cut alike."""
-    line = context_class(max_kv_len)
-    if line == CONTEXT_LINES[0] or nseq > FOLD_ROWS or (line > CONTEXT_LINES[-1] and nseq > 8):
-        return None
-    return (2, 16) if nseq <= 2 else (3, 8) if nseq <= 4 else (8, 4) if nseq <= 8 else (6, 4) if nseq <= 32 else (10, 4)
-
-
-def key_pieces(part, batch, heads: int, head_dim: int, value_dim: int):
-    """(pieces at most, scratch for their partial results or None, pages a piece or 0) for this step: single tokens in bfloat16 are cut
-    sequence by sequence where ``token_pieces`` says so, whatever the plan says; the others, and what the tensor-core kernel
-    does not take, by the plan."""
-    ops = part.rt.ops
-    pieces = None
-    if not part.rt.is_fp32 and value_dim == head_dim and ops.attention_decode_rope_accepts(torch.bfloat16, head_dim, 0, batch.max_q_len):
-        pieces = token_pieces(batch.nseq, batch.max_kv_len)
-    if pieces is None:
-        return part.key_splits(batch) + (0,)
-    pages, most = pieces
-    floats = ops.attention_scratch_floats(batch.nseq, heads, value_dim, most)
-    return most, batch.workspace(("attention key splits", heads, value_dim, most), floats), pages
 
 
 class Attention(Mixer):
@@ -234,13 +193,13 @@ class Attention(Mixer):
         rope_args = (s.heads, s.kv_heads, s.head_dim, self.q_norm, self.k_norm, self.eps, cos, sin, rot, batch.row_pos,
                      batch.row_seq, batch.seq_slot, cache.block_table, cache.k, cache.v, cache.writable)
         ctx = torch.empty((rows, self.q_dim), dtype=x.dtype, device=x.device)
-        splits, scratch, pages = key_pieces(self, batch, s.heads, s.head_dim, s.head_dim)
+        splits, scratch = self.key_splits(batch)
         attn_args = (cache.k, cache.v, cache.block_table, batch.seq_slot, batch.seq_q_start, batch.seq_q_len, batch.seq_kv_len,
                      batch.nseq, batch.max_q_len, s.heads, s.kv_heads, s.head_dim, float(s.scale), int(s.window), splits, scratch)
         if ops.attention_decode_rope_accepts(x.dtype, s.head_dim, rot, batch.max_q_len):
             # single tokens: the attention kernel norms and rotates its queries and places the token's key and value itself
-            ops.attention_decode_rope(qkv, ctx, rope_args, attn_args, piece_pages=pages)
+            ops.attention_decode_rope(qkv, ctx, rope_args, attn_args)
         else:
             ops.qk_norm_rope_kv_write(qkv, *rope_args)
-            ops.attention(qkv[:, :self.q_dim], ctx, *attn_args, piece_pages=pages)
+            ops.attention(qkv[:, :self.q_dim], ctx, *attn_args)
         return ctx

@@ -19,7 +19,7 @@ from typing import List, Mapping
 import torch
 
 from .. import registry
-from .attention import choose_splits, key_pieces
+from .attention import choose_splits
 from .base import KVRequest, Mixer, Runtime, TensorDecl
 
 
@@ -119,10 +119,10 @@ class DiffAttention(Mixer):
                                   batch.row_pos, batch.row_seq, batch.seq_slot, cache.block_table, cache.k, cache.v, cache.writable,
                                   pairs=bool(getattr(self.position, "pairs", False)), value_dim=s.value_dim, v_share=self.MAPS)
         maps = torch.empty((rows, self.q_heads * s.value_dim), dtype=x.dtype, device=x.device)
-        splits, scratch, pages = key_pieces(self, batch, self.q_heads, s.head_dim, s.value_dim)
+        splits, scratch = self.key_splits(batch)
         ops.attention(qkv, maps, cache.k, cache.v, cache.block_table, batch.seq_slot, batch.seq_q_start, batch.seq_q_len, batch.seq_kv_len,
                       batch.nseq, batch.max_q_len, self.q_heads, self.k_heads, s.head_dim, float(s.scale), int(s.window), splits, scratch,
-                      value_dim=s.value_dim, chunk=int(s.chunk), v_share=self.MAPS, piece_pages=pages)
+                      value_dim=s.value_dim, chunk=int(s.chunk), v_share=self.MAPS)
         ctx = torch.empty((rows, s.heads * s.value_dim), dtype=x.dtype, device=x.device)
         ops.diff_combine(maps, ctx, s.heads, self.per_group, s.value_dim, self.lam, float(s.eps), 1.0 - float(s.lambda_init))
         ops.gemm(ctx, self.o, out)

@@ -20,7 +20,7 @@ from typing import List, Mapping
 import torch
 
 from .. import registry
-from .attention import Attention, key_pieces
+from .attention import Attention
 from .base import KVRequest, KVStateRequest, Runtime, StateRequest, TensorDecl
 from .rope import scaled_magnitude
 
@@ -225,11 +225,11 @@ class GatedAttention(Attention):
                                       pairs=bool(getattr(self.position, "pairs", False)), value_dim=s.value_dim, span=self.norm_span,
                                       value_from_key=self.value_from_key)
         ctx = torch.empty((rows, self.o_dim), dtype=x.dtype, device=x.device)
-        splits, scratch, pages = key_pieces(self, batch, s.heads, s.head_dim, s.value_dim)
+        splits, scratch = self.key_splits(batch)
         ops.attention(q, ctx, cache.k, cache.v, cache.block_table, batch.seq_slot, batch.seq_q_start, batch.seq_q_len,
                       batch.seq_kv_len, batch.nseq, batch.max_q_len, s.heads, s.kv_heads, s.head_dim, float(s.scale), int(s.window),
                       splits, scratch, value_dim=s.value_dim, keep_first=int(s.keep_first), sink=bool(s.sink) or self.sinks is not None,
-                      sinks=self.sinks, piece_pages=pages)
+                      sinks=self.sinks)
         if s.gate:
             ops.head_norm_gate(ctx, qkvg[:, self.g_off:self.g_off + self.o_dim], ctx, s.heads, s.value_dim, ops.GATE_SIGMOID)
         return ctx

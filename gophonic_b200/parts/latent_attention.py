@@ -105,16 +105,6 @@ class LatentAttention(Mixer):
         return splits, batch.workspace(("attention key splits", s.heads, s.kv_rank, splits),
                                        self.rt.ops.attention_scratch_floats(batch.nseq, s.heads, s.kv_rank, splits))
 
-    def key_pieces(self, batch, nseq: int, most_rows: int):
-        """(pieces at most, scratch or None, pages a piece or 0): single tokens in bfloat16 are cut by each sequence's own length,
-        short pieces where there are few sequences (an SM holds one CTA)."""
-        s = self.spec
-        if self.rt.is_fp32 or most_rows != 1 or s.kv_rank not in (64, 128, 256, 512) or self.key_dim % 16 or self.key_dim > 640:
-            return self.key_splits(batch) + (0,)
-        pages, most = (1 if nseq <= 8 else 2 if nseq <= 32 else 4), (32 if nseq <= 8 else 16 if nseq <= 32 else 8)
-        return most, batch.workspace(("attention key splits", s.heads, s.kv_rank, most),
-                                     self.rt.ops.attention_scratch_floats(nseq, s.heads, s.kv_rank, most)), pages
-
     def _per_head(self, a: torch.Tensor, w_kn: torch.Tensor, w_nk: torch.Tensor, out: torch.Tensor) -> None:
         """out[:, h, :] = a[:, h, :] @ w_kn[h] for every head (``w_nk`` holds the same matrices transposed)."""
         ops = self.rt.ops
@@ -222,9 +212,9 @@ class LatentAttention(Mixer):
         self._per_head(q.view(rows, H, d + dr)[:, :, :d], self.uk_kn, self.uk_nk, qa.view(rows, H, self.key_dim)[:, :, :R])
         ops.latent_q_rot(q, qa, H, d, dr, cos, sin, row_pos)
         mixed = torch.empty((rows, H * R), dtype=q.dtype, device=q.device)               # per head sum_j p_j c_j
-        splits, scratch, pages = self.key_pieces(batch, end - first, most)
+        splits, scratch = self.key_splits(batch)
         ops.attention(qa, mixed, cache.k, cache.v, cache.block_table, slot, q_start, q_len, kv_len, end - first, most, H, 1, self.key_dim,
-                      float(s.scale), int(s.window), splits, scratch, value_dim=R, chunk=int(s.chunk), piece_pages=pages)
+                      float(s.scale), int(s.window), splits, scratch, value_dim=R, chunk=int(s.chunk))
         self._per_head(mixed.view(rows, H, R), self.uv_kn, self.uv_nk, ctx.view(rows, H, dv))
 
     def forward(self, batch, x: torch.Tensor, out: torch.Tensor, cache) -> None:

@@ -702,6 +702,15 @@ def test_single_token_attention_that_rotates_and_stores_the_token_itself(ops, he
     assert torch.equal(k_a, k0) != write and torch.equal(v_a, v0) != write
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,kvh,d", [(4, 2, 32), (16, 2, 128), (2, 1, 256)])
+@pytest.mark.parametrize("splits", [2, 9, 32, 33, 70, 256])
+def test_partial_results_of_many_key_splits_are_joined(ops, dtype, heads, kvh, d, splits):
+    """Fewer pieces than are asked for ahead, one for every lane of a warp, and more than that; most of them empty where a sequence is short."""
+    out, ref, _ = attention_case(ops, dtype, heads, kvh, d, q_lens=[1] * 4, kv_lens=[1, 640, 2113, 2600], splits=splits)
+    close(out, ref, tol_of(dtype))
+
+
 @pytest.mark.parametrize("heads,kvh,d,dv", [(4, 2, 16, 16), (32, 8, 128, 128), (2, 2, 256, 256), (16, 1, 96, 64), (6, 3, 24, 24)])
 def test_partial_results_of_key_splits_may_begin_at_any_float(ops, heads, kvh, d, dv):
     """Scratch is floats: the bits do not depend on where it begins (the tensor-core kernels' single tokens and latents, the CUDA cores)."""
@@ -722,74 +731,6 @@ def test_partial_results_of_key_splits_may_begin_at_any_float(ops, heads, kvh, d
         outs.append(out)
     assert used == ("latent_mma" if dv != d else "simt" if d % 16 else "decode_mma")
     assert torch.isfinite(outs[0].float()).all() and torch.equal(*outs)
-
-
-@pytest.mark.parametrize("heads,kvh,d", [(4, 2, 16), (32, 8, 128), (20, 1, 32), (2, 2, 256)])
-@pytest.mark.parametrize("pages,most", [(1, 32), (2, 8), (4, 2)])
-@pytest.mark.parametrize("opts", [{}, {"window": 100}, {"window": 130, "keep_first": 70, "sink": True}, {"chunk": 256}])
-def test_single_tokens_cut_by_their_own_lengths(ops, heads, kvh, d, pages, most, opts):
-    """Pieces of a fixed number of pages, more of them the longer the sequence: lengths at the edges of pages and pieces, more
-    pieces than the GPU has places, the options of the uncut kernel.  The uncut kernel's result but for roundings to bfloat16,
-    2^-9 on either side: of every weight, whose reference point is the largest score of its own piece (together at most that
-    share of the weighted mean of |v|), and of the result; and the bits of the sequence alone."""
-    kv_lens = [1, 64, 65, 128, 129, 257, 700, 333, 2049, 512] * 6
-    nseq, n_pages = len(kv_lens), sum((n + 63) // 64 for n in kv_lens)
-    stride = max((n + 63) // 64 for n in kv_lens)
-    perm = torch.randperm(n_pages, generator=torch.Generator().manual_seed(3)).to(torch.int32)
-    table, at = torch.zeros((nseq, stride), dtype=torch.int32), 0
-    for i, n in enumerate(kv_lens):
-        table[i, :(n + 63) // 64] = perm[at:at + (n + 63) // 64]
-        at += (n + 63) // 64
-    table = table.to(DEV)
-    k, v = paged(n_pages, kvh, d, torch.bfloat16, 4)
-    q = rnd(nseq, heads * d, dtype=torch.bfloat16, seed=6)
-    mk = lambda x: torch.tensor(list(x), dtype=torch.int32, device=DEV)
-
-    def run(seqs, splits, v=v, **more):
-        n = len(seqs)
-        out = torch.full((n, heads * d), float("nan"), dtype=torch.bfloat16, device=DEV)
-        scratch = torch.full((ops.attention_scratch_floats(n, heads, d, splits),), float("nan"), device=DEV) if splits > 1 else None
-        ops.attention(q[seqs].contiguous(), out, k, v, table, mk(seqs), mk(range(n)), mk([1] * n), mk(kv_lens[i] for i in seqs), n, 1, heads, kvh, d,
-                      d ** -0.5, opts.get("window", 0), splits, scratch, algo="decode_mma", keep_first=opts.get("keep_first", 0),
-                      sink=opts.get("sink", False), chunk=opts.get("chunk", 0), **more)
-        return out
-
-    everyone = list(range(nseq))
-    got = run(everyone, most, piece_pages=pages)
-    want = run(everyone, 1).float()
-    size = run(everyone, 1, v=v.abs()).float()
-    assert torch.isfinite(got.float()).all()
-    assert ((got.float() - want).abs() <= 2.0 ** -8 * (size + want.abs()) + 1e-5).all()
-    for i in range(0, 10):
-        assert torch.equal(run([i], most, piece_pages=pages)[0], got[i]), kv_lens[i]
-
-
-@pytest.mark.parametrize("heads,kvh,d,rot", [(32, 8, 128, 128), (5, 1, 48, 32), (2, 2, 256, 256)])
-@pytest.mark.parametrize("window", [0, 100])
-def test_pieces_rotate_and_store_the_token_as_the_two_kernels_do(ops, heads, kvh, d, rot, window):
-    kv_lens = [1, 64, 65, 700, 333, 128] * 8
-    nseq, stride = len(kv_lens), 11
-    table = torch.randperm(nseq * stride, generator=torch.Generator().manual_seed(5)).to(torch.int32).reshape(nseq, stride).to(DEV)
-    k0, v0 = paged(nseq * stride, kvh, d, torch.bfloat16, 11)
-    qkv0 = rnd(nseq, (heads + 2 * kvh) * d, dtype=torch.bfloat16, seed=12)
-    qw, kw = 1 + 0.1 * rnd(d, seed=13), 1 + 0.1 * rnd(d, seed=14)
-    cos, sin = torch.cos(rnd(800, rot // 2, seed=15)), torch.sin(rnd(800, rot // 2, seed=15))
-    mk = lambda x: torch.tensor(list(x), dtype=torch.int32, device=DEV)
-    pos, seqs = mk([n - 1 for n in kv_lens]), mk(range(nseq))
-    scratch = torch.empty(ops.attention_scratch_floats(nseq, heads, d, 8), dtype=torch.float32, device=DEV)
-    results = []
-    for fused in (False, True):
-        qkv, k, v = qkv0.clone(), k0.clone(), v0.clone()
-        out = torch.full((nseq, heads * d), float("nan"), dtype=torch.bfloat16, device=DEV)
-        rope_args = (heads, kvh, d, qw, kw, 1e-6, cos, sin, rot, pos, seqs, seqs, table, k, v, True)
-        attn_args = (k, v, table, seqs, seqs, mk([1] * nseq), mk(kv_lens), nseq, 1, heads, kvh, d, d ** -0.5, window, 8, scratch)
-        if fused:
-            ops.attention_decode_rope(qkv, out, rope_args, attn_args, piece_pages=2)
-        else:
-            ops.qk_norm_rope_kv_write(qkv, *rope_args)
-            ops.attention(qkv[:, :heads * d], out, *attn_args, algo="decode_mma", piece_pages=2)
-        results.append((out, k, v))
-    assert all(torch.equal(a, b) for a, b in zip(*results))
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

@@ -4,9 +4,9 @@ from types import SimpleNamespace
 import pytest
 import torch
 
+from gophonic_b200.engine import graphs
 from gophonic_b200.engine.step import build_batch
-from gophonic_b200.engine.graphs import captured_size
-from gophonic_b200.parts.attention import Attention, choose_splits, context_class, few_splits, token_pieces
+from gophonic_b200.parts.attention import Attention, choose_splits, few_splits
 from gophonic_b200.parts.gated_attention import GatedAttention
 from gophonic_b200.parts.latent_attention import LatentAttention
 
@@ -69,10 +69,25 @@ def test_a_batch_of_one_size_asks_for_few_captured_steps():
         assert len({a.plan(n, 1, kv, 148) for kv in range(1, 8193, 7)}) <= most
 
 
-def test_a_step_and_the_captured_one_that_is_replayed_for_it_cut_alike():
-    for n in range(1, 129):
-        for kv in (1, 512, 513, 2048, 2049, 40000):
-            assert token_pieces(n, kv) == token_pieces(captured_size(n), kv) == token_pieces(n, context_class(kv))
+def captured_steps(monkeypatch, plan, nseq, contexts):
+    """How many steps are captured for ``nseq`` sequences as the longest of them grows, with mixers that answer ``plan``."""
+    monkeypatch.setattr(graphs, "DecodeGraph", lambda engine, size, plans, *more: object())
+
+    class Engine:
+        sm_count = 148
+        model = SimpleNamespace(step_plans=lambda *a: (plan(*a),))
+    engine = Engine()        # the graphs refer to it weakly
+    g = graphs.DecodeGraphs(engine, max_graphs=10 ** 6)
+    g.pool = object()
+    return len({id(g.get(nseq, kv)) for kv in contexts})
+
+
+@pytest.mark.parametrize("plan", [part().plan, part(fp32=True).plan, part(window=300).plan, lambda *a: None])
+def test_steps_are_captured_once_for_every_answer_of_the_plans(monkeypatch, plan):
+    contexts = range(1, 12289, 7)
+    for n in (1, 2, 8, 16, 24, 64):
+        answers = {plan(graphs.captured_size(n), 1, kv, 148) for kv in contexts}
+        assert captured_steps(monkeypatch, plan, n, contexts) == len(answers)
 
 
 # ---- latent attention: which sequences of a step go over expanded keys and values -------------------------
@@ -130,3 +145,48 @@ def test_the_rule_of_expanded_latents():
     assert [r[5] > 0 for r in runs_of([(0, 500), (2000, 3), (1200, 3)])] == [True]
     assert not expanded(0, 500, dtype=torch.float32) and not expanded(0, 500, dims=(64, 64, 128)) and not expanded(0, 500, kv_rank=516)
     assert runs_of([(0, 100), (9, 3)], dtype=torch.float32) == [(0, 2, 0, 103, 100, 0)]
+
+
+class RecordingOps:
+    """Stands for the kernels that latent attention calls; keeps what attention was asked for."""
+
+    def __init__(self):
+        from gophonic_b200 import ops
+        self.latent_expanded_accepts, self.LATENT_TC5_MIN_ROWS = ops.latent_expanded_accepts, ops.LATENT_TC5_MIN_ROWS
+        self.attention_scratch_floats = ops.attention_scratch_floats
+        self.cuts = []
+
+    def head_gemm_mma_accepts(self, *a):
+        return True
+
+    def head_gemm_mma(self, *a):
+        pass
+
+    latent_q_rot = head_gemm_mma
+
+    def attention(self, q, out, k, v, table, slot, q_start, q_len, kv_len, nseq, max_q_len, heads, kv_heads, dim, scale, window, splits, scratch, **more):
+        more.pop("value_dim"), more.pop("chunk")
+        self.cuts.append((max_q_len, splits, sorted(more)))
+
+
+def test_a_mixed_steps_single_rows_are_cut_alike_whatever_their_neighbours_hold():
+    """A row that joins other sequences' rows in a step is attended to in one pass over its keys: nothing follows from how many of the others
+    have long contexts, or from how many rows they bring."""
+    prompt = [(0, 1500)]
+    cuts = []
+    for others in ([(1300, 1)] * 10, [(1300, 1)] * 3 + [(100, 1)] * 7, [(1300, 1)] * 9 + [(1300, 2)]):
+        p = object.__new__(LatentAttention)
+        p.spec = SimpleNamespace(heads=4, head_dim=128, rot_dim=64, value_dim=128, kv_rank=512, window=0, chunk=0, scale=1.0)
+        p.rt = SimpleNamespace(ops=RecordingOps(), act_dtype=torch.bfloat16, is_fp32=False)
+        p.key_dim, p.position = 576, SimpleNamespace(kernel_args=lambda: (None, None, 64))
+        p.uk_kn = p.uv_nk = p.uk_nk = p.uv_kn = torch.empty(0, dtype=torch.bfloat16)
+        batch, _ = build_batch([(i, [5] * rows, known) for i, (known, rows) in enumerate(prompt + others)], torch.device("cpu"))
+        q = torch.empty((batch.rows, 4 * 192), dtype=torch.bfloat16)
+        ctx = torch.empty((batch.rows, 4 * 128), dtype=torch.bfloat16)
+        cache = SimpleNamespace(k=torch.empty((1, 1, 64, 576), dtype=torch.bfloat16), v=None, block_table=None)
+        runs = [r for r in LatentAttention.runs(p, batch) if not r[5]]
+        assert runs                          # rows behind many pages stay on the latents
+        for run in runs:
+            LatentAttention._absorbed(p, batch, q, ctx, cache, run)
+        cuts += p.rt.ops.cuts
+    assert cuts and all((splits, more) == (1, []) for _, splits, more in cuts)
