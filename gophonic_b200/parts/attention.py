@@ -62,12 +62,57 @@ def choose_splits(units: int, max_kv_len: int, sm_count: int = 148, page_bytes: 
 def few_splits(units: int, max_kv_len: int, sm_count: int = 148) -> int:
     """Into how many pieces at least, beside ``choose_splits``, a step of few sequences cuts its keys: a power of two (the count then
     changes as seldom as the context doubles, and a changed count means another captured step), as long as a CTA an SM
-    takes all pieces, there are no more than 32 and a piece keeps at least 96 keys.  Whole steps (1.7B sizes), us, in pieces of at
-    least 256 keys and in these: one sequence of 700 keys 1248 and 1186, of 1500 1217 and 1207, four of 1000 1329 and 1284."""
+    takes all pieces, there are no more than 32 and a piece keeps at least 96 keys.  (From 512 keys on ``wave_splits`` goes further
+    but for the longest contexts of very few key heads: one of 4096 keys over two key heads, attention and merge, 11.7 us in 32 pieces.)"""
     s = 1
     while 2 * s <= min(max_kv_len // 96, sm_count // max(1, units), 32):
         s *= 2
     return s
+
+
+def page_class(pages: int) -> int:
+    """``pages`` or up to a half more: 1, 2, 3, 4, 6, 8, 12, 16, 24, ... (counts that follow from it change seldom)."""
+    size = 1
+    while True:
+        for cand in (size, size + size // 2):
+            if pages <= cand:
+                return cand
+        size *= 2
+
+
+def wave_splits(splits: int, units: int, heads: int, seen: int, places: int) -> int:
+    """``splits``, or into how many more pieces single tokens behind more than 512 visible keys are cut by the tensor-core kernel:
+    ``units`` CTAs if uncut, ``heads`` heads of all sequences together, ``places`` CTAs that the GPU holds at once.
+
+    As many pieces as run in one wave, for equal sequences the best number at every length (8 of eight key heads, us: 600 keys 13.1 in
+    two, 12.4 in four, 16.6 in eight; 4096 keys 30.2 in four, 33.4 in eight), but no more than 16, and no more than keep the partial results
+    of all heads to four a place, since the merge reads them all (8 of 1500 over two key heads of 16 heads each: 12.9 in eight, 13.8 in
+    twelve).  A page takes a CTA a little over 1 us, a piece more of every sequence some 0.2, so more pieces have to save a CTA two pages
+    (2 of 900 in eight 9.2, in sixteen 9.7), or one page for a single piece more; the first cut, which brings the merge, five.
+    Where not even two pieces fit, three fill two waves of up to 197 units, if a piece has eight pages.
+    Whole steps, 1.7B sizes, against ``choose_splits`` and ``few_splits`` alone: one sequence of 700 keys -4 %, five of 700 -6, of 4000 0, 12 of 700
+    -3, 16 of 700 -3, 24 of 1500 -1 if they are equal and -11 if they are not."""
+    pages = (seen + 63) // 64
+    if pages <= 8:
+        return splits
+    if 2 * units > places:
+        return max(splits, 3) if 3 * units <= 2 * places and 3 * heads <= 8 * places and pages >= 24 else splits
+    most = min(16, places // max(1, units), 4 * places // max(1, heads))
+    if most <= splits:
+        return splits
+    size = page_class(pages)
+    more = most if pages <= most else -(-size // -(-size // most))       # a page a piece, or pieces of as many whole pages as it takes
+    saved = -(-pages // splits) - -(-pages // more)
+    return more if saved >= (5 if splits == 1 else 2) or (saved == 1 and more == splits + 1) else splits
+
+
+def token_splits(splits: int, part, nseq: int, heads: int, kv_heads: int, value_dim: int, seen: int, sm_count: int) -> int:
+    """``splits`` or more, where the tensor-core single-token kernel takes ``part``'s heads (``wave_splits``)."""
+    d = part.spec.head_dim
+    if part.rt.is_fp32 or value_dim != d or d % 16 or not (d <= 128 or d == 256):
+        return splits
+    units = nseq * kv_heads * -(-heads // (16 * kv_heads))      # a CTA holds up to 16 heads of a key head
+    return wave_splits(splits, units, nseq * heads, seen, sm_count * (2 if d <= 128 else 1))
 
 
 class Attention(Mixer):
@@ -125,7 +170,8 @@ class Attention(Mixer):
         if self.rt.is_fp32:
             return splits
         seen = min(max_kv_len, self.spec.window) if self.spec.window > 0 else max_kv_len
-        return max(splits, few_splits(nseq * self.spec.kv_heads, seen, sm_count))
+        splits = max(splits, few_splits(nseq * self.spec.kv_heads, seen, sm_count))
+        return token_splits(splits, self, nseq, self.spec.heads, self.spec.kv_heads, self.spec.head_dim, seen, sm_count)
 
     def splits_of(self, nseq: int, max_kv_len: int, sm_count: int) -> int:
         elem = 4 if self.rt.is_fp32 else 2

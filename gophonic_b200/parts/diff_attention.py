@@ -19,7 +19,7 @@ from typing import List, Mapping
 import torch
 
 from .. import registry
-from .attention import choose_splits
+from .attention import choose_splits, token_splits
 from .base import KVRequest, Mixer, Runtime, TensorDecl
 
 
@@ -95,7 +95,9 @@ class DiffAttention(Mixer):
             return 1
         elem = 4 if self.rt.is_fp32 else 2
         page_bytes = 64 * (self.spec.head_dim + self.spec.value_dim) * elem
-        return choose_splits(nseq * self.k_heads, self._seen(max_kv_len), sm_count, page_bytes)
+        seen = self._seen(max_kv_len)
+        splits = choose_splits(nseq * self.k_heads, seen, sm_count, page_bytes)
+        return token_splits(splits, self, nseq, self.q_heads, self.k_heads, self.spec.value_dim, seen, sm_count)
 
     def key_splits(self, batch):
         s = self.spec

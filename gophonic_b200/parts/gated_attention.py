@@ -20,7 +20,7 @@ from typing import List, Mapping
 import torch
 
 from .. import registry
-from .attention import Attention
+from .attention import Attention, token_splits
 from .base import KVRequest, KVStateRequest, Runtime, StateRequest, TensorDecl
 from .rope import scaled_magnitude
 
@@ -172,7 +172,7 @@ class GatedAttention(Attention):
             return 1
         s = self.spec
         seen = min(max_kv_len, s.window + s.keep_first) if s.window > 0 else max_kv_len
-        return self.splits_of(nseq, seen, sm_count)
+        return token_splits(self.splits_of(nseq, seen, sm_count), self, nseq, s.heads, s.kv_heads, s.value_dim, seen, sm_count)
 
     def key_splits(self, batch):
         s = self.spec

@@ -711,9 +711,10 @@ def test_partial_results_of_many_key_splits_are_joined(ops, dtype, heads, kvh, d
     close(out, ref, tol_of(dtype))
 
 
-@pytest.mark.parametrize("heads,kvh,d,dv", [(4, 2, 16, 16), (32, 8, 128, 128), (2, 2, 256, 256), (16, 1, 96, 64), (6, 3, 24, 24)])
+@pytest.mark.parametrize("heads,kvh,d,dv", [(4, 2, 16, 16), (32, 8, 128, 128), (2, 2, 256, 256), (16, 1, 96, 64), (40, 1, 576, 512), (6, 3, 24, 24)])
 def test_partial_results_of_key_splits_may_begin_at_any_float(ops, heads, kvh, d, dv):
-    """Scratch is floats: the bits do not depend on where it begins (the tensor-core kernels' single tokens and latents, the CUDA cores)."""
+    """Scratch is floats: the bits do not depend on where it begins (the tensor-core kernels' single tokens and latents, the CUDA cores); and the
+    uncut result, but for the weights' roundings to bfloat16."""
     kv_lens = [1, 64, 700, 333]
     nseq, stride = len(kv_lens), 11
     table = torch.randperm(nseq * stride, generator=torch.Generator().manual_seed(5)).to(torch.int32).reshape(nseq, stride).to(DEV)
@@ -724,13 +725,14 @@ def test_partial_results_of_key_splits_may_begin_at_any_float(ops, heads, kvh, d
     mk = lambda x: torch.tensor(list(x), dtype=torch.int32, device=DEV)
     floats = ops.attention_scratch_floats(nseq, heads, dv, 4)
     outs = []
-    for first in (0, 1):
+    for first, splits in ((0, 4), (1, 4), (0, 1)):
         out = torch.full((nseq, heads * dv), float("nan"), dtype=torch.bfloat16, device=DEV)
-        used = ops.attention(q, out, k, v, table, mk(range(nseq)), mk(range(nseq)), mk([1] * nseq), mk(kv_lens), nseq, 1, heads, kvh, d, d ** -0.5, 0, 4,
-                             torch.full((floats + 1,), float("nan"), device=DEV)[first:first + floats], value_dim=dv)
+        used = ops.attention(q, out, k, v, table, mk(range(nseq)), mk(range(nseq)), mk([1] * nseq), mk(kv_lens), nseq, 1, heads, kvh, d, d ** -0.5, 0, splits,
+                             torch.full((floats + 1,), float("nan"), device=DEV)[first:first + floats] if splits > 1 else None, value_dim=dv)
         outs.append(out)
     assert used == ("latent_mma" if dv != d else "simt" if d % 16 else "decode_mma")
-    assert torch.isfinite(outs[0].float()).all() and torch.equal(*outs)
+    assert torch.isfinite(outs[0].float()).all() and torch.equal(outs[0], outs[1])
+    close(outs[0], outs[2], tol_of(torch.bfloat16))
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

@@ -302,6 +302,31 @@ def test_replayed_graph_steps_equal_eager_steps(model_dirs, plain_models, dtype)
     assert len(graph.graphs.graphs) >= 3  # several batch sizes and split counts were captured
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("lens", [[505], [2033, 500, 3], [505, 2, 64, 130, 500, 7, 300, 1, 501]])
+def test_replayed_steps_equal_eager_ones_where_the_cut_of_the_keys_changes(dtype, lens):
+    """A context that grows past 512 or 2048 keys in mid-generation: another step is captured, and the eager step's bits follow."""
+    from gophonic_b200.config import Qwen3Config
+    from gophonic_b200.engine import Engine, Model
+    cfg = Qwen3Config(hidden_size=128, num_hidden_layers=2, num_attention_heads=8, num_key_value_heads=2, head_dim=64, intermediate_size=256,
+                      vocab_size=600, max_position_embeddings=2304, rms_norm_eps=1e-6, rope_theta=1000000.0, tie_word_embeddings=True)
+    model = Model.from_random(cfg, seed=5, dtype=dtype, device="cuda:0")
+    rng = np.random.default_rng(11)
+    prompts = [rng.integers(0, cfg.vocab_size, size=n).tolist() for n in lens]
+    toks = rng.integers(0, cfg.vocab_size, size=(16, len(lens)))
+    runs = []
+    for graphs in (False, True):
+        eng = Engine(model, max_tokens=8192, max_slots=len(lens), use_graphs=graphs)
+        slots = [eng.new_sequence() for _ in prompts]
+        eng.step(list(zip(slots, prompts)))
+        runs.append([eng.step([(s, [int(t)]) for s, t in zip(slots, row)]).cpu().numpy() for row in toks])
+    assert all(np.array_equal(a, b) for a, b in zip(*runs))
+    plans = {model.step_plans(max(len(lens), 12 if len(lens) > 8 else 1), 1, max(lens) + 1 + i, eng.sm_count) for i in range(16)}
+    assert len(eng.graphs.graphs) == len(plans)
+    if lens[0] == 505:
+        assert len(plans) == (2 if dtype == "bfloat16" else 1)
+
+
 @pytest.mark.parametrize("name,dtype", [("D", "bfloat16"), ("B", "bfloat16"), ("F", "bfloat16"), ("A", "float32")])
 def test_what_an_earlier_request_left_in_a_page_is_never_seen(model_dirs, references, plain_models, name, dtype):
     """Every free page of the cache holds NaN (as if earlier requests had gone wrong) before each

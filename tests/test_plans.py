@@ -6,7 +6,7 @@ import torch
 
 from gophonic_b200.engine import graphs
 from gophonic_b200.engine.step import build_batch
-from gophonic_b200.parts.attention import Attention, choose_splits, few_splits
+from gophonic_b200.parts.attention import Attention, choose_splits, few_splits, page_class, wave_splits
 from gophonic_b200.parts.gated_attention import GatedAttention
 from gophonic_b200.parts.latent_attention import LatentAttention
 
@@ -15,7 +15,7 @@ LENGTHS = [1, 63, 64, 65, 100, 256, 700, 1500, 4096, 12000, 40960]
 
 
 def part(heads=32, kv_heads=8, head_dim=128, window=0, keep_first=0, fp32=False):
-    p = SimpleNamespace(spec=SimpleNamespace(heads=heads, kv_heads=kv_heads, head_dim=head_dim, window=window, keep_first=keep_first),
+    p = SimpleNamespace(spec=SimpleNamespace(heads=heads, kv_heads=kv_heads, head_dim=head_dim, value_dim=head_dim, window=window, keep_first=keep_first),
                         rt=SimpleNamespace(is_fp32=fp32))
     p.splits_of = lambda *a: Attention.splits_of(p, *a)
     p.plan = lambda *a: Attention.plan(p, *a)
@@ -39,17 +39,55 @@ def test_pieces_of_few_sequences():
             assert s & (s - 1) == 0 and ok(s) and not ok(2 * s)
 
 
-@pytest.mark.parametrize("window", [0, 300])
-def test_single_tokens_take_the_finer_of_both_rules(window):
+@pytest.mark.parametrize("window", [0, 300, 1024])
+def test_single_tokens_take_the_finest_of_the_rules(window):
     a, full = part(window=window), part(window=window, fp32=True)
     for n in SIZES:
         for kv in LENGTHS:
-            coarse = choose_splits(8 * n, kv)
-            assert a.plan(n, 1, kv, 148) == max(coarse, few_splits(8 * n, min(kv, window) if window else kv))
+            coarse, seen = choose_splits(8 * n, kv), min(kv, window) if window else kv
+            assert a.plan(n, 1, kv, 148) == wave_splits(max(coarse, few_splits(8 * n, seen)), 8 * n, 32 * n, seen, 296)
             assert full.plan(n, 1, kv, 148) == choose_splits(8 * n, kv, 148, 65536)
-            # the gated form keeps to the one rule, over the keys that a row can see
-            g = part(window=window, keep_first=20)
-            assert GatedAttention.plan(g, n, 1, kv, 148) == choose_splits(8 * n, min(kv, window + 20) if window else kv)
+            # the gated form has two of them, over the keys that a row can see
+            g, seen = part(window=window, keep_first=20), min(kv, window + 20) if window else kv
+            assert GatedAttention.plan(g, n, 1, kv, 148) == wave_splits(choose_splits(8 * n, seen), 8 * n, 32 * n, seen, 296)
+
+
+def test_pieces_that_fill_one_wave():
+    """Nothing up to 512 visible keys; else no more CTAs than one wave holds (or two, nearly full, in three pieces of eight pages), no more than 16
+    pieces, partial results of no more than four heads a place, no piece empty at the largest length of a class, and no more pieces that
+    save a CTA too little."""
+    for places in (148, 296):
+        for units in (1, 2, 7, 8, 9, 24, 32, 64, 74, 75, 96, 148, 149, 192, 197, 198, 400, 4000):
+            for group in (1, 4, 16):
+                for kv_len in LENGTHS + [512, 513, 1472, 1473, 8192]:
+                    for had in (1, 2, 5, 12, 32):
+                        s, pages = wave_splits(had, units, units * group, kv_len, places), -(-kv_len // 64)
+                        if pages <= 8:
+                            assert s == had
+                        elif 2 * units > places:
+                            three = 3 * units <= 2 * places and 3 * group * units <= 8 * places and pages >= 24
+                            assert s == (max(3, had) if three else had)
+                        elif s != had:
+                            assert had < s <= 16 and s * units <= places and s * units * group <= 4 * places
+                            size = page_class(pages)
+                            assert pages <= size <= 3 * pages // 2 and (pages <= s or (s - 1) * -(-size // s) < size)
+                            assert -(-pages // had) - -(-pages // s) >= (5 if had == 1 else 1 if s == had + 1 else 2)
+    rule = lambda n, kv: wave_splits(max(choose_splits(8 * n, kv), few_splits(8 * n, kv)), 8 * n, 32 * n, kv, 296)
+    assert [rule(n, 700) for n in (1, 2, 3, 4, 5, 8, 12, 16, 24, 32, 64)] == [16, 16, 12, 4, 6, 4, 3, 2, 1, 1, 1]      # as measured
+    assert [rule(n, 1500) for n in (1, 2, 3, 5, 8, 12, 16, 24, 32, 64)] == [8, 8, 12, 6, 4, 3, 2, 3, 1, 1]
+    assert [rule(n, 4096) for n in (1, 2, 3, 5, 8, 12, 16, 24, 32, 64)] == [16, 16, 11, 7, 4, 3, 2, 3, 1, 1]
+    assert rule(2, 900) == 8 and rule(16, 530) == 1
+    assert wave_splits(8, 16, 256, 1500, 296) == 8       # eight sequences of two key heads, 16 heads each: the merge reads them all
+
+
+def test_what_the_tensor_core_kernel_does_not_take_is_cut_as_before():
+    wide = part(head_dim=40)
+    unequal = part()
+    unequal.spec.value_dim = 64
+    for p, page in ((wide, 2 * 64 * 40 * 2), (unequal, 32768)):
+        for n in (1, 4, 8):
+            for kv in LENGTHS:
+                assert GatedAttention.plan(p, n, 1, kv, 148) == choose_splits(8 * n, kv, 148, page)
 
 
 def test_the_plan_of_a_step_does_not_depend_on_the_other_lengths():
