@@ -185,6 +185,30 @@ def test_the_rule_of_expanded_latents():
     assert runs_of([(0, 100), (9, 3)], dtype=torch.float32) == [(0, 2, 0, 103, 100, 0)]
 
 
+@pytest.mark.parametrize("heads", [8, 16, 32, 64])
+def test_pieces_of_single_tokens_over_latents(heads):
+    """One wave of an SM a CTA, only where the pages that a CTA is saved are worth the merge; float32, narrow latents and many sequences
+    are cut as the general rule says, and the captured steps of a batch size are few."""
+    p = object.__new__(LatentAttention)
+    p.spec = SimpleNamespace(heads=heads, kv_rank=512, window=0, chunk=0)
+    p.rt, p.key_dim = SimpleNamespace(is_fp32=False), 576
+    ctas = -(-heads // 32)
+    for n in SIZES + [256, 8192, 100000]:
+        for kv in LENGTHS + [129, 192, 193, 250, 350]:
+            rule, got, fine = choose_splits(n, kv, 74, 64 * 576 * 2), p.plan(n, 1, kv, 148), p.fine_splits(n, kv, 148)
+            assert got == max(rule, fine) and p.plan(n, 2, kv, 148) == 1
+            assert fine == 1 or (n * ctas * fine <= 148 and fine <= 32 and kv > 128)
+            if 2 * n * ctas > 148 or kv <= 128:
+                assert got == rule
+        assert len({p.plan(n, 1, kv, 148) for kv in range(1, 8193, 31)}) <= len({choose_splits(n, kv, 74, 64 * 576 * 2) for kv in range(1, 8193, 31)}) + 2
+    if heads == 16:      # as measured
+        assert [p.plan(n, 1, kv, 148) for n, kv in ((1, 700), (8, 1024), (16, 250), (16, 350), (24, 150), (24, 1500), (32, 350), (64, 1024))] == [12, 16, 1, 6, 1, 6, 1, 2]
+    p.spec.kv_rank = 256
+    assert p.fine_splits(1, 700, 148) == 1
+    p.spec.kv_rank, p.rt.is_fp32 = 512, True
+    assert p.plan(1, 1, 700, 148) == choose_splits(1, 700, 74, 64 * 576 * 4)
+
+
 class RecordingOps:
     """Stands for the kernels that latent attention calls; keeps what attention was asked for."""
 
