@@ -664,14 +664,16 @@ __global__ void __launch_bounds__(ST) sample_final_kernel(SampleParams p, const 
     }
     const int n = (int)count;
     const unsigned long long* c = cands + (int64_t)r * MAXC;
-    if (n >= BUCKET_MIN && bucket_candidates(c, n, cand, count_s)) {
-        // sorted
-    } else if (n <= ST)
+    // Short lists first, and the code of one way for them: behind the buckets' code, and with another copy for crowded lists, every
+    // choice took 0.2 to 0.3 us more (8 rows of 32000, the 40 likeliest: 15.6 us so, 15.3 this way).
+    if (n < BUCKET_MIN)
         sort_candidates<1>(c, n, cand);
-    else if (n <= 2 * ST)
-        sort_candidates<2>(c, n, cand);
-    else
-        sort_candidates<4>(c, n, cand);
+    else if (!bucket_candidates(c, n, cand, count_s)) {
+        if (n <= 2 * ST)
+            sort_candidates<2>(c, n, cand);
+        else
+            sort_candidates<4>(c, n, cand);
+    }
     const float* row = p.logits + (int64_t)r * p.stride;
     const float temp = p.temperature[o];
     if (!(temp > 0.f)) {
